@@ -94,19 +94,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 // ---- epilogue: kernel function applied to the register sums -------------------------------------
 // The epilogue is unrolled 128 times (the sums live in registers), so its body has to stay small:
 // with the library expf / powf / tanhf inlined 128 times the code outgrew the instruction cache
-// and one tile's epilogue took as long as two thirds of its main loop. The RBF path therefore uses
-// a 6-instruction exponential: exp(x) = 2^y (1 + r ln2) with y = fl(x log2e) and r the rounding
-// residual of that product (FMA) plus x times the representation error of log2e; ex2.approx is
-// accurate to 2^-22.5 relative, the total stays below 3e-7 relative for |x| <= 100.
+// and one tile's epilogue took as long as two thirds of its main loop. The RBF path evaluates
+// exp(x) = 2^(x log2 e) with the product carried in two floats (the error-free product of T. J. Dekker, "A
+// floating-point technique for extending the available precision", 1971, in its FMA form): y = fl(x H) and
+// r = (x H - y) + x L, where H + L is log2 e split into two floats at compile time; then
+// 2^(y + r) = 2^y + 2^y (r ln 2) + O(r^2), and r^2 < 2^-34 for |x| <= 100. The hardware's 2^y is good to
+// 2^-22.5 relative, the total stays below 3e-7.
 enum { EPI_RBF = 0, EPI_LINEAR = 1, EPI_GENERIC = 2 };
 
 __device__ __forceinline__ float exp_compact(float x) {
-    const float y = x * 1.4426950408889634f;
-    float r = fmaf(x, 1.4426950408889634f, -y);
-    r = fmaf(x, 1.925963033500e-8f, r);
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(y));
-    return fmaf(e, r * 0.6931471805599453f, e);
+    constexpr double LOG2_E = 1.442695040888963407359924681, LN_2 = 0.693147180559945309417232121;
+    constexpr float H = (float) LOG2_E, L = (float) (LOG2_E - (double) H);
+    const float y = x * H;
+    const float r = fmaf(x, L, fmaf(x, H, -y));
+    float p;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(y));
+    return fmaf(p, r * (float) LN_2, p);
 }
 
 template <int EPI>
