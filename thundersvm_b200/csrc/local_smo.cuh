@@ -1,0 +1,362 @@
+// The local solver: SMO on one working set of at most 1,024 instances, one CTA.
+// Reference behaviour: c_smo_solve_kernel of the CPU backend (src/thundersvm/kernel/smo_kernel.cpp:12-125) with ties
+// to the lowest slot, and nu_smo_solve_kernel of the CUDA backend (src/thundersvm/kernel/smo_kernel.cu:118-252): bound
+// held in float, float arithmetic in the curvature term.
+//
+// What bounds it: a chain of dependent steps, about a thousand of them per call. One iteration is
+//   argmin of f over I_up -> row i of the ws x ws block -> second-order argmax over I_low -> row j -> f update
+// and nothing of the next iteration can start before f is updated. The two rows come from L2; the two reductions cross
+// the block. So the kernel is laid out for latency: few warps with many slots each (the slots of a thread overlap, and
+// what every warp has to repeat - the reductions, the step - is repeated by few warps), one barrier per reduction,
+// and everything that is not on the chain is placed into the shadow of a row load.
+//   * The first argmin compares the doubles themselves inside a thread and between warps; inside a warp one float
+//     reduction over the doubles' high words finds the winner, and only if two lanes share the high word the low words
+//     are looked at.
+//   * The largest f over I_low is needed for the stopping rule only. Its high word gives a lower bound of it; the
+//     exact value is reduced when the bound cannot show that the gap is still open.
+//   * The second-order values b^2 / a are compared in FP32 (error below 1e-6 relative: b truncated to 24 bits, a rounded
+//     once, an approximate reciprocal). If the best value of the block stands out by more than 8e-6 it is the
+//     winner in FP64 too; otherwise - near-equal instances, mostly - or if an operand leaves the range in which that
+//     error bound holds, the block repeats the comparison in FP64 (a few ulp), ties to the lower slot.
+// Measured (RBF block, 1,024 slots): 1.00 us per iteration, 1.74 before (512 threads with two slots each, every mirror
+// written in every iteration, FP64 keys and one exact division per thread in the second-order choice); where most
+// values tie (a kernel close to the identity) 1.39 against 2.07; nu 1.48 against 2.58. Of the 1,900 cycles about 740 are
+// the two L2 round trips (372 cycles each), 440 the first reduction, 250 the second.
+#pragma once
+#include "common.cuh"
+
+namespace tsvm {
+
+constexpr int NO_SLOT = 0x7fffffff;
+
+namespace smo {
+constexpr float FAR_POS = 1.7014118e38f;                            // as the high word of a double: 2^1008
+constexpr double NO_MEMBER = 1e300;                                 // |value| above it: no instance in the list
+
+__device__ __forceinline__ float high_as_float(double v) { return __int_as_float(__double2hiint(v)); }
+__device__ __forceinline__ double with_high(float h, double v) { return __hiloint2double(__float_as_int(h), __double2loint(v)); }
+__device__ __forceinline__ float warp_min_f32(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max_f32(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// 1 / a to a few ulp: two Newton steps on the hardware's approximation (which is kept for zero and infinity)
+__device__ __forceinline__ double reciprocal(double a) {
+    double r0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(a));
+    double r = fma(r0, fma(-a, r0, 1.0), r0);
+    r = fma(r, fma(-a, r, 1.0), r);
+    return a != 0.0 && fabs(a) < 1e300 ? r : r0;
+}
+
+struct First { double f; int slot; float low; };        // a warp's smallest f over I_up, its slot; high word of max f over I_low
+struct Second { float best, next; int slot, pad; };     // a warp's largest and second-largest estimate of b^2 / a
+}  // namespace smo
+
+// Slot t of the working set belongs to thread t % T. S slots per thread.
+template <bool NU, int S, int T>
+__global__ void __launch_bounds__(T, 1)
+local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict__ diag_ws,
+                 const int *__restrict__ y_ws, const double *__restrict__ f_ws, double *__restrict__ alpha_ws,
+                 double *__restrict__ alpha_diff, double Cp_in, double Cn_in, double eps, int max_iter,
+                 double *__restrict__ diff, const int *__restrict__ ids, double *__restrict__ alpha_global,
+                 const int *__restrict__ stop) {
+    using namespace smo;
+    constexpr int W = T / 32, CLS = NU ? 2 : 1;             // nu: the lists of I_up and I_low are split by class
+    if (stop && *stop) {            // queued past the end of a solve: no step, so the f update that follows adds zero
+        for (int t = threadIdx.x; t < ws; t += T) alpha_diff[t] = 0;
+        return;
+    }
+    __shared__ double f_sm[S * T], a_sm[S * T];
+    __shared__ float kd_sm[S * T];
+    __shared__ int y_sm[S * T];
+    __shared__ First e1[CLS][W];
+    __shared__ Second e2[W];
+    __shared__ unsigned long long exact_key[CLS][W];
+    __shared__ int exact_slot[CLS][W];
+    __shared__ double exact_low[CLS][W];
+    const double Cp = NU ? (double) (float) Cp_in : Cp_in;
+    const double Cn = NU ? Cp : Cn_in;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    double f[S];
+    float kd[S], pen_up[S], pen_low[S];     // +-FAR_POS: what clamps a non-member's f out of the list
+    bool pos[S];                            // nu: class of the slot
+    int off[S];                             // column of the slot in a row of kww (any valid one where there is no slot)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int t = tid + s * T;
+        double a = 0;
+        int y = 0;                          // y = 0: member of no set
+        f[s] = 0; kd[s] = 0;
+        if (t < ws) { f[s] = f_ws[t]; a = alpha_ws[t]; y = y_ws[t]; kd[s] = diag_ws[t]; }
+        f_sm[t] = f[s]; a_sm[t] = a; y_sm[t] = y; kd_sm[t] = kd[s];
+        pen_up[s] = in_I_up(a, y, Cp, Cn) ? -FAR_POS : FAR_POS;
+        pen_low[s] = in_I_low(a, y, Cp, Cn) ? FAR_POS : -FAR_POS;
+        pos[s] = y > 0;
+        off[s] = t < ws ? t : 0;
+    }
+    __syncthreads();
+
+    double local_eps = 0;
+    int it = 0;
+    // the last step, written to a_sm once every thread has read what it needs for that step
+    int step_i = 0, step_j = 0;
+    double step_ai = a_sm[0], step_aj = step_ai;
+    for (;;) {
+        // ---- smallest f over I_up (with its slot), high word of the largest f over I_low ---------------------
+        float low_h[S];                     // high word of f, clamped to -FAR_POS outside I_low
+#pragma unroll
+        for (int s = 0; s < S; ++s) low_h[s] = fminf(high_as_float(f[s]), pen_low[s]);
+#pragma unroll
+        for (int c = 0; c < CLS; ++c) {
+            double v[S];
+            int slot[S];
+            float lo = -FAR_POS;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const float h = fmaxf(high_as_float(f[s]), pen_up[s]);
+                const bool mine = !NU || pos[s] == (c == 0);
+                v[s] = with_high(mine ? h : FAR_POS, f[s]);
+                slot[s] = tid + s * T;
+                lo = fmaxf(lo, mine ? low_h[s] : -FAR_POS);
+            }
+            // neighbouring slots first: the left operand always holds the lower slots and wins ties
+#pragma unroll
+            for (int d = 1; d < S; d <<= 1)
+#pragma unroll
+                for (int s = 0; s + d < S; s += 2 * d)
+                    if (v[s + d] < v[s]) { v[s] = v[s + d]; slot[s] = slot[s + d]; }
+            const float h = high_as_float(v[0]);
+            const float h_min = warp_min_f32(h), lo_max = warp_max_f32(lo);
+            const unsigned at_min = __ballot_sync(0xffffffffu, h == h_min);
+            int winner = at_min ? __ffs(at_min) - 1 : 0;
+            if (at_min & (at_min - 1)) {
+                unsigned long long key = ordered_key(v[0]);
+                int sl = slot[0];
+                warp_argmin_u64(key, sl);
+                winner = __ffs(__ballot_sync(0xffffffffu, slot[0] == sl)) - 1;
+            }
+            if (lane == winner) { First e; e.f = v[0]; e.slot = slot[0]; e.low = lo_max; e1[c][warp] = e; }
+        }
+        __syncthreads();
+        double up[CLS];
+        int iu[CLS];
+        float lowf[CLS];
+#pragma unroll
+        for (int c = 0; c < CLS; ++c) {
+            double v[W];
+            int slot[W];
+            float lo[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) { const First e = e1[c][w]; v[w] = e.f; slot[w] = e.slot; lo[w] = e.low; }
+#pragma unroll
+            for (int d = 1; d < W; d <<= 1)
+#pragma unroll
+                for (int w = 0; w + d < W; w += 2 * d) {
+                    lo[w] = fmaxf(lo[w], lo[w + d]);
+                    if (v[w + d] < v[w] || (v[w + d] == v[w] && slot[w + d] < slot[w])) { v[w] = v[w + d]; slot[w] = slot[w + d]; }
+                }
+            up[c] = v[0]; iu[c] = (unsigned) slot[0] < (unsigned) ws ? slot[0] : 0; lowf[c] = lo[0];
+        }
+        float kI[CLS][S];
+#pragma unroll
+        for (int c = 0; c < CLS; ++c)
+#pragma unroll
+            for (int s = 0; s < S; ++s) kI[c][s] = __ldg(kww + iu[c] * ws + off[s]);
+        // mirrors of the state after the last step (its readers have passed the barrier above)
+#pragma unroll
+        for (int s = 0; s < S; ++s) f_sm[tid + s * T] = f[s];
+        if (tid == 0) { a_sm[step_i] = step_ai; a_sm[step_j] = step_aj; }
+
+        // ---- stopping rule ---------------------------------------------------------------------------------
+        bool open = it > 0 && it <= max_iter;
+        {
+            double gap = 0;
+#pragma unroll
+            for (int c = 0; c < CLS; ++c) {
+                // the smallest double with this high word
+                const int h = __float_as_int(lowf[c]);
+                const double g = __hiloint2double(h, h < 0 ? -1 : 0) - up[c];
+                gap = c == 0 ? g : fmax(gap, g);
+            }
+            open = open && gap >= local_eps;
+        }
+        if (!open) {
+            // the exact gap: at the first iteration, near the end, and at the end
+#pragma unroll
+            for (int c = 0; c < CLS; ++c) {
+                double m = -INFINITY;
+#pragma unroll
+                for (int s = 0; s < S; ++s)
+                    if (pen_low[s] > 0 && (!NU || pos[s] == (c == 0))) m = fmax(m, f[s]);
+                const double wm = key_to_double(~warp_min_u64(~ordered_key(m)));
+                if (lane == 0) exact_low[c][warp] = wm;
+            }
+            __syncthreads();
+            double local_diff = 0;
+#pragma unroll
+            for (int c = 0; c < CLS; ++c) {
+                double m = exact_low[c][0];
+                for (int w = 1; w < W; ++w) m = fmax(m, exact_low[c][w]);
+                const double d = m - (up[c] > NO_MEMBER ? INFINITY : up[c]);
+                local_diff = c == 0 ? d : fmax(local_diff, d);
+            }
+            if (it == 0) {
+                local_eps = NU ? fmax(eps, 0.1 * local_diff) : fmax(eps, (double) 0.1f * local_diff);
+                if (tid == 0) diff[0] = local_diff;
+            }
+            if (it > max_iter || local_diff < local_eps) break;
+        }
+
+        // ---- second-order choice of j ------------------------------------------------------------------------
+        float q[S], q2[S], q0[S];
+        int qs[S];
+        float kd_i[CLS];
+#pragma unroll
+        for (int c = 0; c < CLS; ++c) kd_i[c] = kd_sm[iu[c]];
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const bool second = NU && !pos[s];
+            const float k = second ? kI[CLS - 1][s] : kI[0][s];
+            const double b = with_high(low_h[s], f[s]) - (second ? up[CLS - 1] : up[0]);    // far below zero outside I_low
+            // b in FP32, truncated, straight from the double's bits; [2^-50, 2^50) keeps its square in range
+            const int bh = __double2hiint(b);
+            const float b32 = __int_as_float(__funnelshift_l((unsigned) __double2loint(b), (unsigned) (bh - 0x38000000), 3));
+            const bool b_ok = (unsigned) (bh - 0x3cd00000) < 0x06400000u;
+            const float a32 = fmaf(-2.0f, k, (second ? kd_i[CLS - 1] : kd_i[0]) + kd[s]);
+            const bool a_ok = a32 > 1e-30f && a32 < 1e30f;
+            float r;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a32));
+            q[s] = b_ok && a_ok ? b32 * b32 * r : (b > 0 ? INFINITY : 0.0f);
+            q0[s] = q[s];
+            q2[s] = 0.0f;
+            qs[s] = tid + s * T;
+        }
+#pragma unroll
+        for (int d = 1; d < S; d <<= 1)
+#pragma unroll
+            for (int s = 0; s + d < S; s += 2 * d) {
+                q2[s] = fmaxf(fminf(q[s], q[s + d]), fmaxf(q2[s], q2[s + d]));
+                if (q[s + d] > q[s]) { q[s] = q[s + d]; qs[s] = qs[s + d]; }
+            }
+        {
+            const float best = warp_max_f32(q[0]);
+            const unsigned at_best = __ballot_sync(0xffffffffu, q[0] == best);
+            const float next = warp_max_f32(q[0] == best ? q2[0] : q[0]);
+            if (lane == (int) __ffs(at_best) - 1) {
+                Second e;
+                e.best = best; e.next = (at_best & (at_best - 1)) ? best : next; e.slot = qs[0]; e.pad = 0;
+                e2[warp] = e;
+            }
+        }
+        __syncthreads();
+        int j;
+        {
+            float best[W], next[W];
+            int slot[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) { const Second e = e2[w]; best[w] = e.best; next[w] = e.next; slot[w] = e.slot; }
+#pragma unroll
+            for (int d = 1; d < W; d <<= 1)
+#pragma unroll
+                for (int w = 0; w + d < W; w += 2 * d) {
+                    next[w] = fmaxf(fminf(best[w], best[w + d]), fmaxf(next[w], next[w + d]));
+                    if (best[w + d] > best[w]) { best[w] = best[w + d]; slot[w] = slot[w + d]; }
+                }
+            j = slot[0];
+            if (!(best[0] > 0.0f && best[0] < INFINITY && next[0] < best[0] * (1.0f - 8e-6f))) {
+                // too close to call in FP32, or out of its range: the same values in FP64, ties to the lower slot
+                const float thr = best[0] < INFINITY ? best[0] * (1.0f - 8e-6f) : 0.0f;
+                double most[CLS];
+                int sl[CLS];
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) { most[c] = -INFINITY; sl[c] = NO_SLOT; }
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    const bool second = NU && !pos[s];
+                    const double b = -(second ? up[CLS - 1] : up[0]) + f[s];
+                    const float k = second ? kI[CLS - 1][s] : kI[0][s], kdi = second ? kd_i[CLS - 1] : kd_i[0];
+                    const double a = NU ? (double) (kdi + kd[s] - 2 * k) : (double) (kdi + kd[s]) - 2.0 * (double) k;
+                    const double e = b * b * reciprocal(a);
+                    const bool asked = q0[s] > 0.0f && q0[s] >= thr;
+#pragma unroll
+                    for (int c = 0; c < CLS; ++c)
+                        if (asked && second == (c > 0) && e > most[c]) { most[c] = e; sl[c] = tid + s * T; }
+                }
+                unsigned long long key[CLS];
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) key[c] = ordered_key(-most[c]);
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) {
+                    warp_argmin_u64(key[c], sl[c]);
+                    if (lane == 0) { exact_key[c][warp] = key[c]; exact_slot[c][warp] = sl[c]; }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) {
+                    key[c] = lane < W ? exact_key[c][lane] : ~0ull;
+                    sl[c] = lane < W ? exact_slot[c][lane] : NO_SLOT;
+                    warp_argmin_u64(key[c], sl[c]);
+                }
+                j = sl[0];
+                // the positive-class pair wins only if its value is strictly smaller (smo_kernel.cu:220-233)
+                if (NU && !(key_to_double(key[0]) < key_to_double(key[CLS - 1]))) j = sl[CLS - 1];
+                if (j == NO_SLOT) j = 0;
+            }
+        }
+        // ---- step, repeated by every thread in the shadow of row j -------------------------------------------
+        float kJ[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) kJ[s] = __ldg(kww + j * ws + off[s]);
+        const int yj = y_sm[j];
+        const bool second = NU && yj < 0;
+        const int i = second ? iu[CLS - 1] : iu[0];
+        const int yi = y_sm[i];
+        const double u = second ? up[CLS - 1] : up[0];
+        const double ai = a_sm[i], aj = a_sm[j], fj = f_sm[j];
+        const float kij = __ldg(kww + i * ws + j);          // row i has just been read: from L1
+        const double room_i = yi > 0 ? Cp - ai : ai;
+        const double curv = NU ? (double) (kd_sm[i] + kd_sm[j] - 2 * kij)
+                               : (double) (kd_sm[i] + kd_sm[j]) - 2.0 * (double) kij;
+        const double room_j = fmin(yj > 0 ? aj : Cn - aj, (-u + fj) / curv);
+        const double l = fmin(room_i, room_j);
+        step_i = i; step_j = j;
+        step_ai = ai + l * yi; step_aj = aj - l * yj;
+        const float up_i = in_I_up(step_ai, yi, Cp, Cn) ? -FAR_POS : FAR_POS, up_j = in_I_up(step_aj, yj, Cp, Cn) ? -FAR_POS : FAR_POS;
+        const float lo_i = in_I_low(step_ai, yi, Cp, Cn) ? FAR_POS : -FAR_POS, lo_j = in_I_low(step_aj, yj, Cp, Cn) ? FAR_POS : -FAR_POS;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const int t = tid + s * T;
+            if (t == i) { pen_up[s] = up_i; pen_low[s] = lo_i; }
+            if (t == j) { pen_up[s] = up_j; pen_low[s] = lo_j; }
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const float k = second ? kI[CLS - 1][s] : kI[0][s];
+            const double d = NU ? (double) (kJ[s] - k) : (double) kJ[s] - (double) k;
+            f[s] = fma(-l, d, f[s]);
+        }
+        ++it;
+    }
+    __syncthreads();                // (the last step's alphas are in a_sm)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int t = tid + s * T;
+        if (t < ws) {
+            const double a = a_sm[t], a_old = alpha_ws[t];
+            alpha_ws[t] = a;
+            alpha_diff[t] = -(a - a_old) * y_sm[t];
+            if (alpha_global && ids[t] >= 0) alpha_global[ids[t]] = a;
+        }
+    }
+    if (tid == 0) diff[1] = it;
+}
+
+}  // namespace tsvm

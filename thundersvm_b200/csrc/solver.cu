@@ -3,6 +3,7 @@
 // termination rules. Reference behaviour: src/thundersvm/solver/csmosolver.cpp:10-239,
 // src/thundersvm/solver/nusmosolver.cpp:9-136, src/thundersvm/kernel/smo_kernel.cu:28-315.
 #include "common.cuh"
+#include "local_smo.cuh"
 #include <cooperative_groups.h>
 #include <chrono>
 #include <limits.h>
@@ -650,258 +651,6 @@ static size_t merge_smem_bytes(int len) {
     return keys + (size_t) MAX_LISTS * MERGE_MAX_WANT * (4 + 2 + 1) + (size_t) HASH_SLOTS * 6 + 64;
 }
 
-// =================================================================================================
-// Local SMO (one CTA per working set)
-// =================================================================================================
-// threads per local solver: 512 (two slots each) for a working set of 1,024 - measured 1.96 us per iteration
-// against 2.14 with 256 threads and 2.10 with 1,024 -, 256 for smaller working sets
-constexpr int SMO_THREADS_MAX = 512, SMO_WARPS_MAX = SMO_THREADS_MAX / 32;
-constexpr unsigned long long KEY_POS_INF = 0xfff0000000000000ull;   // ordered_key(+inf)
-constexpr int NO_SLOT = 0x7fffffff;
-
-struct RedBuf {                     // per-warp partial results of up to four simultaneous reductions
-    unsigned long long key[4][SMO_WARPS_MAX];
-    int slot[4][SMO_WARPS_MAX];
-};
-
-// Block-wide argmin of R (key, slot) pairs: one __syncthreads, result in every thread.
-template <int R, int SMO_WARPS>
-__device__ __forceinline__ void block_argmin(RedBuf &buf, unsigned long long (&key)[R], int (&slot)[R]) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        warp_argmin_u64(key[r], slot[r]);
-        if (lane == 0) { buf.key[r][warp] = key[r]; buf.slot[r][warp] = slot[r]; }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        unsigned long long k = lane < SMO_WARPS ? buf.key[r][lane] : ~0ull;
-        int s = lane < SMO_WARPS ? buf.slot[r][lane] : NO_SLOT;
-        warp_argmin_u64(k, s);
-        key[r] = k; slot[r] = s;
-    }
-}
-
-// Local solver. Slot t of the working set is owned by thread t % 256 (register copies of f, alpha,
-// y, diag); mirrors of f / alpha / y / diag in shared memory serve the few values every thread
-// needs from the selected pair. kww is the ws x ws kernel block, so row loads are coalesced.
-// NU = false: c_smo_solve_kernel semantics of the CPU backend (smo_kernel.cpp:12-125), ties to the
-// lowest slot. NU = true: nu_smo_solve_kernel semantics of the CUDA backend
-// (smo_kernel.cu:118-252): bound held in float, float arithmetic in the curvature term.
-template <bool NU, int SLOTS, int SMO_THREADS>
-__global__ void __launch_bounds__(SMO_THREADS)
-local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict__ diag_ws,
-                 const int *__restrict__ y_ws, const double *__restrict__ f_ws, double *__restrict__ alpha_ws,
-                 double *__restrict__ alpha_diff, double Cp_in, double Cn_in, double eps, int max_iter,
-                 double *__restrict__ diff, const int *__restrict__ ids, double *__restrict__ alpha_global,
-                 const int *__restrict__ stop) {
-    if (stop && *stop) {            // queued past the end of a solve: no step, so the f update that follows adds zero
-        for (int t = threadIdx.x; t < ws; t += SMO_THREADS) alpha_diff[t] = 0;
-        return;
-    }
-    __shared__ RedBuf red[2];
-    __shared__ double f_sm[1024], a_sm[1024];
-    __shared__ float kd_sm[1024];
-    __shared__ int y_sm[1024];
-    const double Cp = NU ? (double) (float) Cp_in : Cp_in;
-    const double Cn = NU ? Cp : Cn_in;
-    const int tid = threadIdx.x;
-    double f[SLOTS], a[SLOTS], aold[SLOTS];
-    int y[SLOTS];
-    float kd[SLOTS];
-#pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-        const int t = tid + s * SMO_THREADS;
-        if (t < ws) {
-            f[s] = f_ws[t]; a[s] = aold[s] = alpha_ws[t]; y[s] = y_ws[t]; kd[s] = diag_ws[t];
-            f_sm[t] = f[s]; a_sm[t] = a[s]; y_sm[t] = y[s]; kd_sm[t] = kd[s];
-        } else { f[s] = 0; a[s] = aold[s] = 0; y[s] = 0; kd[s] = 0; }   // y = 0: member of no set
-    }
-    // Membership of I_up / I_low only changes for the two slots a step moves, so it is kept in registers and
-    // recomputed for those two instead of for every slot in every selection
-    bool in_up[SLOTS], in_low[SLOTS];
-#pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-        in_up[s] = in_I_up(a[s], y[s], Cp, Cn);
-        in_low[s] = in_I_low(a[s], y[s], Cp, Cn);
-    }
-    __syncthreads();
-    double local_eps = 0;
-    int it = 0;
-    for (;;) {
-        // ---- first-order selection --------------------------------------------------------
-        constexpr int R1 = NU ? 4 : 2;
-        unsigned long long key[R1];
-        int slot[R1];
-#pragma unroll
-        for (int r = 0; r < R1; ++r) { key[r] = KEY_POS_INF; slot[r] = NO_SLOT; }
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            const int t = tid + s * SMO_THREADS;
-            const unsigned long long kf = ordered_key(f[s]), knf = ordered_key(-f[s]);
-            if (!NU) {
-                if (in_up[s] && kf < key[0]) { key[0] = kf; slot[0] = t; }
-                if (in_low[s] && knf < key[1]) { key[1] = knf; slot[1] = t; }
-            } else {
-                // the four lists are I_up and I_low split by class (Cn = Cp here)
-                if (y[s] > 0 && in_up[s] && kf < key[0]) { key[0] = kf; slot[0] = t; }       // up, +:  a < C
-                if (y[s] < 0 && in_up[s] && kf < key[1]) { key[1] = kf; slot[1] = t; }       // up, -:  a > 0
-                if (y[s] > 0 && in_low[s] && knf < key[2]) { key[2] = knf; slot[2] = t; }    // low, +: a > 0
-                if (y[s] < 0 && in_low[s] && knf < key[3]) { key[3] = knf; slot[3] = t; }    // low, -: a < C
-            }
-        }
-        block_argmin<R1, SMO_THREADS / 32>(red[0], key, slot);
-        // mirrors written only now: every thread has finished reading them for the last step
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            const int t = tid + s * SMO_THREADS;
-            if (t < ws) { f_sm[t] = f[s]; a_sm[t] = a[s]; }
-        }
-        const int i0 = slot[0] == NO_SLOT ? 0 : slot[0];
-        const int i1 = NU ? (slot[1] == NO_SLOT ? 0 : slot[1]) : 0;
-        const double up0 = key_to_double(key[0]);
-        const double up1 = NU ? key_to_double(key[1]) : 0.0;
-        float kI0[SLOTS], kI1[SLOTS];
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            const int t = tid + s * SMO_THREADS;
-            kI0[s] = t < ws ? __ldg(kww + (size_t) i0 * ws + t) : 0.0f;
-            kI1[s] = (NU && t < ws) ? __ldg(kww + (size_t) i1 * ws + t) : 0.0f;
-        }
-        double local_diff;
-        if (!NU) local_diff = -key_to_double(key[1]) - up0;
-        else local_diff = fmax(-key_to_double(key[2]) - up0, -key_to_double(key[3]) - up1);
-        if (it == 0) {
-            local_eps = NU ? fmax(eps, 0.1 * local_diff) : fmax(eps, (double) 0.1f * local_diff);
-            if (tid == 0) diff[0] = local_diff;
-        }
-        if (it > max_iter || local_diff < local_eps) break;
-
-        // ---- second-order selection ---------------------------------------------------------
-        constexpr int R2 = NU ? 2 : 1;
-        unsigned long long key2[R2];
-        int slot2[R2];
-#pragma unroll
-        for (int r = 0; r < R2; ++r) { key2[r] = KEY_POS_INF; slot2[r] = NO_SLOT; }
-        const float kd_i0 = kd_sm[i0], kd_i1 = NU ? kd_sm[i1] : 0.0f;
-        if (!NU) {
-            // The exact quotient -b^2 / a costs a double-precision division per slot, and only the thread's best
-            // slot matters. An FP32 estimate of b^2 / a (relative error below 5e-7: two roundings to FP32, a
-            // product, a 2-ulp division) first rules out every slot whose estimate is more than 8e-6 below the
-            // thread's largest: its exact quotient is smaller by more than any rounding, so it can neither win nor
-            // tie. What is left - almost always one slot - is divided exactly. Estimates outside the range
-            // where the error bound holds send all of the thread's candidates to the exact path.
-            bool cnd[SLOTS];
-            double aIJ[SLOTS], bIJ[SLOTS];
-            float q32[SLOTS];
-            float m = -1.0f;
-            bool trust = true;
-#pragma unroll
-            for (int s = 0; s < SLOTS; ++s) {
-                cnd[s] = -up0 > -f[s] && in_low[s];
-                aIJ[s] = (double) (kd_i0 + kd[s]) - 2.0 * (double) kI0[s];
-                bIJ[s] = -up0 + f[s];
-                const float b32 = (float) bIJ[s], a32 = (float) aIJ[s];
-                q32[s] = __fdividef(b32 * b32, a32);
-                trust = trust && (!cnd[s] || (b32 > 1e-15f && b32 < 1e15f && a32 > 1e-30f && a32 < 1e30f));
-                if (cnd[s]) m = fmaxf(m, q32[s]);
-            }
-            const float thr = m * (1.0f - 8e-6f);
-            // the first slot that holds the largest estimate, divided without a branch
-            int pick = SLOTS;
-            double pa = 1.0, pb = 0.0;
-#pragma unroll
-            for (int s = SLOTS - 1; s >= 0; --s)
-                if (cnd[s] && q32[s] == m) { pick = s; pa = aIJ[s]; pb = bIJ[s]; }
-            if (pick < SLOTS) {
-                key2[0] = ordered_key(-pb * pb / pa);
-                slot2[0] = tid + pick * SMO_THREADS;
-            }
-            // any other slot the estimate cannot rule out: exact, ties to the lower slot as in a pass in slot order
-            bool more = false;
-#pragma unroll
-            for (int s = 0; s < SLOTS; ++s) more = more || (cnd[s] && s != pick && (!trust || q32[s] >= thr));
-            if (more) {
-#pragma unroll
-                for (int s = 0; s < SLOTS; ++s) {
-                    if (cnd[s] && s != pick && (!trust || q32[s] >= thr)) {
-                        const int t = tid + s * SMO_THREADS;
-                        const unsigned long long k = ordered_key(-bIJ[s] * bIJ[s] / aIJ[s]);
-                        if (k < key2[0] || (k == key2[0] && t < slot2[0])) { key2[0] = k; slot2[0] = t; }
-                    }
-                }
-            }
-        } else {
-#pragma unroll
-            for (int s = 0; s < SLOTS; ++s) {
-                const int t = tid + s * SMO_THREADS;
-                // every slot computes its quotients, candidates or not (the others divide by one and are
-                // discarded): the divisions of a thread's slots then overlap instead of one divergent branch each
-                const bool c0 = -up0 > -f[s] && y[s] > 0 && in_low[s];
-                const bool c1 = -up1 > -f[s] && y[s] < 0 && in_low[s];
-                const double a0 = (double) (kd_i0 + kd[s] - 2 * kI0[s]), a1 = (double) (kd_i1 + kd[s] - 2 * kI1[s]);
-                const double b0 = -up0 + f[s], b1 = -up1 + f[s];
-                const double v0 = -b0 * b0 / (c0 ? a0 : 1.0), v1 = -b1 * b1 / (c1 ? a1 : 1.0);
-                const unsigned long long k0 = ordered_key(v0), k1 = ordered_key(v1);
-                if (c0 && k0 < key2[0]) { key2[0] = k0; slot2[0] = t; }
-                if (c1 && k1 < key2[1]) { key2[1] = k1; slot2[1] = t; }
-            }
-        }
-        block_argmin<R2, SMO_THREADS / 32>(red[1], key2, slot2);
-        int i, j2;
-        double up;
-        bool use1 = false;
-        if (!NU) { i = i0; j2 = slot2[0] == NO_SLOT ? 0 : slot2[0]; up = up0; }
-        else {
-            // the positive-class pair wins only if its value is strictly smaller (smo_kernel.cu:220-233)
-            if (key_to_double(key2[0]) < key_to_double(key2[1])) { i = i0; j2 = slot2[0] == NO_SLOT ? 0 : slot2[0]; up = up0; }
-            else { i = i1; j2 = slot2[1] == NO_SLOT ? 0 : slot2[1]; up = up1; use1 = true; }
-        }
-        // ---- step length, computed redundantly by every thread ---------------------------------
-        const double ai = a_sm[i], aj = a_sm[j2], fj = f_sm[j2];
-        const int yi = y_sm[i], yj = y_sm[j2];
-        const float kij = __ldg(kww + (size_t) i * ws + j2);
-        float kJ[SLOTS];
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            const int t = tid + s * SMO_THREADS;
-            kJ[s] = t < ws ? __ldg(kww + (size_t) j2 * ws + t) : 0.0f;
-        }
-        const double alpha_i_diff = yi > 0 ? Cp - ai : ai;
-        const double curv = NU ? (double) (kd_sm[i] + kd_sm[j2] - 2 * kij)
-                               : (double) (kd_sm[i] + kd_sm[j2]) - 2.0 * (double) kij;
-        const double alpha_j_diff = fmin(yj > 0 ? aj : Cn - aj, (-up + fj) / curv);
-        const double l = fmin(alpha_i_diff, alpha_j_diff);
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            const int t = tid + s * SMO_THREADS;
-            if (t == i) a[s] += l * yi;
-            if (t == j2) a[s] -= l * yj;
-            if (t == i || t == j2) {
-                in_up[s] = in_I_up(a[s], y[s], Cp, Cn);
-                in_low[s] = in_I_low(a[s], y[s], Cp, Cn);
-            }
-            if (t < ws) {
-                const float kI = use1 ? kI1[s] : kI0[s];
-                if (NU) f[s] -= l * (double) (kJ[s] - kI);
-                else f[s] -= l * ((double) kJ[s] - (double) kI);
-            }
-        }
-        ++it;
-    }
-#pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-        const int t = tid + s * SMO_THREADS;
-        if (t < ws) {
-            alpha_ws[t] = a[s];
-            alpha_diff[t] = -(a[s] - aold[s]) * y[s];
-            if (alpha_global && ids[t] >= 0) alpha_global[ids[t]] = a[s];
-        }
-    }
-    if (tid == 0) diff[1] = it;
-}
-
 // ---- gather of the working set's block and vectors ---------------------------------------------
 // Logical slot t of the working set lives in physical row phys(t) of the row buffer (the two
 // halves of the buffer swap roles every outer iteration instead of being copied).
@@ -1401,14 +1150,17 @@ static tsvm_status launch_local_smo(int solver_kind, int ws, const float *kww, c
                                     double eps, int max_iter, double *diff, const int *ids, double *alpha_global,
                                     cudaStream_t st, const int *stop = nullptr) {
     const bool nu = solver_kind != TSVM_SOLVER_C;
-#define SMO_CASE(NU, S, T)                                                                                     \
-    TSVM_LAUNCH((local_smo_kernel<NU, S, T>), 1, T, 0, st, ws, kww, diag_ws, y_ws, f_ws, alpha_ws,             \
-                alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop)
-    if (!nu) {
-        if (ws <= 256) SMO_CASE(false, 1, 256); else if (ws <= 512) SMO_CASE(false, 2, 256); else SMO_CASE(false, 2, 512);
-    } else {
-        if (ws <= 256) SMO_CASE(true, 1, 256); else if (ws <= 512) SMO_CASE(true, 2, 256); else SMO_CASE(true, 2, 512);
-    }
+    // four warps at every size, one to eight slots per thread: measured at 1,024 / 512 / 256 slots 1.00 / 0.84 / 0.73 us
+    // per iteration against 1.12 / 0.99 / 0.86 with eight warps and 1.73 with sixteen (512 slots)
+    constexpr int T = 128;
+#define SMO_CASE(S)                                                                                              \
+    do {                                                                                                         \
+        if (nu) TSVM_LAUNCH((local_smo_kernel<true, S, T>), 1, T, 0, st, ws, kww, diag_ws, y_ws, f_ws, alpha_ws, \
+                            alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop);                   \
+        else TSVM_LAUNCH((local_smo_kernel<false, S, T>), 1, T, 0, st, ws, kww, diag_ws, y_ws, f_ws, alpha_ws,   \
+                         alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop);                      \
+    } while (0)
+    if (ws <= T) SMO_CASE(1); else if (ws <= 2 * T) SMO_CASE(2); else if (ws <= 4 * T) SMO_CASE(4); else SMO_CASE(8);
 #undef SMO_CASE
     return TSVM_OK;
 }
