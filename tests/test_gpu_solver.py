@@ -108,6 +108,28 @@ def test_sorted_runs_merge_equals_select(capi, solver, shards):
     assert np.array_equal(got, exp)
 
 
+@pytest.mark.parametrize("solver", ["c", "nu_svc"])
+@pytest.mark.parametrize("n,want", [(2048, 1024), (2049, 1024), (17, 8), (262145, 512)])
+@pytest.mark.parametrize("law", ["plain", "one_value", "hidden_low", "sampled_low", "few_eligible"])
+def test_working_set_selection_pivot_edges(capi, solver, n, want, law):
+    """The selection's pivot comes from a sample: sizes around the sample's, all keys equal but for the id, and extreme
+    values that the sample does not see (the exact pivot takes over), or almost none to choose from."""
+    y, f, alpha = _state(n, n + want)
+    if law == "one_value":
+        f[:] = -1.0
+    elif law in ("hidden_low", "sampled_low"):       # what the sample sees (128 runs of 16) is not typical
+        runs = np.arange(128)[:, None] * n // 128
+        at = runs + (np.arange(32) + 40 if law == "hidden_low" else np.arange(16))
+        f[at[at < n]] -= 50.0
+    elif law == "few_eligible":
+        alpha = np.where(y > 0, 1.0, 0.0)
+        alpha[:: max(1, n // 40)] = 0.5
+    sel = capi.WorkingSetSelector(n, 1024)
+    got = sel.select(_t(f), _t(alpha), _t(y), 1.0, 1.0, want, solver=solver).cpu().numpy()
+    exp = P.select_working_set("c" if solver == "c" else "nu", f, y, alpha, 1.0, 1.0, None, want)
+    assert np.array_equal(got, exp)
+
+
 @pytest.mark.parametrize("solver,ws", [("c", 1024), ("c", 128), ("c", 64), ("nu_svc", 512), ("nu_svc", 32)])
 def test_local_smo_matches_oracle(capi, solver, ws):
     import torch

@@ -4,7 +4,7 @@
 // src/thundersvm/solver/nusmosolver.cpp:9-136, src/thundersvm/kernel/smo_kernel.cu:28-315.
 #include "common.cuh"
 #include "local_smo.cuh"
-#include <cooperative_groups.h>
+#include "select.cuh"
 #include <chrono>
 #include <limits.h>
 #include <string.h>
@@ -13,680 +13,6 @@
 #include <vector>
 
 namespace tsvm {
-
-// =================================================================================================
-// Working-set selection
-// =================================================================================================
-// The reference sorts all n f-values every outer iteration (smo_kernel.cu:312-315) and then walks
-// the sorted ids from both ends on the host (csmosolver.cpp:123-165). Only the first `want`
-// eligible instances of every walk can ever be taken, so the device keeps, per walk ("list"),
-// the `want` smallest 96-bit keys (f-order, id) among the eligible instances:
-//   C-SMO : list 0 = I_up ascending (f, id);      list 1 = I_low descending (f, id)
-//   nu-SMO: lists 0/1 = I_up for y>0 / y<0;       lists 2/3 = I_low for y>0 / y<0
-// found with a 12-bit radix select of up to 8 passes, followed by a compaction (select_fused_kernel below).
-// One pass = histogram of the current digit over the eligible instances that match the prefix, all lists in
-// one sweep over the data; the last block to finish picks, per list, the digit that holds the wanted rank. A
-// list whose threshold digit holds few enough instances for the whole digit to fit the candidate capacity
-// `cap` is resolved on the spot (the threshold becomes "everything up to and including this digit" and the
-// exact order is left to the sort of the candidates), so that in practice two passes do the work.
-
-constexpr int RADIX_BITS = 12, RADIX_BINS = 1 << RADIX_BITS, RADIX_PASSES = 8, MAX_LISTS = 4;
-typedef unsigned __int128 key96_t;
-
-struct SelectState {            // one per list, lives in device memory
-    unsigned long long prefix_hi;   // bits 95..32 of the threshold key found so far
-    unsigned int prefix_lo;         // bits 31..0
-    int k_rem;                      // rank still to resolve inside the current prefix
-    int take_all;                   // fewer candidates than wanted: take every one
-    int count;                      // compaction cursor
-    int resolved;                   // the threshold is final: later radix passes skip this list
-};
-
-__device__ __forceinline__ int list_count(int solver_kind) { return solver_kind == TSVM_SOLVER_C ? 2 : 4; }
-
-// Is instance (a, y) eligible for list l?
-__device__ __forceinline__ bool in_list(int solver_kind, int l, double a, int y, double Cp, double Cn) {
-    if (solver_kind == TSVM_SOLVER_C) return l == 0 ? in_I_up(a, y, Cp, Cn) : in_I_low(a, y, Cp, Cn);
-    const bool pos = (l & 1) == 0;
-    if (pos != (y > 0)) return false;
-    return l < 2 ? in_I_up(a, y, Cp, Cn) : in_I_low(a, y, Cp, Cn);
-}
-__device__ __forceinline__ bool list_ascending(int solver_kind, int l) {
-    return solver_kind == TSVM_SOLVER_C ? l == 0 : l < 2;
-}
-__device__ __forceinline__ key96_t make_key(bool asc, double f, unsigned id) {
-    unsigned long long h = ordered_key(f);
-    if (!asc) { h = ~h; id = ~id; }
-    return ((key96_t) h << 32) | id;
-}
-
-// ---- merge: sort every candidate list, keep its first `want`, then the reference's alternating
-// walk with "already taken" checks (csmosolver.cpp:123-165 / nusmosolver.cpp:48-118). ------------
-constexpr int MERGE_THREADS = 1024, MERGE_MAX_LEN = 8192, MERGE_MAX_WANT = 1024, HASH_SLOTS = 4096;
-constexpr int MERGE_JOINT_MAX = 2048;          // longest lists that merge_lists sorts side by side
-
-__device__ __forceinline__ bool key_less(unsigned long long ah, unsigned al, unsigned long long bh, unsigned bl) {
-    return ah < bh || (ah == bh && al < bl);
-}
-
-__device__ void merge_lists(int solver_kind, const double *__restrict__ cand_f, const int *__restrict__ cand_id, int len,
-                            int want, int *__restrict__ out_ids, int *__restrict__ out_count, int seg_len,
-                            unsigned char *smem) {
-    const int lists = list_count(solver_kind);
-    int P = 1;
-    while (P < len) P <<= 1;
-    // layout: sort keys (P x 12 B), then per list: top ids / partner positions
-    unsigned long long *kh = reinterpret_cast<unsigned long long *>(smem);
-    unsigned int *kl = reinterpret_cast<unsigned int *>(kh + P);
-    int *top_id = reinterpret_cast<int *>(kl + P);                 // [lists][want]
-    short *partner = reinterpret_cast<short *>(top_id + MAX_LISTS * MERGE_MAX_WANT);   // [lists][want]
-    int *hash_id = reinterpret_cast<int *>(partner + MAX_LISTS * MERGE_MAX_WANT);      // [HASH_SLOTS]
-    short *hash_pos = reinterpret_cast<short *>(hash_id + HASH_SLOTS);
-    __shared__ int top_len[MAX_LISTS];
-    __shared__ unsigned long long last_fkey[MAX_LISTS];
-    __shared__ int real_total;
-    const int tid = threadIdx.x;
-
-    // Lists that are not made of sorted runs and fit the shared memory side by side are sorted together: every
-    // step of the bitonic network handles all lists before its barrier (half the barriers for two lists).
-    const bool joint = seg_len == 0 && P <= MERGE_JOINT_MAX;
-    if (joint) {
-        for (int l = 0; l < lists; ++l) {
-            const bool asc = list_ascending(solver_kind, l);
-            for (int e = tid; e < P; e += MERGE_THREADS) {
-                unsigned long long h = ~0ull;
-                unsigned lo = ~0u;
-                if (e < len) {
-                    const int id = __ldcg(cand_id + (size_t) l * len + e);
-                    if (id >= 0) {
-                        h = ordered_key(__ldcg(cand_f + (size_t) l * len + e));
-                        lo = (unsigned) id;
-                        if (!asc) { h = ~h; lo = ~lo; }
-                    }
-                }
-                kh[(size_t) l * P + e] = h;
-            }
-        }
-        // (kl follows all lists' kh)
-        unsigned int *klj = reinterpret_cast<unsigned int *>(kh + (size_t) lists * P);
-        for (int l = 0; l < lists; ++l) {
-            const bool asc = list_ascending(solver_kind, l);
-            for (int e = tid; e < P; e += MERGE_THREADS) {
-                unsigned lo = ~0u;
-                if (e < len) {
-                    const int id = __ldcg(cand_id + (size_t) l * len + e);
-                    if (id >= 0) lo = asc ? (unsigned) id : ~(unsigned) id;
-                }
-                klj[(size_t) l * P + e] = lo;
-            }
-        }
-        __syncthreads();
-        for (int k = 2; k <= P; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int w = tid; w < lists * (P >> 1); w += MERGE_THREADS) {
-                    // comparison w of this step: list l, lower element e (bit j clear), partner e | j
-                    const int l = w / (P >> 1), c = w - l * (P >> 1);
-                    const int e = ((c & ~(j - 1)) << 1) | (c & (j - 1));
-                    const int x = e | j;
-                    unsigned long long *khl = kh + (size_t) l * P;
-                    unsigned int *kll = klj + (size_t) l * P;
-                    const bool up = (e & k) == 0;
-                    if (key_less(khl[x], kll[x], khl[e], kll[e]) == up) {
-                        unsigned long long th = khl[e]; khl[e] = khl[x]; khl[x] = th;
-                        unsigned tl = kll[e]; kll[e] = kll[x]; kll[x] = tl;
-                    }
-                }
-                __syncthreads();
-            }
-        int *top_id_j = reinterpret_cast<int *>(klj + (size_t) lists * P);
-        top_id = top_id_j;
-        partner = reinterpret_cast<short *>(top_id + MAX_LISTS * MERGE_MAX_WANT);
-        hash_id = reinterpret_cast<int *>(partner + MAX_LISTS * MERGE_MAX_WANT);
-        hash_pos = reinterpret_cast<short *>(hash_id + HASH_SLOTS);
-        for (int l = 0; l < lists; ++l) {
-            const bool asc = list_ascending(solver_kind, l);
-            const unsigned long long *khl = kh + (size_t) l * P;
-            const unsigned int *kll = klj + (size_t) l * P;
-            for (int e = tid; e < want; e += MERGE_THREADS) {
-                int id = -1;
-                if (e < P && !(khl[e] == ~0ull && kll[e] == ~0u)) id = (int) (asc ? kll[e] : ~kll[e]);
-                top_id[l * MERGE_MAX_WANT + e] = id;
-                partner[l * MERGE_MAX_WANT + e] = -1;
-            }
-        }
-        __syncthreads();
-        if (tid < lists) {
-            const int l = tid;
-            const bool asc = list_ascending(solver_kind, l);
-            const unsigned long long *khl = kh + (size_t) l * P;
-            int c = want < P ? want : P;
-            int lo = 0, hi = c;
-            while (lo < hi) { int mid = (lo + hi) >> 1; if (top_id[l * MERGE_MAX_WANT + mid] >= 0) lo = mid + 1; else hi = mid; }
-            top_len[l] = lo;
-            last_fkey[l] = lo > 0 ? (asc ? khl[lo - 1] : ~khl[lo - 1]) : 0ull;
-        }
-        __syncthreads();
-    }
-
-    for (int l = 0; l < lists && !joint; ++l) {
-        const bool asc = list_ascending(solver_kind, l);
-        for (int e = tid; e < P; e += MERGE_THREADS) {
-            unsigned long long h = ~0ull;
-            unsigned lo = ~0u;
-            if (e < len) {
-                const int id = __ldcg(cand_id + (size_t) l * len + e);      // written by other blocks: from L2
-                if (id >= 0) {
-                    h = ordered_key(__ldcg(cand_f + (size_t) l * len + e));
-                    lo = (unsigned) id;
-                    if (!asc) { h = ~h; lo = ~lo; }
-                    // keep real keys distinct from the padding key
-                }
-            }
-            kh[e] = h; kl[e] = lo;
-        }
-        __syncthreads();
-        if (seg_len > 0) {
-            // The list is a sequence of sorted runs (one per rank, padding last): an entry's place in the merged
-            // order is its place in its own run plus, for every other run, the number of smaller keys there
-            // (binary search; keys are distinct because ids are). No sort, a few microseconds for 8 x 512.
-            const int nseg = len / seg_len;
-            for (int e = tid; e < want; e += MERGE_THREADS) {
-                top_id[l * MERGE_MAX_WANT + e] = -1;
-                partner[l * MERGE_MAX_WANT + e] = -1;
-            }
-            if (tid == 0) real_total = 0;
-            __syncthreads();
-            if (tid < nseg) {                       // real entries of run tid: first padding key
-                int lo_i = 0, hi_i = seg_len;
-                while (lo_i < hi_i) {
-                    const int mid = (lo_i + hi_i) >> 1;
-                    const int e = tid * seg_len + mid;
-                    if (kh[e] == ~0ull && kl[e] == ~0u) hi_i = mid; else lo_i = mid + 1;
-                }
-                atomicAdd(&real_total, lo_i);
-            }
-            __syncthreads();
-            const int keep = real_total < want ? real_total : want;
-            for (int e = tid; e < len; e += MERGE_THREADS) {
-                const unsigned long long h = kh[e];
-                const unsigned lo = kl[e];
-                if (h == ~0ull && lo == ~0u) continue;
-                const int r = e / seg_len;
-                int rank = e - r * seg_len;
-                for (int r2 = 0; r2 < nseg && rank < want; ++r2) {
-                    if (r2 == r) continue;
-                    int lo_i = 0, hi_i = seg_len;            // number of keys in run r2 below (h, lo)
-                    while (lo_i < hi_i) {
-                        const int mid = (lo_i + hi_i) >> 1;
-                        const int x = r2 * seg_len + mid;
-                        if (key_less(kh[x], kl[x], h, lo)) lo_i = mid + 1; else hi_i = mid;
-                    }
-                    rank += lo_i;
-                }
-                if (rank < want) {
-                    top_id[l * MERGE_MAX_WANT + rank] = (int) (asc ? lo : ~lo);
-                    if (rank == keep - 1) last_fkey[l] = asc ? h : ~h;
-                }
-            }
-            if (tid == 0) { top_len[l] = keep; if (keep == 0) last_fkey[l] = 0ull; }
-            __syncthreads();
-            continue;
-        }
-        for (int k = 2; k <= P; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int e = tid; e < P; e += MERGE_THREADS) {
-                    const int x = e ^ j;
-                    if (x > e) {
-                        const bool up = (e & k) == 0;
-                        const bool lt = key_less(kh[x], kl[x], kh[e], kl[e]);
-                        if (lt == up) {
-                            unsigned long long th = kh[e]; kh[e] = kh[x]; kh[x] = th;
-                            unsigned tl = kl[e]; kl[e] = kl[x]; kl[x] = tl;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        for (int e = tid; e < want; e += MERGE_THREADS) {
-            int id = -1;
-            if (e < P && !(kh[e] == ~0ull && kl[e] == ~0u)) id = (int) (asc ? kl[e] : ~kl[e]);
-            top_id[l * MERGE_MAX_WANT + e] = id;
-            partner[l * MERGE_MAX_WANT + e] = -1;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            int c = want < P ? want : P;
-            // entries are sorted, padding last: count the real ones
-            int lo = 0, hi = c;
-            while (lo < hi) { int mid = (lo + hi) >> 1; if (top_id[l * MERGE_MAX_WANT + mid] >= 0) lo = mid + 1; else hi = mid; }
-            top_len[l] = lo;
-            // f-order key of the last kept entry: the list's largest f (ascending) / smallest f (descending)
-            last_fkey[l] = lo > 0 ? (asc ? kh[lo - 1] : ~kh[lo - 1]) : 0ull;
-        }
-        __syncthreads();
-    }
-
-    // An instance sits in an "up" list and in the paired "low" list only if the up list's largest f is not
-    // below the low list's smallest f. For large problems that never happens: no instance is then met twice,
-    // the reference's alternating walk takes entry p of every list in round p, and the output position of
-    // every entry follows from the list lengths alone.
-    const int half = lists / 2;
-    bool disjoint = true;
-    for (int u = 0; u < half; ++u)
-        if (top_len[u] > 0 && top_len[u + half] > 0 && !(last_fkey[u] < last_fkey[u + half])) disjoint = false;
-    if (disjoint) {
-        int total = 0;
-        for (int l = 0; l < lists; ++l) total += top_len[l];
-        const int got = total < want ? total : want;
-        for (int e = tid; e < lists * want; e += MERGE_THREADS) {
-            const int l = e / want, p = e - l * want;
-            if (p >= top_len[l]) continue;
-            int pos = 0;
-            for (int o = 0; o < lists; ++o) pos += (top_len[o] < p ? top_len[o] : p) + ((o < l && top_len[o] > p) ? 1 : 0);
-            if (pos < want) out_ids[pos] = top_id[l * MERGE_MAX_WANT + p];
-        }
-        for (int r = got + tid; r < want; r += MERGE_THREADS) out_ids[r] = -1;
-        if (tid == 0 && out_count) *out_count = got;
-        return;
-    }
-
-    // partner positions: an instance can sit in an "up" list and in the "low" list of the same
-    // class. up list u pairs with low list u + lists/2.
-    for (int u = 0; u < half; ++u) {
-        const int lw = u + half;
-        for (int s = tid; s < HASH_SLOTS; s += MERGE_THREADS) hash_id[s] = -1;
-        __syncthreads();
-        for (int e = tid; e < top_len[lw]; e += MERGE_THREADS) {
-            const int id = top_id[lw * MERGE_MAX_WANT + e];
-            unsigned s = ((unsigned) id * 2654435761u) >> 20;
-            for (;;) {
-                const int old = atomicCAS(&hash_id[s], -1, id);
-                if (old == -1) { hash_pos[s] = (short) e; break; }
-                s = (s + 1) & (HASH_SLOTS - 1);
-            }
-        }
-        __syncthreads();
-        for (int e = tid; e < top_len[u]; e += MERGE_THREADS) {
-            const int id = top_id[u * MERGE_MAX_WANT + e];
-            unsigned s = ((unsigned) id * 2654435761u) >> 20;
-            for (;;) {
-                const int cur = hash_id[s];
-                if (cur == -1) break;
-                if (cur == id) {
-                    const short p = hash_pos[s];
-                    partner[u * MERGE_MAX_WANT + e] = p;
-                    partner[lw * MERGE_MAX_WANT + p] = (short) e;
-                    break;
-                }
-                s = (s + 1) & (HASH_SLOTS - 1);
-            }
-        }
-        __syncthreads();
-    }
-
-    // The walk takes the lists in turn, one entry each per round, and steps over an entry whose instance the partner
-    // list has taken. Entry p of a list is reached in round t(p) = p - (entries stepped over before p); the up list,
-    // whose turn comes first in a round, loses a shared instance if the low list reaches it in an earlier round, and
-    // the low list loses it otherwise. Every decision depends on earlier rounds only, so repeating "decide from t,
-    // recompute t by a prefix sum" from t(p) = p settles on the walk's own outcome, in two or three rounds for the
-    // usual case of two lists that run towards each other (one thread walking it took 40 us for 512 ids).
-    static_assert(MERGE_MAX_WANT <= MERGE_THREADS, "one list entry per thread");
-    short *when = reinterpret_cast<short *>(hash_id);                   // [lists][want]: t(p); the hash table is done with
-    static_assert(MAX_LISTS * MERGE_MAX_WANT * sizeof(short) <= HASH_SLOTS * sizeof(int), "t(p) does not fit the hash table");
-    __shared__ int step_over[MAX_LISTS][MERGE_THREADS / 32];
-    __shared__ int n_taken[MAX_LISTS];
-    const int lane = tid & 31, warp = tid >> 5;
-    int t_own[MAX_LISTS];
-    short mate[MAX_LISTS];
-    unsigned stepped = 0;                       // bit l: this thread's entry of list l is stepped over
-#pragma unroll
-    for (int l = 0; l < MAX_LISTS; ++l) {
-        t_own[l] = tid;
-        mate[l] = l < lists && tid < top_len[l] ? partner[l * MERGE_MAX_WANT + tid] : (short) -1;
-    }
-    for (;;) {
-        __syncthreads();                        // (first round: everyone is done with the hash table)
-#pragma unroll
-        for (int l = 0; l < MAX_LISTS; ++l)
-            if (l < lists) when[l * MERGE_MAX_WANT + tid] = (short) t_own[l];
-        __syncthreads();
-        unsigned over[MAX_LISTS];
-#pragma unroll
-        for (int l = 0; l < MAX_LISTS; ++l) {
-            bool skip = false;
-            if (l < lists && mate[l] >= 0) {
-                const int other = when[(l < half ? l + half : l - half) * MERGE_MAX_WANT + mate[l]];
-                skip = l < half ? other < t_own[l] : other <= t_own[l];
-            }
-            over[l] = __ballot_sync(0xffffffffu, skip);
-            if (lane == 0) step_over[l][warp] = __popc(over[l]);
-        }
-        __syncthreads();
-        bool changed = false;
-#pragma unroll
-        for (int l = 0; l < MAX_LISTS; ++l) {
-            if (l >= lists) continue;
-            int before = lane < warp ? step_over[l][lane] : 0;
-            before = __reduce_add_sync(0xffffffffu, before) + __popc(over[l] & ((1u << lane) - 1));
-            changed = changed || (tid < top_len[l] && t_own[l] != tid - before);
-            t_own[l] = tid - before;
-            stepped = (stepped & ~(1u << l)) | (((over[l] >> lane) & 1u) << l);
-        }
-        if (!__syncthreads_or(changed)) break;
-    }
-    if (tid < lists) {
-        int sum = 0;
-        for (int w = 0; w < MERGE_THREADS / 32; ++w) sum += step_over[tid][w];
-        n_taken[tid] = top_len[tid] - sum;
-    }
-    __syncthreads();
-    int total = 0;
-    for (int l = 0; l < lists; ++l) total += n_taken[l];
-    const int got = total < want ? total : want;
-#pragma unroll
-    for (int l = 0; l < MAX_LISTS; ++l) {
-        if (l >= lists || tid >= top_len[l] || ((stepped >> l) & 1u)) continue;
-        const int t = t_own[l];
-        int pos = 0;
-        for (int o = 0; o < lists; ++o) pos += (n_taken[o] < t ? n_taken[o] : t) + ((o < l && n_taken[o] > t) ? 1 : 0);
-        if (pos < want) out_ids[pos] = top_id[l * MERGE_MAX_WANT + tid];
-    }
-    for (int r = got + tid; r < want; r += MERGE_THREADS) out_ids[r] = -1;
-    if (tid == 0 && out_count) *out_count = got;
-}
-
-__global__ void __launch_bounds__(MERGE_THREADS)
-select_merge_kernel(int solver_kind, const double *__restrict__ cand_f, const int *__restrict__ cand_id, int len,
-                    int want, int *__restrict__ out_ids, int *__restrict__ out_count, int seg_len) {
-    extern __shared__ unsigned char smem[];
-    merge_lists(solver_kind, cand_f, cand_id, len, want, out_ids, out_count, seg_len, smem);
-}
-
-// Sorts a candidate list by its list key (padding, id -1, last): one block per list, bitonic in shared
-// memory. The runs of several ranks can then be merged by rank computation instead of a sort.
-__device__ void sort_list(int solver_kind, int l, const double *cand_f, const int *cand_id, int len, double *out_f,
-                          int *out_id, int out_len, unsigned char *smem) {
-    const int tid = threadIdx.x;
-    int P = 1;
-    while (P < len) P <<= 1;
-    unsigned long long *kh = reinterpret_cast<unsigned long long *>(smem);
-    unsigned int *kl = reinterpret_cast<unsigned int *>(kh + P);
-    double *fv = reinterpret_cast<double *>(kl + P + (P & 1));          // the f values travel with their keys
-    const bool asc = list_ascending(solver_kind, l);
-    for (int e = tid; e < P; e += MERGE_THREADS) {
-        unsigned long long h = ~0ull;
-        unsigned lo = ~0u;
-        double v = 0.0;
-        if (e < len) {
-            const int id = __ldcg(cand_id + (size_t) l * len + e);
-            if (id >= 0) {
-                v = __ldcg(cand_f + (size_t) l * len + e);
-                h = ordered_key(v);
-                lo = (unsigned) id;
-                if (!asc) { h = ~h; lo = ~lo; }
-            }
-        }
-        kh[e] = h; kl[e] = lo; fv[e] = v;
-    }
-    __syncthreads();
-    for (int k = 2; k <= P; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int e = tid; e < P; e += MERGE_THREADS) {
-                const int x = e ^ j;
-                if (x > e) {
-                    const bool up = (e & k) == 0;
-                    if (key_less(kh[x], kl[x], kh[e], kl[e]) == up) {
-                        unsigned long long th = kh[e]; kh[e] = kh[x]; kh[x] = th;
-                        unsigned tl = kl[e]; kl[e] = kl[x]; kl[x] = tl;
-                        double tv = fv[e]; fv[e] = fv[x]; fv[x] = tv;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    // the first out_len entries of the sorted list (out_len <= len; the output may be the input)
-    for (int e = tid; e < out_len; e += MERGE_THREADS) {
-        const bool pad = kh[e] == ~0ull && kl[e] == ~0u;
-        out_f[(size_t) l * out_len + e] = pad ? 0.0 : fv[e];
-        out_id[(size_t) l * out_len + e] = pad ? -1 : (int) (asc ? kl[e] : ~kl[e]);
-    }
-}
-
-__global__ void __launch_bounds__(MERGE_THREADS)
-select_sort_candidates_kernel(int solver_kind, const double *cand_f, const int *cand_id, int len, double *out_f,
-                              int *out_id, int out_len) {
-    extern __shared__ unsigned char smem[];
-    sort_list(solver_kind, blockIdx.x, cand_f, cand_id, len, out_f, out_id, out_len, smem);
-}
-
-// ---- the whole selection as ONE cooperative launch -------------------------------------------------------
-// init -> radix passes (as many as the data needs, decided on the device) -> compaction -> sort / merge of the
-// candidates, with grid-wide barriers between the phases instead of one launch per phase. The launch is
-// cooperative (all blocks resident), so the barriers cannot deadlock. Every block takes the same path
-// through the barriers: the decisions between them depend only on state written before the previous barrier.
-namespace cg = cooperative_groups;
-constexpr int FUSED_THREADS = 1024;
-enum { FUSED_CANDIDATES = 0, FUSED_MERGE = 1, FUSED_SORT = 2 };
-
-struct SelectArgs {
-    int solver_kind, n;
-    const double *f, *alpha;
-    const int *y;
-    const unsigned char *in_ws;
-    double Cp, Cn;
-    SelectState *st;
-    int *hist, *ticket;
-    int want, cap, id_offset;
-    double *cand_f;             // [lists][cap]
-    int *cand_id;
-    int mode;                   // FUSED_*
-    int *out_ids, *out_count;   // FUSED_MERGE: the selected ids
-    double *sorted_f;           // FUSED_SORT: the `want` best of every list, sorted, [lists][want]
-    int *sorted_id;
-    // optional rotation of the working set before the selection (plain solver): ids[0..q) <- ids[q..2q),
-    // in-working-set flags of the leaving / staying members
-    int *shift_ids;
-    int shift_q;
-    unsigned char *shift_flags;
-    // optional: when *stop is non-zero the whole launch is a no-op (iterations queued past the end of a solve)
-    const int *stop;
-};
-
-__device__ void merge_lists(int solver_kind, const double *cand_f, const int *cand_id, int len, int want, int *out_ids,
-                            int *out_count, int seg_len, unsigned char *smem);
-__device__ void sort_list(int solver_kind, int l, const double *cand_f, const int *cand_id, int len, double *out_f,
-                          int *out_id, int out_len, unsigned char *smem);
-
-__global__ void __launch_bounds__(FUSED_THREADS, 1) select_fused_kernel(const SelectArgs a) {
-    extern __shared__ unsigned char fused_smem[];
-    int *sh = reinterpret_cast<int *>(fused_smem);
-    __shared__ int scan[256];
-    __shared__ bool is_last;
-    cg::grid_group grid = cg::this_grid();
-    const int lists = list_count(a.solver_kind);
-    // the selection state is written by other blocks between the barriers: always read it from L2
-    volatile SelectState *st = a.st;
-    const int tid = threadIdx.x, gtid = blockIdx.x * FUSED_THREADS + tid, gsize = gridDim.x * FUSED_THREADS;
-    // written by an earlier launch only: every thread of every block reads the same value and leaves before
-    // the first grid barrier
-    if (a.stop && *a.stop) return;
-
-    // ---- phase 0: state, histograms, candidate ids, optional rotation of the working set
-    for (int i = gtid; i < lists * RADIX_BINS; i += gsize) a.hist[i] = 0;
-    for (int i = gtid; i < lists * a.cap; i += gsize) a.cand_id[i] = -1;
-    if (blockIdx.x == 0) {
-        if (tid < lists) {
-            st[tid].prefix_hi = 0; st[tid].prefix_lo = 0; st[tid].k_rem = a.want; st[tid].take_all = 0;
-            st[tid].count = 0; st[tid].resolved = 0;
-        }
-        if (tid == 0) *a.ticket = 0;
-        if (a.shift_ids && tid < a.shift_q) {
-            const int leaving = a.shift_ids[tid], staying = a.shift_ids[a.shift_q + tid];
-            if (leaving >= 0) a.shift_flags[leaving] = 0;
-            if (staying >= 0) a.shift_flags[staying] = 1;
-            a.shift_ids[tid] = staying;
-        }
-    }
-    grid.sync();
-
-    // ---- radix passes: one sweep each; the last block to finish its sweep picks the digits
-    for (int pass = 0; pass < RADIX_PASSES; ++pass) {
-        const int shift = 96 - RADIX_BITS * (pass + 1);
-        unsigned active = 0;
-        key96_t prefix[MAX_LISTS];
-#pragma unroll
-        for (int l = 0; l < MAX_LISTS; ++l) {
-            prefix[l] = 0;
-            if (l < lists && !st[l].take_all && !st[l].resolved) {
-                active |= 1u << l;
-                prefix[l] = ((key96_t) st[l].prefix_hi << 32) | st[l].prefix_lo;
-            }
-        }
-        if (!active) break;                      // the same for every block: the state was final before the barrier
-        for (int b = tid; b < lists * RADIX_BINS; b += FUSED_THREADS) sh[b] = 0;
-        __syncthreads();
-        for (int j = gtid; j < a.n; j += gsize) {
-            if (a.in_ws && a.in_ws[j]) continue;
-            const double al = a.alpha[j], fj = a.f[j];
-            const int yj = a.y[j];
-#pragma unroll
-            for (int l = 0; l < MAX_LISTS; ++l) {
-                if (!((active >> l) & 1u)) continue;
-                if (!in_list(a.solver_kind, l, al, yj, a.Cp, a.Cn)) continue;
-                const key96_t k = make_key(list_ascending(a.solver_kind, l), fj, (unsigned) j);
-                if (pass > 0 && (k >> (shift + RADIX_BITS)) != (prefix[l] >> (shift + RADIX_BITS))) continue;
-                const int bin = l * RADIX_BINS + ((int) (k >> shift) & (RADIX_BINS - 1));
-                if (pass == 0) {
-                    const unsigned peers = __match_any_sync(__activemask(), bin);
-                    if ((int) (tid & 31) == __ffs(peers) - 1) atomicAdd(&sh[bin], __popc(peers));
-                } else {
-                    atomicAdd(&sh[bin], 1);
-                }
-            }
-        }
-        __syncthreads();
-        for (int b = tid; b < lists * RADIX_BINS; b += FUSED_THREADS)
-            if (sh[b]) atomicAdd(&a.hist[b], sh[b]);
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) is_last = (atomicAdd(a.ticket, 1) == (int) gridDim.x - 1);
-        __syncthreads();
-        if (is_last) {
-            __threadfence();
-            // All lists at once: threads 256 l .. 256 l + 255 own list l, 16 consecutive bins each. Exclusive scan of the
-            // per-thread sums inside the list: warp shuffles, then the list's eight warp totals through shared memory.
-            const int l = tid >> 8, t8 = tid & 255, lane = tid & 31;
-            const bool mine = l < lists && ((active >> l) & 1u);
-            int local[16], sum = 0;
-            int *h = a.hist + l * RADIX_BINS + t8 * 16;
-            if (mine) {
-#pragma unroll
-                for (int b4 = 0; b4 < 16; b4 += 4) {
-                    const int4 v = __ldcg(reinterpret_cast<const int4 *>(h + b4));
-                    local[b4] = v.x; local[b4 + 1] = v.y; local[b4 + 2] = v.z; local[b4 + 3] = v.w;
-                    sum += v.x + v.y + v.z + v.w;
-                }
-            }
-            int inc = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += v; }
-            if (lane == 31) scan[tid >> 5] = inc;              // 32 warp totals: 8 per list
-            __syncthreads();
-            if (mine) {
-                int before = inc - sum, total = 0;
-                for (int w = 0; w < 8; ++w) {
-                    const int v = scan[(l << 3) + w];
-                    if (w < (t8 >> 5)) before += v;
-                    total += v;
-                }
-                const int k_rem = st[l].k_rem;
-                if (total < k_rem) {
-                    if (t8 == 0) st[l].take_all = 1;   // can only happen in pass 0
-                } else if (before < k_rem && k_rem <= before + sum) {
-                    int run = before;
-#pragma unroll
-                    for (int b = 0; b < 16; ++b) {
-                        if (run < k_rem && k_rem <= run + local[b]) {
-                            key96_t p = prefix[l] | ((key96_t) (t8 * 16 + b) << shift);
-                            const int k_new = k_rem - run;
-                            if (shift > 0 && (a.want - k_new) + local[b] <= a.cap) {
-                                p |= ((key96_t) 1 << shift) - 1;
-                                st[l].resolved = 1;
-                            }
-                            st[l].prefix_hi = (unsigned long long) (p >> 32);
-                            st[l].prefix_lo = (unsigned int) p;
-                            st[l].k_rem = k_new;
-                        }
-                        run += local[b];
-                    }
-                }
-#pragma unroll
-                for (int b4 = 0; b4 < 16; b4 += 4) *reinterpret_cast<int4 *>(h + b4) = make_int4(0, 0, 0, 0);
-            }
-            __syncthreads();
-            if (tid == 0) *a.ticket = 0;
-            __threadfence();
-        }
-        grid.sync();
-    }
-
-    // ---- compaction of the candidates
-    key96_t threshold[MAX_LISTS];
-    bool take_all[MAX_LISTS];
-#pragma unroll
-    for (int l = 0; l < MAX_LISTS; ++l) {
-        take_all[l] = l < lists ? st[l].take_all != 0 : true;
-        threshold[l] = l < lists ? ((key96_t) st[l].prefix_hi << 32) | st[l].prefix_lo : 0;
-    }
-    for (int j0 = gtid - (tid & 31); j0 < a.n; j0 += gsize) {          // whole warps enter every round (ballots below)
-        const int j = j0 + (tid & 31);
-        const bool live = j < a.n && !(a.in_ws && a.in_ws[j]);
-        const double al = live ? a.alpha[j] : 0.0, fj = live ? a.f[j] : 0.0;
-        const int yj = live ? a.y[j] : 0;
-        unsigned hit = 0;
-#pragma unroll
-        for (int l = 0; l < MAX_LISTS; ++l) {
-            if (l >= lists || !live) continue;
-            if (!in_list(a.solver_kind, l, al, yj, a.Cp, a.Cn)) continue;
-            if (!take_all[l]) {
-                const key96_t thr = threshold[l];
-                if (make_key(list_ascending(a.solver_kind, l), fj, (unsigned) j) > thr) continue;
-            }
-            hit |= 1u << l;
-        }
-        // one atomic per warp and list instead of one per candidate
-#pragma unroll
-        for (int l = 0; l < MAX_LISTS; ++l) {
-            if (l >= lists) continue;
-            const unsigned peers = __ballot_sync(0xffffffffu, (hit >> l) & 1u);
-            if (!peers) continue;
-            int base = 0;
-            if ((tid & 31) == __ffs(peers) - 1) base = atomicAdd(&a.st[l].count, __popc(peers));
-            base = __shfl_sync(0xffffffffu, base, __ffs(peers) - 1);
-            if ((hit >> l) & 1u) {
-                const int pos = base + __popc(peers & ((1u << (tid & 31)) - 1));
-                if (pos < a.cap) { a.cand_f[(size_t) l * a.cap + pos] = fj; a.cand_id[(size_t) l * a.cap + pos] = j + a.id_offset; }
-            }
-        }
-    }
-    if (a.mode == FUSED_CANDIDATES) return;
-    __threadfence();
-    grid.sync();
-    // ---- the candidates are few: one block merges them / one block per list sorts them
-    if (a.mode == FUSED_MERGE) {
-        if (blockIdx.x == 0) merge_lists(a.solver_kind, a.cand_f, a.cand_id, a.cap, a.want, a.out_ids, a.out_count, 0, fused_smem);
-    } else if ((int) blockIdx.x < lists) {
-        sort_list(a.solver_kind, blockIdx.x, a.cand_f, a.cand_id, a.cap, a.sorted_f, a.sorted_id, a.want, fused_smem);
-    }
-}
-
-static size_t merge_smem_bytes(int len) {
-    int P = 1;
-    while (P < len) P <<= 1;
-    // keys of one list, or of all lists side by side where merge_lists sorts them together
-    const size_t keys = (size_t) P * 12 * (P <= MERGE_JOINT_MAX ? MAX_LISTS : 1);
-    return keys + (size_t) MAX_LISTS * MERGE_MAX_WANT * (4 + 2) + (size_t) HASH_SLOTS * 6 + 64;
-}
 
 // ---- gather of the working set's block and vectors ---------------------------------------------
 // Logical slot t of the working set lives in physical row phys(t) of the row buffer (the two
@@ -915,10 +241,24 @@ struct SolverCtl {
 };
 static_assert(offsetof(SolverCtl, stop) == 0, "kernels read the stop flag through a pointer to the struct");
 
+constexpr int STATUS_THREADS = 512;                               // at least half the largest working set
+
 __global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ diff, const int *__restrict__ got,
                                      int wanted, double eps, int max_iter, const long long *__restrict__ cache_ctr,
-                                     const int *__restrict__ engine_status) {
-    if (threadIdx.x != 0 || c->stop) return;
+                                     const int *__restrict__ engine_status, int *__restrict__ ids, int q,
+                                     unsigned char *__restrict__ in_ws) {
+    const int already = c->stop;
+    __syncthreads();
+    if (already) return;
+    // The working set rotates for the next selection: the old second half becomes the first half and keeps its flags,
+    // the old first half leaves. (After the last iteration nothing looks at it again.)
+    if ((int) threadIdx.x < q) {
+        const int leaving = ids[threadIdx.x], staying = ids[q + threadIdx.x];
+        if (leaving >= 0) in_ws[leaving] = 0;
+        if (staying >= 0) in_ws[staying] = 1;
+        ids[threadIdx.x] = staying;
+    }
+    if (threadIdx.x != 0) return;
     const double d = diff[0];
     c->diff0 = d;
     c->local_iter += (long long) diff[1];
@@ -1221,28 +561,49 @@ static size_t row_cache_budget() {
 
 struct tsvm_ws {
     int n_max = 0, ws_max = 0;
-    int cand_cap = 0;               // entries per list of cand_f / cand_id
-    SelectState *state = nullptr;
+    SelectState *state = nullptr;   // zero between calls, like ticket
     int *hist = nullptr, *ticket = nullptr, *count = nullptr;
-    double *cand_f = nullptr;
-    int *cand_id = nullptr;
+    unsigned long long *cand_h = nullptr;       // [4][SELECT_CAP]
+    unsigned int *cand_l = nullptr;
+    double *sorted_f = nullptr;                 // [4][ws_max]
+    int *sorted_id = nullptr;
 };
 
 extern "C" {
 
 void tsvm_set_row_cache_bytes(long long bytes) { g_row_cache_bytes = bytes; }
 
-tsvm_status tsvm_ws_create(int n_max, int ws_max, tsvm_ws **out) {
-    TSVM_REQUIRE(out && n_max > 0 && ws_max > 0 && ws_max <= MERGE_MAX_WANT, "ws_create: bad arguments");
+// (the state still has to be cleared, see clear_select_state)
+static tsvm_status ws_alloc(int n_max, int ws_max, tsvm_ws **out) {
     tsvm_ws *w = new tsvm_ws;
     w->n_max = n_max; w->ws_max = ws_max;
-    w->cand_cap = 2 * ws_max;       // room for the whole threshold digit of an early-resolved list
-    tsvm_status s = dev_alloc(&w->state, MAX_LISTS);
+    tsvm_status s = dev_alloc(&w->state, MAX_LISTS + 1);         // the ticket lies behind the lists
     if (s == TSVM_OK) s = dev_alloc(&w->hist, MAX_LISTS * RADIX_BINS);
-    if (s == TSVM_OK) s = dev_alloc(&w->ticket, 1);
     if (s == TSVM_OK) s = dev_alloc(&w->count, 1);
-    if (s == TSVM_OK) s = dev_alloc(&w->cand_f, (size_t) MAX_LISTS * w->cand_cap);
-    if (s == TSVM_OK) s = dev_alloc(&w->cand_id, (size_t) MAX_LISTS * w->cand_cap);
+    if (s == TSVM_OK) s = dev_alloc(&w->cand_h, (size_t) MAX_LISTS * SELECT_CAP);
+    if (s == TSVM_OK) s = dev_alloc(&w->cand_l, (size_t) MAX_LISTS * SELECT_CAP);
+    if (s == TSVM_OK) s = dev_alloc(&w->sorted_f, (size_t) MAX_LISTS * ws_max);
+    if (s == TSVM_OK) s = dev_alloc(&w->sorted_id, (size_t) MAX_LISTS * ws_max);
+    if (s != TSVM_OK) { tsvm_ws_destroy(w); return s; }
+    w->ticket = reinterpret_cast<int *>(w->state + MAX_LISTS);
+    *out = w;
+    return TSVM_OK;
+}
+static tsvm_status clear_select_state(tsvm_ws *w, cudaStream_t st) {
+    TSVM_CUDA(cudaMemsetAsync(w->state, 0, (MAX_LISTS + 1) * sizeof(SelectState), st));
+    return TSVM_OK;
+}
+
+tsvm_status tsvm_ws_create(int n_max, int ws_max, tsvm_ws **out) {
+    TSVM_REQUIRE(out && n_max > 0 && ws_max > 0 && ws_max <= MERGE_MAX_WANT, "ws_create: bad arguments");
+    *out = nullptr;
+    tsvm_ws *w = nullptr;
+    TSVM_TRY(ws_alloc(n_max, ws_max, &w));
+    tsvm_status s = clear_select_state(w, nullptr);
+    if (s == TSVM_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) {     // the first call may be on any stream
+        set_error("ws_create: clearing the selection state failed");
+        s = TSVM_ERR_CUDA;
+    }
     if (s != TSVM_OK) { tsvm_ws_destroy(w); return s; }
     *out = w;
     return TSVM_OK;
@@ -1250,46 +611,24 @@ tsvm_status tsvm_ws_create(int n_max, int ws_max, tsvm_ws **out) {
 
 void tsvm_ws_destroy(tsvm_ws *w) {
     if (!w) return;
-    pool_free_many({w->state, w->hist, w->ticket, w->count, w->cand_f, w->cand_id});
+    pool_free_many({w->state, w->hist, w->count, w->cand_h, w->cand_l, w->sorted_f, w->sorted_id});
     delete w;
 }
 
-// The selection in one cooperative launch (select_fused_kernel). Candidate lists of `cap` >= want entries each
-// (stride cap): the `want` best of every list are among them; mode says what happens to them on the device.
-struct FusedExtra {
-    int mode = FUSED_CANDIDATES;
-    int *out_ids = nullptr;                       // FUSED_MERGE
-    double *sorted_f = nullptr;                   // FUSED_SORT
-    int *sorted_id = nullptr;
-    int *shift_ids = nullptr;                     // optional rotation of the working set first
-    int shift_q = 0;
-    unsigned char *shift_flags = nullptr;
-    const int *stop = nullptr;
-};
-
-static size_t fused_smem_bytes(int lists, int cap, int mode) {
-    size_t b = (size_t) lists * RADIX_BINS * sizeof(int);
-    int P = 1;
-    while (P < cap) P <<= 1;
-    if (mode == FUSED_MERGE && merge_smem_bytes(cap) > b) b = merge_smem_bytes(cap);
-    if (mode == FUSED_SORT && (size_t) P * 20 + 8 > b) b = (size_t) P * 20 + 8;
-    return b;
-}
-
-static tsvm_status ws_candidates_cap(tsvm_ws *w, int solver_kind, int n, const double *f_dev, const double *alpha_dev,
-                                     const int *y_dev, const unsigned char *in_ws_dev, double Cp, double Cn, int want,
-                                     int cap, int id_offset, double *cand_f_dev, int *cand_id_dev, cudaStream_t st,
-                                     const FusedExtra &x = FusedExtra()) {
+// The selection in one cooperative launch (select_kernel). out_ids: the merged selection; else the sorted lists
+// ([lists][want], padding id -1) in sorted_f / sorted_id are the result.
+static tsvm_status launch_select(tsvm_ws *w, int solver_kind, int n, const double *f_dev, const double *alpha_dev,
+                                 const int *y_dev, const unsigned char *in_ws_dev, double Cp, double Cn, int want,
+                                 int id_offset, double *sorted_f, int *sorted_id, int *out_ids, const int *stop,
+                                 cudaStream_t st) {
     const int lists = solver_kind == TSVM_SOLVER_C ? 2 : 4;
     static int resident_blocks[MAX_DEVICES] = {0};
     int dev = 0;
     TSVM_CUDA(cudaGetDevice(&dev));
     int &max_blocks = resident_blocks[dev & (MAX_DEVICES - 1)];
     if (!max_blocks) {
-        const size_t smem_max = fused_smem_bytes(MAX_LISTS, MERGE_MAX_LEN, FUSED_SORT) > fused_smem_bytes(MAX_LISTS, MERGE_MAX_LEN, FUSED_MERGE)
-                                    ? fused_smem_bytes(MAX_LISTS, MERGE_MAX_LEN, FUSED_SORT)
-                                    : fused_smem_bytes(MAX_LISTS, MERGE_MAX_LEN, FUSED_MERGE);
-        TSVM_CUDA(cudaFuncSetAttribute(select_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_max));
+        TSVM_CUDA(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int) select_smem_bytes(MAX_LISTS, SAMPLE_MAX)));
         int sms = 0, coop = 0;
         TSVM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         TSVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
@@ -1298,16 +637,23 @@ static tsvm_status ws_candidates_cap(tsvm_ws *w, int solver_kind, int n, const d
     }
     SelectArgs a;
     a.solver_kind = solver_kind; a.n = n; a.f = f_dev; a.alpha = alpha_dev; a.y = y_dev; a.in_ws = in_ws_dev;
-    a.Cp = Cp; a.Cn = Cn; a.st = w->state; a.hist = w->hist; a.ticket = w->ticket; a.want = want; a.cap = cap;
-    a.id_offset = id_offset; a.cand_f = cand_f_dev; a.cand_id = cand_id_dev; a.mode = x.mode; a.out_ids = x.out_ids;
-    a.out_count = w->count; a.sorted_f = x.sorted_f; a.sorted_id = x.sorted_id; a.shift_ids = x.shift_ids;
-    a.shift_q = x.shift_q; a.shift_flags = x.shift_flags; a.stop = x.stop;
-    int grid = ceil_div(n, FUSED_THREADS * 2);
+    a.Cp = Cp; a.Cn = Cn; a.st = w->state; a.hist = w->hist; a.ticket = w->ticket; a.want = want;
+    a.id_offset = id_offset; a.cand_h = w->cand_h; a.cand_l = w->cand_l; a.sorted_f = sorted_f; a.sorted_id = sorted_id;
+    a.out_ids = out_ids; a.out_count = w->count; a.stop = stop;
+    a.sample = select_sample(n);
+    if (a.sample == n) { a.rank_low = want; a.rank_high = want + want / 2; }
+    else {
+        // `want` instances put want * sample / n of their own into the sample, give or take the square root of that;
+        // 3.2 of these and two more are added so that the pivot hardly ever falls short
+        const double mean = (double) want * a.sample / n;
+        a.rank_low = (int) (mean + 3.2 * sqrt(mean) + 2.0);
+        a.rank_high = a.rank_low + a.rank_low / 4 + 2;
+    }
+    int grid = select_grid(n);
     if (grid > max_blocks) grid = max_blocks;
-    if (grid < (x.mode == FUSED_SORT ? lists : 1)) grid = x.mode == FUSED_SORT ? lists : 1;
     void *args[] = {&a};
-    TSVM_CUDA(cudaLaunchCooperativeKernel((const void *) select_fused_kernel, dim3(grid), dim3(FUSED_THREADS), args,
-                                          fused_smem_bytes(lists, cap, x.mode), st));
+    TSVM_CUDA(cudaLaunchCooperativeKernel((const void *) select_kernel, dim3(grid), dim3(SELECT_THREADS), args,
+                                          select_smem_bytes(lists, a.sample), st));
     count_launch();
     return TSVM_OK;
 }
@@ -1317,8 +663,8 @@ tsvm_status tsvm_ws_candidates(tsvm_ws *w, int solver_kind, int n, const double 
                                int id_offset, double *cand_f_dev, int *cand_id_dev, void *stream) {
     TSVM_REQUIRE(w && f_dev && alpha_dev && y_dev && cand_f_dev && cand_id_dev && n > 0 && want > 0 &&
                  want <= w->ws_max && solver_kind >= 0 && solver_kind <= 2, "ws_candidates: bad arguments");
-    return ws_candidates_cap(w, solver_kind, n, f_dev, alpha_dev, y_dev, in_ws_dev, Cp, Cn, want, want, id_offset,
-                             cand_f_dev, cand_id_dev, (cudaStream_t) stream);
+    return launch_select(w, solver_kind, n, f_dev, alpha_dev, y_dev, in_ws_dev, Cp, Cn, want, id_offset, cand_f_dev,
+                         cand_id_dev, nullptr, nullptr, (cudaStream_t) stream);
 }
 
 static tsvm_status ws_merge_impl(tsvm_ws *w, int solver_kind, const double *cand_f_dev, const int *cand_id_dev, int len,
@@ -1371,13 +717,8 @@ tsvm_status tsvm_select_working_set(tsvm_ws *w, int solver_kind, int n, const do
                                     int *out_ids_dev, void *stream) {
     TSVM_REQUIRE(w && f_dev && alpha_dev && y_dev && out_ids_dev && n > 0 && want > 0 && want <= w->ws_max &&
                  solver_kind >= 0 && solver_kind <= 2, "select_working_set: bad arguments");
-    const int cap = 2 * want <= w->cand_cap ? 2 * want : (want <= w->cand_cap ? w->cand_cap : want);
-    TSVM_REQUIRE(cap >= want, "select_working_set: candidate buffers hold %d entries, %d wanted", w->cand_cap, want);
-    FusedExtra x;
-    x.mode = FUSED_MERGE;
-    x.out_ids = out_ids_dev;
-    return ws_candidates_cap(w, solver_kind, n, f_dev, alpha_dev, y_dev, in_ws_dev, Cp, Cn, want, cap, 0, w->cand_f,
-                             w->cand_id, (cudaStream_t) stream, x);
+    return launch_select(w, solver_kind, n, f_dev, alpha_dev, y_dev, in_ws_dev, Cp, Cn, want, 0, w->sorted_f, w->sorted_id,
+                         out_ids_dev, nullptr, (cudaStream_t) stream);
 }
 
 // ---- working-set selection without any allocation --------------------------------------------------
@@ -1390,9 +731,11 @@ constexpr size_t STATIC_OFF_STATE = 0;                                          
 constexpr size_t STATIC_OFF_HIST = 256;                                                  // int[4 * 4096]
 constexpr size_t STATIC_OFF_TICKET = STATIC_OFF_HIST + sizeof(int) * MAX_LISTS * RADIX_BINS;   // int
 constexpr size_t STATIC_OFF_COUNT = STATIC_OFF_TICKET + 128;                             // int
-constexpr size_t STATIC_OFF_CAND_F = STATIC_OFF_COUNT + 128;                             // double[4 * 1024]
-constexpr size_t STATIC_OFF_CAND_ID = STATIC_OFF_CAND_F + sizeof(double) * MAX_LISTS * STATIC_WS_MAX;
-constexpr size_t STATIC_SCRATCH_BYTES = STATIC_OFF_CAND_ID + sizeof(int) * MAX_LISTS * STATIC_WS_MAX;
+constexpr size_t STATIC_OFF_CAND_H = STATIC_OFF_COUNT + 128;                             // uint64[4 * SELECT_CAP]
+constexpr size_t STATIC_OFF_CAND_L = STATIC_OFF_CAND_H + 8 * MAX_LISTS * SELECT_CAP;     // uint32[4 * SELECT_CAP]
+constexpr size_t STATIC_OFF_SORTED_F = STATIC_OFF_CAND_L + 4 * MAX_LISTS * SELECT_CAP;   // double[4 * 1024]
+constexpr size_t STATIC_OFF_SORTED_ID = STATIC_OFF_SORTED_F + sizeof(double) * MAX_LISTS * STATIC_WS_MAX;
+constexpr size_t STATIC_SCRATCH_BYTES = STATIC_OFF_SORTED_ID + sizeof(int) * MAX_LISTS * STATIC_WS_MAX;
 static_assert(sizeof(SelectState) * MAX_LISTS <= STATIC_OFF_HIST, "selection state does not fit its slot");
 static __device__ __align__(256) unsigned char g_static_select_scratch[STATIC_SCRATCH_BYTES];
 
@@ -1423,15 +766,16 @@ tsvm_status tsvm_select_working_set_static(int solver_kind, int n, const double 
     tsvm_ws view;                      // a view over the static array; owns nothing, frees nothing
     view.n_max = n;
     view.ws_max = STATIC_WS_MAX;
-    view.cand_cap = STATIC_WS_MAX;
     view.state = reinterpret_cast<SelectState *>(base + STATIC_OFF_STATE);
     view.hist = reinterpret_cast<int *>(base + STATIC_OFF_HIST);
     view.ticket = reinterpret_cast<int *>(base + STATIC_OFF_TICKET);
     view.count = reinterpret_cast<int *>(base + STATIC_OFF_COUNT);
-    view.cand_f = reinterpret_cast<double *>(base + STATIC_OFF_CAND_F);
-    view.cand_id = reinterpret_cast<int *>(base + STATIC_OFF_CAND_ID);
-    // the selection kernel's first phase zeroes the state, the histograms and the ticket and resets the
-    // candidate ids on every call, so nothing of an earlier call's contents is read.
+    view.cand_h = reinterpret_cast<unsigned long long *>(base + STATIC_OFF_CAND_H);
+    view.cand_l = reinterpret_cast<unsigned int *>(base + STATIC_OFF_CAND_L);
+    view.sorted_f = reinterpret_cast<double *>(base + STATIC_OFF_SORTED_F);
+    view.sorted_id = reinterpret_cast<int *>(base + STATIC_OFF_SORTED_ID);
+    // the counters that have to be zero at the start of a call are zero in the image and are cleared again by the last
+    // block of every call; nothing else of an earlier call's contents is read.
     return tsvm_select_working_set(&view, solver_kind, n, f_dev, alpha_dev, y_dev, in_ws_dev, Cp, Cn, want,
                                    out_ids_dev, stream);
 }
@@ -1611,7 +955,8 @@ struct tsvm_solver {
         TSVM_TRY(dev_alloc(&red, 16));   // >= RHO_VALS
         TSVM_TRY(dev_alloc(&in_ws, (size_t) n));
         TSVM_CUDA(cudaMemsetAsync(in_ws, 0, (size_t) n, st));
-        TSVM_TRY(tsvm_ws_create(n, ws, &sel));
+        TSVM_TRY(ws_alloc(n, ws, &sel));
+        TSVM_TRY(clear_select_state(sel, st));
         TSVM_TRY(pinned_alloc((void **) &diff_host, 16 * sizeof(double)));
         TSVM_TRY(dev_alloc(&ctl, 1));
         TSVM_TRY(pinned_alloc((void **) &ctl_host, sizeof(SolverCtl)));
@@ -1678,19 +1023,9 @@ struct tsvm_solver {
         const int *n_miss_dev = reinterpret_cast<const int *>(cache_ctr);
         const int *stop = &ctl->stop;
         TSVM_CUDA(cudaEventRecord(E.ph[0], st));
-        if (it == 0) {
-            TSVM_TRY(tsvm_select_working_set(sel, kind, n, f, alpha, y, nullptr, Cp, Cn, ws, ids, st));
-        } else {
-            // rotation of the working set (old second half -> first half, flags) and the selection of the new
-            // second half: one cooperative launch
-            FusedExtra x;
-            x.mode = FUSED_MERGE;
-            x.out_ids = ids + q;
-            x.shift_ids = ids; x.shift_q = q; x.shift_flags = in_ws;
-            x.stop = stop;
-            TSVM_TRY(ws_candidates_cap(sel, kind, n, f, alpha, y, in_ws, Cp, Cn, q, 2 * q <= sel->cand_cap ? 2 * q : q, 0,
-                                       sel->cand_f, sel->cand_id, st, x));
-        }
+        // (the status kernel of the previous iteration has rotated the working set)
+        TSVM_TRY(launch_select(sel, kind, n, f, alpha, y, it == 0 ? nullptr : in_ws, Cp, Cn, n_new, 0, sel->sorted_f,
+                               sel->sorted_id, ids + t0, it == 0 ? nullptr : stop, st));
         if (overlapped) {
             // The block's new rows need the members' planes and nothing else: the second stream starts on them
             // (new members against all members, from the members' own operand planes) while the first one still
@@ -1769,8 +1104,8 @@ struct tsvm_solver {
                         rows_vec_ok(rows, ld), q, ws, update_f_cols(n), row_slot);
         }
         TSVM_CUDA(cudaEventRecord(E.ph[4], st));
-        TSVM_LAUNCH(solver_status_kernel, 1, 32, 0, st, ctl, diff, sel->count, n_new, eps, max_iter, cache_ctr,
-                    km->status_dev);
+        TSVM_LAUNCH(solver_status_kernel, 1, STATUS_THREADS, 0, st, ctl, diff, sel->count, n_new, eps, max_iter, cache_ctr,
+                    km->status_dev, ids, q, in_ws);
         return TSVM_OK;
     }
 
@@ -2059,7 +1394,8 @@ struct tsvm_shard {
         TSVM_TRY(dev_alloc(&grp_id, (size_t) world * MAX_LISTS * ws));
         TSVM_TRY(dev_alloc(&in_ws, (size_t) n_local));
         TSVM_CUDA(cudaMemsetAsync(in_ws, 0, (size_t) n_local, st));
-        TSVM_TRY(tsvm_ws_create(n_local, ws, &sel));
+        TSVM_TRY(ws_alloc(n_local, ws, &sel));
+        TSVM_TRY(clear_select_state(sel, st));
         TSVM_TRY(dev_alloc(&ctl, 1));
         TSVM_TRY(pinned_alloc((void **) &ctl_host, sizeof(SolverCtl)));
         memset(ctl_host, 0, sizeof(SolverCtl));
@@ -2089,16 +1425,9 @@ struct tsvm_shard {
             TSVM_CUDA(cudaMemcpyAsync(m_lo, (char *) m_lo + (size_t) q * row_bytes, (size_t) q * row_bytes,
                                       cudaMemcpyDeviceToDevice, st));
         }
-        // Candidates into the selector's own lists with twice the wanted capacity where it fits (the radix
-        // select then stops after two sweeps, see select_fused_kernel), sorted, and the best n_new of every
-        // list handed over: the merge of the gathered sorted runs needs no sort.
-        const int cap = 2 * n_new <= sel->cand_cap ? 2 * n_new : n_new;
-        FusedExtra x;
-        x.mode = FUSED_SORT;
-        x.sorted_f = cand_f; x.sorted_id = cand_id;
-        x.stop = &ctl->stop;
-        TSVM_TRY(ws_candidates_cap(sel, kind, n_local, f, alpha, y, it == 0 ? nullptr : in_ws, Cp, Cn, n_new, cap, lo,
-                                   sel->cand_f, sel->cand_id, st, x));
+        // the best n_new of every list, sorted: the merge of the gathered sorted runs needs no sort
+        TSVM_TRY(launch_select(sel, kind, n_local, f, alpha, y, it == 0 ? nullptr : in_ws, Cp, Cn, n_new, lo, cand_f, cand_id,
+                               nullptr, &ctl->stop, st));
         *lists_out = lists;
         *want_out = n_new;
         phase = 1;
@@ -2176,7 +1505,7 @@ struct tsvm_shard {
                     rows, ld, rows_vec_ok(rows, ld), it == 0 ? 0 : q, ws, update_f_cols(n_local), (const int *) nullptr);
         TSVM_LAUNCH(shard_scatter_kernel, ceil_div(ws, 256), 256, 0, st, ids, ws, lo, hi, a_ws, alpha);
         TSVM_LAUNCH(solver_status_kernel, 1, 32, 0, st, ctl, diff, sel->count, n_new, eps, -1, (const long long *) nullptr,
-                    km->status_dev);
+                    km->status_dev, (int *) nullptr, 0, (unsigned char *) nullptr);
         ++queued;
         phase = 0;
         return TSVM_OK;
