@@ -70,7 +70,8 @@ __device__ __forceinline__ int cache_bin(int stamp, int now) {
 
 __global__ void __launch_bounds__(CACHE_THREADS, 1)
 cache_assign_kernel(const int *__restrict__ ids, int t0, int n_new, int now, int *__restrict__ slot_of,
-                    int *__restrict__ inst_of, int *__restrict__ stamp, int cap, int *__restrict__ row_slot,
+                    int *__restrict__ inst_of, int *__restrict__ stamp, int cap,
+                    const int *__restrict__ row_slot_before, int *__restrict__ row_slot,
                     int *__restrict__ miss_ids, int *__restrict__ miss_slot, int *__restrict__ victims,
                     long long *__restrict__ ctr, int row_block, const int *__restrict__ stop) {
     if (stop && *stop) {            // queued past the end of a solve: no member changes, no row to compute
@@ -84,7 +85,7 @@ cache_assign_kernel(const int *__restrict__ ids, int t0, int n_new, int now, int
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // the members that stay move to the front; their rows are in use now
     int keep = 0;
-    if (tid < t0) keep = row_slot[t0 + tid];
+    if (tid < t0) keep = row_slot_before[t0 + tid];
     for (int b = tid; b < CACHE_BINS; b += CACHE_THREADS) hist[b] = 0;
     if (tid == 0) { n_miss_s = 0; n_hit_s = 0; }
     __syncthreads();
@@ -864,7 +865,7 @@ struct tsvm_solver {
     float *ws_hi = nullptr, *ws_lo = nullptr, *ws_sd = nullptr, *ws_unscale = nullptr;
     // kernel-row cache (cache_assign_kernel): the row buffer holds cache_cap rows; directory and per-iteration lists
     long long cache_cap = 0;
-    int *slot_of = nullptr, *inst_of = nullptr, *stamp = nullptr, *row_slot = nullptr, *miss_ids = nullptr,
+    int *slot_of = nullptr, *inst_of = nullptr, *stamp = nullptr, *row_slots = nullptr, *miss_ids = nullptr,
         *miss_slot = nullptr, *victims = nullptr;
     long long *cache_ctr = nullptr;
     float *miss_hi = nullptr, *miss_lo = nullptr, *miss_sd = nullptr, *miss_unscale = nullptr;
@@ -879,7 +880,7 @@ struct tsvm_solver {
 
     ~tsvm_solver() {
         pool_free_many({ids, y_ws, rows, kww, diag_ws, f_ws, a_ws, alpha_diff, diff, red, in_ws, ws_hi, ws_lo, ws_sd,
-                        ws_unscale, slot_of, inst_of, stamp, row_slot, miss_ids, miss_slot, victims, cache_ctr, miss_hi,
+                        ws_unscale, slot_of, inst_of, stamp, row_slots, miss_ids, miss_slot, victims, cache_ctr, miss_hi,
                         miss_lo, miss_sd, miss_unscale, ctl});
         tsvm_ws_destroy(sel);
         if (diff_host) pinned_free(diff_host);
@@ -929,7 +930,7 @@ struct tsvm_solver {
         TSVM_TRY(dev_alloc(&slot_of, (size_t) n));
         TSVM_TRY(dev_alloc(&inst_of, (size_t) cache_cap));
         TSVM_TRY(dev_alloc(&stamp, (size_t) cache_cap));
-        TSVM_TRY(dev_alloc(&row_slot, (size_t) ws));
+        TSVM_TRY(dev_alloc(&row_slots, (size_t) 2 * ws));      // this iteration's and the previous one's
         TSVM_TRY(dev_alloc(&miss_ids, (size_t) ws));
         TSVM_TRY(dev_alloc(&miss_slot, (size_t) ws));
         TSVM_TRY(dev_alloc(&victims, (size_t) ws));
@@ -937,7 +938,7 @@ struct tsvm_solver {
         TSVM_LAUNCH(fill_int_kernel, 296, 256, 0, st, slot_of, (long long) n, -1);
         TSVM_LAUNCH(fill_int_kernel, 296, 256, 0, st, inst_of, cache_cap, -1);
         TSVM_CUDA(cudaMemsetAsync(stamp, 0, sizeof(int) * (size_t) cache_cap, st));
-        TSVM_CUDA(cudaMemsetAsync(row_slot, 0, sizeof(int) * (size_t) ws, st));
+        TSVM_CUDA(cudaMemsetAsync(row_slots, 0, sizeof(int) * (size_t) 2 * ws, st));
         TSVM_CUDA(cudaMemsetAsync(cache_ctr, 0, sizeof(long long) * CACHE_CTRS, st));
         return TSVM_OK;
     }
@@ -1022,29 +1023,39 @@ struct tsvm_solver {
         const int row_block = km_pair_engine(km, st) ? 256 : 64;           // requested rows per tile of the engine
         const int *n_miss_dev = reinterpret_cast<const int *>(cache_ctr);
         const int *stop = &ctl->stop;
+        int *row_slot = row_slots + (it & 1) * ws;                         // row of every working-set slot
+        const int *row_slot_before = row_slots + ((it + 1) & 1) * ws;
         TSVM_CUDA(cudaEventRecord(E.ph[0], st));
         // (the status kernel of the previous iteration has rotated the working set)
         TSVM_TRY(launch_select(sel, kind, n, f, alpha, y, it == 0 ? nullptr : in_ws, Cp, Cn, n_new, 0, sel->sorted_f,
                                sel->sorted_id, ids + t0, it == 0 ? nullptr : stop, st));
         if (overlapped) {
-            // The block's new rows need the members' planes and nothing else: the second stream starts on them
-            // (new members against all members, from the members' own operand planes) while the first one still
-            // runs the cache directory, i.e. before the big launch takes all SM pairs but one.
+            // The block needs the members' planes and the old members' rows, both known now: the second stream starts on
+            // it while the first one still runs the cache directory, i.e. before the big launch takes all SM pairs
+            // but one (started after it, the gather alone took 240 us at 200,000 instances; now 20). Rows 0..q-1 come
+            // from the row buffer (where the previous iteration left them), rows q..ws-1 are computed from the members' own
+            // operand planes.
             TSVM_TRY(ensure_ws_planes());
             TSVM_TRY(ensure_miss_planes());
             TSVM_TRY(km_gather_planes(km, ids, ws, nullptr, ws_hi, ws_lo, ws_sd, ws_unscale, st));
             TSVM_CUDA(cudaEventRecord(ev_fork, st));
             TSVM_CUDA(cudaStreamWaitEvent(st2, ev_fork, 0));
+            TSVM_LAUNCH(gather_ws_kernel, ws, 256, 0, st2, ws, q, 0, ids, rows, ld, km->diag, y, f, alpha, kww, diag_ws,
+                        y_ws, f_ws, a_ws, q, row_slot_before + q);
             const size_t rb = km_plane_row_bytes(km);
             const InstancePlanes members{ws_hi, ws_lo, ws_sd, ws_unscale, ws};
             const RowPlanes new_members{reinterpret_cast<const float *>(reinterpret_cast<const char *>(ws_hi) + (size_t) q * rb),
                                         reinterpret_cast<const float *>(reinterpret_cast<const char *>(ws_lo) + (size_t) q * rb),
                                         ws_sd + q, ws_unscale + q};
             TSVM_TRY(km_rows_planes_on(km, members, new_members, q, kww + (size_t) q * ws, ws, st2));
+            TSVM_CUDA(cudaEventRecord(E.l0, st2));
+            TSVM_TRY(launch_local_smo(kind, ws, kww, diag_ws, y_ws, f_ws, a_ws, alpha_diff, Cp, Cn, eps, local_max_iter,
+                                      diff, ids, alpha, st2, stop));
+            TSVM_CUDA(cudaEventRecord(E.l1, st2));
         }
         // cache directory: hits point at their rows, misses get the least recently used rows
         TSVM_LAUNCH(cache_assign_kernel, 1, CACHE_THREADS, 0, st, ids, t0, n_new, (int) (it + 1), slot_of, inst_of, stamp,
-                    (int) cache_cap, row_slot, miss_ids, miss_slot, victims, cache_ctr, row_block, stop);
+                    (int) cache_cap, row_slot_before, row_slot, miss_ids, miss_slot, victims, cache_ctr, row_block, stop);
         TSVM_CUDA(cudaEventRecord(E.ph[1], st));
         if (!overlapped) {
             // the engine computes the missing rows only (their number is read on the device) into their cache rows
@@ -1055,15 +1066,7 @@ struct tsvm_solver {
         } else {
             TSVM_TRY(km_gather_planes(km, miss_ids, q, n_miss_dev, miss_hi, miss_lo, miss_sd, miss_unscale, st));
             TSVM_CUDA(cudaEventRecord(ev_fork2, st));
-            // second stream, after the directory: block rows 0..q-1 and the slot vectors by gather from the rows in
-            // the buffer, then the local solver
             TSVM_CUDA(cudaStreamWaitEvent(st2, ev_fork2, 0));
-            TSVM_LAUNCH(gather_ws_kernel, ws, 256, 0, st2, ws, q, 0, ids, rows, ld, km->diag, y, f, alpha, kww, diag_ws,
-                        y_ws, f_ws, a_ws, q, row_slot);
-            TSVM_CUDA(cudaEventRecord(E.l0, st2));
-            TSVM_TRY(launch_local_smo(kind, ws, kww, diag_ws, y_ws, f_ws, a_ws, alpha_diff, Cp, Cn, eps, local_max_iter,
-                                      diff, ids, alpha, st2, stop));
-            TSVM_CUDA(cudaEventRecord(E.l1, st2));
             // the rows that were in the buffer already can be applied to f at once (HBM-bound, next to the
             // tensor-bound launch); the new rows follow on the first stream
             TSVM_LAUNCH(update_f_kernel, update_f_grid(n), 128, 0, st2, f, n, alpha_diff, ws, q, 0, rows, ld,
