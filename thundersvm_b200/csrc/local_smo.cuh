@@ -55,22 +55,112 @@ __device__ __forceinline__ double reciprocal(double a) {
     return a != 0.0 && fabs(a) < 1e300 ? r : r0;
 }
 
+// Row ring: rows of kww that the next iterations are likely to need, copied to shared memory by a warp of its own.
+constexpr int RING = 32;                // one ring slot per lane of the copying warp
+constexpr int RING_SPARE = 10;          // slots kept free for the next copies
+constexpr int NOT_THERE = -1, ON_THE_WAY = -2;
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
+__device__ __forceinline__ int load_acquire(const int *p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_release(int *p, int v) {
+    asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ bool copy_done(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+template <int T>
+__device__ __forceinline__ void solver_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory"); }
+
 struct First { double f; int slot; float low; };        // a warp's smallest f over I_up, its slot; high word of max f over I_low
 struct Second { float best, next; int slot, pad; };     // a warp's largest and second-largest estimate of b^2 / a
+
+// The copying warp. Which rows the next iterations need can be guessed: the winner of an argmin is usually among the best
+// few of the argmin before. Every warp of the solver leaves its best two slots of both argmins in `cand` (n_cand ids);
+// whichever of them has no row in the ring is copied there, and a row that has not been wanted for longest makes room.
+//   where[t]: ring slot of row t, NOT_THERE or ON_THE_WAY. It is set only when the copy has arrived, so a solver thread
+//   either finds the row or reads kww; both hold the same values.
+//   A row is taken out of `where` first and its slot is overwritten three windows later (a window: from one barrier of the
+//   solver to the next): a row that a solver thread finds in a window is read in that window and the next.
+__device__ void copy_rows_ahead(const float *__restrict__ kww, int ws, float *ring, int *where, const int *cand, int n_cand,
+                                const int *window, const int *done, unsigned long long *bars, int *stamp, int *stage) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu, bar = smem_addr(bars + lane), row_bytes = (unsigned) ws * 4;
+    enum { FREE, COMING, READY };
+    int state = FREE, row = 0, freed = -4, used = 0, seen = -1;
+    unsigned parity = 0;
+    auto arrived = [&](int now) {
+        if (state == COMING && copy_done(bar, parity)) {
+            parity ^= 1;
+            state = READY;
+            used = now;
+            store_release(where + row, lane);
+        }
+    };
+    // (bounded: a solver that runs longer than this goes on without new rows)
+    for (int polls = 0; polls < (1 << 26); ++polls) {
+        const int now = load_acquire(window);
+        if (load_acquire(done)) break;
+        arrived(now);
+        if (__all_sync(full, now == seen)) { __nanosleep(32); continue; }
+        seen = now;
+        // candidates without a row, each once
+        const int x = lane < n_cand ? *(volatile const int *) (cand + lane) : -1;
+        const bool valid = (unsigned) x < (unsigned) ws;
+        const int at = valid ? *(volatile int *) (where + x) : (int) ON_THE_WAY;
+        const unsigned same = __match_any_sync(full, valid ? x : -1 - lane);
+        const bool need = valid && at == NOT_THERE && lane == __ffs(same) - 1;
+        if (valid && at >= 0) stamp[at] = now;
+        const unsigned needs = __ballot_sync(full, need);
+        if (need) stage[__popc(needs & ((1u << lane) - 1))] = x;
+        __syncwarp();
+        if (state == READY && stamp[lane] == now) used = now;
+        const bool open = state == FREE && now - freed >= 3;
+        const unsigned opens = __ballot_sync(full, open);
+        const int k = __popc(opens & ((1u << lane) - 1));
+        if (open && k < __popc(needs)) {
+            row = stage[k];
+            *(volatile int *) (where + row) = ON_THE_WAY;
+            state = COMING;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(row_bytes) : "memory");
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_addr(ring + (size_t) lane * ws)), "l"(kww + (size_t) row * ws), "r"(row_bytes), "r"(bar) : "memory");
+        }
+        // make room: the row that has not been wanted for longest
+        const int spare = __popc(__ballot_sync(full, state == FREE));
+        const int oldest = __reduce_min_sync(full, state == READY ? used : 0x7fffffff);
+        const unsigned olds = __ballot_sync(full, state == READY && used == oldest);
+        if (spare < RING_SPARE && state == READY && used == oldest && oldest < now &&
+            __popc(olds & ((1u << lane) - 1)) < RING_SPARE - spare) {
+            store_release(where + row, NOT_THERE);
+            __threadfence_block();
+            state = FREE;
+            freed = load_acquire(window);
+        }
+        __syncwarp();
+    }
+    for (int polls = 0; polls < (1 << 24) && __any_sync(full, state == COMING); ++polls) arrived(0);
+}
 }  // namespace smo
 
-// Slot t of the working set belongs to thread t % T. S slots per thread.
+// Slot t of the working set belongs to thread t % T. S slots per thread; 32 more threads copy rows ahead.
 template <bool NU, int S, int T>
-__global__ void __launch_bounds__(T, 1)
+__global__ void __launch_bounds__(T + 32, 1)
 local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict__ diag_ws,
                  const int *__restrict__ y_ws, const double *__restrict__ f_ws, double *__restrict__ alpha_ws,
                  double *__restrict__ alpha_diff, double Cp_in, double Cn_in, double eps, int max_iter,
                  double *__restrict__ diff, const int *__restrict__ ids, double *__restrict__ alpha_global,
-                 const int *__restrict__ stop) {
+                 const int *__restrict__ stop, int use_ring) {
     using namespace smo;
     constexpr int W = T / 32, CLS = NU ? 2 : 1;             // nu: the lists of I_up and I_low are split by class
     if (stop && *stop) {            // queued past the end of a solve: no step, so the f update that follows adds zero
-        for (int t = threadIdx.x; t < ws; t += T) alpha_diff[t] = 0;
+        for (int t = threadIdx.x; t < ws; t += T + 32) alpha_diff[t] = 0;
         return;
     }
     __shared__ double f_sm[S * T], a_sm[S * T];
@@ -81,9 +171,26 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
     __shared__ unsigned long long exact_key[CLS][W];
     __shared__ int exact_slot[CLS][W];
     __shared__ double exact_low[CLS][W];
+    // row ring (use_ring): ring [RING][ws] floats in dynamic shared memory
+    extern __shared__ __align__(128) float ring[];
+    constexpr int N_CAND = 2 * (CLS + 1) * W;
+    __shared__ int where[S * T], cand[N_CAND], ring_stamp[RING], ring_stage[32], window, done;
+    __shared__ __align__(8) unsigned long long ring_bar[RING];
+    static_assert(N_CAND <= 32, "one candidate per lane of the copying warp");
     const double Cp = NU ? (double) (float) Cp_in : Cp_in;
     const double Cn = NU ? Cp : Cn_in;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid >= T) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(ring_bar + lane)) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        ring_stamp[lane] = -1;
+        if (lane < N_CAND) cand[lane] = -1;
+        if (lane == 0) { window = 0; done = 0; }
+        for (int t = lane; t < S * T; t += 32) where[t] = NOT_THERE;
+        __syncthreads();
+        if (use_ring) copy_rows_ahead(kww, ws, ring, where, cand, N_CAND, &window, &done, ring_bar, ring_stamp, ring_stage);
+        return;
+    }
 
     double f[S];
     float kd[S], pen_up[S], pen_low[S];     // +-FAR_POS: what clamps a non-member's f out of the list
@@ -103,6 +210,15 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         off[s] = t < ws ? t : 0;
     }
     __syncthreads();
+    auto read_row = [&](int r, int at, float (&k)[S]) {
+        if (at >= 0) {
+#pragma unroll
+            for (int s = 0; s < S; ++s) k[s] = ring[at * ws + off[s]];
+        } else {
+#pragma unroll
+            for (int s = 0; s < S; ++s) k[s] = __ldg(kww + r * ws + off[s]);
+        }
+    };
 
     double local_eps = 0;
     int it = 0;
@@ -110,6 +226,8 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
     int step_i = 0, step_j = 0;
     double step_ai = a_sm[0], step_aj = step_ai;
     for (;;) {
+        float first_h[CLS];                 // the lane's best, without the warp's winner
+        int first_slot[CLS];
         // ---- smallest f over I_up (with its slot), high word of the largest f over I_low ---------------------
         float low_h[S];                     // high word of f, clamped to -FAR_POS outside I_low
 #pragma unroll
@@ -143,9 +261,12 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                 warp_argmin_u64(key, sl);
                 winner = __ffs(__ballot_sync(0xffffffffu, slot[0] == sl)) - 1;
             }
-            if (lane == winner) { First e; e.f = v[0]; e.slot = slot[0]; e.low = lo_max; e1[c][warp] = e; }
+            if (lane == winner) { First e; e.f = v[0]; e.slot = slot[0]; e.low = lo_max; e1[c][warp] = e; cand[c * W + warp] = slot[0]; }
+            first_h[c] = lane == winner ? FAR_POS : h;
+            first_slot[c] = slot[0];
         }
-        __syncthreads();
+        solver_barrier<T>();
+        if (tid == 0) *(volatile int *) &window = 2 * it + 1;
         double up[CLS];
         int iu[CLS];
         float lowf[CLS];
@@ -166,10 +287,13 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
             up[c] = v[0]; iu[c] = (unsigned) slot[0] < (unsigned) ws ? slot[0] : 0; lowf[c] = lo[0];
         }
         float kI[CLS][S];
+        int at_i[CLS];
+#pragma unroll
+        for (int c = 0; c < CLS; ++c) { at_i[c] = *(volatile int *) (where + iu[c]); read_row(iu[c], at_i[c], kI[c]); }
+        // second-best lanes of the first argmin: rows to copy ahead
 #pragma unroll
         for (int c = 0; c < CLS; ++c)
-#pragma unroll
-            for (int s = 0; s < S; ++s) kI[c][s] = __ldg(kww + iu[c] * ws + off[s]);
+            if (first_h[c] == warp_min_f32(first_h[c])) cand[(CLS + 1 + c) * W + warp] = first_slot[c];
         // mirrors of the state after the last step (its readers have passed the barrier above)
 #pragma unroll
         for (int s = 0; s < S; ++s) f_sm[tid + s * T] = f[s];
@@ -199,7 +323,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                 const double wm = key_to_double(~warp_min_u64(~ordered_key(m)));
                 if (lane == 0) exact_low[c][warp] = wm;
             }
-            __syncthreads();
+            solver_barrier<T>();
             double local_diff = 0;
 #pragma unroll
             for (int c = 0; c < CLS; ++c) {
@@ -249,14 +373,18 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         {
             const float best = warp_max_f32(q[0]);
             const unsigned at_best = __ballot_sync(0xffffffffu, q[0] == best);
-            const float next = warp_max_f32(q[0] == best ? q2[0] : q[0]);
+            const float mine = q[0] == best ? q2[0] : q[0];
+            const float next = warp_max_f32(mine);
+            if (mine == next && q[0] != best) cand[(2 * CLS + 1) * W + warp] = qs[0];
             if (lane == (int) __ffs(at_best) - 1) {
                 Second e;
                 e.best = best; e.next = (at_best & (at_best - 1)) ? best : next; e.slot = qs[0]; e.pad = 0;
                 e2[warp] = e;
+                cand[CLS * W + warp] = qs[0];
             }
         }
-        __syncthreads();
+        solver_barrier<T>();
+        if (tid == 0) *(volatile int *) &window = 2 * it + 2;
         int j;
         {
             float best[W], next[W];
@@ -298,7 +426,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                     warp_argmin_u64(key[c], sl[c]);
                     if (lane == 0) { exact_key[c][warp] = key[c]; exact_slot[c][warp] = sl[c]; }
                 }
-                __syncthreads();
+                solver_barrier<T>();
 #pragma unroll
                 for (int c = 0; c < CLS; ++c) {
                     key[c] = lane < W ? exact_key[c][lane] : ~0ull;
@@ -313,15 +441,15 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         }
         // ---- step, repeated by every thread in the shadow of row j -------------------------------------------
         float kJ[S];
-#pragma unroll
-        for (int s = 0; s < S; ++s) kJ[s] = __ldg(kww + j * ws + off[s]);
+        read_row(j, *(volatile int *) (where + j), kJ);
         const int yj = y_sm[j];
         const bool second = NU && yj < 0;
         const int i = second ? iu[CLS - 1] : iu[0];
         const int yi = y_sm[i];
         const double u = second ? up[CLS - 1] : up[0];
         const double ai = a_sm[i], aj = a_sm[j], fj = f_sm[j];
-        const float kij = __ldg(kww + i * ws + j);          // row i has just been read: from L1
+        const int at = second ? at_i[CLS - 1] : at_i[0];
+        const float kij = at >= 0 ? ring[at * ws + j] : __ldg(kww + i * ws + j);      // row i has just been read: from L1
         const double room_i = yi > 0 ? Cp - ai : ai;
         const double curv = NU ? (double) (kd_sm[i] + kd_sm[j] - 2 * kij)
                                : (double) (kd_sm[i] + kd_sm[j]) - 2.0 * (double) kij;
@@ -345,7 +473,8 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         }
         ++it;
     }
-    __syncthreads();                // (the last step's alphas are in a_sm)
+    if (tid == 0) store_release(&done, 1);
+    solver_barrier<T>();            // (the last step's alphas are in a_sm)
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         const int t = tid + s * T;

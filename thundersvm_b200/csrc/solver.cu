@@ -531,15 +531,20 @@ static tsvm_status launch_local_smo(int solver_kind, int ws, const float *kww, c
     // four warps at every size, one to eight slots per thread: measured at 1,024 / 512 / 256 slots 1.00 / 0.84 / 0.73 us
     // per iteration against 1.12 / 0.99 / 0.86 with eight warps and 1.73 with sixteen (512 slots)
     constexpr int T = 128;
-#define SMO_CASE(S)                                                                                              \
-    do {                                                                                                         \
-        if (nu) TSVM_LAUNCH((local_smo_kernel<true, S, T>), 1, T, 0, st, ws, kww, diag_ws, y_ws, f_ws, alpha_ws, \
-                            alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop);                   \
-        else TSVM_LAUNCH((local_smo_kernel<false, S, T>), 1, T, 0, st, ws, kww, diag_ws, y_ws, f_ws, alpha_ws,   \
-                         alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop);                      \
+    const int use_ring = ws >= 256 && (ws & 3) == 0 && ((uintptr_t) kww & 15) == 0;
+    const size_t ring_bytes = use_ring ? (size_t) smo::RING * ws * sizeof(float) : 0;
+#define SMO_LAUNCH(NU, S)                                                                                          \
+    do {                                                                                                           \
+        TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute(local_smo_kernel<NU, S, T>,                            \
+                                                            cudaFuncAttributeMaxDynamicSharedMemorySize,           \
+                                                            (int) (smo::RING * S * T * sizeof(float)))));          \
+        TSVM_LAUNCH((local_smo_kernel<NU, S, T>), 1, T + 32, ring_bytes, st, ws, kww, diag_ws, y_ws, f_ws,         \
+                    alpha_ws, alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop, use_ring);         \
     } while (0)
+#define SMO_CASE(S) do { if (nu) SMO_LAUNCH(true, S); else SMO_LAUNCH(false, S); } while (0)
     if (ws <= T) SMO_CASE(1); else if (ws <= 2 * T) SMO_CASE(2); else if (ws <= 4 * T) SMO_CASE(4); else SMO_CASE(8);
 #undef SMO_CASE
+#undef SMO_LAUNCH
     return TSVM_OK;
 }
 
