@@ -159,6 +159,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                  const int *__restrict__ stop, int use_ring) {
     using namespace smo;
     constexpr int W = T / 32, CLS = NU ? 2 : 1;             // nu: the lists of I_up and I_low are split by class
+    constexpr bool AHEAD = !NU;                             // (nu reads two rows i and guesses j badly: 5 % slower with the ring)
     if (stop && *stop) {            // queued past the end of a solve: no step, so the f update that follows adds zero
         for (int t = threadIdx.x; t < ws; t += T + 32) alpha_diff[t] = 0;
         return;
@@ -188,7 +189,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         if (lane == 0) { window = 0; done = 0; }
         for (int t = lane; t < S * T; t += 32) where[t] = NOT_THERE;
         __syncthreads();
-        if (use_ring) copy_rows_ahead(kww, ws, ring, where, cand, N_CAND, &window, &done, ring_bar, ring_stamp, ring_stage);
+        if (AHEAD && use_ring) copy_rows_ahead(kww, ws, ring, where, cand, N_CAND, &window, &done, ring_bar, ring_stamp, ring_stage);
         return;
     }
 
@@ -245,28 +246,35 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                 slot[s] = tid + s * T;
                 lo = fmaxf(lo, mine ? low_h[s] : -FAR_POS);
             }
-            // neighbouring slots first: the left operand always holds the lower slots and wins ties
+            // The warp's reduction runs over the high words and needs only their minimum; the exact minimum and its slot
+            // are found next to it. Neighbouring slots first: the left operand always holds the lower slots and wins ties.
+            float h = high_as_float(v[0]);
+#pragma unroll
+            for (int s = 1; s < S; ++s) h = fminf(h, high_as_float(v[s]));
+            const float h_min = warp_min_f32(h), lo_max = warp_max_f32(lo);
 #pragma unroll
             for (int d = 1; d < S; d <<= 1)
 #pragma unroll
                 for (int s = 0; s + d < S; s += 2 * d)
                     if (v[s + d] < v[s]) { v[s] = v[s + d]; slot[s] = slot[s + d]; }
-            const float h = high_as_float(v[0]);
-            const float h_min = warp_min_f32(h), lo_max = warp_max_f32(lo);
-            const unsigned at_min = __ballot_sync(0xffffffffu, h == h_min);
-            int winner = at_min ? __ffs(at_min) - 1 : 0;
-            if (at_min & (at_min - 1)) {
+            bool winner = h == h_min;
+            First e;
+            e.f = v[0]; e.slot = slot[0]; e.low = lo_max;
+            if (winner) { e1[c][warp] = e; if (AHEAD) cand[c * W + warp] = slot[0]; }
+            const unsigned at_min = __ballot_sync(0xffffffffu, winner);
+            if (at_min & (at_min - 1)) {            // several lanes share the high word: the lane with the exact minimum writes again
                 unsigned long long key = ordered_key(v[0]);
                 int sl = slot[0];
                 warp_argmin_u64(key, sl);
-                winner = __ffs(__ballot_sync(0xffffffffu, slot[0] == sl)) - 1;
+                winner = slot[0] == sl;
+                __syncwarp();
+                if (winner) { e1[c][warp] = e; if (AHEAD) cand[c * W + warp] = slot[0]; }
             }
-            if (lane == winner) { First e; e.f = v[0]; e.slot = slot[0]; e.low = lo_max; e1[c][warp] = e; cand[c * W + warp] = slot[0]; }
-            first_h[c] = lane == winner ? FAR_POS : h;
+            first_h[c] = winner ? FAR_POS : h;
             first_slot[c] = slot[0];
         }
         solver_barrier<T>();
-        if (tid == 0) *(volatile int *) &window = 2 * it + 1;
+        if (AHEAD && tid == 0) *(volatile int *) &window = 2 * it + 1;
         double up[CLS];
         int iu[CLS];
         float lowf[CLS];
@@ -289,11 +297,11 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         float kI[CLS][S];
         int at_i[CLS];
 #pragma unroll
-        for (int c = 0; c < CLS; ++c) { at_i[c] = *(volatile int *) (where + iu[c]); read_row(iu[c], at_i[c], kI[c]); }
+        for (int c = 0; c < CLS; ++c) { at_i[c] = AHEAD ? *(volatile int *) (where + iu[c]) : (int) NOT_THERE; read_row(iu[c], at_i[c], kI[c]); }
         // second-best lanes of the first argmin: rows to copy ahead
 #pragma unroll
         for (int c = 0; c < CLS; ++c)
-            if (first_h[c] == warp_min_f32(first_h[c])) cand[(CLS + 1 + c) * W + warp] = first_slot[c];
+            if (AHEAD && first_h[c] == warp_min_f32(first_h[c])) cand[(CLS + 1 + c) * W + warp] = first_slot[c];
         // mirrors of the state after the last step (its readers have passed the barrier above)
 #pragma unroll
         for (int s = 0; s < S; ++s) f_sm[tid + s * T] = f[s];
@@ -375,16 +383,16 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
             const unsigned at_best = __ballot_sync(0xffffffffu, q[0] == best);
             const float mine = q[0] == best ? q2[0] : q[0];
             const float next = warp_max_f32(mine);
-            if (mine == next && q[0] != best) cand[(2 * CLS + 1) * W + warp] = qs[0];
+            if (AHEAD && mine == next && q[0] != best) cand[(2 * CLS + 1) * W + warp] = qs[0];
             if (lane == (int) __ffs(at_best) - 1) {
                 Second e;
                 e.best = best; e.next = (at_best & (at_best - 1)) ? best : next; e.slot = qs[0]; e.pad = 0;
                 e2[warp] = e;
-                cand[CLS * W + warp] = qs[0];
+                if (AHEAD) cand[CLS * W + warp] = qs[0];
             }
         }
         solver_barrier<T>();
-        if (tid == 0) *(volatile int *) &window = 2 * it + 2;
+        if (AHEAD && tid == 0) *(volatile int *) &window = 2 * it + 2;
         int j;
         {
             float best[W], next[W];
@@ -441,7 +449,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         }
         // ---- step, repeated by every thread in the shadow of row j -------------------------------------------
         float kJ[S];
-        read_row(j, *(volatile int *) (where + j), kJ);
+        read_row(j, AHEAD ? *(volatile int *) (where + j) : (int) NOT_THERE, kJ);
         const int yj = y_sm[j];
         const bool second = NU && yj < 0;
         const int i = second ? iu[CLS - 1] : iu[0];

@@ -531,7 +531,7 @@ static tsvm_status launch_local_smo(int solver_kind, int ws, const float *kww, c
     // four warps at every size, one to eight slots per thread: measured at 1,024 / 512 / 256 slots 1.00 / 0.84 / 0.73 us
     // per iteration against 1.12 / 0.99 / 0.86 with eight warps and 1.73 with sixteen (512 slots)
     constexpr int T = 128;
-    const int use_ring = ws >= 256 && (ws & 3) == 0 && ((uintptr_t) kww & 15) == 0;
+    const int use_ring = !nu && ws >= 256 && (ws & 3) == 0 && ((uintptr_t) kww & 15) == 0;
     const size_t ring_bytes = use_ring ? (size_t) smo::RING * ws * sizeof(float) : 0;
 #define SMO_LAUNCH(NU, S)                                                                                          \
     do {                                                                                                           \
