@@ -70,9 +70,13 @@ constexpr int MAX_DEVICES = 64;
 // driver's allocation calls cost more than such a sub-problem's whole solve.
 tsvm_status pool_alloc(void **p, size_t bytes);
 void pool_free(void *p);                      // waits for the block's device, like cudaFree
-// Several blocks at once: one wait per device that owns any of them, then all are filed.
-void pool_free_many(std::initializer_list<void *> blocks);
+// Several blocks at once: one wait per device that owns any of them, then all are filed. idle: the caller knows that
+// nothing in flight uses them (it has waited for the only stream that did), and nothing is waited for.
+void pool_free_many(std::initializer_list<void *> blocks, bool idle = false);
+int device_sm_count();                        // SMs of the current device (asked once per device)
+size_t device_memory_bytes();                 // total memory of the current device (asked once per device)
 void pool_release();                          // returns every cached block to the driver
+void release_solver_streams();                // solver.cu: destroys the cached streams and events
 tsvm_status pinned_alloc(void **p, size_t bytes);
 void pinned_free(void *p);
 
@@ -221,6 +225,17 @@ struct tsvm_km {
     const int *rows_m_dev = nullptr, *rows_slot_dev = nullptr;
     int *status_dev = nullptr;      // device status word written by kernels with bounded waits
     int *status_host = nullptr;     // pinned mirror
+    // Work that may still be in flight on the handle's buffers: on one stream, or (streams_mixed) who knows where. The
+    // calls that end by waiting for their stream clear it, so that destroying the handle has nothing to wait for.
+    bool in_flight = false, streams_mixed = false;
+    cudaStream_t flight_stream = nullptr;
+    bool exposed = false;           // a caller has a device pointer of the handle's own
+    void launched(cudaStream_t st) {
+        if (in_flight && flight_stream != st) streams_mixed = true;
+        in_flight = true;
+        flight_stream = st;
+    }
+    void waited(cudaStream_t st) { if (in_flight && !streams_mixed && flight_stream == st) in_flight = false; }
 };
 
 namespace tsvm {

@@ -14,6 +14,7 @@
 namespace thundersvm {
 void *device_alloc(size_t bytes);                 // throws std::bad_alloc when the device is out of memory
 void device_free(void *p);
+bool device_has_room(double bytes);               // less than 60 % of the free device memory
 void copy_to_device(void *dst, const void *src, size_t bytes);
 void copy_to_host(void *dst, const void *src, size_t bytes);
 void copy_on_device(void *dst, const void *src, size_t bytes);

@@ -4,7 +4,7 @@
 #include <thundersvm/solver/csmosolver.h>
 #include <thundersvm/solver/nusmosolver.h>
 #include <cuda_runtime.h>
-#include "../../../include/thundersvm_b200.h"
+#include "../common.cuh"
 
 namespace {
 void b200_check(tsvm_status s) {
@@ -49,10 +49,8 @@ KernelMatrix::KernelMatrix(const DataSet::node2d &instances, SvmParam param) : p
     // is very sparse (then the CSR engine touches far fewer bytes) or the three dense planes would
     // not fit next to the kernel-row buffer.
     const double density = (double) nnz_ / ((double) n_instances_ * n_features_);
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
     const double dense_bytes = 3.0 * n_instances_ * ((n_features_ + 3) & ~3ul) * 4.0 + 1024.0 * n_instances_ * 4.0;
-    dense_ = (density >= 0.02 || n_features_ <= 256) && dense_bytes < 0.6 * (double) free_b;
+    dense_ = (density >= 0.02 || n_features_ <= 256) && thundersvm::device_has_room(dense_bytes);
     if (dense_) {
         vector<float> X(n_instances_ * n_features_, 0.0f);
 #pragma omp parallel for schedule(static)
@@ -69,7 +67,7 @@ KernelMatrix::KernelMatrix(const DataSet::node2d &instances, SvmParam param) : p
     cudaStreamSynchronize(thundersvm::work_stream());    // the host staging buffers above go out of scope
     thundersvm::total_memory_size() += (dense_ ? (size_t) dense_bytes : nnz_ * 8 + n_instances_ * 12);
     diag_.resize(n_instances_);
-    thundersvm::copy_to_host(diag_.host_data(), tsvm_km_diag_dev(km_), sizeof(kernel_type) * n_instances_);
+    thundersvm::copy_to_host(diag_.host_data(), km_->diag, sizeof(kernel_type) * n_instances_);
 }
 
 KernelMatrix::KernelMatrix(const float *X_dev, size_t d, size_t ld, size_t r0, size_t n0, size_t r1, size_t n1,
@@ -87,7 +85,7 @@ KernelMatrix::KernelMatrix(const float *X_dev, size_t d, size_t ld, size_t r0, s
     const double dense_bytes = 3.0 * n_instances_ * ((n_features_ + 3) & ~3ul) * 4.0 + 1024.0 * n_instances_ * 4.0;
     thundersvm::total_memory_size() += (size_t) dense_bytes;
     diag_.resize(n_instances_);
-    thundersvm::copy_to_host(diag_.host_data(), tsvm_km_diag_dev(km_), sizeof(kernel_type) * n_instances_);
+    thundersvm::copy_to_host(diag_.host_data(), km_->diag, sizeof(kernel_type) * n_instances_);
 }
 
 KernelMatrix::~KernelMatrix() {

@@ -389,10 +389,8 @@ void SVC::build_device_rows(const DataSet &ds) {
     }
     const size_t d = (size_t) mx + 1, ld = (d + 3) & ~(size_t) 3;
     const double density = (double) nnz / ((double) n * d);
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
     const double bytes = 4.0 * n * ld * 4.0 + 1024.0 * n * 4.0;      // this copy + a pair's matrix and planes + rows
-    if (!((density >= 0.02 || d <= 256) && bytes < 0.6 * (double) free_b)) return;
+    if (!((density >= 0.02 || d <= 256) && thundersvm::device_has_room(bytes))) return;
     vector<float> X(n * ld, 0.0f);
     const vector<int> perm = ds.original_index();
     const DataSet::node2d &ins = ds.instances();

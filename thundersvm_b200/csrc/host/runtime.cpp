@@ -25,7 +25,6 @@ void *device_alloc(size_t bytes) {
     if (s != TSVM_OK) LOG(FATAL) << "device allocation: " << tsvm_last_error();
     return p;
 }
-void device_free(void *p) { tsvm::pool_free(p); }
 static thread_local cudaStream_t tl_stream = nullptr;
 cudaStream_t work_stream() { return tl_stream; }
 void set_work_stream(cudaStream_t s) { tl_stream = s; }
@@ -41,6 +40,19 @@ void copy_to_host(void *dst, const void *src, size_t bytes) {
 }
 void copy_on_device(void *dst, const void *src, size_t bytes) {
     cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, tl_stream), "D2D copy");
+}
+// The owner of such memory works on its thread's stream only, so that is all there is to wait for.
+void device_free(void *p) {
+    if (!p) return;
+    cudaStreamSynchronize(tl_stream);
+    tsvm::pool_free_many({p}, true);
+}
+// The driver is asked for the free memory only where it matters (a driver lock, at times tens of milliseconds): what fits
+// a hundredth of the device is allocated in any case, and a device that full fails the allocation.
+bool device_has_room(double bytes) {
+    if (bytes < 0.01 * (double) tsvm::device_memory_bytes()) return true;
+    size_t free_b = 0, total_b = 0;
+    return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes < 0.6 * (double) free_b;
 }
 void device_zero(void *p, size_t bytes) { cuda_ok(cudaMemsetAsync(p, 0, bytes, tl_stream), "cudaMemset"); }
 std::atomic<size_t> &total_memory_size() {

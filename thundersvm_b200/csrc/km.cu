@@ -96,14 +96,38 @@ static size_t pool_cache_cap() {
     // should come back from the pool when the next solver of the same problem is created)
     static const size_t cap = [] {
         if (const char *e = getenv("TSVM_POOL_CACHE_MB")) return (size_t) strtoull(e, nullptr, 10) << 20;
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return (size_t) 32 << 30; }
-        return (size_t) ((double) total_b * 0.6);
+        return (size_t) ((double) device_memory_bytes() * 0.6);
     }();
     return cap;
 }
 
-void pool_free_many(std::initializer_list<void *> blocks) {
+// cudaMemGetInfo takes a driver lock that other processes of the machine hold too: usually 100 us, at times 40 ms. What
+// the library wants to know is the size of the device, which does not change.
+int device_sm_count() {
+    static std::atomic<int> count[MAX_DEVICES];
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return sms; }
+    std::atomic<int> &known = count[dev & (MAX_DEVICES - 1)];
+    if (const int k = known.load(std::memory_order_relaxed)) return k;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) cudaGetLastError();
+    known.store(sms, std::memory_order_relaxed);
+    return sms;
+}
+
+size_t device_memory_bytes() {
+    static std::atomic<size_t> bytes[MAX_DEVICES];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return (size_t) 32 << 30; }
+    std::atomic<size_t> &known = bytes[dev & (MAX_DEVICES - 1)];
+    size_t total = known.load(std::memory_order_relaxed);
+    if (total) return total;
+    size_t free_b = 0;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) { cudaGetLastError(); return (size_t) 32 << 30; }
+    known.store(total, std::memory_order_relaxed);
+    return total;
+}
+
+void pool_free_many(std::initializer_list<void *> blocks, bool idle) {
     int cur = 0;
     bool have_cur = false;
     unsigned long long synced = 0;
@@ -114,7 +138,7 @@ void pool_free_many(std::initializer_list<void *> blocks) {
             if (!p) continue;
             auto it = g_pool_live.find(p);
             if (it == g_pool_live.end()) { foreign.push_back(p); continue; }
-            synced |= 1ull << (it->second.dev & (MAX_DEVICES - 1));
+            if (!idle) synced |= 1ull << (it->second.dev & (MAX_DEVICES - 1));
         }
     }
     for (int dev = 0; dev < MAX_DEVICES; ++dev) {
@@ -183,39 +207,26 @@ tsvm_status launch_dense_tc(tsvm_km *km, int m, float *out, long long ld_out, cu
 
 // ---- construction kernels ---------------------------------------------------------------
 
-// self_dot[i] = float(sum_k double(x_ik)^2), one warp per row (kernelmatrix.cpp:194-204).
-__global__ void self_dot_dense_kernel(const float *__restrict__ X, int n, int d, int ld, float *__restrict__ out) {
-    int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const float *x = X + (size_t) row * ld;
-    double s = 0;
-    for (int k = lane; k < d; k += 32) { double v = x[k]; s += v * v; }
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[row] = (float) s;
+// diag (kernelmatrix.cpp:225-247)
+__device__ __forceinline__ float diag_value(const KernelFn &fn, float v) {
+    switch (fn.type) {
+        case TSVM_RBF: case TSVM_PRECOMPUTED: return 1.0f;
+        case TSVM_POLY: return powf(fn.gamma * v + fn.coef0, (float) fn.degree);
+        case TSVM_SIGMOID: return tanhf(fn.gamma * v + fn.coef0);
+        default: return v;
+    }
 }
 
-__global__ void self_dot_csr_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, int n,
-                                    float *__restrict__ out) {
+// Self dots float(sum_k double(x_ik)^2) and diagonal of CSR instances, one warp per row (kernelmatrix.cpp:194-247).
+__global__ void self_dot_csr_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, int n, KernelFn fn,
+                                    float *__restrict__ sd, float *__restrict__ diag, int *__restrict__ status) {
     int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
     if (row >= n) return;
     double s = 0;
     for (int p = row_ptr[row] + lane; p < row_ptr[row + 1]; p += 32) { double v = val[p]; s += v * v; }
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[row] = (float) s;
-}
-
-// diag (kernelmatrix.cpp:225-247)
-__global__ void diag_kernel(const float *__restrict__ sd, int n, KernelFn fn, float *__restrict__ out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float v = sd[i];
-    switch (fn.type) {
-        case TSVM_RBF: case TSVM_PRECOMPUTED: v = 1.0f; break;
-        case TSVM_POLY: v = powf(fn.gamma * v + fn.coef0, (float) fn.degree); break;
-        case TSVM_SIGMOID: v = tanhf(fn.gamma * v + fn.coef0); break;
-        default: break;
-    }
-    out[i] = v;
+    if (lane == 0) { sd[row] = (float) s; diag[row] = diag_value(fn, (float) s); }
 }
 
 // Self dot of a batch of new instances, accumulated sequentially in float in storage order
@@ -301,20 +312,35 @@ struct RowDst {
     int kind, ld;                  // plane kind (0 = FP32 W) and row length in elements
 };
 
-// Planes of all instances: one warp per row; columns d..pld-1 are zero.
-__global__ void split_rows_kernel(const float *__restrict__ X, int n, int d, int ld, int kind, int pld,
-                                  float *__restrict__ hi, float *__restrict__ lo, float *__restrict__ x_unscale) {
+// Self dots, diagonal and operand planes of all instances: one warp per row, one pass over X (the second look at a row
+// comes from L1). kind 0: no planes. sd == nullptr: planes only. Columns d..pld-1 of the planes are zero.
+__global__ void prepare_rows_kernel(const float *__restrict__ X, int n, int d, int ld, int kind, int pld,
+                                    float *__restrict__ hi, float *__restrict__ lo, float *__restrict__ x_unscale, KernelFn fn,
+                                    float *__restrict__ sd, float *__restrict__ diag, int *__restrict__ status) {
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    if (sd && blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
     for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < n; row += gridDim.x * wpb) {
         const float *x = X + (size_t) row * ld;
+        float amax = 0.0f;
+        double s = 0;
+#pragma unroll 4
+        for (int k = lane; k < d; k += 32) {
+            const float v = x[k];
+            amax = fmaxf(amax, fabsf(v));
+            s += (double) v * v;
+        }
+        if (sd) {
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) { sd[row] = (float) s; diag[row] = diag_value(fn, (float) s); }
+        }
+        if (kind == 0) continue;
         float scale = 1.0f, unscale = 1.0f;
         if (kind == 2) {
-            float amax = 0.0f;
-            for (int k = lane; k < d; k += 32) amax = fmaxf(amax, fabsf(x[k]));
             amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
             row_scale_from_max(amax, scale, unscale);
             if (lane == 0) x_unscale[row] = unscale;
         }
+#pragma unroll 4
         for (int k = lane; k < pld; k += 32)
             store_planes(kind, hi, lo, (size_t) row * pld + k, k < d ? x[k] : 0.0f, scale);
     }
@@ -755,10 +781,10 @@ static inline int wanted_plane_kind(const tsvm_km *km) {
     return (km->engine == 2 || km->engine == 3) ? 1 : 2;
 }
 
-// Builds the planes the selected engine reads, once; a change of engine rebuilds them.
-static tsvm_status ensure_planes(tsvm_km *km, cudaStream_t st) {
-    const int kind = wanted_plane_kind(km);
-    if (kind == 0 || kind == km->plane_kind) return TSVM_OK;
+static inline int prepare_grid(int n) { const int b = ceil_div(n, 8); return b < 148 * 8 ? b : 148 * 8; }
+
+// Buffers of the planes the selected engine reads.
+static tsvm_status alloc_planes(tsvm_km *km, int kind) {
     pool_free_many({km->Xhi, km->Xlo});
     km->Xhi = km->Xlo = nullptr;
     km->plane_kind = 0;
@@ -767,8 +793,16 @@ static tsvm_status ensure_planes(tsvm_km *km, cudaStream_t st) {
     TSVM_TRY(dev_alloc(&km->Xhi, words));
     TSVM_TRY(dev_alloc(&km->Xlo, words));
     if (!km->x_unscale) TSVM_TRY(dev_alloc(&km->x_unscale, (size_t) km->n));
-    TSVM_LAUNCH(split_rows_kernel, 148 * 8, 256, 0, st, km->X, km->n, km->d, km->ldx, kind, km->plane_ld, km->Xhi,
-                km->Xlo, km->x_unscale);
+    return TSVM_OK;
+}
+
+// Builds the planes, once; a change of engine rebuilds them.
+static tsvm_status ensure_planes(tsvm_km *km, cudaStream_t st) {
+    const int kind = wanted_plane_kind(km);
+    if (kind == 0 || kind == km->plane_kind) return TSVM_OK;
+    TSVM_TRY(alloc_planes(km, kind));
+    TSVM_LAUNCH(prepare_rows_kernel, prepare_grid(km->n), 256, 0, st, km->X, km->n, km->d, km->ldx, kind, km->plane_ld,
+                km->Xhi, km->Xlo, km->x_unscale, km->fn, (float *) nullptr, (float *) nullptr, (int *) nullptr);
     km->plane_kind = kind;
     return TSVM_OK;
 }
@@ -785,15 +819,19 @@ static tsvm_status finish_create(tsvm_km *km, cudaStream_t st) {
     TSVM_TRY(dev_alloc(&km->self_dot, (size_t) km->n));
     TSVM_TRY(dev_alloc(&km->diag, (size_t) km->n));
     TSVM_TRY(dev_alloc(&km->status_dev, 4));
-    TSVM_CUDA(cudaMemsetAsync(km->status_dev, 0, 4 * sizeof(int), st));
     TSVM_TRY(pinned_alloc((void **) &km->status_host, 4 * sizeof(int)));
-    const int blocks = ceil_div((long long) km->n * 32, 256);
-    if (km->dense)
-        TSVM_LAUNCH(self_dot_dense_kernel, blocks, 256, 0, st, km->X, km->n, km->d, km->ldx, km->self_dot);
-    else
-        TSVM_LAUNCH(self_dot_csr_kernel, blocks, 256, 0, st, km->val, km->row_ptr, km->n, km->self_dot);
-    TSVM_LAUNCH(diag_kernel, ceil_div(km->n, 256), 256, 0, st, km->self_dot, km->n, km->fn, km->diag);
-    return ensure_planes(km, st);
+    km->launched(st);
+    if (!km->dense) {
+        TSVM_LAUNCH(self_dot_csr_kernel, ceil_div((long long) km->n * 32, 256), 256, 0, st, km->val, km->row_ptr, km->n,
+                    km->fn, km->self_dot, km->diag, km->status_dev);
+        return TSVM_OK;
+    }
+    const int kind = wanted_plane_kind(km);
+    if (kind) TSVM_TRY(alloc_planes(km, kind));
+    TSVM_LAUNCH(prepare_rows_kernel, prepare_grid(km->n), 256, 0, st, km->X, km->n, km->d, km->ldx, kind, km->plane_ld,
+                km->Xhi, km->Xlo, km->x_unscale, km->fn, km->self_dot, km->diag, km->status_dev);
+    km->plane_kind = kind;
+    return TSVM_OK;
 }
 
 // TSVM_CSR_SMEM=0 keeps the L2-panel engine for every CSR matrix (used to compare the two engines)
@@ -821,12 +859,7 @@ static tsvm_status csr_engine_launch(tsvm_km *km, const CsrView &X, const float 
         TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute(csr_rows_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                             (int) (((size_t) CSR_SMEM_MAX_D * CSR_SMEM_PART + 2 * CSR_SMEM_TILE) * sizeof(float)))));
         const int parts = ceil_div(m, CSR_SMEM_PART);
-        int sms = 148;
-        {
-            int dev = 0;
-            TSVM_CUDA(cudaGetDevice(&dev));
-            TSVM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        }
+        int sms = device_sm_count();
         sms = sms - spare_sms > 0 ? sms - spare_sms : 1;
         int bx = sms / parts > 0 ? sms / parts : 1;
         const int n_tiles = ceil_div(X.n, 32);
@@ -958,7 +991,10 @@ extern "C" {
 
 const char *tsvm_last_error(void) { return tsvm::g_err; }
 int tsvm_abi_version(void) { return 2; }
-void tsvm_release_cached_memory(void) { tsvm::pool_release(); }
+void tsvm_release_cached_memory(void) {
+    tsvm::release_solver_streams();
+    tsvm::pool_release();
+}
 
 tsvm_status tsvm_km_create_dense(const float *X, int n, int d, int ld, int loc, int kernel_type, int degree,
                                  float gamma, float coef0, void *stream, tsvm_km **out) {
@@ -1005,12 +1041,12 @@ tsvm_status tsvm_km_create_csr(const float *val, const int *row_ptr, const int *
     km->n = n; km->d = d; km->dense = false;
     km->fn = KernelFn{kernel_type, degree, gamma, coef0};
     tsvm_status s = TSVM_OK;
-    int last = 0;
-    if (loc == TSVM_HOST) last = row_ptr[n];
-    else if (cudaMemcpy(&last, row_ptr + n, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) s = TSVM_ERR_CUDA;
-    km->nnz = last;
-    if (s == TSVM_OK && loc == TSVM_DEVICE) { km->val = val; km->row_ptr = row_ptr; km->col = col; }
-    else if (s == TSVM_OK) {
+    if (loc == TSVM_DEVICE) {
+        km->nnz = -1;                     // read from row_ptr when someone asks (tsvm_km_nnz)
+        km->val = val; km->row_ptr = row_ptr; km->col = col;
+    } else {
+        const int last = row_ptr[n];
+        km->nnz = last;
         s = dev_alloc(&km->val_owned, (size_t) last);
         if (s == TSVM_OK) s = dev_alloc(&km->col_owned, (size_t) last);
         if (s == TSVM_OK) s = dev_alloc(&km->row_ptr_owned, (size_t) n + 1);
@@ -1033,17 +1069,34 @@ void tsvm_km_destroy(tsvm_km *km) {
     if (!km) return;
     pool_free_many({km->X_owned, km->Xhi, km->Xlo, km->x_unscale, km->w_unscale, km->val_owned, km->row_ptr_owned,
                     km->col_owned, km->self_dot, km->diag, km->W, km->Whi, km->Wlo, km->WT, km->sd_rows,
-                    km->status_dev});
+                    km->status_dev}, !km->in_flight && !km->exposed);
     if (km->status_host) pinned_free(km->status_host);
     delete km;
 }
 
 int tsvm_km_n_instances(const tsvm_km *km) { return km ? km->n : 0; }
 int tsvm_km_n_features(const tsvm_km *km) { return km ? km->d : 0; }
-long long tsvm_km_nnz(const tsvm_km *km) { return km ? km->nnz : 0; }
+long long tsvm_km_nnz(const tsvm_km *km) {
+    if (!km) return 0;
+    if (km->nnz >= 0) return km->nnz;
+    int last = 0;
+    if (cudaMemcpy(&last, km->row_ptr + km->n, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return last;
+}
 int tsvm_km_is_dense(const tsvm_km *km) { return km && km->dense; }
-const float *tsvm_km_diag_dev(const tsvm_km *km) { return km ? km->diag : nullptr; }
-const float *tsvm_km_self_dot_dev(const tsvm_km *km) { return km ? km->self_dot : nullptr; }
+const float *tsvm_km_diag_dev(const tsvm_km *km) {
+    if (!km) return nullptr;
+    const_cast<tsvm_km *>(km)->exposed = true;      // the caller's own work may read it until the handle is destroyed
+    return km->diag;
+}
+const float *tsvm_km_self_dot_dev(const tsvm_km *km) {
+    if (!km) return nullptr;
+    const_cast<tsvm_km *>(km)->exposed = true;
+    return km->self_dot;
+}
 
 tsvm_status tsvm_km_set_dense_engine(tsvm_km *km, int engine) {
     TSVM_REQUIRE(km && engine >= 0 && engine <= 4, "set_dense_engine: bad arguments");
@@ -1055,6 +1108,7 @@ tsvm_status tsvm_km_rows_by_index(tsvm_km *km, const int *idx_dev, int q, float 
                                   void *stream) {
     TSVM_REQUIRE(km && idx_dev && out_dev && q > 0 && ld_out >= km->n, "rows_by_index: bad arguments (q=%d)", q);
     cudaStream_t st = (cudaStream_t) stream;
+    km->launched(st);
     TSVM_TRY(ensure_scratch(km, q));
     if (km->dense) {
         TSVM_TRY(ensure_planes(km, st));
@@ -1076,6 +1130,7 @@ tsvm_status tsvm_km_rows_by_instances_dense(tsvm_km *km, const float *T_dev, int
     TSVM_REQUIRE(km && T_dev && out_dev && m > 0 && dt > 0 && ldt >= dt && ld_out >= km->n,
                  "rows_by_instances_dense: bad arguments");
     cudaStream_t st = (cudaStream_t) stream;
+    km->launched(st);
     const int chunk = km->dense ? 4096 : 1024;
     for (int r0 = 0; r0 < m; r0 += chunk) {
         const int mm = min(chunk, m - r0);
@@ -1103,6 +1158,7 @@ tsvm_status tsvm_km_rows_for_features_dense(tsvm_km *km, const float *T_dev, int
     TSVM_REQUIRE(km && km->dense && T_dev && sd_T_dev && out_dev && m > 0 && ldt >= km->d && ld_out >= km->n,
                  "rows_for_features_dense: bad arguments (dense kernel matrix required)");
     cudaStream_t st = (cudaStream_t) stream;
+    km->launched(st);
     for (int r0 = 0; r0 < m; r0 += 4096) {
         const int mm = min(4096, m - r0);
         TSVM_TRY(ensure_scratch(km, mm));
@@ -1121,6 +1177,7 @@ tsvm_status tsvm_km_rows_by_instances_csr(tsvm_km *km, const float *tval_dev, co
     (void) tnnz;
     TSVM_REQUIRE(km && trow_ptr_dev && out_dev && m > 0 && ld_out >= km->n, "rows_by_instances_csr: bad arguments");
     cudaStream_t st = (cudaStream_t) stream;
+    km->launched(st);
     const int chunk = km->dense ? 4096 : 1024;
     for (int r0 = 0; r0 < m; r0 += chunk) {
         const int mm = min(chunk, m - r0);

@@ -10,6 +10,7 @@
 #include <string.h>
 #include <stdlib.h>
 #include <dlfcn.h>
+#include <mutex>
 #include <vector>
 
 namespace tsvm {
@@ -282,6 +283,13 @@ __global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ di
     if (cache_ctr)
         for (int k = 0; k < CACHE_CTRS; ++k) c->ctr[k] = cache_ctr[k];
     c->stop = stop;
+}
+
+// *any becomes non-zero if one of a[0..n) is
+__global__ void any_nonzero_kernel(const double *__restrict__ a, int n, int *__restrict__ any) {
+    bool mine = false;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) mine = mine || a[i] != 0.0;
+    if (__syncthreads_or(mine) && threadIdx.x == 0) *any = 1;
 }
 
 __global__ void fill_int_kernel(int *p, long long n, int v) {
@@ -560,9 +568,7 @@ static long long g_row_cache_bytes = -1;
 static size_t row_cache_budget() {
     if (g_row_cache_bytes >= 0) return (size_t) g_row_cache_bytes;
     if (const char *e = getenv("TSVM_ROW_CACHE_MB")) return (size_t) strtoull(e, nullptr, 10) << 20;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return (size_t) 8 << 30; }
-    return (size_t) ((double) total_b * 0.45);
+    return (size_t) ((double) device_memory_bytes() * 0.45);
 }
 
 struct tsvm_ws {
@@ -615,11 +621,12 @@ tsvm_status tsvm_ws_create(int n_max, int ws_max, tsvm_ws **out) {
     return TSVM_OK;
 }
 
-void tsvm_ws_destroy(tsvm_ws *w) {
+static void ws_destroy(tsvm_ws *w, bool idle) {
     if (!w) return;
-    pool_free_many({w->state, w->hist, w->count, w->cand_h, w->cand_l, w->sorted_f, w->sorted_id});
+    pool_free_many({w->state, w->hist, w->count, w->cand_h, w->cand_l, w->sorted_f, w->sorted_id}, idle);
     delete w;
 }
+void tsvm_ws_destroy(tsvm_ws *w) { ws_destroy(w, false); }
 
 // The selection in one cooperative launch (select_kernel). out_ids: the merged selection; else the sorted lists
 // ([lists][want], padding id -1) in sorted_f / sorted_id are the result.
@@ -838,11 +845,95 @@ static int sync_every() {
     return k;
 }
 
-struct tsvm_solver {
+// The second stream of a solver and its events. Creating them costs more than the rest of a small solve's set-up (a stream
+// 0.2 - 2 ms), so a finished solver leaves them to the next one of the same device: 16 sets at most are kept, and
+// tsvm_release_cached_memory destroys them. A set belongs to one solver at a time and is idle when it comes back.
+struct SolverStreams {
     // Events of one queued iteration: phase boundaries on the first stream, start and end of the local solver
     struct IterEvents {
         cudaEvent_t ph[5] = {nullptr, nullptr, nullptr, nullptr, nullptr}, l0 = nullptr, l1 = nullptr;
     };
+    int dev = 0;
+    cudaStream_t st2 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_fork2 = nullptr, ev_join = nullptr;
+    IterEvents evs[MAX_QUEUED];
+
+    ~SolverStreams() {
+        for (auto &E : evs) {
+            for (auto e : E.ph) if (e) cudaEventDestroy(e);
+            for (auto e : {E.l0, E.l1}) if (e) cudaEventDestroy(e);
+        }
+        for (auto e : {ev_fork, ev_fork2, ev_join}) if (e) cudaEventDestroy(e);
+        if (st2) cudaStreamDestroy(st2);
+    }
+    tsvm_status create() {
+        TSVM_CUDA(cudaGetDevice(&dev));
+        TSVM_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+        TSVM_CUDA(cudaEventCreateWithFlags(&ev_fork2, cudaEventDisableTiming));
+        TSVM_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+        int lo_prio = 0, hi_prio = 0;
+        TSVM_CUDA(cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio));
+        TSVM_CUDA(cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, hi_prio));
+        return TSVM_OK;
+    }
+    tsvm_status ensure_events(int j) {
+        IterEvents &E = evs[j];
+        if (E.l1) return TSVM_OK;
+        for (auto &e : E.ph) if (!e) TSVM_CUDA(cudaEventCreate(&e));
+        if (!E.l0) TSVM_CUDA(cudaEventCreate(&E.l0));
+        TSVM_CUDA(cudaEventCreate(&E.l1));
+        return TSVM_OK;
+    }
+};
+namespace {
+constexpr size_t MAX_STREAM_SETS = 16;
+std::mutex &g_streams_mu = *new std::mutex;
+auto &g_streams_free = *new std::vector<SolverStreams *>;
+
+tsvm_status take_streams(SolverStreams **out) {
+    int dev = 0;
+    TSVM_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lk(g_streams_mu);
+        for (size_t k = g_streams_free.size(); k-- > 0;)
+            if (g_streams_free[k]->dev == dev) {
+                *out = g_streams_free[k];
+                g_streams_free.erase(g_streams_free.begin() + k);
+                return TSVM_OK;
+            }
+    }
+    SolverStreams *s = new SolverStreams;
+    const tsvm_status r = s->create();
+    if (r != TSVM_OK) { delete s; return r; }
+    *out = s;
+    return TSVM_OK;
+}
+// idle: nothing is pending on the set's stream
+void give_streams(SolverStreams *s, bool idle) {
+    if (!s) return;
+    if (idle) {
+        std::lock_guard<std::mutex> lk(g_streams_mu);
+        if (g_streams_free.size() < MAX_STREAM_SETS) { g_streams_free.push_back(s); return; }
+    }
+    delete s;
+}
+}  // namespace
+namespace tsvm {
+void release_solver_streams() {
+    std::lock_guard<std::mutex> lk(g_streams_mu);
+    int cur = 0;
+    const bool have = cudaGetDevice(&cur) == cudaSuccess;
+    for (auto *s : g_streams_free) {
+        cudaSetDevice(s->dev);
+        delete s;
+    }
+    g_streams_free.clear();
+    if (have) cudaSetDevice(cur);
+}
+}  // namespace tsvm
+
+struct tsvm_solver {
+    typedef SolverStreams::IterEvents IterEvents;
 
     tsvm_km *km = nullptr;
     int kind = 0, ws = 0, q = 0, n = 0;
@@ -860,12 +951,13 @@ struct tsvm_solver {
     double *diff_host = nullptr;
     // end-of-iteration state on the device, its pinned copy, and the events of the queued iterations
     SolverCtl *ctl = nullptr, *ctl_host = nullptr;
-    IterEvents evs[MAX_QUEUED];
+    SolverStreams *streams = nullptr;
+    bool idle = true;               // nothing of this solver is in flight (the last call ended with a wait)
     int max_iter = -1;              // iteration cap applied on the device; -1: none
     bool stopped = false;           // the device stopped the queue (done, capped or an error)
     // overlapped iteration: second stream, fork / join events, operand planes of the working set
     bool overlap = true;
-    cudaStream_t st2 = nullptr;
+    cudaStream_t st2 = nullptr;     // of `streams`, like the events
     cudaEvent_t ev_fork = nullptr, ev_fork2 = nullptr, ev_join = nullptr;
     float *ws_hi = nullptr, *ws_lo = nullptr, *ws_sd = nullptr, *ws_unscale = nullptr;
     // kernel-row cache (cache_assign_kernel): the row buffer holds cache_cap rows; directory and per-iteration lists
@@ -886,16 +978,11 @@ struct tsvm_solver {
     ~tsvm_solver() {
         pool_free_many({ids, y_ws, rows, kww, diag_ws, f_ws, a_ws, alpha_diff, diff, red, in_ws, ws_hi, ws_lo, ws_sd,
                         ws_unscale, slot_of, inst_of, stamp, row_slots, miss_ids, miss_slot, victims, cache_ctr, miss_hi,
-                        miss_lo, miss_sd, miss_unscale, ctl});
-        tsvm_ws_destroy(sel);
+                        miss_lo, miss_sd, miss_unscale, ctl}, idle);
+        ws_destroy(sel, idle);
         if (diff_host) pinned_free(diff_host);
         if (ctl_host) pinned_free(ctl_host);
-        for (auto &E : evs) {
-            for (auto e : E.ph) if (e) cudaEventDestroy(e);
-            for (auto e : {E.l0, E.l1}) if (e) cudaEventDestroy(e);
-        }
-        for (auto e : {ev_fork, ev_fork2, ev_join}) if (e) cudaEventDestroy(e);
-        if (st2) cudaStreamDestroy(st2);
+        give_streams(streams, idle);
     }
 
     tsvm_status ensure_ws_planes() {
@@ -949,6 +1036,7 @@ struct tsvm_solver {
     }
 
     tsvm_status init() {
+        idle = false;
         TSVM_TRY(dev_alloc(&ids, (size_t) ws));
         TSVM_TRY(dev_alloc(&y_ws, (size_t) ws));
         TSVM_TRY(alloc_rows());
@@ -969,14 +1057,8 @@ struct tsvm_solver {
         memset(ctl_host, 0, sizeof(SolverCtl));
         ctl_host->prev = ctl_host->last = ctl_host->second_last = INFINITY;     // csmosolver.cpp:51-57
         TSVM_CUDA(cudaMemcpyAsync(ctl, ctl_host, sizeof(SolverCtl), cudaMemcpyHostToDevice, st));
-        TSVM_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-        TSVM_CUDA(cudaEventCreateWithFlags(&ev_fork2, cudaEventDisableTiming));
-        TSVM_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-        {
-            int lo_prio = 0, hi_prio = 0;
-            TSVM_CUDA(cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio));
-            TSVM_CUDA(cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, hi_prio));
-        }
+        TSVM_TRY(take_streams(&streams));
+        st2 = streams->st2; ev_fork = streams->ev_fork; ev_fork2 = streams->ev_fork2; ev_join = streams->ev_join;
         // local iteration cap: max(100000, 100 * ws) (csmosolver.cpp:49)
         local_max_iter = ws > INT_MAX / 100 ? INT_MAX : (100 * ws > 100000 ? 100 * ws : 100000);
         return init_f();
@@ -984,6 +1066,13 @@ struct tsvm_solver {
 
     // init_f (csmosolver.cpp:189-214): f -= sum over the initially non-zero alphas
     tsvm_status init_f() {
+        // all zero, as C-SVC starts: nothing to add, and no need for the alphas on the host
+        int *nonzero = reinterpret_cast<int *>(red);
+        TSVM_CUDA(cudaMemsetAsync(nonzero, 0, sizeof(int), st));
+        TSVM_LAUNCH(any_nonzero_kernel, ceil_div(n, 4096) < 296 ? ceil_div(n, 4096) : 296, 256, 0, st, alpha, n, nonzero);
+        TSVM_CUDA(cudaMemcpyAsync(diff_host, nonzero, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TSVM_CUDA(cudaStreamSynchronize(st));
+        if (*reinterpret_cast<const int *>(diff_host) == 0) { idle = true; return TSVM_OK; }
         std::vector<double> a_h(n);
         std::vector<int> y_h(n);
         TSVM_CUDA(cudaMemcpyAsync(a_h.data(), alpha, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
@@ -1008,7 +1097,9 @@ struct tsvm_solver {
             if (a_h[i] != 0) { bi.push_back(i); bd.push_back(-a_h[i] * y_h[i]); }
             if ((int) bi.size() == ws) TSVM_TRY(flush());
         }
-        return flush();
+        TSVM_TRY(flush());
+        idle = true;
+        return TSVM_OK;
     }
 
     // Queues one outer iteration of csmosolver.cpp:59-120, number `it`, without waiting for it. Its last launch
@@ -1123,17 +1214,15 @@ struct tsvm_solver {
     tsvm_status run_iterations(int count) {
         if (count > sync_every()) count = sync_every();
         if (iter == 0) count = 1;                   // the first iteration is read back on its own
+        idle = false;
         for (int j = 0; j < count; ++j) {
-            IterEvents &E = evs[j];
-            if (!E.l0) {
-                for (auto &e : E.ph) TSVM_CUDA(cudaEventCreate(&e));
-                TSVM_CUDA(cudaEventCreate(&E.l0));
-                TSVM_CUDA(cudaEventCreate(&E.l1));
-            }
-            TSVM_TRY(enqueue_iteration(iter + j, E));
+            TSVM_TRY(streams->ensure_events(j));
+            TSVM_TRY(enqueue_iteration(iter + j, streams->evs[j]));
         }
         TSVM_CUDA(cudaMemcpyAsync(ctl_host, ctl, sizeof(SolverCtl), cudaMemcpyDeviceToHost, st));
-        TSVM_CUDA(cudaStreamSynchronize(st));
+        TSVM_CUDA(cudaStreamSynchronize(st));            // (the second stream has joined the first)
+        idle = true;
+        km->waited(st);
         const SolverCtl &c = *ctl_host;
         if (c.engine_status != 0) {
             set_error("dense kernel-row engine reported status %d (a bounded wait ran out)", c.engine_status);
@@ -1141,7 +1230,7 @@ struct tsvm_solver {
         }
         const int ran = (int) (c.iter - iter);
         for (int j = 0; j < ran; ++j) {
-            const IterEvents &E = evs[j];
+            const IterEvents &E = streams->evs[j];
             float ms;
             cudaEventElapsedTime(&ms, E.ph[0], E.ph[1]); t_sel += ms;
             cudaEventElapsedTime(&ms, E.ph[1], E.ph[2]); t_rows += ms;
@@ -1188,6 +1277,7 @@ struct tsvm_solver {
 
     // rho and objective (csmosolver.cpp:167-187,227-239; nusmosolver.cpp:9-46,120-126)
     tsvm_status finish(double *rho_host, tsvm_solve_stats *stats_host) {
+        idle = false;
         TSVM_LAUNCH(rho_obj_kernel, 1, 1024, 0, st, n, f, alpha, y, Cp, Cn, red);
         TSVM_CUDA(cudaMemcpyAsync(diff_host, red, RHO_VALS * sizeof(double), cudaMemcpyDeviceToHost, st));
         TSVM_CUDA(cudaStreamSynchronize(st));
@@ -1210,6 +1300,7 @@ struct tsvm_solver {
                 rho /= r;
             }
         }
+        idle = true;
         *rho_host = rho;
         if (stats_host) fill_stats(stats_host, obj);
         return TSVM_OK;
@@ -1383,6 +1474,8 @@ struct tsvm_shard {
     tsvm_status init() {
         TSVM_REQUIRE(km_pair_engine(km, st), "shard solver: needs dense data on the CTA-pair tensor engine "
                                              "(more than 32 features)");
+        km->launched(st);
+        km->streams_mixed = true;        // (this solver's two streams; its calls do not note their work on the matrix one by one)
         row_bytes = km_plane_row_bytes(km);
         const size_t plane_words = (row_bytes * (size_t) ws + 3) / 4;
         TSVM_TRY(dev_alloc(&ids, (size_t) ws));
