@@ -114,3 +114,36 @@ def test_fused_prediction_many_classes(capi):
     """20 classes: 19 coefficient rows per support vector (more than the shared-memory table holds) and 190 pairs;
     several launches over the test rows."""
     _fused_case(capi, 20, [17 + 3 * c for c in range(20)], d=64, m=4500)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 64, 65])
+@pytest.mark.parametrize("storage", ["dense", "dense_sv_csr_rows", "csr"])
+@pytest.mark.parametrize("nc,n_sv,d,kernel", [(2, 1, 1, "rbf"), (2, 700, 35, "rbf"), (3, 129, 4, "linear"),
+                                              (32, 300, 70, "poly")])
+def test_prediction_of_few_rows(capi, m, storage, nc, n_sv, d, kernel):
+    """Up to eight tiles of eight rows go through one launch; sizes around its row tiles, one and several support vectors
+    per block, more blocks than support vectors, features that are no multiple of four, test rows with features beyond
+    the support vectors'."""
+    rng = np.random.default_rng(m * 7 + nc)
+    dt = d + 3                                       # the extra features count in the test rows' self dots only
+    SVd = (rng.standard_normal((n_sv, d)) * (rng.random((n_sv, d)) < 0.7)).astype(np.float32)
+    T = (rng.standard_normal((m, dt)) * (rng.random((m, dt)) < 0.7)).astype(np.float32)
+    cnt = np.bincount(np.arange(n_sv) % nc, minlength=nc).astype(np.int32)
+    coef = rng.standard_normal((nc - 1, n_sv))
+    rho = rng.standard_normal(nc * (nc - 1) // 2)
+    kw = dict(kernel=kernel, gamma=0.05, coef0=0.5, degree=2)
+    want = P.predict_dec(P.Csr(dense=SVd), coef.reshape(-1), cnt, rho, nc, P.Csr(dense=T), **kw)
+
+    def csr(a):
+        nz = a != 0
+        rp = np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32)
+        return _t(a[nz]), _t(rp), _t(np.nonzero(nz)[1].astype(np.int32))
+
+    km = capi.KernelMatrix(csr=csr(SVd), d=d, **kw) if storage == "csr" else capi.KernelMatrix(dense=_t(SVd), **kw)
+    batch = dict(dense=_t(T)) if storage == "dense" else dict(csr=csr(T))
+    for _ in range(2):                               # the second call finds the first one's sums cleared
+        dec = capi.predict_dec(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, **batch)
+        assert np.max(np.abs(dec.cpu().numpy() - want)) < 1e-4 * max(1.0, np.max(np.abs(want)))
+        lab = capi.predict_labels(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, **batch)
+        assert np.array_equal(lab.cpu().numpy(), capi.vote(dec, nc).cpu().numpy())
+    km.close()

@@ -223,6 +223,8 @@ struct tsvm_km {
     // requested rows is read from the device (at most the q of the call) and requested row i goes to row
     // rows_slot_dev[i] of the output buffer instead of row i.
     const int *rows_m_dev = nullptr, *rows_slot_dev = nullptr;
+    double *few_acc = nullptr;      // predict_few: sums of a call (zero between calls), and the tickets behind them
+    size_t few_cap = 0;             // doubles in few_acc
     int *status_dev = nullptr;      // device status word written by kernels with bounded waits
     int *status_host = nullptr;     // pinned mirror
     // Work that may still be in flight on the handle's buffers: on one stream, or (streams_mixed) who knows where. The
@@ -241,6 +243,7 @@ struct tsvm_km {
 namespace tsvm {
 // Pieces of tsvm_km_rows_by_index (km.cu) for callers that overlap them with other work.
 bool km_pair_engine(tsvm_km *km, cudaStream_t st);
+bool km_automatic_engine(const tsvm_km *km);
 size_t km_plane_row_bytes(const tsvm_km *km);
 tsvm_status km_stage_rows_by_index(tsvm_km *km, const int *idx_dev, int q, cudaStream_t st);
 tsvm_status km_rows_staged(tsvm_km *km, int q, float *out, long long ld_out, cudaStream_t st);

@@ -906,6 +906,7 @@ tsvm_status launch_dense_tc2_on(tsvm_km *km, const InstancePlanes &X, int m, flo
 
 // True when kernel rows of this matrix run on the CTA-pair tensor engine, whose requested-row staging and
 // launch can be issued separately and against a caller-chosen subset of instances.
+bool km_automatic_engine(const tsvm_km *km) { return km->engine == 0; }
 bool km_pair_engine(tsvm_km *km, cudaStream_t st) {
     if (!km->dense || !use_tensor_engine(km)) return false;
     return ensure_planes(km, st) == TSVM_OK && km->plane_kind != 0;
@@ -1069,7 +1070,7 @@ void tsvm_km_destroy(tsvm_km *km) {
     if (!km) return;
     pool_free_many({km->X_owned, km->Xhi, km->Xlo, km->x_unscale, km->w_unscale, km->val_owned, km->row_ptr_owned,
                     km->col_owned, km->self_dot, km->diag, km->W, km->Whi, km->Wlo, km->WT, km->sd_rows,
-                    km->status_dev}, !km->in_flight && !km->exposed);
+                    km->few_acc, km->status_dev}, !km->in_flight && !km->exposed);
     if (km->status_host) pinned_free(km->status_host);
     delete km;
 }

@@ -10,6 +10,7 @@
 // vectors, at most 32 features) compute the block in slabs of test rows and reduce it with
 // sum_kernel_values_kernel.
 #include "common.cuh"
+#include "predict_few.cuh"
 #include <vector>
 
 namespace tsvm {
@@ -101,16 +102,86 @@ static tsvm_status fused_slab(tsvm_km *km_sv, const double *coef_dev, const int 
     return launch_dense_tc2_predict(km_sv, mm, coef_dev, sv_class, n_classes, dec, st);
 }
 
+// Few rows: one launch (predict_few.cuh; 62 -> 33 us per call at 8 rows x 3,001 x 100, 104 -> 45 us at 1 x 5,000 x 784 with
+// ten classes, 190 -> 42 us at 5 CSR rows x 8,000). *taken: the path was taken and the results are there.
+// Where the line lies: eight rows cost one read of the support vectors, which no other path undercuts; more rows cost
+// one read (from L2) per eight, so that they pay as long as that stays below the 15 - 20 us that the general path's
+// extra launches take - about 1.6e7 features read.
+template <int R>
+static tsvm_status launch_few(const FewArgs &a, bool csr, cudaStream_t st) {
+    const int tiles = ceil_div(a.m, R);
+    int bx = ceil_div(a.n_sv, 8), most = 2 * device_sm_count() / tiles;
+    if (most < 1) most = 1;
+    if (bx > most) bx = most;
+    if (csr) {
+        const size_t smem = sizeof(float) * FEW_ENTRIES * R + (sizeof(int) + sizeof(short)) * FEW_SLOTS + FewShared<R>::bytes(a.n_pairs);
+        TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute(predict_few_csr_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)));
+        TSVM_LAUNCH(predict_few_csr_kernel<R>, dim3(bx, tiles), FEW_THREADS + 32, smem, st, a);
+    } else {
+        const size_t smem = sizeof(float) * R * ((a.d + 3) & ~3) + FewShared<R>::bytes(a.n_pairs);
+        TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute(predict_few_dense_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)));
+        TSVM_LAUNCH(predict_few_dense_kernel<R>, dim3(bx, tiles), FEW_THREADS + 32, smem, st, a);
+    }
+    return TSVM_OK;
+}
+
+static tsvm_status predict_few(tsvm_km *km, const double *coef_dev, const int *sv_count_host, const double *rho_dev,
+                               int n_classes, int m, const float *T_dev, int dt, int ldt, const float *tval_dev,
+                               const int *trow_ptr_dev, const int *tcol_dev, long long tnnz, double *dec_dev, int *labels_dev,
+                               cudaStream_t st, bool *taken) {
+    *taken = false;
+    const int R = m == 1 ? 1 : (m == 2 ? 2 : (m <= 4 ? 4 : 8)), tiles = ceil_div(m, R);
+    if (n_classes > FEW_CLASSES || tiles > FEW_TILES || (km->dense && !km_automatic_engine(km))) return TSVM_OK;
+    const double per_sv = km->dense ? (double) km->d_pad : (double) km->nnz / km->n;
+    if (tiles > 1 && (double) tiles * km->n * (km->nnz < 0 ? 64.0 : per_sv) > 1.6e7) return TSVM_OK;
+    const int n_pairs = n_classes * (n_classes - 1) / 2;
+    if (km->dense) {
+        if (sizeof(float) * (size_t) R * km->d_pad + FewShared<8>::bytes(n_pairs) > 190 * 1024) return TSVM_OK;
+    } else if (T_dev || tnnz <= 0 || tnnz > FEW_ENTRIES) return TSVM_OK;
+    const size_t need = (size_t) FEW_TILES * 8 * n_pairs + FEW_TILES;
+    if (km->few_cap < need) {
+        pool_free(km->few_acc);
+        km->few_acc = nullptr;
+        km->few_cap = 0;
+        TSVM_TRY(dev_alloc(&km->few_acc, need));
+        TSVM_CUDA(cudaMemsetAsync(km->few_acc, 0, need * sizeof(double), st));
+        km->few_cap = need;
+    }
+    FewArgs a;
+    a.X = km->dense ? km->X : nullptr; a.ldx = km->ldx; a.val = km->val; a.row_ptr = km->row_ptr; a.col = km->col;
+    a.n_sv = km->n; a.d = km->d; a.sd_sv = km->self_dot;
+    a.T = T_dev; a.dt = dt; a.ldt = ldt; a.tval = tval_dev; a.trow_ptr = trow_ptr_dev; a.tcol = tcol_dev; a.m = m;
+    a.fn = km->fn; a.coef = coef_dev; a.rho = rho_dev; a.n_classes = n_classes; a.n_pairs = n_pairs;
+    a.start[0] = 0;
+    for (int c = 0; c < n_classes; ++c) a.start[c + 1] = a.start[c] + sv_count_host[c];
+    // the tickets lie at the end of the buffer, whatever the number of sums in front of them
+    a.acc = km->few_acc; a.ticket = reinterpret_cast<int *>(km->few_acc + km->few_cap - FEW_TILES);
+    a.dec = dec_dev; a.labels = labels_dev; a.overflow = km->status_host + 1;
+    km->status_host[1] = 0;
+    if (R == 1) TSVM_TRY(launch_few<1>(a, !km->dense, st));
+    else if (R == 2) TSVM_TRY(launch_few<2>(a, !km->dense, st));
+    else if (R == 4) TSVM_TRY(launch_few<4>(a, !km->dense, st));
+    else TSVM_TRY(launch_few<8>(a, !km->dense, st));
+    TSVM_CUDA(cudaStreamSynchronize(st));
+    *taken = *(volatile int *) (km->status_host + 1) == 0;
+    return TSVM_OK;
+}
+
 // labels_dev != nullptr: only the vote leaves the slab (sum_kernel_values_instant); dec_dev is then unused.
 static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host, const double *rho_dev,
                                 int n_classes, int m, const float *T_dev, int dt, int ldt, const float *tval_dev,
-                                const int *trow_ptr_dev, const int *tcol_dev, double *dec_dev, int *labels_dev,
-                                size_t max_mem_bytes, cudaStream_t st) {
+                                const int *trow_ptr_dev, const int *tcol_dev, long long tnnz, double *dec_dev,
+                                int *labels_dev, size_t max_mem_bytes, cudaStream_t st) {
     const int n_sv = km_sv->n;
     int total = 0;
     std::vector<int> start(n_classes), count(n_classes);
     for (int c = 0; c < n_classes; ++c) { start[c] = total; count[c] = sv_count_host[c]; total += count[c]; }
     TSVM_REQUIRE(total == n_sv, "predict: support-vector counts sum to %d but the matrix holds %d", total, n_sv);
+    km_sv->launched(st);
+    bool taken = false;
+    TSVM_TRY(predict_few(km_sv, coef_dev, sv_count_host, rho_dev, n_classes, m, T_dev, dt, ldt, tval_dev, trow_ptr_dev,
+                         tcol_dev, tnnz, dec_dev, labels_dev, st, &taken));
+    if (taken) { km_sv->waited(st); return TSVM_OK; }
     const int nb = n_classes * (n_classes - 1) / 2;
     const bool fused = km_pair_engine(km_sv, st);
     const long long ldk = ((long long) n_sv + 3) & ~3ll;
@@ -171,7 +242,8 @@ static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const in
             s = TSVM_ERR_DEVICE;
         }
     } else cudaStreamSynchronize(st);
-    pool_free_many({K, meta, sv_class, dec_slab});
+    pool_free_many({K, meta, sv_class, dec_slab}, s == TSVM_OK);      // (only this stream has used them)
+    if (s == TSVM_OK) km_sv->waited(st);
     return s;
 }
 
@@ -181,24 +253,22 @@ tsvm_status tsvm_predict_dec(tsvm_km *km_sv, const double *coef_dev, const int *
                              int n_classes, int m, const float *T_dev, int dt, int ldt, const float *tval_dev,
                              const int *trow_ptr_dev, const int *tcol_dev, long long tnnz, double *dec_dev,
                              size_t max_mem_bytes, void *stream) {
-    (void) tnnz;
     TSVM_REQUIRE(km_sv && coef_dev && sv_count_host && rho_dev && dec_dev && n_classes >= 2 && m > 0,
                  "predict_dec: bad arguments");
     TSVM_REQUIRE(T_dev || trow_ptr_dev, "predict_dec: neither a dense nor a CSR test batch was given");
     return predict_impl(km_sv, coef_dev, sv_count_host, rho_dev, n_classes, m, T_dev, dt, ldt, tval_dev, trow_ptr_dev,
-                        tcol_dev, dec_dev, nullptr, max_mem_bytes, (cudaStream_t) stream);
+                        tcol_dev, tnnz, dec_dev, nullptr, max_mem_bytes, (cudaStream_t) stream);
 }
 
 tsvm_status tsvm_predict_labels(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host,
                                 const double *rho_dev, int n_classes, int m, const float *T_dev, int dt, int ldt,
                                 const float *tval_dev, const int *trow_ptr_dev, const int *tcol_dev, long long tnnz,
                                 int *labels_dev, size_t max_mem_bytes, void *stream) {
-    (void) tnnz;
     TSVM_REQUIRE(km_sv && coef_dev && sv_count_host && rho_dev && labels_dev && n_classes >= 2 && m > 0,
                  "predict_labels: bad arguments");
     TSVM_REQUIRE(T_dev || trow_ptr_dev, "predict_labels: neither a dense nor a CSR test batch was given");
     return predict_impl(km_sv, coef_dev, sv_count_host, rho_dev, n_classes, m, T_dev, dt, ldt, tval_dev, trow_ptr_dev,
-                        tcol_dev, nullptr, labels_dev, max_mem_bytes, (cudaStream_t) stream);
+                        tcol_dev, tnnz, nullptr, labels_dev, max_mem_bytes, (cudaStream_t) stream);
 }
 
 tsvm_status tsvm_vote(const double *dec_dev, int m, int n_classes, int *out_dev, void *stream) {
