@@ -251,3 +251,35 @@ def test_csr_engines_agree_bit_for_bit():
         assert r.returncode == 0, r.stderr[-2000:]
         digests.append(r.stdout.strip().splitlines()[-1])
     assert len(digests[0]) == 64 and digests[0] == digests[1]
+
+
+@pytest.mark.parametrize("q", [1, 128, 129, 700])
+@pytest.mark.parametrize("d,kernel", [(378, "linear"), (379, "rbf"), (5000, "rbf"), (300000, "rbf")])
+def test_csr_rows_places_of_the_panel(capi, q, d, kernel):
+    """The largest panel that fits shared memory, one feature more, more features than the skip bitmap covers; one requested
+    row, a full part, one row more, several parts; instances with no entries, with one batch of 32 and with more; a
+    number of instances that is no multiple of a warp's unit."""
+    import torch
+    rng = np.random.default_rng(q + d)
+    n = 1003
+    lens = rng.integers(0, 90, n)
+    p = 1.0 / np.arange(1, d + 1)
+    cdf = np.cumsum(p / p.sum())
+    rows = [np.unique(np.minimum(np.searchsorted(cdf, rng.random(k)), d - 1)) for k in lens]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    col = np.concatenate(rows).astype(np.int32)
+    val = rng.standard_normal(len(col)).astype(np.float32) * 0.3
+    ids = rng.choice(n, q, replace=False).astype(np.int32)
+    want = P.kernel_rows_idx(P.Csr(csr=(val, rp, col), d=d), ids, kernel=kernel, gamma=0.1)
+    km = capi.KernelMatrix(csr=(torch.from_numpy(val).cuda(), torch.from_numpy(rp).cuda(), torch.from_numpy(col).cuda()), d=d,
+                           kernel=kernel, gamma=0.1)
+    for _ in range(2):                               # the staging panel and its bitmap are clear again after a call
+        got = km.get_rows(torch.from_numpy(ids).cuda()).cpu().numpy()
+        assert np.max(np.abs(got - want) / np.maximum(np.abs(want), 0.05)) < 1e-5   # linear products cancel
+    if d == 5000:                                    # the same rows as a dense batch: no bitmap
+        T = np.zeros((q, d), np.float32)
+        for i, r in enumerate(ids):
+            T[i, col[rp[r]:rp[r + 1]]] = val[rp[r]:rp[r + 1]]
+        got = km.get_rows_instances(dense=torch.from_numpy(T).cuda()).cpu().numpy()
+        assert np.max(np.abs(got - want) / np.maximum(np.abs(want), 0.05)) < 1e-5   # linear products cancel
+    km.close()

@@ -211,13 +211,15 @@ struct tsvm_km {
     int *row_ptr_owned = nullptr, *col_owned = nullptr;
     float *self_dot = nullptr, *diag = nullptr;
     // scratch for the rows whose kernel values are requested
-    int w_cap = 0;                  // rows the scratch below can hold
+    int w_cap = 0;                  // rows the dense engines' scratch can hold
     float *W = nullptr;             // dense engines: w_cap x d_pad (row-major), FP32
     float *Whi = nullptr, *Wlo = nullptr;   // two-plane split of W, same kind as the X planes
     float *w_unscale = nullptr;     // FP16 planes: 1 / scale of every requested row [w_cap]
     float *WT = nullptr;            // CSR engine: d x wt_ld, column = requested row
-    int wt_ld = 0;
-    float *sd_rows = nullptr;       // self dots of the requested rows [w_cap]
+    int wt_ld = 0;                  // rows the panel can hold
+    unsigned *csr_bits = nullptr;   // bitmap of the features staged in every part of the panel
+    float *sd_rows = nullptr;       // self dots of the requested rows [sd_cap]
+    int sd_cap = 0;
     int reserve_clusters = 0;       // SM pairs the pair engine leaves free (a concurrent stream's kernels run there)
     // Set by a caller around tsvm_km_rows_by_index-style launches (the solver's row cache): the number of
     // requested rows is read from the device (at most the q of the call) and requested row i goes to row

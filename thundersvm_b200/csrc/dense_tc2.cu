@@ -445,7 +445,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                             // takes one column (test row) and half of the instances and multiplies their values by all
                             // coefficients (16-byte reads of four instances' coefficients). Element (c, l) of the block
                             // lies at column (l + c) mod 32, so that the 16 columns are read from 16 banks. Ten
-                            // classes, 8,003 x 784: 290 -> 130 us per 4,096 rows.
+                            // classes, 8,003 x 784: 290 -> 247 us per 4,096 rows.
                             float *block = priv - lane;
                             const float *cf_block = coef_priv - lane;
                             __syncwarp();                    // everyone has read its own sums

@@ -232,7 +232,7 @@ __global__ void self_dot_csr_kernel(const float *__restrict__ val, const int *__
 // Self dots of a batch of new instances, accumulated sequentially in float in storage order as kernelmatrix.cpp:288-296
 // does: one thread per row keeps that order. What bounds it is that chain, 4 cycles per feature; the rows have to be
 // there in time. A warp copies 32 rows x 64 features at a time (asynchronous copies, coalesced, four stages in flight) to
-// shared memory and each lane adds up its own row from there: 4,096 rows x 2,000 155 -> 9 us against loads that every lane
+// shared memory and each lane adds up its own row from there: 4,096 rows x 2,000 155 -> 23 us against loads that every lane
 // made from its own row. VEC: 16-byte copies (aligned rows), else 4-byte ones.
 constexpr int SEQ_COLS = 64, SEQ_STAGES = 4, SEQ_LD = SEQ_COLS + 4;      // row stride: 16-byte reads without bank conflicts
 template <bool VEC>
@@ -456,12 +456,16 @@ __global__ void scatter_csr_to_w_kernel(const float *__restrict__ val, const int
     }
 }
 
-// CSR engine staging: WT[c * wt_ld + i] = value of feature c in requested row i. WT is kept
-// all-zero between calls: `clear` = true writes zeros back at the same places.
+constexpr int CSR_PART = 128;               // requested rows per part of the CSR engine
+
+// CSR engine staging: WT[c * wt_ld + i] = value of feature c in requested row i, and a bit for feature c in the bitmap
+// of row i's part (bits [parts][words], words == 0: none). Both are kept all-zero between calls: `clear` = true writes
+// zeros back at the same places.
 __global__ void scatter_csr_to_wt_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr,
                                          const int *__restrict__ col, const int *__restrict__ idx, int m, int d,
                                          int wt_ld, float *__restrict__ WT, const float *__restrict__ sd,
-                                         float *__restrict__ sd_rows, bool clear, const int *__restrict__ m_dev) {
+                                         float *__restrict__ sd_rows, bool clear, const int *__restrict__ m_dev,
+                                         unsigned *__restrict__ bits, int words) {
     int i = blockIdx.x;
     if (i >= m || (m_dev && i >= *m_dev)) return;
     int r = idx ? idx[i] : i;
@@ -469,9 +473,15 @@ __global__ void scatter_csr_to_wt_kernel(const float *__restrict__ val, const in
         if (!clear && sd && threadIdx.x == 0) sd_rows[i] = 0.0f;
         return;
     }
+    unsigned *mine = bits + (size_t) (i / CSR_PART) * words;
     for (int p = row_ptr[r] + threadIdx.x; p < row_ptr[r + 1]; p += blockDim.x) {
         int c = col[p];
-        if (c < d) WT[(size_t) c * wt_ld + i] = clear ? 0.0f : val[p];
+        if (c >= d) continue;
+        WT[(size_t) c * wt_ld + i] = clear ? 0.0f : val[p];
+        if (words) {
+            if (clear) mine[c >> 5] = 0u;
+            else atomicOr(mine + (c >> 5), 1u << (c & 31));
+        }
     }
     if (!clear && sd && threadIdx.x == 0) sd_rows[i] = sd[r];
 }
@@ -566,248 +576,210 @@ dense_rows_simt_kernel(const float *__restrict__ X, int ldx, int n, const float 
 }
 
 // ---- CSR engine ------------------------------------------------------------------------------
-// One warp per stored instance; lanes own requested rows c = 4*lane + 128*v (float4 each). For
-// every stored entry (col, val) in storage order: acc[c] += val * WT[col][c], the same FP32
-// recurrence as the reference's sparse x dense product (kernelmatrix_kernel.cpp:149-160).
-// A block covers 32 consecutive instances and transposes its results through shared memory so
-// that every requested row receives 128-byte coalesced stores.
-template <int NV>
-__global__ void __launch_bounds__(256)
-csr_rows_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, const int *__restrict__ col, int n,
-                const float *__restrict__ WT, int wt_ld, int m_launch, const float *__restrict__ sd,
-                const float *__restrict__ sd_rows, KernelFn fn, float *__restrict__ out, long long ld_out,
-                const int *__restrict__ m_dev, const int *__restrict__ row_slot) {
-    extern __shared__ float tile[];   // [NV*128][33]
-    const int m = m_dev ? min(m_launch, max(*m_dev, 0)) : m_launch;     // the count found on the device, if any
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int j0 = blockIdx.x * 32;
-    for (int jj = warp; jj < 32; jj += 8) {
-        const int j = j0 + jj;
-        float4 acc[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v] = make_float4(0, 0, 0, 0);
-        if (j < n) {
-            const int b = row_ptr[j], e = row_ptr[j + 1];
-            for (int p0 = b; p0 < e; p0 += 32) {
-                int cc = 0;
-                float vv = 0;
-                if (p0 + lane < e) { cc = col[p0 + lane]; vv = val[p0 + lane]; }
-                const int cnt = min(32, e - p0);
-                for (int t = 0; t < cnt; ++t) {
-                    const int c = __shfl_sync(0xffffffffu, cc, t);
-                    const float x = __shfl_sync(0xffffffffu, vv, t);
-                    const float4 *w = reinterpret_cast<const float4 *>(WT + (size_t) c * wt_ld) + lane;
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) {
-                        float4 wv = __ldg(w + 32 * v);
-                        acc[v].x = fmaf(x, wv.x, acc[v].x);
-                        acc[v].y = fmaf(x, wv.y, acc[v].y);
-                        acc[v].z = fmaf(x, wv.z, acc[v].z);
-                        acc[v].w = fmaf(x, wv.w, acc[v].w);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const int c = 128 * v + 4 * lane;
-            tile[(c + 0) * 33 + jj] = acc[v].x;
-            tile[(c + 1) * 33 + jj] = acc[v].y;
-            tile[(c + 2) * 33 + jj] = acc[v].z;
-            tile[(c + 3) * 33 + jj] = acc[v].w;
-        }
-    }
-    __syncthreads();
-    const int j = j0 + lane;
-    const float sdj = j < n ? sd[j] : 0.0f;
-    if ((ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && j0 + 32 <= n) {
-        // four consecutive instances of one row per thread, one 16-byte store: a warp covers four rows
-        const int jq = 4 * (lane & 7);
-        const float s0 = __shfl_sync(0xffffffffu, sdj, jq), s1 = __shfl_sync(0xffffffffu, sdj, jq + 1),
-                    s2 = __shfl_sync(0xffffffffu, sdj, jq + 2), s3 = __shfl_sync(0xffffffffu, sdj, jq + 3);
-#pragma unroll 2
-        for (int c = 4 * warp + (lane >> 3); c < m; c += 32) {
-            const float *tr = tile + c * 33 + jq;
-            const float sr = sd_rows[c];
-            const size_t orow = row_slot ? (size_t) row_slot[c] : (size_t) c;
-            float4 o;
-            o.x = apply_kernel(fn, tr[0], sr, s0); o.y = apply_kernel(fn, tr[1], sr, s1);
-            o.z = apply_kernel(fn, tr[2], sr, s2); o.w = apply_kernel(fn, tr[3], sr, s3);
-            *reinterpret_cast<float4 *>(out + orow * ld_out + j0 + jq) = o;
-        }
-        return;
-    }
-    for (int c = warp; c < m; c += 8) {
-        const size_t orow = row_slot ? (size_t) row_slot[c] : (size_t) c;
-        if (j < n) out[orow * ld_out + j] = apply_kernel(fn, tile[c * 33 + lane], sd_rows[c], sdj);
-    }
+// out[i][j] = kfn(sum over the stored entries (c, x) of instance j, in storage order, of x * panel[c][i]): the same FP32
+// recurrence per value as the reference's sparse x dense product (kernelmatrix_kernel.cpp:149-160). The requested rows are
+// staged as a panel [feature][requested row] (zero where a row has no such feature).
+//
+// A warp takes an instance at a time and a part of 128 requested rows, a lane four of them: an entry costs one 512-byte
+// read of the panel and four FMAs per lane. What bounds it is first the number of instructions around these, then the
+// latency of the reads, then L2:
+//   * the live entries of 32 are packed (place, value) into shared memory, from where the loop reads two with one
+//     broadcast load: 8 instructions per entry instead of 28 with a shuffle each for place and value;
+//   * an entry whose panel row is all zero in this part is skipped (a bitmap over the features, filled by the staging
+//     kernel): adding x * 0 does not change a sum, and text-like data has mostly such entries;
+//   * with few features (ALL) the part's panel is copied to shared memory first; else the frequent features come from L1
+//     (keeping the most frequent ones in shared memory took half of the warps' room and was slower);
+//   * bounds, entries and self dots of the following instances are fetched while one is computed;
+//   * blocks are dealt to the parts that exist: the number of requested rows is only known on the device (the row cache
+//     asks for what it misses, often 100 of 512), and every block takes part;
+//   * a warp works on `unit` consecutive instances and then stores up to 16 bytes per requested row at once. Larger units
+//     store better, smaller ones leave fewer warps without work at the end: the largest one with four rounds or more.
+// Measured, staging included, before and after: 120 / 512 / 1,000 requested rows of 20,242 x 47,236 (74 entries each) 80 /
+// 306 / 1,344 -> 68 / 157 / 279 us; of 32,561 x 123 (14 entries each) 56 / 96 / 171 -> 56 / 103 / 184 us, where the former
+// engine could not tell that only 120 of 512 rows were wanted.
+constexpr int CSR_THREADS = 512, CSR_WARPS = CSR_THREADS / 32, CSR_UNIT = 4;
+constexpr int CSR_WARP_SMEM = CSR_UNIT * 33 * 16 + 32 * 8;                       // results of a unit, packed entries
+constexpr int CSR_FIXED_SMEM = CSR_WARPS * CSR_WARP_SMEM + CSR_PART * 4;         // and the output row of every requested row
+constexpr int CSR_BITMAP_MAX_D = 1 << 18;                                        // 32 KB of bitmap; more features: no skipping
+constexpr int CSR_SMEM_MAX = 227 * 1024 - 256;
+__host__ __device__ constexpr int csr_bitmap_words(int d) { return d <= CSR_BITMAP_MAX_D ? (d + 31) / 32 : 0; }
+
+struct CsrPanel {
+    const float *WT;                // [d][ld]
+    int ld, d;
+    const unsigned *bits;           // [parts][words]: features that some row of the part has
+    int words;                      // 0: no bitmap
+};
+
+template <bool RBF>
+__device__ __forceinline__ float csr_value(const KernelFn &fn, float dot, float sd_i, float sd_j) {
+    if constexpr (RBF) return expf(-(sd_i + sd_j - dot * 2.0f) * fn.gamma);
+    else return apply_kernel(fn, dot, sd_i, sd_j);
 }
 
-// ---- CSR engine for few features: the panel in shared memory ---------------------------------------
-// csr_rows_kernel reads a 2 KB panel row from L2 for every stored entry; with d features the panel is only
-// d x 1 KB per 256 requested rows, which fits in shared memory for d <= CSR_SMEM_MAX_D. A block then loads
-// its 256-row part of the panel once and sweeps instance tiles with it (grid: blocks x parts, every block a
-// strided share of the 32-instance tiles): a stored entry costs two 16-byte shared-memory loads and eight
-// multiply-adds per lane instead of a trip to L2. Same FP32 recurrence in storage order per (row, instance),
-// so the values are those of csr_rows_kernel bit for bit. Results go through a double-buffered transposed
-// tile so that every requested row receives 128-byte coalesced stores.
-constexpr int CSR_SMEM_THREADS = 512, CSR_SMEM_PART = 256, CSR_SMEM_TILE = CSR_SMEM_PART * 33;
-constexpr int CSR_SMEM_MAX_D = (227 * 1024 - 2 * CSR_SMEM_TILE * 4 - 2 * CSR_SMEM_PART * 4 - 64) / (CSR_SMEM_PART * 4);
-
-__global__ void __launch_bounds__(CSR_SMEM_THREADS, 1)
-csr_rows_smem_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, const int *__restrict__ col, int n,
-                     int d, const float *__restrict__ WT, int wt_ld, int m_launch, const float *__restrict__ sd,
-                     const float *__restrict__ sd_rows, KernelFn fn, float *__restrict__ out, long long ld_out,
-                     const int *__restrict__ m_dev, const int *__restrict__ row_slot) {
-    extern __shared__ __align__(16) float csr_sm[];          // panel [d][256] | tile [2][256][33]
+template <bool RBF, bool ALL>
+__global__ void __launch_bounds__(CSR_THREADS, 2)
+csr_rows_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, const int *__restrict__ col, int n,
+                const CsrPanel P, int m_launch, const float *__restrict__ sd, const float *__restrict__ sd_rows, KernelFn fn,
+                float *__restrict__ out, long long ld_out, const int *__restrict__ m_dev, const int *__restrict__ row_slot) {
+    extern __shared__ __align__(16) unsigned char csr_sm[];  // results | packed entries | output rows | panel or bitmap
     const int m = m_dev ? min(m_launch, max(*m_dev, 0)) : m_launch;     // the count found on the device, if any
-    const int c0 = blockIdx.y * CSR_SMEM_PART;
-    if (c0 >= m) return;
-    const int mh = min(CSR_SMEM_PART, m - c0);
-    float4 *panel4 = reinterpret_cast<float4 *>(csr_sm);
-    float *tiles = csr_sm + (size_t) d * CSR_SMEM_PART;
+    const int parts = (m + CSR_PART - 1) / CSR_PART;
+    if (parts == 0) return;
+    const int part = blockIdx.x % parts, share = blockIdx.x / parts, shares = ((int) gridDim.x - part + parts - 1) / parts;
+    const int c0 = part * CSR_PART, mh = min(CSR_PART, m - c0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    __shared__ int orow_sm[CSR_SMEM_PART];
-    __shared__ float sdr_sm[CSR_SMEM_PART];
-    if (tid < mh) {
-        orow_sm[tid] = row_slot ? row_slot[c0 + tid] : c0 + tid;
-        sdr_sm[tid] = sd_rows[c0 + tid];
+    float4 *res = reinterpret_cast<float4 *>(csr_sm) + (size_t) warp * CSR_UNIT * 33;
+    uint2 *packed = reinterpret_cast<uint2 *>(csr_sm + CSR_WARPS * CSR_UNIT * 33 * 16) + warp * 32;
+    int *orow_sm = reinterpret_cast<int *>(csr_sm + CSR_WARPS * CSR_WARP_SMEM);
+    unsigned char *rest = csr_sm + CSR_FIXED_SMEM;
+    const unsigned *bits = reinterpret_cast<const unsigned *>(rest);
+    if constexpr (ALL) {
+        float4 *panel = reinterpret_cast<float4 *>(rest);
+#pragma unroll 4
+        for (int i = tid; i < P.d * (CSR_PART / 4); i += CSR_THREADS)
+            panel[i] = __ldg(reinterpret_cast<const float4 *>(P.WT + (size_t) (i / (CSR_PART / 4)) * P.ld + c0) + i % (CSR_PART / 4));
+    } else {
+        for (int w = tid; w < P.words; w += CSR_THREADS)
+            reinterpret_cast<unsigned *>(rest)[w] = P.bits[(size_t) part * P.words + w];
     }
-    for (int i = tid; i < d * (CSR_SMEM_PART / 4); i += CSR_SMEM_THREADS) {
-        const int c = i / (CSR_SMEM_PART / 4), v = i % (CSR_SMEM_PART / 4);
-        panel4[i] = __ldg(reinterpret_cast<const float4 *>(WT + (size_t) c * wt_ld + c0) + v);
-    }
+    // this lane's requested rows: c0 + 4 * lane + k
+    float sdr[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sdr[k] = 4 * lane + k < mh ? sd_rows[c0 + 4 * lane + k] : 0.0f;
+    if (tid < CSR_PART) orow_sm[tid] = tid < mh ? (row_slot ? row_slot[c0 + tid] : c0 + tid) : -1;
     __syncthreads();
-    const int n_tiles = (n + 31) / 32;
     const bool vec_ok = (ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    constexpr int PER_WARP = 32 / (CSR_SMEM_THREADS / 32);        // instances of a tile per warp
-    // The CSR entries of the next tile's instances are fetched (row bounds, then the first 32 entries) while
-    // this tile is computed: the two dependent trips to memory per instance stay off the critical path.
-    int nb[PER_WARP], ne[PER_WARP], ncc[PER_WARP];
-    float nvv[PER_WARP], nsd = 0.0f;
-    auto fetch = [&](int ti) {
-#pragma unroll
-        for (int u = 0; u < PER_WARP; ++u) {
-            const int j = ti * 32 + warp + u * (CSR_SMEM_THREADS / 32);
-            nb[u] = ne[u] = 0; ncc[u] = 0; nvv[u] = 0.0f;
-            if (ti < n_tiles && j < n) { nb[u] = row_ptr[j]; ne[u] = row_ptr[j + 1]; }
-        }
-#pragma unroll
-        for (int u = 0; u < PER_WARP; ++u)
-            if (nb[u] + lane < ne[u]) { ncc[u] = col[nb[u] + lane]; nvv[u] = val[nb[u] + lane]; }
-        const int j = ti * 32 + lane;
-        nsd = (ti < n_tiles && j < n) ? sd[j] : 0.0f;
+    const long long rounds = (long long) n * parts / ((long long) gridDim.x * CSR_WARPS);
+    const int unit = rounds >= 16 ? 4 : (rounds >= 8 ? 2 : 1);
+    const int step = shares * CSR_WARPS * unit;
+    auto after = [&](int j) { return ((j + 1) & (unit - 1)) != 0 && j + 1 < n ? j + 1 : j - (j & (unit - 1)) + step; };
+    auto bounds = [&](int j, int &b, int &e, float &s) {
+        b = e = 0; s = 0.0f;
+        if (j < n) { b = row_ptr[j]; e = row_ptr[j + 1]; s = sd[j]; }
     };
-    fetch(blockIdx.x);
-    int buf = 0;
-    for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, buf ^= 1) {
-        const int j0 = ti * 32;
-        float *T = tiles + buf * CSR_SMEM_TILE;
-        int cb[PER_WARP], ce[PER_WARP], ccc[PER_WARP];
-        float cvv[PER_WARP];
-#pragma unroll
-        for (int u = 0; u < PER_WARP; ++u) { cb[u] = nb[u]; ce[u] = ne[u]; ccc[u] = ncc[u]; cvv[u] = nvv[u]; }
-        const float sdj = nsd;
-        fetch(ti + gridDim.x);
-#pragma unroll
-        for (int u = 0; u < PER_WARP; ++u) {
-            const int jj = warp + u * (CSR_SMEM_THREADS / 32);
-            // rows c0 + 4 * lane + 0..3 and c0 + 128 + 4 * lane + 0..3: a warp's 16-byte loads cover 512 contiguous bytes
-            float4 a0 = make_float4(0, 0, 0, 0), a1 = make_float4(0, 0, 0, 0);
-            for (int p0 = cb[u]; p0 < ce[u]; p0 += 32) {
-                int cc = ccc[u];
-                float vv = cvv[u];
-                if (p0 != cb[u]) {                  // beyond the prefetched entries
-                    cc = 0; vv = 0;
-                    if (p0 + lane < ce[u]) { cc = col[p0 + lane]; vv = val[p0 + lane]; }
-                }
-                const int cnt = min(32, ce[u] - p0);
-                int t = 0;
-                // four stored entries at a time: their panel loads are independent, the sums keep the storage order
-                for (; t + 4 <= cnt; t += 4) {
-                    float x[4];
-                    float4 w0[4], w1[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int c = __shfl_sync(0xffffffffu, cc, t + k);
-                        x[k] = __shfl_sync(0xffffffffu, vv, t + k);
-                        const float4 *w = panel4 + (size_t) c * (CSR_SMEM_PART / 4) + lane;
-                        w0[k] = w[0]; w1[k] = w[32];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        a0.x = fmaf(x[k], w0[k].x, a0.x); a0.y = fmaf(x[k], w0[k].y, a0.y);
-                        a0.z = fmaf(x[k], w0[k].z, a0.z); a0.w = fmaf(x[k], w0[k].w, a0.w);
-                        a1.x = fmaf(x[k], w1[k].x, a1.x); a1.y = fmaf(x[k], w1[k].y, a1.y);
-                        a1.z = fmaf(x[k], w1[k].z, a1.z); a1.w = fmaf(x[k], w1[k].w, a1.w);
-                    }
-                }
-                for (; t < cnt; ++t) {
-                    const int c = __shfl_sync(0xffffffffu, cc, t);
-                    const float x = __shfl_sync(0xffffffffu, vv, t);
-                    const float4 *w = panel4 + (size_t) c * (CSR_SMEM_PART / 4) + lane;
-                    const float4 w0 = w[0], w1 = w[32];
-                    a0.x = fmaf(x, w0.x, a0.x); a0.y = fmaf(x, w0.y, a0.y);
-                    a0.z = fmaf(x, w0.z, a0.z); a0.w = fmaf(x, w0.w, a0.w);
-                    a1.x = fmaf(x, w1.x, a1.x); a1.y = fmaf(x, w1.y, a1.y);
-                    a1.z = fmaf(x, w1.z, a1.z); a1.w = fmaf(x, w1.w, a1.w);
-                }
+    auto entry = [&](int p, int e, int &c, float &v) {
+        c = 0; v = 0.0f;
+        if (p < e) { c = col[p]; v = val[p]; }
+    };
+    auto panel_row = [&](unsigned place) -> float4 {
+        if constexpr (ALL) return *reinterpret_cast<const float4 *>(rest + place + lane * 16);
+        return __ldg(reinterpret_cast<const float4 *>(P.WT + (size_t) place * P.ld + c0) + lane);
+    };
+    auto add = [](float4 &acc, unsigned v, const float4 &w) {
+        const float x = __uint_as_float(v);
+        acc.x = fmaf(x, w.x, acc.x); acc.y = fmaf(x, w.y, acc.y);
+        acc.z = fmaf(x, w.z, acc.z); acc.w = fmaf(x, w.w, acc.w);
+    };
+    int j = (share * CSR_WARPS + warp) * unit, j1 = after(j);
+    int b, e, b1, e1, cc;
+    float s, s1, vv;
+    if (j >= n) return;
+    bounds(j, b, e, s);
+    bounds(j1, b1, e1, s1);
+    entry(b + lane, e, cc, vv);
+    for (;;) {
+        const int j2 = after(j1);
+        int b2, e2, cc1;
+        float s2, vv1;
+        bounds(j2, b2, e2, s2);
+        entry(b1 + lane, e1, cc1, vv1);
+        float4 acc = make_float4(0, 0, 0, 0);
+        for (int p0 = b; p0 < e; p0 += 32) {
+            const int c = cc;
+            const float v = vv;
+            if (p0 + 32 < e) entry(p0 + 32 + lane, e, cc, vv);
+            bool live = p0 + lane < e;
+            if constexpr (!ALL)
+                if (live && P.words) live = (bits[c >> 5] >> (c & 31)) & 1u;
+            const unsigned mask = __ballot_sync(0xffffffffu, live);
+            const int count = __popc(mask);
+            if (live) packed[__popc(mask & ((1u << lane) - 1))] = make_uint2(ALL ? (unsigned) c * (CSR_PART * 4) : (unsigned) c, __float_as_uint(v));
+            __syncwarp();
+            int t = 0;
+            for (; t + 4 <= count; t += 4) {             // four panel rows in flight, added in storage order
+                const uint4 p01 = *reinterpret_cast<const uint4 *>(packed + t), p23 = *reinterpret_cast<const uint4 *>(packed + t + 2);
+                const float4 w0 = panel_row(p01.x), w1 = panel_row(p01.z), w2 = panel_row(p23.x), w3 = panel_row(p23.z);
+                add(acc, p01.y, w0); add(acc, p01.w, w1); add(acc, p23.y, w2); add(acc, p23.w, w3);
             }
-            // row 4 * lane + k (+ 128) sits in tile row 32 * k + lane (+ 128): a warp's stores hit 32 banks each
-            T[(0 * 32 + lane) * 33 + jj] = a0.x; T[(1 * 32 + lane) * 33 + jj] = a0.y;
-            T[(2 * 32 + lane) * 33 + jj] = a0.z; T[(3 * 32 + lane) * 33 + jj] = a0.w;
-            T[(4 * 32 + lane) * 33 + jj] = a1.x; T[(5 * 32 + lane) * 33 + jj] = a1.y;
-            T[(6 * 32 + lane) * 33 + jj] = a1.z; T[(7 * 32 + lane) * 33 + jj] = a1.w;
+            if (t < count) {
+                const uint2 e0 = packed[t], ea = packed[t + (t + 1 < count ? 1 : 0)], eb = packed[t + (t + 2 < count ? 2 : 0)];
+                const float4 w0 = panel_row(e0.x), w1 = panel_row(ea.x), w2 = panel_row(eb.x);
+                add(acc, e0.y, w0);
+                if (t + 1 < count) add(acc, ea.y, w1);
+                if (t + 2 < count) add(acc, eb.y, w2);
+            }
+            __syncwarp();
         }
-        __syncthreads();
-        // (the other buffer is written next; this one again only after the next barrier, which every warp
-        // reaches after it has read its rows here)
-        if (vec_ok && j0 + 32 <= n) {
-            // four consecutive instances of one row per thread, one 16-byte store: a warp covers four rows
-            const int jq = 4 * (lane & 7);
-            const float s0 = __shfl_sync(0xffffffffu, sdj, jq), s1 = __shfl_sync(0xffffffffu, sdj, jq + 1),
-                        s2 = __shfl_sync(0xffffffffu, sdj, jq + 2), s3 = __shfl_sync(0xffffffffu, sdj, jq + 3);
-#pragma unroll 2
-            for (int c = 4 * warp + (lane >> 3); c < mh; c += 4 * (CSR_SMEM_THREADS / 32)) {
-                const float *tr = T + ((((c >> 7) << 2) + (c & 3)) * 32 + ((c & 127) >> 2)) * 33 + jq;
-                const float sr = sdr_sm[c];
-                float4 o;
-                o.x = apply_kernel(fn, tr[0], sr, s0); o.y = apply_kernel(fn, tr[1], sr, s1);
-                o.z = apply_kernel(fn, tr[2], sr, s2); o.w = apply_kernel(fn, tr[3], sr, s3);
-                *reinterpret_cast<float4 *>(out + (size_t) orow_sm[c] * ld_out + j0 + jq) = o;
+        acc.x = csr_value<RBF>(fn, acc.x, sdr[0], s); acc.y = csr_value<RBF>(fn, acc.y, sdr[1], s);
+        acc.z = csr_value<RBF>(fn, acc.z, sdr[2], s); acc.w = csr_value<RBF>(fn, acc.w, sdr[3], s);
+        const int u = j & (unit - 1), first = j - u;
+        res[u * 33 + lane] = acc;
+        if (j1 != j + 1 || u + 1 == unit) {              // the last one of its unit: store them
+            const int have = u + 1;
+            __syncwarp();
+            if (vec_ok && have == 4) {
+                // a lane stores four instances of its four requested rows
+                const int4 o = reinterpret_cast<const int4 *>(orow_sm)[lane];
+                const float4 r0 = res[lane], r1 = res[33 + lane], r2 = res[66 + lane];
+                if (o.x >= 0) *reinterpret_cast<float4 *>(out + o.x * ld_out + first) = make_float4(r0.x, r1.x, r2.x, acc.x);
+                if (o.y >= 0) *reinterpret_cast<float4 *>(out + o.y * ld_out + first) = make_float4(r0.y, r1.y, r2.y, acc.y);
+                if (o.z >= 0) *reinterpret_cast<float4 *>(out + o.z * ld_out + first) = make_float4(r0.z, r1.z, r2.z, acc.z);
+                if (o.w >= 0) *reinterpret_cast<float4 *>(out + o.w * ld_out + first) = make_float4(r0.w, r1.w, r2.w, acc.w);
+            } else {
+                // a lane stores one value: the instances of a row next to each other
+                const int sh = unit == 4 ? 2 : unit - 1, w = lane & (unit - 1);
+                for (int r = lane >> sh; r < mh; r += 32 >> sh)
+                    if (w < have) out[orow_sm[r] * ld_out + first + w] = reinterpret_cast<const float *>(res)[w * 132 + r];
             }
-        } else {
-            const int j = j0 + lane;
-            for (int c = warp; c < mh; c += CSR_SMEM_THREADS / 32) {
-                const float dot = T[((((c >> 7) << 2) + (c & 3)) * 32 + ((c & 127) >> 2)) * 33 + lane];
-                if (j < n) out[(size_t) orow_sm[c] * ld_out + j] = apply_kernel(fn, dot, sdr_sm[c], sdj);
-            }
+            __syncwarp();
         }
+        j = j1; j1 = j2;
+        if (j >= n) return;
+        b = b1; e = e1; s = s1; b1 = b2; e1 = e2; s1 = s2;
+        cc = cc1; vv = vv1;
     }
 }
 
 // ---- host side ----------------------------------------------------------------------------------
 
-static tsvm_status ensure_scratch(tsvm_km *km, int m) {
-    if (m <= km->w_cap) return TSVM_OK;
+// Staging buffers for m requested rows: as rows in the operand form of the dense engines, or (panel) as the CSR engine's
+// panel.
+static tsvm_status ensure_scratch(tsvm_km *km, int m, bool panel) {
+    if (m <= (panel ? km->wt_ld : km->w_cap)) return TSVM_OK;
     int cap = 128;
     while (cap < m) cap *= 2;
-    pool_free_many({km->W, km->Whi, km->Wlo, km->WT, km->sd_rows, km->w_unscale});
-    km->W = km->Whi = km->Wlo = km->WT = km->sd_rows = km->w_unscale = nullptr;
-    km->w_cap = 0;
-    TSVM_TRY(dev_alloc(&km->sd_rows, (size_t) cap));
-    if (km->dense) {
+    if (cap > km->sd_cap) {
+        pool_free(km->sd_rows);
+        km->sd_rows = nullptr;
+        km->sd_cap = 0;
+        TSVM_TRY(dev_alloc(&km->sd_rows, (size_t) cap));
+        km->sd_cap = cap;
+    }
+    if (!panel) {
+        pool_free_many({km->W, km->Whi, km->Wlo, km->w_unscale});
+        km->W = km->Whi = km->Wlo = km->w_unscale = nullptr;
+        km->w_cap = 0;
         // either plane kind fits cap x d_pad words: round_up(d, 8) halves <= d_pad floats
         TSVM_TRY(dev_alloc(&km->w_unscale, (size_t) cap));
         TSVM_TRY(dev_alloc(&km->W, (size_t) cap * km->d_pad));
         TSVM_TRY(dev_alloc(&km->Whi, (size_t) cap * km->d_pad));
         TSVM_TRY(dev_alloc(&km->Wlo, (size_t) cap * km->d_pad));
-    } else {
-        km->wt_ld = cap;
-        TSVM_TRY(dev_alloc(&km->WT, (size_t) km->d * cap));
-        TSVM_CUDA(cudaMemset(km->WT, 0, sizeof(float) * (size_t) km->d * cap));
+        km->w_cap = cap;
+        return TSVM_OK;
     }
-    km->w_cap = cap;
+    pool_free_many({km->WT, km->csr_bits});
+    km->WT = nullptr;
+    km->csr_bits = nullptr;
+    km->wt_ld = 0;
+    TSVM_TRY(dev_alloc(&km->WT, (size_t) km->d * cap));
+    // (an allocation that other streams know nothing of: cleared and waited for here)
+    TSVM_CUDA(cudaMemset(km->WT, 0, sizeof(float) * (size_t) km->d * cap));
+    const size_t words = (size_t) csr_bitmap_words(km->d) * ceil_div(cap, CSR_PART);
+    TSVM_TRY(dev_alloc(&km->csr_bits, words));
+    TSVM_CUDA(cudaMemset(km->csr_bits, 0, sizeof(unsigned) * words));
+    TSVM_CUDA(cudaStreamSynchronize(nullptr));
+    km->wt_ld = cap;
     return TSVM_OK;
 }
 
@@ -858,8 +830,8 @@ static inline size_t row_dst_bytes(const RowDst &r, int m) {
 static tsvm_status finish_create(tsvm_km *km, cudaStream_t st) {
     TSVM_TRY(dev_alloc(&km->self_dot, (size_t) km->n));
     TSVM_TRY(dev_alloc(&km->diag, (size_t) km->n));
-    TSVM_TRY(dev_alloc(&km->status_dev, 4));
-    TSVM_TRY(pinned_alloc((void **) &km->status_host, 4 * sizeof(int)));
+    if (!km->status_dev) TSVM_TRY(dev_alloc(&km->status_dev, 4));
+    if (!km->status_host) TSVM_TRY(pinned_alloc((void **) &km->status_host, 4 * sizeof(int)));
     km->launched(st);
     if (!km->dense) {
         TSVM_LAUNCH(self_dot_csr_kernel, ceil_div((long long) km->n * 32, 256), 256, 0, st, km->val, km->row_ptr, km->n,
@@ -874,55 +846,35 @@ static tsvm_status finish_create(tsvm_km *km, cudaStream_t st) {
     return TSVM_OK;
 }
 
-// TSVM_CSR_SMEM=0 keeps the L2-panel engine for every CSR matrix (used to compare the two engines)
-static bool csr_smem_engine_allowed() {
+// TSVM_CSR_SMEM=0 leaves the panel in L2 (used to check that its place changes no result)
+static bool csr_smem_allowed() {
     static const bool on = [] { const char *e = getenv("TSVM_CSR_SMEM"); return !e || atoi(e) != 0; }();
     return on;
 }
 
-// A set of stored instances the CSR engines sweep: the kernel matrix's own, or a gathered subset of them.
-struct CsrView {
-    const float *val;
-    const int *row_ptr, *col;
-    int n;
-    const float *sd;                // self dots of the instances
-};
-
-// Kernel rows of the m requested rows staged in `panel` (feature-major, row stride km->wt_ld; self dots in
-// sd_rows) against the instances of X. spare_sms: SMs the persistent engine leaves free.
-static tsvm_status csr_engine_launch(tsvm_km *km, const CsrView &X, const float *panel, const float *sd_rows, int m,
-                                     float *out, long long ld_out, const int *m_dev, const int *row_slot, int spare_sms,
-                                     cudaStream_t st) {
-    if (km->d <= CSR_SMEM_MAX_D && csr_smem_engine_allowed()) {
-        // few features: the panel of 256 requested rows fits in shared memory
-        const size_t smem = ((size_t) km->d * CSR_SMEM_PART + 2 * CSR_SMEM_TILE) * sizeof(float);
-        TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute(csr_rows_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                            (int) (((size_t) CSR_SMEM_MAX_D * CSR_SMEM_PART + 2 * CSR_SMEM_TILE) * sizeof(float)))));
-        const int parts = ceil_div(m, CSR_SMEM_PART);
-        int sms = device_sm_count();
-        sms = sms - spare_sms > 0 ? sms - spare_sms : 1;
-        int bx = sms / parts > 0 ? sms / parts : 1;
-        const int n_tiles = ceil_div(X.n, 32);
-        if (bx > n_tiles) bx = n_tiles;
-        TSVM_LAUNCH(csr_rows_smem_kernel, dim3(bx, parts), CSR_SMEM_THREADS, smem, st, X.val, X.row_ptr, X.col, X.n, km->d,
-                    panel, km->wt_ld, m, X.sd, sd_rows, km->fn, out, ld_out, m_dev, row_slot);
-        return TSVM_OK;
-    }
-    const int nv = ceil_div(m, 128);
-    const int grid = ceil_div(X.n, 32);
-#define CSR_CASE(NV)                                                                                             \
-    {                                                                                                            \
-        size_t smem = (size_t) (NV) * 128 * 33 * sizeof(float);                                                  \
-        TSVM_CUDA(cudaFuncSetAttribute(csr_rows_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
-                                       (int) smem));                                                             \
-        TSVM_LAUNCH(csr_rows_kernel<NV>, grid, 256, smem, st, X.val, X.row_ptr, X.col, X.n, panel, km->wt_ld, m, \
-                    X.sd, sd_rows, km->fn, out, ld_out, m_dev, row_slot);                                        \
-    }
-    if (nv <= 1) CSR_CASE(1)
-    else if (nv <= 2) CSR_CASE(2)
-    else if (nv <= 4) CSR_CASE(4)
-    else if (nv <= 8) CSR_CASE(8)
-    else { set_error("CSR engine handles at most 1024 rows per call, got %d", m); return TSVM_ERR_INVALID; }
+// Kernel rows of the m requested rows staged in WT / sd_rows against all stored instances. with_bits: the staging filled
+// the bitmap.
+static tsvm_status csr_engine_launch(tsvm_km *km, int m, bool with_bits, float *out, long long ld_out, cudaStream_t st) {
+    TSVM_REQUIRE(m <= 1024, "CSR engine handles at most 1024 rows per call, got %d", m);
+    const bool all = csr_smem_allowed() && km->d <= (CSR_SMEM_MAX - CSR_FIXED_SMEM) / (CSR_PART * 4);
+    CsrPanel P;
+    P.WT = km->WT; P.ld = km->wt_ld; P.d = km->d;
+    P.words = with_bits && !all ? csr_bitmap_words(km->d) : 0;
+    P.bits = km->csr_bits;
+    const size_t smem = CSR_FIXED_SMEM + (all ? (size_t) km->d * CSR_PART * 4 : (size_t) P.words * 4);
+    const bool rbf = km->fn.type == TSVM_RBF || km->fn.type == TSVM_PRECOMPUTED;
+    const int per_sm = smem <= 112 * 1024 ? 2 : 1;
+    const int units = ceil_div(km->n, CSR_WARPS) * ceil_div(m, CSR_PART);
+    const int grid = device_sm_count() * per_sm < units ? device_sm_count() * per_sm : units;
+#define CSR_CASE(RBF, ALL)                                                                                                \
+    do {                                                                                                                  \
+        TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute((csr_rows_kernel<RBF, ALL>),                                  \
+                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, CSR_SMEM_MAX))); \
+        TSVM_LAUNCH((csr_rows_kernel<RBF, ALL>), grid, CSR_THREADS, smem, st, km->val, km->row_ptr, km->col, km->n, P, m, \
+                    km->self_dot, km->sd_rows, km->fn, out, ld_out, km->rows_m_dev, km->rows_slot_dev);                   \
+    } while (0)
+    if (rbf) { if (all) CSR_CASE(true, true); else CSR_CASE(true, false); }
+    else if (all) CSR_CASE(false, true); else CSR_CASE(false, false);
 #undef CSR_CASE
     return TSVM_OK;
 }
@@ -936,8 +888,7 @@ static tsvm_status rows_common(tsvm_km *km, int m, float *out, long long ld_out,
                     km->self_dot, km->sd_rows, km->fn, out, ld_out, km->rows_m_dev, km->rows_slot_dev);
         return TSVM_OK;
     }
-    return csr_engine_launch(km, CsrView{km->val, km->row_ptr, km->col, km->n, km->self_dot}, km->WT, km->sd_rows, m, out,
-                             ld_out, km->rows_m_dev, km->rows_slot_dev, 0, st);
+    return csr_engine_launch(km, m, true, out, ld_out, st);
 }
 
 // ---- pieces of tsvm_km_rows_by_index for callers that overlap them (the solver) -------------------
@@ -957,7 +908,7 @@ size_t km_plane_row_bytes(const tsvm_km *km) {
 }
 
 tsvm_status km_stage_rows_by_index(tsvm_km *km, const int *idx_dev, int q, cudaStream_t st) {
-    TSVM_TRY(ensure_scratch(km, q));
+    TSVM_TRY(ensure_scratch(km, q, false));
     TSVM_TRY(ensure_planes(km, st));
     TSVM_LAUNCH(gather_rows_dense_kernel, q, 256, 0, st, km->X, km->ldx, km->d, idx_dev, q, km->self_dot, row_dst(km),
                 km->sd_rows, km->rows_m_dev);
@@ -991,7 +942,7 @@ tsvm_status km_rows_planes_on(tsvm_km *km, const InstancePlanes &X, const RowPla
 // Stages m explicit feature rows (m x n_features, stride ldt) with their self dots as the requested rows.
 tsvm_status km_stage_rows_features(tsvm_km *km, const float *T_dev, int ldt, const float *sd_T_dev, int m,
                                    cudaStream_t st) {
-    TSVM_TRY(ensure_scratch(km, m));
+    TSVM_TRY(ensure_scratch(km, m, false));
     TSVM_TRY(ensure_planes(km, st));
     TSVM_CUDA(cudaMemcpyAsync(km->sd_rows, sd_T_dev, sizeof(float) * m, cudaMemcpyDeviceToDevice, st));
     TSVM_LAUNCH(stage_rows_dense_kernel, m, 256, 0, st, T_dev, ldt, km->d, km->d, m, row_dst(km));
@@ -1002,7 +953,7 @@ tsvm_status km_stage_rows_features(tsvm_km *km, const float *T_dev, int ldt, con
 // order as kernelmatrix.cpp:288-296 does, rows in the engine's operand form): the first half of
 // tsvm_km_rows_by_instances_*, shared with the fused prediction.
 tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt, int ldt, cudaStream_t st) {
-    TSVM_TRY(ensure_scratch(km, mm));
+    TSVM_TRY(ensure_scratch(km, mm, false));
     TSVM_TRY(launch_self_dot_seq_dense(T, mm, dt, ldt, km->sd_rows, st));
     TSVM_TRY(ensure_planes(km, st));
     TSVM_LAUNCH(stage_rows_dense_kernel, mm, 256, 0, st, T, ldt, dt, km->d, mm, row_dst(km));
@@ -1011,7 +962,7 @@ tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt
 
 tsvm_status km_stage_instances_csr(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int mm,
                                    cudaStream_t st) {
-    TSVM_TRY(ensure_scratch(km, mm));
+    TSVM_TRY(ensure_scratch(km, mm, false));
     TSVM_LAUNCH(self_dot_seq_csr_kernel, ceil_div(mm, 128), 128, 0, st, tval, rp, mm, km->sd_rows);
     TSVM_TRY(ensure_planes(km, st));
     const RowDst dst = row_dst(km);
@@ -1110,7 +1061,7 @@ void tsvm_km_destroy(tsvm_km *km) {
     if (!km) return;
     pool_free_many({km->X_owned, km->Xhi, km->Xlo, km->x_unscale, km->w_unscale, km->val_owned, km->row_ptr_owned,
                     km->col_owned, km->self_dot, km->diag, km->W, km->Whi, km->Wlo, km->WT, km->sd_rows,
-                    km->few_acc, km->status_dev}, !km->in_flight && !km->exposed);
+                    km->few_acc, km->csr_bits, km->status_dev}, !km->in_flight && !km->exposed);
     if (km->status_host) pinned_free(km->status_host);
     delete km;
 }
@@ -1150,7 +1101,7 @@ tsvm_status tsvm_km_rows_by_index(tsvm_km *km, const int *idx_dev, int q, float 
     TSVM_REQUIRE(km && idx_dev && out_dev && q > 0 && ld_out >= km->n, "rows_by_index: bad arguments (q=%d)", q);
     cudaStream_t st = (cudaStream_t) stream;
     km->launched(st);
-    TSVM_TRY(ensure_scratch(km, q));
+    TSVM_TRY(ensure_scratch(km, q, !km->dense));
     if (km->dense) {
         TSVM_TRY(ensure_planes(km, st));
         TSVM_LAUNCH(gather_rows_dense_kernel, q, 256, 0, st, km->X, km->ldx, km->d, idx_dev, q, km->self_dot,
@@ -1159,10 +1110,10 @@ tsvm_status tsvm_km_rows_by_index(tsvm_km *km, const int *idx_dev, int q, float 
     }
     TSVM_REQUIRE(q <= 1024, "CSR engine handles at most 1024 rows per call, got %d", q);
     TSVM_LAUNCH(scatter_csr_to_wt_kernel, q, 128, 0, st, km->val, km->row_ptr, km->col, idx_dev, q, km->d, km->wt_ld,
-                km->WT, km->self_dot, km->sd_rows, false, km->rows_m_dev);
+                km->WT, km->self_dot, km->sd_rows, false, km->rows_m_dev, km->csr_bits, csr_bitmap_words(km->d));
     TSVM_TRY(rows_common(km, q, out_dev, ld_out, st));
     TSVM_LAUNCH(scatter_csr_to_wt_kernel, q, 128, 0, st, km->val, km->row_ptr, km->col, idx_dev, q, km->d, km->wt_ld,
-                km->WT, nullptr, nullptr, true, km->rows_m_dev);
+                km->WT, nullptr, nullptr, true, km->rows_m_dev, km->csr_bits, csr_bitmap_words(km->d));
     return TSVM_OK;
 }
 
@@ -1172,21 +1123,22 @@ tsvm_status tsvm_km_rows_by_instances_dense(tsvm_km *km, const float *T_dev, int
                  "rows_by_instances_dense: bad arguments");
     cudaStream_t st = (cudaStream_t) stream;
     km->launched(st);
-    const int chunk = km->dense ? 4096 : 1024;
+    const bool dense = km->dense;
+    const int chunk = dense ? 4096 : 1024;
     for (int r0 = 0; r0 < m; r0 += chunk) {
         const int mm = min(chunk, m - r0);
         const float *T = T_dev + (size_t) r0 * ldt;
         float *o = out_dev + (size_t) r0 * ld_out;
-        if (km->dense) {
+        if (dense) {
             TSVM_TRY(km_stage_instances_dense(km, T, mm, dt, ldt, st));
             TSVM_TRY(rows_common(km, mm, o, ld_out, st));
         } else {
-            TSVM_TRY(ensure_scratch(km, mm));
+            TSVM_TRY(ensure_scratch(km, mm, true));
             TSVM_TRY(launch_self_dot_seq_dense(T, mm, dt, ldt, km->sd_rows, st));
             dim3 grid(ceil_div(km->d, 32), ceil_div(mm, 32)), block(32, 8);
             TSVM_LAUNCH(transpose_dense_to_wt_kernel, grid, block, 0, st, T, ldt, dt, km->d, mm, km->wt_ld, km->WT,
                         false);
-            TSVM_TRY(rows_common(km, mm, o, ld_out, st));
+            TSVM_TRY(csr_engine_launch(km, mm, false, o, ld_out, st));
             TSVM_LAUNCH(transpose_dense_to_wt_kernel, grid, block, 0, st, T, ldt, dt, km->d, mm, km->wt_ld, km->WT,
                         true);
         }
@@ -1202,7 +1154,7 @@ tsvm_status tsvm_km_rows_for_features_dense(tsvm_km *km, const float *T_dev, int
     km->launched(st);
     for (int r0 = 0; r0 < m; r0 += 4096) {
         const int mm = min(4096, m - r0);
-        TSVM_TRY(ensure_scratch(km, mm));
+        TSVM_TRY(ensure_scratch(km, mm, false));
         TSVM_CUDA(cudaMemcpyAsync(km->sd_rows, sd_T_dev + r0, sizeof(float) * mm, cudaMemcpyDeviceToDevice, st));
         TSVM_TRY(ensure_planes(km, st));
         TSVM_LAUNCH(stage_rows_dense_kernel, mm, 256, 0, st, T_dev + (size_t) r0 * ldt, ldt, km->d, km->d, mm,
@@ -1219,22 +1171,25 @@ tsvm_status tsvm_km_rows_by_instances_csr(tsvm_km *km, const float *tval_dev, co
     TSVM_REQUIRE(km && trow_ptr_dev && out_dev && m > 0 && ld_out >= km->n, "rows_by_instances_csr: bad arguments");
     cudaStream_t st = (cudaStream_t) stream;
     km->launched(st);
-    const int chunk = km->dense ? 4096 : 1024;
+    const bool dense = km->dense;
+    const int chunk = dense ? 4096 : 1024;
     for (int r0 = 0; r0 < m; r0 += chunk) {
         const int mm = min(chunk, m - r0);
         const int *rp = trow_ptr_dev + r0;     // row_ptr entries stay absolute offsets into tval/tcol
         float *o = out_dev + (size_t) r0 * ld_out;
-        if (km->dense) {
+        if (dense) {
             TSVM_TRY(km_stage_instances_csr(km, tval_dev, rp, tcol_dev, mm, st));
             TSVM_TRY(rows_common(km, mm, o, ld_out, st));
         } else {
-            TSVM_TRY(ensure_scratch(km, mm));
+            TSVM_TRY(ensure_scratch(km, mm, true));
             TSVM_LAUNCH(self_dot_seq_csr_kernel, ceil_div(mm, 128), 128, 0, st, tval_dev, rp, mm, km->sd_rows);
             TSVM_LAUNCH(scatter_csr_to_wt_kernel, mm, 128, 0, st, tval_dev, rp, tcol_dev, (const int *) nullptr, mm,
-                        km->d, km->wt_ld, km->WT, (const float *) nullptr, (float *) nullptr, false, (const int *) nullptr);
-            TSVM_TRY(rows_common(km, mm, o, ld_out, st));
+                        km->d, km->wt_ld, km->WT, (const float *) nullptr, (float *) nullptr, false, (const int *) nullptr, km->csr_bits,
+                        csr_bitmap_words(km->d));
+            TSVM_TRY(csr_engine_launch(km, mm, true, o, ld_out, st));
             TSVM_LAUNCH(scatter_csr_to_wt_kernel, mm, 128, 0, st, tval_dev, rp, tcol_dev, (const int *) nullptr, mm,
-                        km->d, km->wt_ld, km->WT, (const float *) nullptr, (float *) nullptr, true, (const int *) nullptr);
+                        km->d, km->wt_ld, km->WT, (const float *) nullptr, (float *) nullptr, true, (const int *) nullptr, km->csr_bits,
+                        csr_bitmap_words(km->d));
         }
     }
     return TSVM_OK;

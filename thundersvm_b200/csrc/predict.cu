@@ -80,7 +80,7 @@ __global__ void sv_class_kernel(int *__restrict__ cls, int n_sv, const int *__re
 }
 
 // votes -> index of the winning class, first maximum wins. One warp per row: the signs of the row's decision values are
-// packed into words (coalesced reads), then every lane counts the votes of its classes. 4,096 rows of ten classes: 25 -> 3 us
+// packed into words (coalesced reads), then every lane counts the votes of its classes. 4,096 rows of ten classes: 25 -> 3.5 us
 // against one thread per row.
 constexpr int VOTE_WARPS = 8, VOTE_WORDS = 256;            // at most 8,192 pairs
 __global__ void __launch_bounds__(VOTE_WARPS * 32)
