@@ -147,3 +147,40 @@ def test_prediction_of_few_rows(capi, m, storage, nc, n_sv, d, kernel):
         lab = capi.predict_labels(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, **batch)
         assert np.array_equal(lab.cpu().numpy(), capi.vote(dec, nc).cpu().numpy())
     km.close()
+
+
+@pytest.mark.parametrize("d,fill,values", [(33, 0.3, "ones"), (256, 0.01, "ones"), (257, 0.01, "ones"), (300, 0.1, "halves"),
+                                           (120, 0.1, "thirds"), (120, 0.1, "large"), (120, 0.1, "descending")])
+@pytest.mark.parametrize("batch", ["ones", "thirds"])
+def test_sparse_data_worked_on_as_dense_rows(capi, d, fill, values, batch):
+    """CSR data that one FP16 number per entry holds exactly may go through the dense engine: the first and the last
+    feature count, a fill below the line, values and orders of the entries that rule it out, batches that do. Kernel
+    rows by index and by instance, decision values of 200 rows (more than the few-row launch takes)."""
+    rng = np.random.default_rng(d)
+
+    def csr(n, width, kind):
+        nz = rng.random((n, width)) < fill
+        rp = np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32)
+        col = np.nonzero(nz)[1].astype(np.int32)
+        v = rng.integers(1, 8, len(col)).astype(np.float32)
+        v = {"halves": v * 0.5, "thirds": v / 3, "large": v * 100}.get(kind, np.ones(len(col))).astype(np.float32)
+        if kind == "descending":
+            for i in range(n):
+                col[rp[i]:rp[i + 1]] = col[rp[i]:rp[i + 1]][::-1].copy()
+        return v, rp, col
+
+    n, m, gamma = 301, 200, 0.05 if values != "large" else 1e-6
+    sv, t = csr(n, d, values), csr(m, d + 5, batch)
+    km = capi.KernelMatrix(csr=tuple(map(_t, sv)), d=d, gamma=gamma)
+    assert not km.is_dense
+    ids = rng.choice(n, 130, replace=False).astype(np.int32)
+    want = P.kernel_rows_idx(P.Csr(csr=sv, d=d), ids, gamma=gamma)
+    assert np.max(np.abs(km.get_rows(_t(ids)).cpu().numpy() - want)) < 1e-5
+    want = P.kernel_rows_ins(P.Csr(csr=sv, d=d), P.Csr(csr=t, d=d + 5), gamma=gamma)
+    assert np.max(np.abs(km.get_rows_instances(csr=tuple(map(_t, t))).cpu().numpy() - want)) < 1e-5
+    cnt = np.array([100, 150, 51], np.int32)
+    coef, rho = rng.standard_normal((2, n)), rng.standard_normal(3)
+    want = P.predict_dec(P.Csr(csr=sv, d=d), coef.reshape(-1), cnt, rho, 3, P.Csr(csr=t, d=d + 5), gamma=gamma)
+    dec = capi.predict_dec(km, _t(coef.reshape(-1)), cnt, _t(rho), 3, csr=tuple(map(_t, t)))
+    assert np.max(np.abs(dec.cpu().numpy() - want)) < 1e-4 * max(1.0, np.max(np.abs(want)))
+    km.close()

@@ -190,6 +190,7 @@ struct tsvm_km {
     int n = 0, d = 0;
     long long nnz = 0;
     bool dense = true;
+    bool from_csr = false;          // X is a copy made of CSR data, which stays next to it
     tsvm::KernelFn fn{};
     // 0 = automatic, 1 = CUDA-core FP32, 2 = tcgen05 TF32 planes single CTA, 3 = tcgen05 TF32 planes CTA pairs,
     // 4 = tcgen05 row-scaled FP16 planes CTA pairs
@@ -245,6 +246,8 @@ struct tsvm_km {
 namespace tsvm {
 // Pieces of tsvm_km_rows_by_index (km.cu) for callers that overlap them with other work.
 bool km_pair_engine(tsvm_km *km, cudaStream_t st);
+tsvm_status km_pair_engine_takes(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int m, cudaStream_t st,
+                                 bool *takes);
 bool km_automatic_engine(const tsvm_km *km);
 size_t km_plane_row_bytes(const tsvm_km *km);
 tsvm_status km_stage_rows_by_index(tsvm_km *km, const int *idx_dev, int q, cudaStream_t st);

@@ -432,6 +432,47 @@ __global__ void stage_rows_dense_kernel(const float *__restrict__ T, int ldt, in
     }
 }
 
+// Which storage CSR data is worked on in. With at least CSR_DENSE_SHARE of the entries present (or at most 256 features)
+// the tensor-core engine needs less time for whole rows than the CSR engine for the entries: 512 rows of 32,561 instances,
+// 14 of 123 features set, take 103 us with the entries and 51 us as dense rows; predicting 16,281 rows with 12,001 of
+// them 1.7 and 0.53 ms. That engine splits a value into two FP16 planes, so the rule asks for data that one FP16 number
+// holds exactly (one-hot and binary features, small counts): the products are exact and nothing is rounded that the CSR
+// engine does not round. The features of a row also have to be strictly ascending: one that occurs twice counts twice
+// in the CSR engine. Below 33 features dense rows run on CUDA cores.
+constexpr double CSR_DENSE_SHARE = 0.02;
+constexpr int CSR_DENSE_MIN_D = 33, CSR_DENSE_ANY_D = 256, CSR_DENSE_MAX_D = 4096;
+
+// out[0] = 1 if some entry rules the dense form out, out[1] = row_ptr[n] (both zeroed before). batch: rows to predict,
+// staged by assignment and cut at d in either form, so only their values count.
+__global__ void inspect_entries_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr,
+                                       const int *__restrict__ col, int n, int d, bool batch, int *__restrict__ out) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[1] = row_ptr[n];
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    bool bad = false;
+    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < n && !bad; row += gridDim.x * wpb) {
+        const int b = row_ptr[row], e = row_ptr[row + 1];
+        for (int p = b + lane; p < e; p += 32) {
+            const float v = val[p], a = fabsf(v);
+            // 2^-10 .. 2^5: inside one row's scaling every such value keeps its eleven bits
+            const bool exact = v == 0.0f || (a >= 0.0009765625f && a <= 32.0f && __half2float(__float2half_rn(v)) == v);
+            bad |= !exact || (!batch && (col[p] < 0 || col[p] >= d || (p > b && col[p - 1] >= col[p])));
+        }
+        bad = __any_sync(0xffffffffu, bad);
+    }
+    if (bad && lane == 0) out[0] = 1;
+}
+
+__global__ void dense_from_csr_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr,
+                                      const int *__restrict__ col, int n, int ld, float *__restrict__ X) {
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < n; row += gridDim.x * wpb) {
+        float *x = X + (size_t) row * ld;
+        for (int k = lane; k < ld; k += 32) x[k] = 0.0f;
+        __syncwarp();
+        for (int p = row_ptr[row] + lane; p < row_ptr[row + 1]; p += 32) x[col[p]] = val[p];
+    }
+}
+
 // CSR rows -> zero-initialised dense rows for the dense engines.
 __global__ void scatter_csr_to_w_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr,
                                         const int *__restrict__ col, const int *__restrict__ idx, int m, int d,
@@ -827,6 +868,37 @@ static inline size_t row_dst_bytes(const RowDst &r, int m) {
     return (size_t) m * r.ld * (r.kind == 2 ? sizeof(__half) : sizeof(float));
 }
 
+static tsvm_status inspect_entries(tsvm_km *km, const float *val, const int *row_ptr, const int *col, int n, bool batch,
+                                   cudaStream_t st, bool *exact) {
+    int *found = km->status_dev + 2;                     // (the first word is the engines' status)
+    TSVM_CUDA(cudaMemsetAsync(found, 0, 2 * sizeof(int), st));
+    TSVM_LAUNCH(inspect_entries_kernel, prepare_grid(n), 256, 0, st, val, row_ptr, col, n, km->d, batch, found);
+    TSVM_CUDA(cudaMemcpyAsync(km->status_host + 2, found, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    TSVM_CUDA(cudaStreamSynchronize(st));
+    *exact = km->status_host[2] == 0;
+    return TSVM_OK;
+}
+
+// Makes the dense copy of CSR data whose kernel rows the tensor-core engine computes faster and as exactly.
+static tsvm_status choose_csr_storage(tsvm_km *km, cudaStream_t st) {
+    const int d_pad = (km->d + 3) & ~3;
+    const double dense_bytes = (double) km->n * d_pad * 8.0;             // the rows and their two planes
+    if (km->d < CSR_DENSE_MIN_D || km->d > CSR_DENSE_MAX_D || dense_bytes > device_memory_bytes() / 8.0) return TSVM_OK;
+    TSVM_TRY(dev_alloc(&km->status_dev, 4));
+    TSVM_TRY(pinned_alloc((void **) &km->status_host, 4 * sizeof(int)));
+    km->launched(st);
+    bool exact = false;
+    TSVM_TRY(inspect_entries(km, km->val, km->row_ptr, km->col, km->n, false, st, &exact));
+    km->nnz = km->status_host[3];
+    if (!exact || (km->d > CSR_DENSE_ANY_D && km->nnz < CSR_DENSE_SHARE * (double) km->n * km->d)) return TSVM_OK;
+    TSVM_TRY(dev_alloc(&km->X_owned, (size_t) km->n * d_pad));
+    TSVM_LAUNCH(dense_from_csr_kernel, prepare_grid(km->n), 256, 0, st, km->val, km->row_ptr, km->col, km->n, d_pad, km->X_owned);
+    km->X = km->X_owned;
+    km->ldx = km->d_pad = d_pad;
+    km->dense = km->from_csr = true;
+    return TSVM_OK;
+}
+
 static tsvm_status finish_create(tsvm_km *km, cudaStream_t st) {
     TSVM_TRY(dev_alloc(&km->self_dot, (size_t) km->n));
     TSVM_TRY(dev_alloc(&km->diag, (size_t) km->n));
@@ -960,6 +1032,18 @@ tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt
     return TSVM_OK;
 }
 
+// Can this batch go through the fused prediction? Where the matrix is the dense copy of CSR data, only if the engine's
+// operand form holds the batch exactly too.
+tsvm_status km_pair_engine_takes(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int m, cudaStream_t st,
+                                 bool *takes) {
+    *takes = km_pair_engine(km, st);
+    if (*takes && km->from_csr) {
+        *takes = false;
+        if (rp) TSVM_TRY(inspect_entries(km, tval, rp, tcol, m, true, st, takes));
+    }
+    return TSVM_OK;
+}
+
 tsvm_status km_stage_instances_csr(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int mm,
                                    cudaStream_t st) {
     TSVM_TRY(ensure_scratch(km, mm, false));
@@ -1051,6 +1135,7 @@ tsvm_status tsvm_km_create_csr(const float *val, const int *row_ptr, const int *
         }
         km->val = km->val_owned; km->col = km->col_owned; km->row_ptr = km->row_ptr_owned;
     }
+    if (s == TSVM_OK) s = choose_csr_storage(km, st);
     if (s == TSVM_OK) s = finish_create(km, st);
     if (s != TSVM_OK) { tsvm_km_destroy(km); return s; }
     *out = km;
@@ -1078,7 +1163,7 @@ long long tsvm_km_nnz(const tsvm_km *km) {
     }
     return last;
 }
-int tsvm_km_is_dense(const tsvm_km *km) { return km && km->dense; }
+int tsvm_km_is_dense(const tsvm_km *km) { return km && km->dense && !km->from_csr; }
 const float *tsvm_km_diag_dev(const tsvm_km *km) {
     if (!km) return nullptr;
     const_cast<tsvm_km *>(km)->exposed = true;      // the caller's own work may read it until the handle is destroyed
@@ -1092,6 +1177,7 @@ const float *tsvm_km_self_dot_dev(const tsvm_km *km) {
 
 tsvm_status tsvm_km_set_dense_engine(tsvm_km *km, int engine) {
     TSVM_REQUIRE(km && engine >= 0 && engine <= 4, "set_dense_engine: bad arguments");
+    if (km->from_csr) return TSVM_OK;        // the choice concerns matrices that were given as dense ones
     km->engine = engine;
     return TSVM_OK;
 }
@@ -1123,7 +1209,7 @@ tsvm_status tsvm_km_rows_by_instances_dense(tsvm_km *km, const float *T_dev, int
                  "rows_by_instances_dense: bad arguments");
     cudaStream_t st = (cudaStream_t) stream;
     km->launched(st);
-    const bool dense = km->dense;
+    const bool dense = km->dense && !km->from_csr;       // (any values may come: entries of the matrix x panel of the batch)
     const int chunk = dense ? 4096 : 1024;
     for (int r0 = 0; r0 < m; r0 += chunk) {
         const int mm = min(chunk, m - r0);
@@ -1148,7 +1234,7 @@ tsvm_status tsvm_km_rows_by_instances_dense(tsvm_km *km, const float *T_dev, int
 
 tsvm_status tsvm_km_rows_for_features_dense(tsvm_km *km, const float *T_dev, int ldt, const float *sd_T_dev, int m,
                                             float *out_dev, long long ld_out, void *stream) {
-    TSVM_REQUIRE(km && km->dense && T_dev && sd_T_dev && out_dev && m > 0 && ldt >= km->d && ld_out >= km->n,
+    TSVM_REQUIRE(km && km->dense && !km->from_csr && T_dev && sd_T_dev && out_dev && m > 0 && ldt >= km->d && ld_out >= km->n,
                  "rows_for_features_dense: bad arguments (dense kernel matrix required)");
     cudaStream_t st = (cudaStream_t) stream;
     km->launched(st);
@@ -1171,7 +1257,7 @@ tsvm_status tsvm_km_rows_by_instances_csr(tsvm_km *km, const float *tval_dev, co
     TSVM_REQUIRE(km && trow_ptr_dev && out_dev && m > 0 && ld_out >= km->n, "rows_by_instances_csr: bad arguments");
     cudaStream_t st = (cudaStream_t) stream;
     km->launched(st);
-    const bool dense = km->dense;
+    const bool dense = km->dense && !km->from_csr;       // (any values may come: entries of the matrix x panel of the batch)
     const int chunk = dense ? 4096 : 1024;
     for (int r0 = 0; r0 < m; r0 += chunk) {
         const int mm = min(chunk, m - r0);

@@ -185,12 +185,13 @@ static tsvm_status predict_few(tsvm_km *km, const double *coef_dev, const int *s
                                const int *trow_ptr_dev, const int *tcol_dev, long long tnnz, double *dec_dev, int *labels_dev,
                                cudaStream_t st, bool *taken) {
     *taken = false;
+    const bool dense = km->dense && !km->from_csr;      // few rows: the entries are read once, and there are fewer of them
     const int R = m == 1 ? 1 : (m == 2 ? 2 : (m <= 4 ? 4 : 8)), tiles = ceil_div(m, R);
-    if (n_classes > FEW_CLASSES || tiles > FEW_TILES || (km->dense && !km_automatic_engine(km))) return TSVM_OK;
-    const double per_sv = km->dense ? (double) km->d_pad : (double) km->nnz / km->n;
+    if (n_classes > FEW_CLASSES || tiles > FEW_TILES || (dense && !km_automatic_engine(km))) return TSVM_OK;
+    const double per_sv = dense ? (double) km->d_pad : (double) km->nnz / km->n;
     if (tiles > 1 && (double) tiles * km->n * (km->nnz < 0 ? 64.0 : per_sv) > 1.6e7) return TSVM_OK;
     const int n_pairs = n_classes * (n_classes - 1) / 2;
-    if (km->dense) {
+    if (dense) {
         if (sizeof(float) * (size_t) R * km->d_pad + FewShared<8>::bytes(n_pairs) > 190 * 1024) return TSVM_OK;
     } else if (T_dev || tnnz <= 0 || tnnz > FEW_ENTRIES) return TSVM_OK;
     const size_t need = (size_t) FEW_TILES * 8 * n_pairs + FEW_TILES;
@@ -203,7 +204,7 @@ static tsvm_status predict_few(tsvm_km *km, const double *coef_dev, const int *s
         km->few_cap = need;
     }
     FewArgs a;
-    a.X = km->dense ? km->X : nullptr; a.ldx = km->ldx; a.val = km->val; a.row_ptr = km->row_ptr; a.col = km->col;
+    a.X = dense ? km->X : nullptr; a.ldx = km->ldx; a.val = km->val; a.row_ptr = km->row_ptr; a.col = km->col;
     a.n_sv = km->n; a.d = km->d; a.sd_sv = km->self_dot;
     a.T = T_dev; a.dt = dt; a.ldt = ldt; a.tval = tval_dev; a.trow_ptr = trow_ptr_dev; a.tcol = tcol_dev; a.m = m;
     a.fn = km->fn; a.coef = coef_dev; a.rho = rho_dev; a.n_classes = n_classes; a.n_pairs = n_pairs;
@@ -213,10 +214,10 @@ static tsvm_status predict_few(tsvm_km *km, const double *coef_dev, const int *s
     a.acc = km->few_acc; a.ticket = reinterpret_cast<int *>(km->few_acc + km->few_cap - FEW_TILES);
     a.dec = dec_dev; a.labels = labels_dev; a.overflow = km->status_host + 1;
     km->status_host[1] = 0;
-    if (R == 1) TSVM_TRY(launch_few<1>(a, !km->dense, st));
-    else if (R == 2) TSVM_TRY(launch_few<2>(a, !km->dense, st));
-    else if (R == 4) TSVM_TRY(launch_few<4>(a, !km->dense, st));
-    else TSVM_TRY(launch_few<8>(a, !km->dense, st));
+    if (R == 1) TSVM_TRY(launch_few<1>(a, !dense, st));
+    else if (R == 2) TSVM_TRY(launch_few<2>(a, !dense, st));
+    else if (R == 4) TSVM_TRY(launch_few<4>(a, !dense, st));
+    else TSVM_TRY(launch_few<8>(a, !dense, st));
     TSVM_CUDA(cudaStreamSynchronize(st));
     *taken = *(volatile int *) (km->status_host + 1) == 0;
     return TSVM_OK;
@@ -238,7 +239,8 @@ static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const in
                          tcol_dev, tnnz, dec_dev, labels_dev, st, &taken));
     if (taken) { km_sv->waited(st); return TSVM_OK; }
     const int nb = n_classes * (n_classes - 1) / 2;
-    const bool fused = km_pair_engine(km_sv, st);
+    bool fused = false;
+    TSVM_TRY(km_pair_engine_takes(km_sv, T_dev ? nullptr : tval_dev, T_dev ? nullptr : trow_ptr_dev, tcol_dev, m, st, &fused));
     const long long ldk = ((long long) n_sv + 3) & ~3ll;
     long long batch = FUSED_ROWS;
     if (!fused) {

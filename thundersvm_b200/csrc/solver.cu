@@ -1472,7 +1472,7 @@ struct tsvm_shard {
     }
 
     tsvm_status init() {
-        TSVM_REQUIRE(km_pair_engine(km, st), "shard solver: needs dense data on the CTA-pair tensor engine "
+        TSVM_REQUIRE(!km->from_csr && km_pair_engine(km, st), "shard solver: needs dense data on the CTA-pair tensor engine "
                                              "(more than 32 features)");
         km->launched(st);
         km->streams_mixed = true;        // (this solver's two streams; its calls do not note their work on the matrix one by one)
