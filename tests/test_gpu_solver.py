@@ -172,6 +172,24 @@ def test_update_f_matches_oracle(capi, n, ws):
     assert np.allclose(got, exp, rtol=0, atol=1e-11)
 
 
+@pytest.mark.parametrize("n", [1, 33, 28288, 28289, 28420, 60003])
+@pytest.mark.parametrize("ws,nonzero", [(1, 1), (8, 7), (128, 128), (130, 129), (1024, 1000), (512, 0)])
+def test_update_f_runs_and_tiles(capi, n, ws, nonzero):
+    """Runs of rows shorter and longer than the loads in flight, empty runs; the last size in 32-column blocks, the first
+    in 128-column ones (with 148 SMs), more tiles than blocks, rows that are not 16-byte aligned. Column 0 must have the same
+    bits whatever the form."""
+    rng = np.random.default_rng(n + ws)
+    rows = rng.random((ws, (n + 3) // 4 * 4), dtype=np.float32)
+    ad = np.zeros(ws)
+    ad[rng.choice(ws, nonzero, replace=False)] = rng.standard_normal(nonzero)
+    f = rng.standard_normal(n)
+    exp = P.update_f(f, ad, np.ascontiguousarray(rows[:, :n]))
+    got = [capi.update_f(_t(f), _t(ad), _t(rows)).cpu().numpy(), capi.update_f(_t(f), _t(ad), _t(rows[:, :n])).cpu().numpy(),
+           capi.update_f(_t(f[:1]), _t(ad), _t(rows[:, :1])).cpu().numpy()]
+    assert np.allclose(got[0], exp, rtol=0, atol=1e-11)
+    assert np.array_equal(got[0], got[1]) and got[0][0] == got[2][0]
+
+
 CASES = {"c1": (lambda: synth.config1(1500), None, None), "c1_soft": (lambda: dict(synth.config1(1500), gamma=0.025), None, None),
          "c2": (lambda: synth.config2(1200), None, None), "c2_dense": (lambda: synth.config2(1200), None, "dense"),
          "c3": (lambda: synth.config3(900), 5, None), "c4": (lambda: synth.config4(700), None, None),
