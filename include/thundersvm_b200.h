@@ -130,7 +130,7 @@ typedef struct {
     long long local_iters;      /* "total local iter"                                        */
     double final_diff;          /* last diff[0] (global maximal violation)                   */
     double objective;           /* calculate_obj, csmosolver.cpp:227-239 (before nu scaling) */
-    double seconds_select;      /* host-observed phase times, seconds                        */
+    double seconds_select;      /* device-observed phase times, seconds                      */
     double seconds_rows;
     double seconds_local;
     double seconds_update;

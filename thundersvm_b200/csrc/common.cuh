@@ -91,6 +91,17 @@ inline int ceil_div(long long a, long long b) { return (int) ((a + b - 1) / b); 
 
 // ---- device helpers ------------------------------------------------------------------
 
+__device__ __forceinline__ long long device_ns() {
+    long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// When the phases of an outer iteration began and ended (device_ns), noted by the kernels themselves: timing events between
+// launches delay the next kernel by 3 - 4 us each, seven of them took 25 of the 370 us of an iteration at 10,000 x 20.
+struct PhaseTimes {
+    long long select_begin, select_end, rows_end, local_begin, local_end, update_begin;
+};
+
 // Monotone map double -> uint64 (ascending); -0.0 is folded onto +0.0 so that equal values
 // get equal keys.
 __host__ __device__ __forceinline__ unsigned long long ordered_key(double v) {
@@ -226,6 +237,7 @@ struct tsvm_km {
     // requested rows is read from the device (at most the q of the call) and requested row i goes to row
     // rows_slot_dev[i] of the output buffer instead of row i.
     const int *rows_m_dev = nullptr, *rows_slot_dev = nullptr;
+    long long *rows_end_dev = nullptr;  // where the pair engine notes when it ended, if anyone asks
     double *few_acc = nullptr;      // predict_few: sums of a call (zero between calls), and the tickets behind them
     size_t few_cap = 0;             // doubles in few_acc
     int *status_dev = nullptr;      // device status word written by kernels with bounded waits

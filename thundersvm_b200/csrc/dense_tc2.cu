@@ -149,6 +149,7 @@ struct PredictArgs {
 struct RowsExtra {
     const int *m_dev;
     const int *row_slot;
+    long long *end;                 // device_ns() when the last block left (never taken back), or nullptr
 };
 
 __device__ __forceinline__ int pair_index(int n_classes, int i, int j) {      // i < j, pairs ordered (0,1),(0,2),...
@@ -536,8 +537,8 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     }
 
     if (*abort_flag) {
-        const long long t0 = global_ns();
-        while (global_ns() - t0 < 1000000ll) __nanosleep(1000);
+        const long long t0 = device_ns();
+        while (device_ns() - t0 < 1000000ll) __nanosleep(1000);
     }
     tc_fence_before();
     __syncthreads();
@@ -545,6 +546,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     tc_fence_after();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    if (threadIdx.x == 0 && ex.end) atomicMax(ex.end, device_ns());
     if (threadIdx.x == 0 && *abort_flag) *(volatile int *) status = *abort_flag;      // (may be a word of pinned host memory)
 }
 
@@ -618,7 +620,7 @@ static tsvm_status launch_pair_any(tsvm_km *km, const InstancePlanes &X, const R
 // (kind 1 = TF32 words, 2 = row-scaled FP16, the handle's plane kind), self dots and 1/scale.
 tsvm_status launch_dense_tc2_planes(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
                                     long long ld_out, cudaStream_t st) {
-    return launch_pair_any<false>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev}, st);
+    return launch_pair_any<false>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, km->rows_end_dev}, st);
 }
 
 // Prediction form: the m staged rows are test rows, the kernel matrix holds the support vectors; adds
@@ -628,7 +630,7 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
     const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
     const RowPlanes staged{km->Whi, km->Wlo, km->sd_rows, km->w_unscale};
     const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, n_classes, n_classes * (n_classes - 1) / 2};
-    return launch_pair_any<true>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr}, st);
+    return launch_pair_any<true>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, nullptr}, st);
 }
 
 // Requested rows = the m rows staged in the handle's scratch.

@@ -156,7 +156,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                  const int *__restrict__ y_ws, const double *__restrict__ f_ws, double *__restrict__ alpha_ws,
                  double *__restrict__ alpha_diff, double Cp_in, double Cn_in, double eps, int max_iter,
                  double *__restrict__ diff, const int *__restrict__ ids, double *__restrict__ alpha_global,
-                 const int *__restrict__ stop, int use_ring) {
+                 const int *__restrict__ stop, int use_ring, PhaseTimes *times) {
     using namespace smo;
     constexpr int W = T / 32, CLS = NU ? 2 : 1;             // nu: the lists of I_up and I_low are split by class
     constexpr bool AHEAD = !NU;                             // (nu reads two rows i and guesses j badly: 5 % slower with the ring)
@@ -164,6 +164,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         for (int t = threadIdx.x; t < ws; t += T + 32) alpha_diff[t] = 0;
         return;
     }
+    if (times && threadIdx.x == 0) times->local_begin = device_ns();
     __shared__ double f_sm[S * T], a_sm[S * T];
     __shared__ float kd_sm[S * T];
     __shared__ int y_sm[S * T];
@@ -493,7 +494,10 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
             if (alpha_global && ids[t] >= 0) alpha_global[ids[t]] = a;
         }
     }
-    if (tid == 0) diff[1] = it;
+    if (tid == 0) {
+        diff[1] = it;
+        if (times) times->local_end = device_ns();
+    }
 }
 
 }  // namespace tsvm

@@ -504,6 +504,7 @@ struct SelectArgs {
     int *sorted_id;
     int *out_ids, *out_count;           // the merged selection, or nullptr: the sorted lists are the result
     const int *stop;                    // optional: when *stop is non-zero the whole launch is a no-op
+    PhaseTimes *times;                  // optional
 };
 
 // Resolves one 12-bit digit of every active list from histograms of 4,096 bins each (threads 256 l .. 256 l + 255 own list
@@ -756,6 +757,7 @@ __global__ void __launch_bounds__(SELECT_THREADS, 1) select_kernel(const SelectA
     // written by an earlier launch only: every thread of every block reads the same value and leaves before
     // the first grid barrier
     if (a.stop && *a.stop) return;
+    if (a.times && blockIdx.x == 0 && tid == 0) a.times->select_begin = device_ns();
 
     sample_pivots(a, lists, pv, select_smem);
     collect_candidates(a, lists, pv);

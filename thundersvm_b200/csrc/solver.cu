@@ -9,6 +9,7 @@
 #include <limits.h>
 #include <string.h>
 #include <stdlib.h>
+#include <sched.h>
 #include <dlfcn.h>
 #include <mutex>
 #include <vector>
@@ -27,8 +28,10 @@ __global__ void gather_ws_kernel(int ws, int q, int first_half_phys, const int *
                                  const int *__restrict__ y, const double *__restrict__ f,
                                  const double *__restrict__ alpha, float *__restrict__ kww,
                                  float *__restrict__ diag_ws, int *__restrict__ y_ws, double *__restrict__ f_ws,
-                                 double *__restrict__ alpha_ws, int block_rows, const int *__restrict__ row_slot) {
+                                 double *__restrict__ alpha_ws, int block_rows, const int *__restrict__ row_slot,
+                                 PhaseTimes *times) {
     const int a = blockIdx.x;                      // logical slot of the row
+    if (times && a == 0 && threadIdx.x == 0) times->rows_end = device_ns();
     // rows >= block_rows of the block are written by someone else (the overlapped iteration computes them
     // directly); the slot vectors are gathered for every slot
     // a slot without an instance (id -1: fewer eligible instances than slots) is inert: y = 0 puts it in no set
@@ -74,7 +77,7 @@ cache_assign_kernel(const int *__restrict__ ids, int t0, int n_new, int now, int
                     int *__restrict__ inst_of, int *__restrict__ stamp, int cap,
                     const int *__restrict__ row_slot_before, int *__restrict__ row_slot,
                     int *__restrict__ miss_ids, int *__restrict__ miss_slot, int *__restrict__ victims,
-                    long long *__restrict__ ctr, int row_block, const int *__restrict__ stop) {
+                    long long *__restrict__ ctr, int row_block, const int *__restrict__ stop, PhaseTimes *times) {
     if (stop && *stop) {            // queued past the end of a solve: no member changes, no row to compute
         if (threadIdx.x == 0) reinterpret_cast<int *>(ctr)[0] = 0;
         return;
@@ -217,6 +220,7 @@ cache_assign_kernel(const int *__restrict__ ids, int t0, int n_new, int now, int
         }
     }
     if (tid == 0) {
+        times->select_end = device_ns();
         reinterpret_cast<int *>(ctr)[0] = n_miss;                 // CACHE_N_MISS, read by the engines as an int
         ctr[CACHE_HITS] += n_hit_s;
         ctr[CACHE_MISSES] += n_miss;
@@ -240,6 +244,8 @@ struct SolverCtl {
     double prev, last, second_last, diff0;
     long long local_iter;
     long long ctr[CACHE_CTRS];      // cache counters as of the last iteration that ran
+    PhaseTimes times;               // of the running iteration
+    long long ns_select, ns_rows, ns_local, ns_update;     // sums over the iterations that ran
 };
 static_assert(offsetof(SolverCtl, stop) == 0, "kernels read the stop flag through a pointer to the struct");
 
@@ -248,10 +254,11 @@ constexpr int STATUS_THREADS = 512;                               // at least ha
 __global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ diff, const int *__restrict__ got,
                                      int wanted, double eps, int max_iter, const long long *__restrict__ cache_ctr,
                                      const int *__restrict__ engine_status, int *__restrict__ ids, int q,
-                                     unsigned char *__restrict__ in_ws) {
+                                     unsigned char *__restrict__ in_ws, volatile unsigned long long *progress) {
     const int already = c->stop;
     __syncthreads();
     if (already) return;
+    const long long now = device_ns();
     // The working set rotates for the next selection: the old second half becomes the first half and keeps its flags,
     // the old first half leaves. (After the last iteration nothing looks at it again.)
     if ((int) threadIdx.x < q) {
@@ -283,6 +290,15 @@ __global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ di
     if (cache_ctr)
         for (int k = 0; k < CACHE_CTRS; ++k) c->ctr[k] = cache_ctr[k];
     c->stop = stop;
+    if (progress) {
+        // how far the solve is, for the host that waits for it: a word of pinned host memory
+        *progress = ((unsigned long long) c->iter << 1) | (unsigned) stop;
+        const PhaseTimes t = c->times;
+        c->ns_select += t.select_end - t.select_begin;
+        c->ns_rows += t.rows_end - t.select_end;
+        c->ns_local += t.local_end - t.local_begin;
+        c->ns_update += now - t.update_begin;
+    }
 }
 
 // *any becomes non-zero if one of a[0..n) is
@@ -310,7 +326,9 @@ constexpr int UPD_WIDE_PER_SM = 2;           // blocks of the V = 4 form that fi
 template <int V>
 __global__ void __launch_bounds__(UPD_WARPS * 32, V == 4 ? UPD_WIDE_PER_SM : 3)
 update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_diff, int q, int first_half_phys,
-                const float *__restrict__ rows, long long ld, int t_begin, int t_end, const int *__restrict__ row_slot) {
+                const float *__restrict__ rows, long long ld, int t_begin, int t_end, const int *__restrict__ row_slot,
+                PhaseTimes *times) {
+    if (times && blockIdx.x == 0 && threadIdx.x == 0) times->update_begin = device_ns();
     constexpr int U = V == 1 ? 16 : 8;
     __shared__ double ad[UPD_SLOTS], part[2][UPD_WARPS][32 * V];
     __shared__ int prow[UPD_SLOTS], count[UPD_WARPS];
@@ -552,21 +570,21 @@ __global__ void shard_scatter_kernel(const int *__restrict__ ids, int ws, int lo
 // 23 us at 32,768 columns, but 18.5 against 16.4 at 20,000. Below that, and for rows that are not aligned, 32 columns per
 // block.
 static tsvm_status launch_update_f(double *f, int n, const double *alpha_diff, int q, int first_half_phys, const float *rows,
-                                   long long ld, int t0, int t1, const int *row_slot, cudaStream_t st) {
+                                   long long ld, int t0, int t1, const int *row_slot, PhaseTimes *times, cudaStream_t st) {
     const int wide_tiles = ceil_div(n, 128), sms = device_sm_count();
     if (((uintptr_t) rows & 15) == 0 && (ld & 3) == 0 && 2 * wide_tiles >= 3 * sms)
         TSVM_LAUNCH(update_f_kernel<4>, wide_tiles < UPD_WIDE_PER_SM * sms ? wide_tiles : UPD_WIDE_PER_SM * sms, UPD_WARPS * 32,
-                    0, st, f, n, alpha_diff, q, first_half_phys, rows, ld, t0, t1, row_slot);
+                    0, st, f, n, alpha_diff, q, first_half_phys, rows, ld, t0, t1, row_slot, times);
     else
         TSVM_LAUNCH(update_f_kernel<1>, ceil_div(n, 32), UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows,
-                    ld, t0, t1, row_slot);
+                    ld, t0, t1, row_slot, times);
     return TSVM_OK;
 }
 
 static tsvm_status launch_local_smo(int solver_kind, int ws, const float *kww, const float *diag_ws, const int *y_ws,
                                     const double *f_ws, double *alpha_ws, double *alpha_diff, double Cp, double Cn,
                                     double eps, int max_iter, double *diff, const int *ids, double *alpha_global,
-                                    cudaStream_t st, const int *stop = nullptr) {
+                                    cudaStream_t st, const int *stop = nullptr, PhaseTimes *times = nullptr) {
     const bool nu = solver_kind != TSVM_SOLVER_C;
     // four warps at every size, one to eight slots per thread: measured at 1,024 / 512 / 256 slots 1.00 / 0.84 / 0.73 us
     // per iteration against 1.12 / 0.99 / 0.86 with eight warps and 1.73 with sixteen (512 slots)
@@ -579,7 +597,7 @@ static tsvm_status launch_local_smo(int solver_kind, int ws, const float *kww, c
                                                             cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                                                             (int) (smo::RING * S * T * sizeof(float)))));          \
         TSVM_LAUNCH((local_smo_kernel<NU, S, T>), 1, T + 32, ring_bytes, st, ws, kww, diag_ws, y_ws, f_ws,         \
-                    alpha_ws, alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop, use_ring);         \
+                    alpha_ws, alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop, use_ring, times);  \
     } while (0)
 #define SMO_CASE(S) do { if (nu) SMO_LAUNCH(true, S); else SMO_LAUNCH(false, S); } while (0)
     if (ws <= T) SMO_CASE(1); else if (ws <= 2 * T) SMO_CASE(2); else if (ws <= 4 * T) SMO_CASE(4); else SMO_CASE(8);
@@ -665,7 +683,7 @@ void tsvm_ws_destroy(tsvm_ws *w) { ws_destroy(w, false); }
 static tsvm_status launch_select(tsvm_ws *w, int solver_kind, int n, const double *f_dev, const double *alpha_dev,
                                  const int *y_dev, const unsigned char *in_ws_dev, double Cp, double Cn, int want,
                                  int id_offset, double *sorted_f, int *sorted_id, int *out_ids, const int *stop,
-                                 cudaStream_t st) {
+                                 cudaStream_t st, PhaseTimes *times = nullptr) {
     const int lists = solver_kind == TSVM_SOLVER_C ? 2 : 4;
     static int resident_blocks[MAX_DEVICES] = {0};
     int dev = 0;
@@ -684,7 +702,7 @@ static tsvm_status launch_select(tsvm_ws *w, int solver_kind, int n, const doubl
     a.solver_kind = solver_kind; a.n = n; a.f = f_dev; a.alpha = alpha_dev; a.y = y_dev; a.in_ws = in_ws_dev;
     a.Cp = Cp; a.Cn = Cn; a.st = w->state; a.hist = w->hist; a.ticket = w->ticket; a.want = want;
     a.id_offset = id_offset; a.cand_h = w->cand_h; a.cand_l = w->cand_l; a.sorted_f = sorted_f; a.sorted_id = sorted_id;
-    a.out_ids = out_ids; a.out_count = w->count; a.stop = stop;
+    a.out_ids = out_ids; a.out_count = w->count; a.stop = stop; a.times = times;
     a.sample = select_sample(n);
     if (a.sample == n) { a.rank_low = want; a.rank_high = want + want / 2; }
     else {
@@ -845,7 +863,7 @@ tsvm_status tsvm_update_f(double *f_dev, int n, const double *alpha_diff_dev, in
                           long long ld, void *stream) {
     TSVM_REQUIRE(f_dev && alpha_diff_dev && rows_dev && n > 0 && ws_size > 0 && ws_size <= 1024 && ld >= n,
                  "update_f: bad arguments (at most 1024 rows per call)");
-    TSVM_TRY(launch_update_f(f_dev, n, alpha_diff_dev, 0, 0, rows_dev, ld, 0, ws_size, nullptr, (cudaStream_t) stream));
+    TSVM_TRY(launch_update_f(f_dev, n, alpha_diff_dev, 0, 0, rows_dev, ld, 0, ws_size, nullptr, nullptr, (cudaStream_t) stream));
     return TSVM_OK;
 }
 
@@ -863,37 +881,30 @@ int tsvm_working_set_size(int n_instances, int n_features, size_t max_mem_bytes,
 }  // extern "C"
 
 // Solver state that persists across outer iterations.
-// How many iterations are queued between two reads of the device's verdict. The queue hides the host's wake-up
-// and launch latency behind the device's work; the price is at most that many no-op iterations after the one
-// that ends the solve.
+// How many iterations are queued before the device has finished the first of them: enough that the next one is there when
+// one ends (the host needs 30 - 60 us to queue an iteration, more with several solvers at a time); every one queued past
+// the end of a solve is a no-op of some 20 us.
 enum { MAX_QUEUED = 32 };
-static int sync_every() {
+static int queued_iterations(int otherwise) {
     static const int k = [] {
         const char *e = getenv("TSVM_SYNC_EVERY");
-        const int v = e ? atoi(e) : 8;
-        return v < 1 ? 1 : (v > MAX_QUEUED ? (int) MAX_QUEUED : v);
+        const int v = e ? atoi(e) : 0;
+        return !e ? 0 : (v < 1 ? 1 : (v > MAX_QUEUED ? (int) MAX_QUEUED : v));
     }();
-    return k;
+    return k ? k : otherwise;
 }
+static int queue_depth() { return queued_iterations(3); }
+static int sync_every() { return queued_iterations(8); }          // shard solver: iterations between two reads of the verdict
 
 // The second stream of a solver and its events. Creating them costs more than the rest of a small solve's set-up (a stream
 // 0.2 - 2 ms), so a finished solver leaves them to the next one of the same device: 16 sets at most are kept, and
 // tsvm_release_cached_memory destroys them. A set belongs to one solver at a time and is idle when it comes back.
 struct SolverStreams {
-    // Events of one queued iteration: phase boundaries on the first stream, start and end of the local solver
-    struct IterEvents {
-        cudaEvent_t ph[5] = {nullptr, nullptr, nullptr, nullptr, nullptr}, l0 = nullptr, l1 = nullptr;
-    };
     int dev = 0;
     cudaStream_t st2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_fork2 = nullptr, ev_join = nullptr;
-    IterEvents evs[MAX_QUEUED];
 
     ~SolverStreams() {
-        for (auto &E : evs) {
-            for (auto e : E.ph) if (e) cudaEventDestroy(e);
-            for (auto e : {E.l0, E.l1}) if (e) cudaEventDestroy(e);
-        }
         for (auto e : {ev_fork, ev_fork2, ev_join}) if (e) cudaEventDestroy(e);
         if (st2) cudaStreamDestroy(st2);
     }
@@ -905,14 +916,6 @@ struct SolverStreams {
         int lo_prio = 0, hi_prio = 0;
         TSVM_CUDA(cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio));
         TSVM_CUDA(cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, hi_prio));
-        return TSVM_OK;
-    }
-    tsvm_status ensure_events(int j) {
-        IterEvents &E = evs[j];
-        if (E.l1) return TSVM_OK;
-        for (auto &e : E.ph) if (!e) TSVM_CUDA(cudaEventCreate(&e));
-        if (!E.l0) TSVM_CUDA(cudaEventCreate(&E.l0));
-        TSVM_CUDA(cudaEventCreate(&E.l1));
         return TSVM_OK;
     }
 };
@@ -963,9 +966,13 @@ void release_solver_streams() {
 }
 }  // namespace tsvm
 
-struct tsvm_solver {
-    typedef SolverStreams::IterEvents IterEvents;
+static inline void cpu_pause() {
+#if defined(__x86_64__) || defined(__i386__)
+    __builtin_ia32_pause();
+#endif
+}
 
+struct tsvm_solver {
     tsvm_km *km = nullptr;
     int kind = 0, ws = 0, q = 0, n = 0;
     const int *y = nullptr;
@@ -986,6 +993,8 @@ struct tsvm_solver {
     bool idle = true;               // nothing of this solver is in flight (the last call ended with a wait)
     int max_iter = -1;              // iteration cap applied on the device; -1: none
     bool stopped = false;           // the device stopped the queue (done, capped or an error)
+    bool uncollected = false;       // iterations have run since the control block was last copied back
+    long long iter_collected = 0;   // iterations as of then
     // overlapped iteration: second stream, fork / join events, operand planes of the working set
     bool overlap = true;
     cudaStream_t st2 = nullptr;     // of `streams`, like the events
@@ -1086,6 +1095,7 @@ struct tsvm_solver {
         TSVM_TRY(dev_alloc(&ctl, 1));
         TSVM_TRY(pinned_alloc((void **) &ctl_host, sizeof(SolverCtl)));
         memset(ctl_host, 0, sizeof(SolverCtl));
+        *progress() = 0;
         ctl_host->prev = ctl_host->last = ctl_host->second_last = INFINITY;     // csmosolver.cpp:51-57
         TSVM_CUDA(cudaMemcpyAsync(ctl, ctl_host, sizeof(SolverCtl), cudaMemcpyHostToDevice, st));
         TSVM_TRY(take_streams(&streams));
@@ -1117,7 +1127,7 @@ struct tsvm_solver {
             TSVM_CUDA(cudaMemcpyAsync(ids, bi.data(), sizeof(int) * m, cudaMemcpyHostToDevice, st));
             TSVM_CUDA(cudaMemcpyAsync(alpha_diff, bd.data(), sizeof(double) * m, cudaMemcpyHostToDevice, st));
             TSVM_TRY(tsvm_km_rows_by_index(km, ids, m, rows, ld, st));
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, 0, 0, rows, ld, 0, m, nullptr, st));
+            TSVM_TRY(launch_update_f(f, n, alpha_diff, 0, 0, rows, ld, 0, m, nullptr, nullptr, st));
             TSVM_CUDA(cudaStreamSynchronize(st));
             rows_made += m;
             bi.clear(); bd.clear();
@@ -1143,18 +1153,18 @@ struct tsvm_solver {
     // gathered from the rows already in the buffer, and the one-CTA local solver then runs on a second stream
     // while the q x n launch - which leaves one SM pair free for it - fills the row buffer. Both meet before
     // the f update.
-    tsvm_status enqueue_iteration(long long it, const IterEvents &E) {
+    tsvm_status enqueue_iteration(long long it) {
         const int t0 = it == 0 ? 0 : q, n_new = it == 0 ? ws : q;          // iteration 0 fills the whole working set
         const bool overlapped = overlap && it > 0 && st2 && km_pair_engine(km, st);
         const int row_block = km_pair_engine(km, st) ? 256 : 64;           // requested rows per tile of the engine
         const int *n_miss_dev = reinterpret_cast<const int *>(cache_ctr);
         const int *stop = &ctl->stop;
+        PhaseTimes *times = &ctl->times;
         int *row_slot = row_slots + (it & 1) * ws;                         // row of every working-set slot
         const int *row_slot_before = row_slots + ((it + 1) & 1) * ws;
-        TSVM_CUDA(cudaEventRecord(E.ph[0], st));
         // (the status kernel of the previous iteration has rotated the working set)
         TSVM_TRY(launch_select(sel, kind, n, f, alpha, y, it == 0 ? nullptr : in_ws, Cp, Cn, n_new, 0, sel->sorted_f,
-                               sel->sorted_id, ids + t0, it == 0 ? nullptr : stop, st));
+                               sel->sorted_id, ids + t0, it == 0 ? nullptr : stop, st, times));
         if (overlapped) {
             // The block needs the members' planes and the old members' rows, both known now: the second stream starts on
             // it while the first one still runs the cache directory, i.e. before the big launch takes all SM pairs
@@ -1167,22 +1177,19 @@ struct tsvm_solver {
             TSVM_CUDA(cudaEventRecord(ev_fork, st));
             TSVM_CUDA(cudaStreamWaitEvent(st2, ev_fork, 0));
             TSVM_LAUNCH(gather_ws_kernel, ws, 256, 0, st2, ws, q, 0, ids, rows, ld, km->diag, y, f, alpha, kww, diag_ws,
-                        y_ws, f_ws, a_ws, q, row_slot_before + q);
+                        y_ws, f_ws, a_ws, q, row_slot_before + q, (PhaseTimes *) nullptr);
             const size_t rb = km_plane_row_bytes(km);
             const InstancePlanes members{ws_hi, ws_lo, ws_sd, ws_unscale, ws};
             const RowPlanes new_members{reinterpret_cast<const float *>(reinterpret_cast<const char *>(ws_hi) + (size_t) q * rb),
                                         reinterpret_cast<const float *>(reinterpret_cast<const char *>(ws_lo) + (size_t) q * rb),
                                         ws_sd + q, ws_unscale + q};
             TSVM_TRY(km_rows_planes_on(km, members, new_members, q, kww + (size_t) q * ws, ws, st2));
-            TSVM_CUDA(cudaEventRecord(E.l0, st2));
             TSVM_TRY(launch_local_smo(kind, ws, kww, diag_ws, y_ws, f_ws, a_ws, alpha_diff, Cp, Cn, eps, local_max_iter,
-                                      diff, ids, alpha, st2, stop));
-            TSVM_CUDA(cudaEventRecord(E.l1, st2));
+                                      diff, ids, alpha, st2, stop, times));
         }
         // cache directory: hits point at their rows, misses get the least recently used rows
         TSVM_LAUNCH(cache_assign_kernel, 1, CACHE_THREADS, 0, st, ids, t0, n_new, (int) (it + 1), slot_of, inst_of, stamp,
-                    (int) cache_cap, row_slot_before, row_slot, miss_ids, miss_slot, victims, cache_ctr, row_block, stop);
-        TSVM_CUDA(cudaEventRecord(E.ph[1], st));
+                    (int) cache_cap, row_slot_before, row_slot, miss_ids, miss_slot, victims, cache_ctr, row_block, stop, times);
         if (!overlapped) {
             // the engine computes the missing rows only (their number is read on the device) into their cache rows
             km->rows_m_dev = n_miss_dev; km->rows_slot_dev = miss_slot;
@@ -1195,78 +1202,96 @@ struct tsvm_solver {
             TSVM_CUDA(cudaStreamWaitEvent(st2, ev_fork2, 0));
             // the rows that were in the buffer already can be applied to f at once (HBM-bound, next to the
             // tensor-bound launch); the new rows follow on the first stream
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, q, row_slot, st2));
+            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, q, row_slot, nullptr, st2));
             TSVM_CUDA(cudaEventRecord(ev_join, st2));
             // first stream: the missing rows against all instances, on all SM pairs but one
             const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
             const RowPlanes miss_rows{miss_hi, miss_lo, miss_sd, miss_unscale};
             km->reserve_clusters = 1;
-            km->rows_m_dev = n_miss_dev; km->rows_slot_dev = miss_slot;
+            km->rows_m_dev = n_miss_dev; km->rows_slot_dev = miss_slot; km->rows_end_dev = &times->rows_end;
             const tsvm_status rs = km_rows_planes_on(km, all, miss_rows, q, rows, ld, st);
             km->reserve_clusters = 0;
-            km->rows_m_dev = nullptr; km->rows_slot_dev = nullptr;
+            km->rows_m_dev = nullptr; km->rows_slot_dev = nullptr; km->rows_end_dev = nullptr;
             TSVM_TRY(rs);
         }
-        TSVM_CUDA(cudaEventRecord(E.ph[2], st));
         if (!overlapped) {
             TSVM_LAUNCH(gather_ws_kernel, ws, 256, 0, st, ws, q, 0, ids, rows, ld, km->diag, y, f, alpha, kww, diag_ws,
-                        y_ws, f_ws, a_ws, ws, row_slot);
-            TSVM_CUDA(cudaEventRecord(E.l0, st));
+                        y_ws, f_ws, a_ws, ws, row_slot, times);
             TSVM_TRY(launch_local_smo(kind, ws, kww, diag_ws, y_ws, f_ws, a_ws, alpha_diff, Cp, Cn, eps, local_max_iter,
-                                      diff, ids, alpha, st, stop));
-            TSVM_CUDA(cudaEventRecord(E.l1, st));
+                                      diff, ids, alpha, st, stop, times));
         } else {
             TSVM_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
         }
-        TSVM_CUDA(cudaEventRecord(E.ph[3], st));
         // f -= sum over the old half's rows, then f -= sum over the new half's rows: two launches in every
         // form of the iteration, so that all of them round alike (the first iteration has new rows only)
         if (it == 0) {
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, ws, row_slot, st));
+            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, ws, row_slot, times, st));
         } else {
             if (!overlapped)
-                TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, q, row_slot, st));
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, q, ws, row_slot, st));
+                TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, q, row_slot, nullptr, st));
+            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, q, ws, row_slot, times, st));
         }
-        TSVM_CUDA(cudaEventRecord(E.ph[4], st));
         TSVM_LAUNCH(solver_status_kernel, 1, STATUS_THREADS, 0, st, ctl, diff, sel->count, n_new, eps, max_iter, cache_ctr,
-                    km->status_dev, ids, q, in_ws);
+                    km->status_dev, ids, q, in_ws, progress());
         return TSVM_OK;
     }
 
 
-    // Queues up to `count` outer iterations, waits once and takes over what the device decided. Fewer than
-    // `count` may have run: the termination rules, the iteration cap or an error stop the queue on the device.
+    // Up to `count` outer iterations; fewer if the termination rules, the iteration cap or an error stop the queue on the
+    // device. The device tells after every iteration how far it is, and the host keeps `queue_depth()` iterations queued:
+    // there is always one ready when another ends, and few no-op ones follow the last. collect() has to come next.
     tsvm_status run_iterations(int count) {
-        if (count > sync_every()) count = sync_every();
-        if (iter == 0) count = 1;                   // the first iteration is read back on its own
+        const long long end = iter + count;
+        long long queued = iter;
         idle = false;
-        for (int j = 0; j < count; ++j) {
-            TSVM_TRY(streams->ensure_events(j));
-            TSVM_TRY(enqueue_iteration(iter + j, streams->evs[j]));
+        uncollected = true;
+        while (!stopped && iter < end) {
+            const int ahead = iter == 0 ? 1 : queue_depth();      // (many small solves end with their first iteration)
+            while (queued < end && queued < iter + ahead) TSVM_TRY(enqueue_iteration(queued++));
+            TSVM_TRY(await_progress());
         }
-        TSVM_CUDA(cudaMemcpyAsync(ctl_host, ctl, sizeof(SolverCtl), cudaMemcpyDeviceToHost, st));
+        return TSVM_OK;
+    }
+
+    volatile unsigned long long *progress() const { return reinterpret_cast<volatile unsigned long long *>(diff_host + 15); }
+
+    // Waits until the device has finished more iterations than `iter`, or has stopped.
+    tsvm_status await_progress() {
+        for (unsigned k = 1;; ++k) {
+            const unsigned long long p = *progress();
+            if ((long long) (p >> 1) > iter || (p & 1)) {
+                iter = (long long) (p >> 1);
+                stopped = (p & 1) != 0;
+                return TSVM_OK;
+            }
+            if (k & 255) { cpu_pause(); continue; }
+            const cudaError_t e = cudaStreamQuery(st);            // a failed launch or kernel makes no progress
+            if (e == cudaErrorNotReady) { cudaGetLastError(); sched_yield(); continue; }
+            TSVM_CUDA(e);
+            const unsigned long long last = *progress();
+            TSVM_REQUIRE((long long) (last >> 1) > iter || (last & 1), "solver: the queue ended without progress");
+        }
+    }
+
+    // Waits for the queue and takes over what the device decided. `more`: enqueues further copies to wait for as well.
+    template <typename More> tsvm_status collect(More more) {
+        if (uncollected) TSVM_CUDA(cudaMemcpyAsync(ctl_host, ctl, sizeof(SolverCtl), cudaMemcpyDeviceToHost, st));
+        TSVM_TRY(more());
         TSVM_CUDA(cudaStreamSynchronize(st));            // (the second stream has joined the first)
         idle = true;
         km->waited(st);
+        if (!uncollected) return TSVM_OK;
+        uncollected = false;
         const SolverCtl &c = *ctl_host;
         if (c.engine_status != 0) {
             set_error("dense kernel-row engine reported status %d (a bounded wait ran out)", c.engine_status);
             return TSVM_ERR_DEVICE;
         }
-        const int ran = (int) (c.iter - iter);
-        for (int j = 0; j < ran; ++j) {
-            const IterEvents &E = streams->evs[j];
-            float ms;
-            cudaEventElapsedTime(&ms, E.ph[0], E.ph[1]); t_sel += ms;
-            cudaEventElapsedTime(&ms, E.ph[1], E.ph[2]); t_rows += ms;
-            cudaEventElapsedTime(&ms, E.l0, E.l1); t_loc += ms;      // overlapped with the rows phase when both streams run
-            cudaEventElapsedTime(&ms, E.ph[3], E.ph[4]); t_upd += ms;
-            rows_made += iter + j == 0 ? ws : q;
-        }
+        t_sel = c.ns_select * 1e-9; t_rows = c.ns_rows * 1e-9; t_loc = c.ns_local * 1e-9; t_upd = c.ns_update * 1e-9;
         hits = c.ctr[CACHE_HITS]; misses = c.ctr[CACHE_MISSES];
         row_blocks = c.ctr[CACHE_BLOCKS]; row_blocks_saved = c.ctr[CACHE_BLOCKS_SAVED];
-        iter = c.iter;
+        rows_made += (c.iter - iter_collected) * q + (iter_collected == 0 && c.iter > 0 ? ws - q : 0);
+        iter = iter_collected = c.iter;
         local_iter = c.local_iter;
         diff0 = c.diff0;
         done = c.done != 0;
@@ -1279,18 +1304,17 @@ struct tsvm_solver {
         }
         return TSVM_OK;
     }
-
-    tsvm_status outer_iteration() { return run_iterations(1); }
+    tsvm_status collect() { return collect([] { return TSVM_OK; }); }
 
     void fill_stats(tsvm_solve_stats *out, double obj) const {
         out->outer_iters = iter;
         out->local_iters = local_iter;
         out->final_diff = diff0;
         out->objective = obj;
-        out->seconds_select = t_sel * 1e-3;
-        out->seconds_rows = t_rows * 1e-3;
-        out->seconds_local = t_loc * 1e-3;
-        out->seconds_update = t_upd * 1e-3;
+        out->seconds_select = t_sel;
+        out->seconds_rows = t_rows;
+        out->seconds_local = t_loc;
+        out->seconds_update = t_upd;
         out->seconds_total = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_begin).count();
         out->kernel_rows = rows_made;
         out->gpu_launches = launch_count() - launches0;
@@ -1305,8 +1329,10 @@ struct tsvm_solver {
     tsvm_status finish(double *rho_host, tsvm_solve_stats *stats_host) {
         idle = false;
         TSVM_LAUNCH(rho_obj_kernel, 1, 1024, 0, st, n, f, alpha, y, Cp, Cn, red);
-        TSVM_CUDA(cudaMemcpyAsync(diff_host, red, RHO_VALS * sizeof(double), cudaMemcpyDeviceToHost, st));
-        TSVM_CUDA(cudaStreamSynchronize(st));
+        TSVM_TRY(collect([&]() -> tsvm_status {
+            TSVM_CUDA(cudaMemcpyAsync(diff_host, red, RHO_VALS * sizeof(double), cudaMemcpyDeviceToHost, st));
+            return TSVM_OK;
+        }));
         const double *R = diff_host;
         const double obj = -R[4];
         double rho;
@@ -1322,6 +1348,7 @@ struct tsvm_solver {
             if (kind == TSVM_SOLVER_NU_SVC) {
                 const double r = (r1 + r2) / 2;
                 TSVM_LAUNCH(scale_kernel, ceil_div(n, 256), 256, 0, st, alpha, n, r);
+                idle = false;
                 TSVM_CUDA(cudaStreamSynchronize(st));
                 rho /= r;
             }
@@ -1359,7 +1386,11 @@ tsvm_status tsvm_solver_create(tsvm_km *km, int solver_kind, const int *y_dev, d
 
 tsvm_status tsvm_solver_iterate(tsvm_solver *S, int n_iters, int *done_host) {
     TSVM_REQUIRE(S && n_iters > 0, "solver_iterate: bad arguments");
-    for (long long end = S->iter + n_iters; S->iter < end && !S->done;) TSVM_TRY(S->run_iterations((int) (end - S->iter)));
+    if (!S->done) {
+        S->stopped = false;              // (an error may have ended the last call; the device says so again)
+        TSVM_TRY(S->run_iterations(n_iters));
+        TSVM_TRY(S->collect());
+    }
     if (done_host) *done_host = S->done ? 1 : 0;
     return TSVM_OK;
 }
@@ -1392,7 +1423,7 @@ tsvm_status tsvm_smo_solve(tsvm_km *km, int solver_kind, const int *y_dev, doubl
     tsvm_status s = TSVM_OK;
     // max_iter = k stops after outer iteration k, i.e. k + 1 iterations (csmosolver.cpp:110); applied on the device
     S->max_iter = max_iter;
-    while (s == TSVM_OK && !S->stopped) s = S->run_iterations(MAX_QUEUED);
+    while (s == TSVM_OK && !S->stopped) s = S->run_iterations(INT_MAX);
     if (s == TSVM_OK) s = S->finish(rho_host, stats_host);
     delete S;
     return s;
@@ -1615,7 +1646,7 @@ struct tsvm_shard {
                                   nullptr, nullptr, st2, &ctl->stop));
         TSVM_CUDA(cudaEventRecord(E.b1, st2));
         if (it > 0)        // the old half's rows are in the buffer already
-            TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, 0, q, nullptr, st2));
+            TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, 0, q, nullptr, nullptr, st2));
         TSVM_CUDA(cudaEventRecord(ev_join, st2));
         // first stream: the new rows against this rank's columns
         float *new_rows = rows + (size_t) (it == 0 ? 0 : (1 - first_half_phys) * q) * ld;
@@ -1627,10 +1658,10 @@ struct tsvm_shard {
         TSVM_TRY(rs);
         TSVM_CUDA(cudaEventRecord(E.r1, st));
         TSVM_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
-        TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, it == 0 ? 0 : q, ws, nullptr, st));
+        TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, it == 0 ? 0 : q, ws, nullptr, nullptr, st));
         TSVM_LAUNCH(shard_scatter_kernel, ceil_div(ws, 256), 256, 0, st, ids, ws, lo, hi, a_ws, alpha);
         TSVM_LAUNCH(solver_status_kernel, 1, 32, 0, st, ctl, diff, sel->count, n_new, eps, -1, (const long long *) nullptr,
-                    km->status_dev, (int *) nullptr, 0, (unsigned char *) nullptr);
+                    km->status_dev, (int *) nullptr, 0, (unsigned char *) nullptr, (volatile unsigned long long *) nullptr);
         ++queued;
         phase = 0;
         return TSVM_OK;

@@ -30,21 +30,16 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-__device__ __forceinline__ long long global_ns() {
-    long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
 // Bounded wait: false when another role gave up or the time budget ran out (the caller
 // then leaves its loop; nothing spins forever).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int code) {
     if (mbar_try(bar, parity)) return true;
-    const long long t0 = global_ns();
+    const long long t0 = device_ns();
     for (;;) {
         for (int i = 0; i < 64; ++i)
             if (mbar_try(bar, parity)) return true;
         if (*abort_flag) return false;
-        if (global_ns() - t0 > tcc::WAIT_NS) { *abort_flag = code; return false; }
+        if (device_ns() - t0 > tcc::WAIT_NS) { *abort_flag = code; return false; }
     }
 }
 
