@@ -110,6 +110,13 @@ def test_fused_prediction_other_kernels(capi, kernel, kw):
     _fused_case(capi, 3, [150, 200, 90], d=96, m=333, kernel=kernel, **kw)
 
 
+@pytest.mark.parametrize("nc", [3, 4, 5, 10, 11, 32, 33])
+def test_fused_prediction_numbers_of_classes(capi, nc):
+    """Around the numbers of coefficients and classes where the fused path changes: 3 and 4 coefficients, 9 and 10, 32 and 33
+    classes; rows that are no multiple of 32, classes of one and of 33 support vectors."""
+    _fused_case(capi, nc, [1 + 32 * (c % 2) for c in range(nc)], d=40, m=97)
+
+
 def test_fused_prediction_many_classes(capi):
     """20 classes: 19 coefficient rows per support vector (more than the shared-memory table holds) and 190 pairs;
     several launches over the test rows."""

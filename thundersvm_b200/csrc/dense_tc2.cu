@@ -139,8 +139,9 @@ __device__ __forceinline__ void stage_chunk(const float (&sum)[tc2::COLS_PER_THR
 struct PredictArgs {
     const double *coef;        // (n_classes - 1) x n_sv, the model's layout (include/thundersvm/model/svmmodel.h:155-164)
     const int *sv_class;       // class of every support vector [n_sv]
-    double *dec;               // [m][n_pairs], preset to -rho; this launch adds its sums
-    int n_classes, n_pairs;
+    double *dec;               // the sums are added to dec[r * row_stride + pair * pair_stride]
+    long long row_stride, pair_stride;
+    int n_classes;
 };
 
 // Optional indirections of the kernel-row form, both read on the device so that a caller can decide them
@@ -152,6 +153,21 @@ struct RowsExtra {
     long long *end;                 // device_ns() when the last block left (never taken back), or nullptr
 };
 
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float sum2(unsigned long long v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return lo + hi;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;                // two FP32 multiply-adds
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
 __device__ __forceinline__ int pair_index(int n_classes, int i, int j) {      // i < j, pairs ordered (0,1),(0,2),...
     return i * (2 * n_classes - i - 1) / 2 + (j - i - 1);
 }
@@ -160,6 +176,65 @@ __device__ __forceinline__ int pair_index(int n_classes, int i, int j) {      //
 __device__ __forceinline__ int block_columns(int m, int nb) {
     const int left = m - nb * tc2::BN;
     return left >= tc2::BN ? tc2::BN : ((left + 31) & ~31);
+}
+
+__device__ __forceinline__ void red_add_if(bool take, double *p, double v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p red.global.add.f64 [%1], %2;\n\t}" ::"r"((int) take), "l"(p), "d"(v) : "memory");
+}
+
+// Prediction: the warp's block of kernel values (32 instances x 16 test rows r0 .. r0 + 15, element (c, l) at column
+// (l + c / 2) mod 32 of row c) times the instances' NC coefficients (zero beyond the real ones), added to the decision
+// values of the pairs. A lane takes two test rows and eight instances; the four lanes of a pair of rows then add up with
+// halving exchanges and end with half of the coefficients of one row.
+template <int NC, int CHUNK, int LD>
+__device__ __forceinline__ void reduce_chunk(const float *block, const float *coef, int cls_own, int cls_lo, int cls_hi, int r0,
+                                             int m, const PredictArgs &pa) {
+    static_assert(CHUNK == 16, "eight pairs of rows x four groups of instances");
+    constexpr int HALF = (NC + 1) / 2;
+    const int lane = threadIdx.x & 31, pair = lane & 7, l0 = (lane >> 3) * 8, odd = (lane >> 3) & 1, high = lane >> 4;
+    const int r = r0 + 2 * pair + odd, nc = pa.n_classes - 1;
+    for (int cl = cls_lo; cl <= cls_hi; ++cl) {
+        const unsigned mine = __ballot_sync(0xffffffffu, cls_own == cl);
+        float k[2][8];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) k[e][u] = block[(2 * pair + e) * LD + ((l0 + u + pair) & 31)];
+        if (mine != 0xffffffffu)
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (!((mine >> (l0 + u)) & 1u)) k[0][u] = k[1][u] = 0.0f;
+        unsigned long long k2[2][4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) k2[e][u] = pack2(k[e][2 * u], k[e][2 * u + 1]);
+        float w[NC];
+#pragma unroll
+        for (int cr = 0; cr < NC; ++cr) {
+            const ulonglong2 ca = *reinterpret_cast<const ulonglong2 *>(coef + cr * LD + l0);
+            const ulonglong2 cb = *reinterpret_cast<const ulonglong2 *>(coef + cr * LD + l0 + 4);
+            float s[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                s[e] = sum2(fma2(cb.y, k2[e][3], fma2(cb.x, k2[e][2], fma2(ca.y, k2[e][1], fma2(ca.x, k2[e][0], 0ull)))));
+            w[cr] = (odd ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, odd ? s[0] : s[1], 8);
+        }
+        double total[HALF];
+#pragma unroll
+        for (int t = 0; t < HALF; ++t) {
+            const float lo = w[t], hi = HALF + t < NC ? w[HALF + t < NC ? HALF + t : t] : 0.0f;
+            total[t] = (double) ((high ? hi : lo) + __shfl_xor_sync(0xffffffffu, high ? lo : hi, 16));
+        }
+        // (no branches: the five exchanges, conversions and additions of ten classes overlap)
+        const int above = pair_index(pa.n_classes, cl, cl + 1) - cl;           // pairs (cl, cr + 1) for cr >= cl
+#pragma unroll
+        for (int t = 0; t < HALF; ++t) {
+            const int cr = high * HALF + t;
+            const int kp = cr < cl ? pair_index(pa.n_classes, cr, cl) : above + cr;
+            red_add_if(cr < nc && r < m, pa.dec + r * pa.row_stride + kp * pa.pair_stride, total[t]);
+        }
+    }
 }
 
 template <int EPI, bool F16, bool PREDICT>
@@ -303,8 +378,9 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                 cls_own = pa.sv_class[j < n ? j : n - 1];
                 if (nc == 1) coef_one = j < n ? (float) pa.coef[j] : 0.0f;
                 else if (nc <= PRED_NC_SMEM)
-                    for (int cr = 0; cr < nc; ++cr)
-                        coef_priv[cr * (EPI_WARPS * 32)] = j < n ? (float) pa.coef[(size_t) cr * n + j] : 0.0f;
+#pragma unroll
+                    for (int cr = 0; cr < PRED_NC_SMEM; ++cr)
+                        coef_priv[cr * (EPI_WARPS * 32)] = cr < nc && j < n ? (float) pa.coef[(size_t) cr * n + j] : 0.0f;
             }
             {
                 // Self dot and 1/scale of this warp's 128 requested rows go to shared memory by asynchronous
@@ -442,54 +518,26 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                         }
                         if (nc > 1 && nc <= PRED_NC_SMEM) {
                             // Several coefficients per instance: the butterfly below would repeat its 31 shuffles for
-                            // each of them. Instead the warp's 32 x 16 kernel values go back to shared memory, every lane
-                            // takes one column (test row) and half of the instances and multiplies their values by all
-                            // coefficients (16-byte reads of four instances' coefficients). Element (c, l) of the block
-                            // lies at column (l + c) mod 32, so that the 16 columns are read from 16 banks. Ten
-                            // classes, 8,003 x 784: 290 -> 247 us per 4,096 rows.
+                            // each of them. Instead the warp's 32 x 16 kernel values go back to shared memory and a lane
+                            // takes two columns (test rows) and eight instances (reduce_chunk). Element (c, l) of the block
+                            // lies at column (l + c / 2) mod 32, so that stores and reads meet no bank twice. What bounds it
+                            // is the chain of these steps, with two such warps per scheduler. Ten classes, 8,003 x 784, per
+                            // 4,096 rows: 290 us with the butterfly, 247 with one column and 16 instances per lane (36
+                            // instead of 18 reads of coefficients, each as long as four stores), 189 with two, 177 with a
+                            // fixed number of coefficients, 173 without branches around the additions, 157 with the
+                            // additions side by side. (With one coefficient the butterfly is faster, 93 against 109 us at
+                            // 12,001 x 123.)
                             float *block = priv - lane;
                             const float *cf_block = coef_priv - lane;
                             __syncwarp();                    // everyone has read its own sums
 #pragma unroll
-                            for (int c = 0; c < EPI_CHUNK; ++c) block[c * (EPI_WARPS * 32) + ((lane + c) & 31)] = kv[c];
+                            for (int c = 0; c < EPI_CHUNK; ++c) block[c * (EPI_WARPS * 32) + ((lane + c / 2) & 31)] = kv[c];
                             __syncwarp();
-                            const int c = lane & (EPI_CHUNK - 1), h = lane / EPI_CHUNK, r = i0 + cbase + c;
-                            constexpr int PART = EPI_CHUNK;  // instances per lane: 32 / (32 / EPI_CHUNK)
-                            for (int cl = cls_lo; cl <= cls_hi; ++cl) {
-                                const unsigned mine = __ballot_sync(0xffffffffu, cls_own == cl);
-                                float acc_c[PRED_NC_SMEM];
-#pragma unroll
-                                for (int cr = 0; cr < PRED_NC_SMEM; ++cr) acc_c[cr] = 0.0f;
-#pragma unroll
-                                for (int l = 0; l < PART; l += 4) {
-                                    float k4[4];
-#pragma unroll
-                                    for (int u = 0; u < 4; ++u) {
-                                        const int ll = h * PART + l + u;
-                                        k4[u] = block[c * (EPI_WARPS * 32) + ((ll + c) & 31)];
-                                        k4[u] = (mine >> ll) & 1u ? k4[u] : 0.0f;
-                                    }
-#pragma unroll
-                                    for (int cr = 0; cr < PRED_NC_SMEM; ++cr) {
-                                        if (cr >= nc) break;
-                                        const float4 cf = *reinterpret_cast<const float4 *>(cf_block + cr * (EPI_WARPS * 32) + h * PART + l);
-                                        acc_c[cr] = fmaf(cf.w, k4[3], fmaf(cf.z, k4[2], fmaf(cf.y, k4[1], fmaf(cf.x, k4[0], acc_c[cr]))));
-                                    }
-                                }
-#pragma unroll
-                                for (int cr = 0; cr < PRED_NC_SMEM; ++cr) {
-                                    if (cr >= nc) break;
-                                    float total = acc_c[cr];
-#pragma unroll
-                                    for (int o = EPI_CHUNK; o < 32; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-                                    if ((cr & (32 / EPI_CHUNK - 1)) == h && r < m && total != 0.0f) {
-                                        const int other = cr < cl ? cr : cr + 1;
-                                        const int k = other > cl ? pair_index(pa.n_classes, cl, other)
-                                                                 : pair_index(pa.n_classes, other, cl);
-                                        atomicAdd(pa.dec + (size_t) r * pa.n_pairs + k, (double) total);
-                                    }
-                                }
-                            }
+                            // (coefficients beyond the real ones are zero: a fixed number keeps the reads in flight together)
+                            if (nc <= 3)
+                                reduce_chunk<3, EPI_CHUNK, EPI_WARPS * 32>(block, cf_block, cls_own, cls_lo, cls_hi, i0 + cbase, m, pa);
+                            else
+                                reduce_chunk<PRED_NC_SMEM, EPI_CHUNK, EPI_WARPS * 32>(block, cf_block, cls_own, cls_lo, cls_hi, i0 + cbase, m, pa);
                             __syncwarp();                    // the next chunk's sums overwrite the block
                             continue;
                         }
@@ -526,7 +574,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                                     const int other = cr < cl ? cr : cr + 1;
                                     const int k = other > cl ? pair_index(pa.n_classes, cl, other)
                                                              : pair_index(pa.n_classes, other, cl);
-                                    atomicAdd(pa.dec + (size_t) r * pa.n_pairs + k, (double) total);
+                                    atomicAdd(pa.dec + r * pa.row_stride + k * pa.pair_stride, (double) total);
                                 }
                             }
                     }
@@ -626,10 +674,10 @@ tsvm_status launch_dense_tc2_planes(tsvm_km *km, const InstancePlanes &X, const 
 // Prediction form: the m staged rows are test rows, the kernel matrix holds the support vectors; adds
 // sum_sv coef * K(sv, test row) to dec_dev[r * n_pairs + pair] (preset by the caller) without writing K.
 tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev, const int *sv_class_dev,
-                                     int n_classes, double *dec_dev, cudaStream_t st) {
+                                     int n_classes, double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st) {
     const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
     const RowPlanes staged{km->Whi, km->Wlo, km->sd_rows, km->w_unscale};
-    const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, n_classes, n_classes * (n_classes - 1) / 2};
+    const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes};
     return launch_pair_any<true>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, nullptr}, st);
 }
 
