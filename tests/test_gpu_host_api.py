@@ -191,3 +191,35 @@ def test_pairs_on_several_host_threads_give_the_same_model_file():
         assert r.returncode == 0, r.stderr[-2000:]
         digests.append(r.stdout.strip().splitlines()[-1])
     assert len(digests[0]) == 64 and len(set(digests)) == 1
+
+
+@pytest.mark.parametrize("d,fill", [(2001, 0.3), (60000, 0.005)])
+def test_instances_larger_than_the_upload_blocks(capi, d, fill):
+    """Rows that go to the device in several page-locked blocks, the last one partly filled, with empty rows among them:
+    stored as dense rows (feature ids up to 2,001) and as CSR. Sparse and dense input give the same two-class and
+    three-class predictions, and the kernel separates the classes."""
+    H = host_api
+    L = H.load()
+    rng = np.random.default_rng(d)
+    n, k = 1801, 3
+    y = rng.integers(0, k, n).astype(np.float32)
+    block = d // k
+    nz = rng.random((n, d)) < fill * 0.1
+    for c in range(k):
+        nz[np.ix_(y == c, np.arange(c * block, (c + 1) * block))] |= rng.random(((y == c).sum(), block)) < fill
+    nz[7] = False
+    X = (nz * rng.random((n, d))).astype(np.float32)
+    rp = np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32)
+    csr = (X[nz], rp, np.nonzero(nz)[1].astype(np.int32))
+    for classes in (2, 3):
+        rows = y < classes
+        keep = nz[rows]
+        part = (X[rows][keep], np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32), np.nonzero(keep)[1].astype(np.int32))
+        m1 = H.train(L, 0, csr=part, y=y[rows], gamma=1.0 / (fill * d), C_=10.0)[0]
+        m2 = H.train(L, 0, X=X[rows], y=y[rows], gamma=1.0 / (fill * d), C_=10.0)[0]
+        a, b = H.predict_dense(L, m1, X), H.predict_dense(L, m2, X)
+        s = H.predict_sparse(L, m1, csr)
+        assert np.mean(a == b) > 0.998 and np.mean(a == s) > 0.998
+        assert np.mean(a[rows] == y[rows]) > 0.97
+        L.model_free(m1)
+        L.model_free(m2)

@@ -77,7 +77,7 @@ int device_sm_count();                        // SMs of the current device (aske
 size_t device_memory_bytes();                 // total memory of the current device (asked once per device)
 void pool_release();                          // returns every cached block to the driver
 void release_solver_streams();                // solver.cu: destroys the cached streams and events
-tsvm_status pinned_alloc(void **p, size_t bytes);
+tsvm_status pinned_alloc(void **p, size_t bytes);         // at most 64 MB of freed blocks are kept
 void pinned_free(void *p);
 
 template <typename T>
@@ -257,6 +257,8 @@ struct tsvm_km {
 
 namespace tsvm {
 // Pieces of tsvm_km_rows_by_index (km.cu) for callers that overlap them with other work.
+tsvm_status km_create_dense(const float *X, int n, int d, int ld, int loc, bool zero_padded, int kernel_type, int degree,
+                            float gamma, float coef0, void *stream, tsvm_km **out);
 bool km_pair_engine(tsvm_km *km, cudaStream_t st);
 tsvm_status km_pair_engine_takes(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int m, cudaStream_t st,
                                  bool *takes);

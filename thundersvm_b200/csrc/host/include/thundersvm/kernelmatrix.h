@@ -7,6 +7,8 @@
 #include "syncarray.h"
 #include "dataset.h"
 #include "svmparam.h"
+#include "util/upload.h"
+#include <memory>
 
 struct tsvm_km;
 
@@ -15,7 +17,7 @@ public:
     explicit KernelMatrix(const DataSet::node2d &instances, SvmParam param);
     /// rows [r0, r0 + n0) followed by rows [r1, r1 + n1) of a dense row-major matrix that is already on the
     /// device (d features, row stride ld floats): the binary sub-problem of two classes of a grouped data set
-    /// without a host round trip. No counterpart in the reference, which rebuilds every sub-problem from the
+    /// without a host round trip; columns d .. ld - 1 of X_dev are zero. No counterpart in the reference, which rebuilds every sub-problem from the
     /// host instances (svc.cpp:147-178).
     KernelMatrix(const float *X_dev, size_t d, size_t ld, size_t r0, size_t n0, size_t r1, size_t n1, SvmParam param);
     ~KernelMatrix();
@@ -39,7 +41,8 @@ private:
     bool dense_ = false;
     SvmParam param_;
     tsvm_km *km_ = nullptr;
-    float *pair_x_ = nullptr;          // device copy of the two row blocks (second constructor)
+    thundersvm::DevicePtr<float> own_x_;    // the dense rows on the device, zero in the padding
+    std::unique_ptr<thundersvm::DeviceCsr> own_csr_;
     mutable SyncArray<kernel_type> diag_;
 };
 #endif

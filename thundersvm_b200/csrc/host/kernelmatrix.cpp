@@ -12,39 +12,14 @@ void b200_check(tsvm_status s) {
     if (s == TSVM_ERR_OOM) throw std::bad_alloc();
     LOG(FATAL) << "thundersvm_b200: " << tsvm_last_error();
 }
-
-// node2d -> CSR with the ids as they are (1-based from LibSVM text); returns max id + 1
-struct HostCsr {
-    vector<float> val;
-    vector<int> col, row_ptr;
-    int n_features = 0;
-};
-HostCsr to_csr(const DataSet::node2d &ins) {
-    HostCsr c;
-    size_t nnz = 0;
-    for (auto &r : ins) nnz += r.size();
-    c.val.reserve(nnz); c.col.reserve(nnz); c.row_ptr.reserve(ins.size() + 1);
-    c.row_ptr.push_back(0);
-    int mx = 0;
-    for (auto &r : ins) {
-        for (auto &nd : r) {
-            c.val.push_back(nd.value);
-            c.col.push_back(nd.index);
-            if (nd.index > mx) mx = nd.index;
-        }
-        c.row_ptr.push_back((int) c.val.size());
-    }
-    c.n_features = mx + 1;            // column 0 stays empty for one-based data (kernelmatrix.cpp:200-206)
-    return c;
-}
 }  // namespace
 
 KernelMatrix::KernelMatrix(const DataSet::node2d &instances, SvmParam param) : param_(param) {
     n_instances_ = instances.size();
     CHECK(n_instances_ > 0) << "KernelMatrix needs at least one instance";
-    HostCsr c = to_csr(instances);
-    n_features_ = c.n_features;
-    nnz_ = c.val.size();
+    const thundersvm::Extent ext = thundersvm::extent_of(instances);
+    n_features_ = (size_t) ext.max_index + 1;   // column 0 stays empty for one-based data (kernelmatrix.cpp:200-206)
+    nnz_ = ext.nnz;
     // Storage: the tensor-core engine wants a dense row-major matrix; it pays off unless the data
     // is very sparse (then the CSR engine touches far fewer bytes) or the three dense planes would
     // not fit next to the kernel-row buffer.
@@ -52,19 +27,20 @@ KernelMatrix::KernelMatrix(const DataSet::node2d &instances, SvmParam param) : p
     const double dense_bytes = 3.0 * n_instances_ * ((n_features_ + 3) & ~3ul) * 4.0 + 1024.0 * n_instances_ * 4.0;
     dense_ = (density >= 0.02 || n_features_ <= 256) && thundersvm::device_has_room(dense_bytes);
     if (dense_) {
-        vector<float> X(n_instances_ * n_features_, 0.0f);
-#pragma omp parallel for schedule(static)
-        for (long i = 0; i < (long) n_instances_; ++i)
-            for (int p = c.row_ptr[i]; p < c.row_ptr[i + 1]; ++p) X[(size_t) i * n_features_ + c.col[p]] = c.val[p];
-        b200_check(tsvm_km_create_dense(X.data(), (int) n_instances_, (int) n_features_, (int) n_features_, TSVM_HOST,
-                                        param.kernel_type, param.degree, (float) param.gamma, (float) param.coef0,
-                                        thundersvm::work_stream(), &km_));
+        const size_t ld = (n_features_ + 3) & ~(size_t) 3;
+        own_x_ = thundersvm::device_array<float>(n_instances_ * ld);
+        thundersvm::upload_dense(own_x_.get(), n_instances_, ld,
+                                 [&](size_t r) -> const vector<DataSet::node> & { return instances[r]; });
+        b200_check(tsvm::km_create_dense(own_x_.get(), (int) n_instances_, (int) n_features_, (int) ld, TSVM_DEVICE, true,
+                                         param.kernel_type, param.degree, (float) param.gamma, (float) param.coef0,
+                                         thundersvm::work_stream(), &km_));
     } else {
-        b200_check(tsvm_km_create_csr(c.val.data(), c.row_ptr.data(), c.col.data(), (int) n_instances_,
-                                      (int) n_features_, TSVM_HOST, param.kernel_type, param.degree,
+        own_csr_.reset(new thundersvm::DeviceCsr(instances));
+        b200_check(tsvm_km_create_csr(own_csr_->val(), own_csr_->row_ptr(), own_csr_->col(), (int) n_instances_,
+                                      (int) n_features_, TSVM_DEVICE, param.kernel_type, param.degree,
                                       (float) param.gamma, (float) param.coef0, thundersvm::work_stream(), &km_));
+        km_->nnz = (long long) nnz_;
     }
-    cudaStreamSynchronize(thundersvm::work_stream());    // the host staging buffers above go out of scope
     thundersvm::total_memory_size() += (dense_ ? (size_t) dense_bytes : nnz_ * 8 + n_instances_ * 12);
     diag_.resize(n_instances_);
     thundersvm::copy_to_host(diag_.host_data(), km_->diag, sizeof(kernel_type) * n_instances_);
@@ -77,11 +53,11 @@ KernelMatrix::KernelMatrix(const float *X_dev, size_t d, size_t ld, size_t r0, s
     nnz_ = n_instances_ * d;
     dense_ = true;
     CHECK(n_instances_ > 0) << "KernelMatrix needs at least one instance";
-    pair_x_ = static_cast<float *>(thundersvm::device_alloc(n_instances_ * ld * sizeof(float)));
-    thundersvm::copy_on_device(pair_x_, X_dev + r0 * ld, n0 * ld * sizeof(float));
-    thundersvm::copy_on_device(pair_x_ + n0 * ld, X_dev + r1 * ld, n1 * ld * sizeof(float));
-    b200_check(tsvm_km_create_dense(pair_x_, (int) n_instances_, (int) d, (int) ld, TSVM_DEVICE, param.kernel_type,
-                                    param.degree, (float) param.gamma, (float) param.coef0, thundersvm::work_stream(), &km_));
+    own_x_ = thundersvm::device_array<float>(n_instances_ * ld);
+    thundersvm::copy_on_device(own_x_.get(), X_dev + r0 * ld, n0 * ld * sizeof(float));
+    thundersvm::copy_on_device(own_x_.get() + n0 * ld, X_dev + r1 * ld, n1 * ld * sizeof(float));
+    b200_check(tsvm::km_create_dense(own_x_.get(), (int) n_instances_, (int) d, (int) ld, TSVM_DEVICE, true, param.kernel_type,
+                                     param.degree, (float) param.gamma, (float) param.coef0, thundersvm::work_stream(), &km_));
     const double dense_bytes = 3.0 * n_instances_ * ((n_features_ + 3) & ~3ul) * 4.0 + 1024.0 * n_instances_ * 4.0;
     thundersvm::total_memory_size() += (size_t) dense_bytes;
     diag_.resize(n_instances_);
@@ -94,7 +70,6 @@ KernelMatrix::~KernelMatrix() {
         thundersvm::total_memory_size() -= (dense_ ? (size_t) dense_bytes : nnz_ * 8 + n_instances_ * 12);
         tsvm_km_destroy(km_);
     }
-    thundersvm::device_free(pair_x_);
 }
 
 void KernelMatrix::get_rows(const SyncArray<int> &idx, SyncArray<kernel_type> &kernel_rows) const {
@@ -106,13 +81,9 @@ void KernelMatrix::get_rows(const SyncArray<int> &idx, SyncArray<kernel_type> &k
 void KernelMatrix::get_rows(const DataSet::node2d &instances, SyncArray<kernel_type> &kernel_rows) const {
     CHECK_GE(kernel_rows.size(), instances.size() * n_instances_) << "kernel_rows memory is too small";
     if (instances.empty()) return;
-    HostCsr c = to_csr(instances);
-    SyncArray<kernel_type> val(std::max<size_t>(c.val.size(), 1));
-    SyncArray<int> col(std::max<size_t>(c.col.size(), 1)), rp(c.row_ptr.size());
-    if (!c.val.empty()) { val.copy_from(c.val.data(), c.val.size()); col.copy_from(c.col.data(), c.col.size()); }
-    rp.copy_from(c.row_ptr.data(), c.row_ptr.size());
-    b200_check(tsvm_km_rows_by_instances_csr(km_, val.device_data(), rp.device_data(), col.device_data(),
-                                             (int) instances.size(), (long long) c.val.size(), kernel_rows.device_data(),
+    const thundersvm::DeviceCsr c(instances);
+    b200_check(tsvm_km_rows_by_instances_csr(km_, c.val(), c.row_ptr(), c.col(), (int) instances.size(),
+                                             (long long) c.nnz(), kernel_rows.device_data(),
                                              (long long) n_instances_, thundersvm::work_stream()));
     cudaStreamSynchronize(thundersvm::work_stream());
 }

@@ -14,6 +14,7 @@
 #include <thundersvm/model/oneclass_svc.h>
 #include <thundersvm/solver/csmosolver.h>
 #include <thundersvm/solver/nusmosolver.h>
+#include <thundersvm/util/upload.h>
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -103,48 +104,13 @@ void SvmModel::predict_dec_values(const DataSet::node2d &instances, SyncArray<fl
         return;
     }
     const KernelMatrix &k_mat = sv_matrix();
-    // test batch as CSR on the device
-    size_t nnz = 0;
-    for (auto &r : instances) nnz += r.size();
-    SyncArray<kernel_type> tval(std::max<size_t>(nnz, 1));
-    SyncArray<int> tcol(std::max<size_t>(nnz, 1)), trp(m + 1);
-    {
-        kernel_type *v = tval.host_data();
-        int *c = tcol.host_data(), *rp = trp.host_data();
-        size_t p = 0;
-        rp[0] = 0;
-        for (size_t r = 0; r < m; ++r) {
-            for (auto &nd : instances[r]) { v[p] = nd.value; c[p] = nd.index; ++p; }
-            rp[r + 1] = (int) p;
-        }
-    }
+    const thundersvm::DeviceCsr batch(instances);
     size_t budget = 0;                      // 0 = library default; a positive batch size bounds the K buffer
     if (batch_size > 0) budget = (size_t) batch_size * (((size_t) sv.size() + 3) & ~3ul) * sizeof(kernel_type);
     b200_check(tsvm_predict_dec(k_mat.handle(), coef.device_data(), n_sv.host_data(), rho.device_data(), n_classes,
-                                (int) m, nullptr, 0, 0, tval.device_data(), trp.device_data(), tcol.device_data(),
-                                (long long) nnz, dec_values.device_data(), budget, nullptr));
+                                (int) m, nullptr, 0, 0, batch.val(), batch.row_ptr(), batch.col(), (long long) batch.nnz(),
+                                dec_values.device_data(), budget, nullptr));
 }
-
-// Test batch as CSR arrays on the device.
-struct DeviceBatch {
-    SyncArray<kernel_type> val;
-    SyncArray<int> col, row_ptr;
-    size_t nnz = 0;
-    explicit DeviceBatch(const DataSet::node2d &instances) {
-        for (auto &r : instances) nnz += r.size();
-        val.resize(std::max<size_t>(nnz, 1));
-        col.resize(std::max<size_t>(nnz, 1));
-        row_ptr.resize(instances.size() + 1);
-        kernel_type *v = val.host_data();
-        int *c = col.host_data(), *rp = row_ptr.host_data();
-        size_t p = 0;
-        rp[0] = 0;
-        for (size_t r = 0; r < instances.size(); ++r) {
-            for (auto &nd : instances[r]) { v[p] = nd.value; c[p] = nd.index; ++p; }
-            rp[r + 1] = (int) p;
-        }
-    }
-};
 
 void SvmModel::predict_dec_values_instant(const DataSet::node2d &instances, SyncArray<float_type> &predict_instant,
                                           int batch_size) const {
@@ -164,14 +130,13 @@ void SvmModel::predict_dec_values_instant(const DataSet::node2d &instances, Sync
         return;
     }
     const KernelMatrix &k_mat = sv_matrix();
-    DeviceBatch batch(instances);
+    const thundersvm::DeviceCsr batch(instances);
     size_t budget = 0;
     if (batch_size > 0) budget = (size_t) batch_size * (((size_t) sv.size() + 3) & ~3ul) * sizeof(kernel_type);
     SyncArray<int> winner(m);
     b200_check(tsvm_predict_labels(k_mat.handle(), coef.device_data(), n_sv.host_data(), rho.device_data(), n_classes,
-                                   (int) m, nullptr, 0, 0, batch.val.device_data(), batch.row_ptr.device_data(),
-                                   batch.col.device_data(), (long long) batch.nnz, winner.device_data(), budget,
-                                   nullptr));
+                                   (int) m, nullptr, 0, 0, batch.val(), batch.row_ptr(), batch.col(),
+                                   (long long) batch.nnz(), winner.device_data(), budget, nullptr));
     const int *w = winner.host_data();
     for (size_t r = 0; r < m; ++r) out[r] = w[r];
 }
@@ -377,28 +342,15 @@ void SVC::build_device_rows(const DataSet &ds) {
     free_device_rows();
     const size_t n = ds.n_instances();
     if (n == 0) return;
-    size_t nnz = 0;
-    int mx = 0;
-    {
-        const DataSet::node2d &all = ds.instances();
-#pragma omp parallel for schedule(static) reduction(+ : nnz) reduction(max : mx)
-        for (long r = 0; r < (long) all.size(); ++r) {
-            nnz += all[r].size();
-            for (auto &nd : all[r]) if (nd.index > mx) mx = nd.index;
-        }
-    }
-    const size_t d = (size_t) mx + 1, ld = (d + 3) & ~(size_t) 3;
-    const double density = (double) nnz / ((double) n * d);
+    const thundersvm::Extent ext = thundersvm::extent_of(ds.instances());
+    const size_t d = (size_t) ext.max_index + 1, ld = (d + 3) & ~(size_t) 3;
+    const double density = (double) ext.nnz / ((double) n * d);
     const double bytes = 4.0 * n * ld * 4.0 + 1024.0 * n * 4.0;      // this copy + a pair's matrix and planes + rows
     if (!((density >= 0.02 || d <= 256) && thundersvm::device_has_room(bytes))) return;
-    vector<float> X(n * ld, 0.0f);
     const vector<int> perm = ds.original_index();
     const DataSet::node2d &ins = ds.instances();
-#pragma omp parallel for schedule(static)
-    for (long k = 0; k < (long) n; ++k)
-        for (auto &nd : ins[perm[k]]) X[(size_t) k * ld + nd.index] = nd.value;
     dev_rows_.X = static_cast<float *>(thundersvm::device_alloc(n * ld * sizeof(float)));
-    thundersvm::copy_to_device(dev_rows_.X, X.data(), n * ld * sizeof(float));
+    thundersvm::upload_dense(dev_rows_.X, n, ld, [&](size_t k) -> const vector<DataSet::node> & { return ins[perm[k]]; });
     dev_rows_.n = n; dev_rows_.d = d; dev_rows_.ld = ld;
 }
 
@@ -471,7 +423,13 @@ void SVC::train(const DataSet &dataset, SvmParam param) {
     for (int c = 0; c < n_classes; ++c) {
         cnt[c] = 0;
         for (int id : ds.original_index(c))
-            if (is_sv[id]) { cnt[c]++; sv.push_back(ds.instances()[id]); sv_indices.push_back(id); }
+            if (is_sv[id]) { cnt[c]++; sv_indices.push_back(id); }
+    }
+    sv.resize(sv_indices.size());
+    {
+        const DataSet::node2d &all = ds.instances();
+#pragma omp parallel for schedule(static) if (sv.size() > 256)
+        for (long k = 0; k < (long) sv.size(); ++k) sv[k] = all[sv_indices[k]];
     }
     n_total_sv = (int) sv.size();
     LOG(INFO) << "#total unique sv = " << n_total_sv;

@@ -4,6 +4,7 @@
 #include <thundersvm/syncarray.h>
 #include <thundersvm/svmparam.h>
 #include <thundersvm/util/metric.h>
+#include <thundersvm/util/upload.h>
 #include <cuda_runtime.h>
 #include "../common.cuh"
 
@@ -55,6 +56,70 @@ bool device_has_room(double bytes) {
     return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes < 0.6 * (double) free_b;
 }
 void device_zero(void *p, size_t bytes) { cuda_ok(cudaMemsetAsync(p, 0, bytes, tl_stream), "cudaMemset"); }
+
+UploadBlocks::UploadBlocks(size_t bytes, bool two) {
+    for (int b = 0; b < (two ? 2 : 1); ++b) {
+        if (tsvm::pinned_alloc(reinterpret_cast<void **>(block_ + b), bytes) != TSVM_OK)
+            LOG(FATAL) << "page-locked memory: " << tsvm_last_error();
+        if (two) cuda_ok(cudaEventCreateWithFlags(sent_ + b, cudaEventDisableTiming), "event");
+    }
+}
+UploadBlocks::~UploadBlocks() {
+    if (busy_[0] || busy_[1]) cudaStreamSynchronize(tl_stream);
+    for (int b = 0; b < 2; ++b) {
+        if (sent_[b]) cudaEventDestroy(sent_[b]);
+        if (block_[b]) tsvm::pinned_free(block_[b]);
+    }
+}
+char *UploadBlocks::next() {
+    at_ = block_[1] ? 1 - at_ : 0;
+    if (busy_[at_]) cuda_ok(sent_[at_] ? cudaEventSynchronize(sent_[at_]) : cudaStreamSynchronize(tl_stream), "H2D copy");
+    busy_[at_] = false;
+    return block_[at_];
+}
+void UploadBlocks::send(void *dst, size_t bytes) {
+    cuda_ok(cudaMemcpyAsync(dst, block_[at_], bytes, cudaMemcpyHostToDevice, tl_stream), "H2D copy");
+    if (sent_[at_]) cuda_ok(cudaEventRecord(sent_[at_], tl_stream), "event");
+    busy_[at_] = true;
+}
+void UploadBlocks::finish() {
+    cuda_ok(cudaStreamSynchronize(tl_stream), "H2D copy");
+    busy_[0] = busy_[1] = false;
+}
+
+Extent extent_of(const DataSet::node2d &rows) {
+    size_t nnz = 0;
+    int mx = 0;
+#pragma omp parallel for schedule(static) reduction(+ : nnz) reduction(max : mx) if (rows.size() > 1024)
+    for (long r = 0; r < (long) rows.size(); ++r) {
+        nnz += rows[r].size();
+        for (auto &nd : rows[r]) if (nd.index > mx) mx = nd.index;
+    }
+    Extent e;
+    e.nnz = nnz; e.max_index = mx;
+    return e;
+}
+
+DeviceCsr::DeviceCsr(const DataSet::node2d &rows) {
+    const size_t m = rows.size();
+    vector<int> rp(m + 1, 0);
+    for (size_t r = 0; r < m; ++r) rp[r + 1] = rp[r] + (int) rows[r].size();
+    nnz_ = rp[m];
+    auto offset = [&](size_t r) { return (size_t) rp[r] * 4; };
+    row_ptr_ = device_array<int>(m + 1);
+    val_ = device_array<float>(nnz_);
+    col_ = device_array<int>(nnz_);
+    copy_to_device(row_ptr_.get(), rp.data(), (m + 1) * sizeof(int));
+    upload_rows(val_.get(), m, offset, [&](size_t r, char *p) {
+        float *v = reinterpret_cast<float *>(p);
+        for (auto &nd : rows[r]) *v++ = nd.value;
+    });
+    upload_rows(col_.get(), m, offset, [&](size_t r, char *p) {
+        int *c = reinterpret_cast<int *>(p);
+        for (auto &nd : rows[r]) *c++ = nd.index;
+    });
+}
+
 std::atomic<size_t> &total_memory_size() {
     static std::atomic<size_t> bytes{0};
     return bytes;

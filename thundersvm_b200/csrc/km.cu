@@ -36,6 +36,8 @@ auto &g_pinned_live = *new std::unordered_map<void *, PoolBlock>;
 auto &g_pool_free = *new std::map<std::pair<int, size_t>, std::vector<void *>>;
 auto &g_pinned_free = *new std::map<size_t, std::vector<void *>>;
 size_t g_pool_cached = 0;               // bytes in g_pool_free
+size_t g_pinned_cached = 0;             // bytes in g_pinned_free
+constexpr size_t MAX_PINNED_CACHED = 64 << 20;
 
 size_t size_class(size_t bytes) {
     if (bytes < 512) return 512;
@@ -58,6 +60,11 @@ void pool_release() {
     }
     g_pool_cached = 0;
     cudaSetDevice(cur);
+    for (auto &kv : g_pinned_free) {
+        for (void *q : kv.second) cudaFreeHost(q);
+        kv.second.clear();
+    }
+    g_pinned_cached = 0;
 }
 
 tsvm_status pool_alloc(void **p, size_t bytes) {
@@ -186,7 +193,13 @@ tsvm_status pinned_alloc(void **p, size_t bytes) {
     {
         std::lock_guard<std::mutex> lk(g_pool_mu);
         auto &v = g_pinned_free[cls];
-        if (!v.empty()) { *p = v.back(); v.pop_back(); g_pinned_live[*p] = PoolBlock{0, cls}; return TSVM_OK; }
+        if (!v.empty()) {
+            *p = v.back();
+            v.pop_back();
+            g_pinned_cached -= cls;
+            g_pinned_live[*p] = PoolBlock{0, cls};
+            return TSVM_OK;
+        }
     }
     TSVM_CUDA(cudaMallocHost(p, cls));
     std::lock_guard<std::mutex> lk(g_pool_mu);
@@ -199,7 +212,11 @@ void pinned_free(void *p) {
     std::lock_guard<std::mutex> lk(g_pool_mu);
     auto it = g_pinned_live.find(p);
     if (it == g_pinned_live.end()) { cudaFreeHost(p); return; }
-    g_pinned_free[it->second.cls].push_back(p);
+    if (g_pinned_cached + it->second.cls > MAX_PINNED_CACHED) cudaFreeHost(p);
+    else {
+        g_pinned_free[it->second.cls].push_back(p);
+        g_pinned_cached += it->second.cls;
+    }
     g_pinned_live.erase(it);
 }
 
@@ -1063,17 +1080,9 @@ tsvm_status km_stage_instances_csr(tsvm_km *km, const float *tval, const int *rp
 
 using namespace tsvm;
 
-extern "C" {
-
-const char *tsvm_last_error(void) { return tsvm::g_err; }
-int tsvm_abi_version(void) { return 2; }
-void tsvm_release_cached_memory(void) {
-    tsvm::release_solver_streams();
-    tsvm::pool_release();
-}
-
-tsvm_status tsvm_km_create_dense(const float *X, int n, int d, int ld, int loc, int kernel_type, int degree,
-                                 float gamma, float coef0, void *stream, tsvm_km **out) {
+// zero_padded: a device X whose columns d .. ld - 1 are zero is worked on in place whatever d is.
+tsvm_status tsvm::km_create_dense(const float *X, int n, int d, int ld, int loc, bool zero_padded, int kernel_type, int degree,
+                                  float gamma, float coef0, void *stream, tsvm_km **out) {
     TSVM_REQUIRE(out && X && n > 0 && d > 0 && ld >= d, "km_create_dense: bad arguments (n=%d d=%d ld=%d)", n, d, ld);
     TSVM_REQUIRE(kernel_type >= TSVM_LINEAR && kernel_type <= TSVM_PRECOMPUTED, "unknown kernel type %d", kernel_type);
     cudaStream_t st = (cudaStream_t) stream;
@@ -1083,7 +1092,7 @@ tsvm_status tsvm_km_create_dense(const float *X, int n, int d, int ld, int loc, 
     km->fn = KernelFn{kernel_type, degree, gamma, coef0};
     km->d_pad = (d + 3) & ~3;
     tsvm_status s = TSVM_OK;
-    bool in_place = loc == TSVM_DEVICE && (d % 4 == 0) && (ld % 4 == 0) && (((uintptr_t) X & 15) == 0) && ld >= km->d_pad;
+    bool in_place = loc == TSVM_DEVICE && (d % 4 == 0 || zero_padded) && (ld % 4 == 0) && (((uintptr_t) X & 15) == 0) && ld >= km->d_pad;
     if (in_place) { km->X = X; km->ldx = ld; }
     else {
         km->ldx = km->d_pad;
@@ -1105,6 +1114,20 @@ tsvm_status tsvm_km_create_dense(const float *X, int n, int d, int ld, int loc, 
     if (s != TSVM_OK) { tsvm_km_destroy(km); return s; }
     *out = km;
     return TSVM_OK;
+}
+
+extern "C" {
+
+const char *tsvm_last_error(void) { return tsvm::g_err; }
+int tsvm_abi_version(void) { return 2; }
+void tsvm_release_cached_memory(void) {
+    tsvm::release_solver_streams();
+    tsvm::pool_release();
+}
+
+tsvm_status tsvm_km_create_dense(const float *X, int n, int d, int ld, int loc, int kernel_type, int degree,
+                                 float gamma, float coef0, void *stream, tsvm_km **out) {
+    return tsvm::km_create_dense(X, n, d, ld, loc, false, kernel_type, degree, gamma, coef0, stream, out);
 }
 
 tsvm_status tsvm_km_create_csr(const float *val, const int *row_ptr, const int *col, int n, int d, int loc,
