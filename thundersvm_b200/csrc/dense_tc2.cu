@@ -571,10 +571,11 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
 #pragma unroll
                                 for (int o = REST >> 1; o >= 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
                                 if ((lane & (REST - 1)) == 0 && r < m && total != 0.0f) {
-                                    const int other = cr < cl ? cr : cr + 1;
-                                    const int k = other > cl ? pair_index(pa.n_classes, cl, other)
-                                                             : pair_index(pa.n_classes, other, cl);
-                                    atomicAdd(pa.dec + r * pa.row_stride + k * pa.pair_stride, (double) total);
+                                    if (nc == 1) atomicAdd(pa.dec + r, (double) total);          // (one pair: its sums lie side by side)
+                                    else {
+                                        const int k = cr < cl ? pair_index(pa.n_classes, cr, cl) : pair_index(pa.n_classes, cl, cr + 1);
+                                        atomicAdd(pa.dec + r * pa.row_stride + k * pa.pair_stride, (double) total);
+                                    }
                                 }
                             }
                     }
