@@ -283,3 +283,18 @@ def test_csr_rows_places_of_the_panel(capi, q, d, kernel):
         got = km.get_rows_instances(dense=torch.from_numpy(T).cuda()).cpu().numpy()
         assert np.max(np.abs(got - want) / np.maximum(np.abs(want), 0.05)) < 1e-5   # linear products cancel
     km.close()
+
+
+@pytest.mark.parametrize("n,q", [(1, 1), (256, 33), (257, 511), (1024, 512), (1025, 65), (5000, 300), (9400, 129)])
+@pytest.mark.parametrize("d", [40, 129, 400])
+def test_dense_rows_block_widths(capi, n, q, d):
+    """Requested rows in blocks of 32, 64, 128 and 256 columns, the last block partly filled, one k slab and several,
+    fewer slabs than stages and more."""
+    rng = np.random.default_rng(n + q + d)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    ids = rng.integers(0, n, q).astype(np.int32)
+    import torch
+    km = capi.KernelMatrix(dense=torch.from_numpy(X).cuda(), kernel="rbf", gamma=0.3 / d)
+    want = P.kernel_rows_idx(P.Csr(dense=X), ids, kernel="rbf", gamma=0.3 / d)
+    assert rel_err(km.get_rows(torch.from_numpy(ids).cuda()).cpu().numpy(), want) < REL_TOL
+    km.close()

@@ -232,6 +232,7 @@ struct tsvm_km {
     unsigned *csr_bits = nullptr;   // bitmap of the features staged in every part of the panel
     float *sd_rows = nullptr;       // self dots of the requested rows [sd_cap]
     int sd_cap = 0;
+    bool whole_blocks = false;      // the pair engine keeps to its widest tiles, whatever it leaves idle
     int reserve_clusters = 0;       // SM pairs the pair engine leaves free (a concurrent stream's kernels run there)
     // Set by a caller around tsvm_km_rows_by_index-style launches (the solver's row cache): the number of
     // requested rows is read from the device (at most the q of the call) and requested row i goes to row

@@ -34,6 +34,10 @@ constexpr int BM = 128, BN = 256, BN_HALF = 128, STAGES = 3, K_STEPS = 4;
 constexpr uint32_t A_BYTES = BM * 128;               // 16 KB per plane (this CTA's instances)
 constexpr uint32_t B_BYTES = BN_HALF * 128;          // 16 KB per plane (this CTA's half of the requested rows)
 constexpr uint32_t STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;   // 64 KB per CTA
+// Where 256-column blocks of requested rows would leave most SM pairs idle, the blocks are 128, 64 or 32 columns wide
+// (block_width): a tile of few columns is done sooner - its stages are smaller, so that up to five of them are in
+// flight, and its epilogue is shorter.
+constexpr int MAX_STAGES = 5, MIN_WIDTH = 32;
 // Warpgroup 0 holds the TMA producer (warp 0), the MMA issuer (warp 1) and two idle warps and gives most of its
 // registers back; the other warpgroups are the promotion / epilogue warps and take them. Default: 8 epilogue
 // warps (two per tensor-memory lane quarter, 128 columns = 128 sums per thread; a 384-thread CTA is compiled
@@ -150,6 +154,7 @@ struct PredictArgs {
 struct RowsExtra {
     const int *m_dev;
     const int *row_slot;
+    int width;                      // requested rows per block (set by the launch)
     long long *end;                 // device_ns() when the last block left (never taken back), or nullptr
 };
 
@@ -173,9 +178,9 @@ __device__ __forceinline__ int pair_index(int n_classes, int i, int j) {      //
 }
 
 // Columns (requested rows) of row block nb that the MMAs cover: all 256, or the rows left rounded up to 32
-__device__ __forceinline__ int block_columns(int m, int nb) {
-    const int left = m - nb * tc2::BN;
-    return left >= tc2::BN ? tc2::BN : ((left + 31) & ~31);
+__device__ __forceinline__ int block_columns(int m, int nb, int width) {
+    const int left = m - nb * width;
+    return left >= width ? width : ((left + 31) & ~31);
 }
 
 __device__ __forceinline__ void red_add_if(bool take, double *p, double v) {
@@ -254,21 +259,24 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
     uint64_t *bars = reinterpret_cast<uint64_t *>(ring_ptr + STAGES * STAGE_BYTES);
-    const uint32_t full_bar = smem_u32(bars), empty_bar = full_bar + 8 * STAGES;
-    const uint32_t tfull_bar = empty_bar + 8 * STAGES, tempty_bar = tfull_bar + 16;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+    const uint32_t full_bar = smem_u32(bars), empty_bar = full_bar + 8 * MAX_STAGES;
+    const uint32_t tfull_bar = empty_bar + 8 * MAX_STAGES, tempty_bar = tfull_bar + 16;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * MAX_STAGES + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-    const int pair_tiles = (n + 2 * BM - 1) / (2 * BM), n_blocks = (m + BN - 1) / BN, k_blocks = (row_len + BK - 1) / BK;
+    const int width = ex.width;
+    const uint32_t b_bytes = (uint32_t) width * 64, stage_bytes = 2 * A_BYTES + 2 * b_bytes;     // half a block's rows of 128 bytes
+    const uint32_t n_stages = min((uint32_t) MAX_STAGES, STAGES * STAGE_BYTES / stage_bytes);
+    const int pair_tiles = (n + 2 * BM - 1) / (2 * BM), n_blocks = (m + width - 1) / width, k_blocks = (row_len + BK - 1) / BK;
     // Work items are (pair tile, row block) with the row block fastest, so neighbouring clusters stream the
     // same instance slabs at the same time and the second reader finds them in L2.
     const int n_items = pair_tiles * n_blocks;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
+        for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar + 8 * a, 1); mbar_init(tempty_bar + 8 * a, 2 * EPI_WARPS); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -296,16 +304,16 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                     const int pt = item / n_blocks, nb = item - pt * n_blocks;
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         if (!mbar_wait(empty_bar + 8 * stage, phase ^ 1, abort_flag, 1)) { ok = false; break; }
-                        const uint32_t base = ring + stage * STAGE_BYTES;
+                        const uint32_t base = ring + stage * stage_bytes;
                         const uint32_t leader_full = mapa_u32(full_bar + 8 * stage, 0);
-                        if (rank == 0) mbar_expect_tx(full_bar + 8 * stage, 2 * STAGE_BYTES);
+                        if (rank == 0) mbar_expect_tx(full_bar + 8 * stage, 2 * stage_bytes);
                         // this CTA's half of the block's requested rows (a narrow last block has narrow halves)
-                        const int xrow = pt * 2 * BM + (int) rank * BM, wrow = nb * BN + (int) rank * (block_columns(m, nb) >> 1);
+                        const int xrow = pt * 2 * BM + (int) rank * BM, wrow = nb * width + (int) rank * (block_columns(m, nb, width) >> 1);
                         tma_load_2d_pair(base, &map_xhi, leader_full, kb * BK, xrow);
                         tma_load_2d_pair(base + A_BYTES, &map_xlo, leader_full, kb * BK, xrow);
                         tma_load_2d_pair(base + 2 * A_BYTES, &map_whi, leader_full, kb * BK, wrow);
-                        tma_load_2d_pair(base + 2 * A_BYTES + B_BYTES, &map_wlo, leader_full, kb * BK, wrow);
-                        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                        tma_load_2d_pair(base + 2 * A_BYTES + b_bytes, &map_wlo, leader_full, kb * BK, wrow);
+                        if (++stage == n_stages) { stage = 0; phase ^= 1; }
                     }
             }
         }
@@ -315,21 +323,21 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             for (int item = cluster_id; item < n_items && ok; item += n_clusters) {
-                    const uint32_t idesc_n = (uint32_t) (block_columns(m, item % n_blocks) >> 3) << 17;
+                    const uint32_t idesc_n = (uint32_t) (block_columns(m, item % n_blocks, width) >> 3) << 17;
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         const bool unit_start = kb % PROMO == 0, unit_end = kb % PROMO == PROMO - 1 || kb == k_blocks - 1;
                         if (unit_start && !mbar_wait(tempty_bar + 8 * acc, acc_phase ^ 1, abort_flag, 2)) { ok = false; break; }
                         if (!mbar_wait(full_bar + 8 * stage, phase, abort_flag, 3)) { ok = false; break; }
                         tc_fence_after();
                         const uint32_t d_tmem = tmem_base + acc * BN;
-                        const uint32_t base = ring + stage * STAGE_BYTES;
+                        const uint32_t base = ring + stage * stage_bytes;
 #pragma unroll
                         for (int k = 0; k < K_STEPS; ++k) {
                             const uint32_t koff = k * 32;
                             umma_pair<F16>(d_tmem, smem_desc_sw128(base + A_BYTES + koff),
                                            smem_desc_sw128(base + 2 * A_BYTES + koff), k != 0 || !unit_start, idesc_n);
                             umma_pair<F16>(d_tmem, smem_desc_sw128(base + koff),
-                                           smem_desc_sw128(base + 2 * A_BYTES + B_BYTES + koff), 1, idesc_n);
+                                           smem_desc_sw128(base + 2 * A_BYTES + b_bytes + koff), 1, idesc_n);
                         }
 #pragma unroll
                         for (int k = 0; k < K_STEPS; ++k) {
@@ -339,7 +347,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                         // stage free / slab complete, signalled in both CTAs
                         umma_commit_pair(mapa_u32(empty_bar + 8 * stage, 0));
                         umma_commit_pair(mapa_u32(empty_bar + 8 * stage, 1));
-                        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                        if (++stage == n_stages) { stage = 0; phase ^= 1; }
                         if (unit_end) {
                             umma_commit_pair(mapa_u32(tfull_bar + 8 * acc, 0));
                             umma_commit_pair(mapa_u32(tfull_bar + 8 * acc, 1));
@@ -369,7 +377,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
             const int j = pt * 2 * BM + (int) rank * BM + quarter * 32 + lane;
             const float sdj = j < n ? sd[j] : 0.0f;
             const float uxj = (F16 && j < n) ? x_unscale[j] : 1.0f;
-            const int n_cols = block_columns(m, nb);
+            const int n_cols = block_columns(m, nb, width);
             int cls_own = 0, cls_lo = 0, cls_hi = -1;
             float coef_one = 0.0f;
             if constexpr (PREDICT) {
@@ -386,7 +394,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                 // Self dot and 1/scale of this warp's 128 requested rows go to shared memory by asynchronous
                 // copies while the k loop runs: with nearly all of the SM's memory configured as shared, the
                 // L1 left over does not keep them across the epilogue's stores.
-                const int i0 = nb * BN + half * COLS_PER_THREAD;
+                const int i0 = nb * width + half * COLS_PER_THREAD;
 #pragma unroll
                 for (int c = lane; c < COLS_PER_THREAD; c += 32) {
                     if (i0 + c < m) {
@@ -602,9 +610,19 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
 tsvm_status make_map(CUtensorMap *map, const void *ptr, int rows, int row_len, long long ld, int box_rows,
                      bool f16);   // dense_tc.cu
 
+// Columns per block: halved while every tile still gets an SM pair of its own, i.e. as long as it costs no second round. A
+// tile takes 5 us, 0.73 (32 columns) to 0.87 us per k slab and 1 to 5 us of epilogue. 512 requested rows of 1,024 x 64 /
+// 784 / 2,000: 11.6 / 22.3 / 38.8 -> 6.5 / 15.6 / 29.8 us; predicting 100 rows with 1,000 x 100 70 -> 64 us, 300 with 2,000
+// x 2,000 104 -> 93 us.
+static int block_width(int pair_tiles, int m, int avail) {
+    int width = tc2::BN;
+    while (width > tc2::MIN_WIDTH && (long long) pair_tiles * ceil_div(m, width / 2) <= avail) width /= 2;
+    return width;
+}
+
 template <int EPI, bool F16, bool PREDICT>
 static tsvm_status launch_pair_kernel(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
-                                      long long ld_out, const PredictArgs &pa, const RowsExtra &ex, cudaStream_t st) {
+                                      long long ld_out, const PredictArgs &pa, const RowsExtra &ex_in, cudaStream_t st) {
     auto kernel = dense_rows_tc2_kernel<EPI, F16, PREDICT>;
     constexpr uint32_t smem_bytes = PREDICT ? tc2::SMEM_BYTES_PREDICT : tc2::SMEM_BYTES;
     static int clusters_of_device[MAX_DEVICES] = {0};      // per instantiation and per device ordinal
@@ -632,11 +650,13 @@ static tsvm_status launch_pair_kernel(tsvm_km *km, const InstancePlanes &X, cons
     const int len = km->plane_ld;
     TSVM_TRY(make_map(&mxh, X.hi, X.n, len, len, tc2::BM, F16));
     TSVM_TRY(make_map(&mxl, X.lo, X.n, len, len, tc2::BM, F16));
-    TSVM_TRY(make_map(&mwh, W.hi, m, len, len, tc2::BN_HALF, F16));
-    TSVM_TRY(make_map(&mwl, W.lo, m, len, len, tc2::BN_HALF, F16));
-    const int n_items = ceil_div(X.n, 2 * tc2::BM) * ceil_div(m, tc2::BN);
     int avail = max_clusters - km->reserve_clusters;     // SM pairs left free for a concurrent stream
     if (avail < 1) avail = 1;
+    RowsExtra ex = ex_in;
+    ex.width = km->whole_blocks ? tc2::BN : block_width(ceil_div(X.n, 2 * tc2::BM), m, avail);
+    TSVM_TRY(make_map(&mwh, W.hi, m, len, len, ex.width / 2, F16));
+    TSVM_TRY(make_map(&mwl, W.lo, m, len, len, ex.width / 2, F16));
+    const int n_items = ceil_div(X.n, 2 * tc2::BM) * ceil_div(m, ex.width);
     const int clusters = n_items < avail ? n_items : avail;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -669,7 +689,7 @@ static tsvm_status launch_pair_any(tsvm_km *km, const InstancePlanes &X, const R
 // (kind 1 = TF32 words, 2 = row-scaled FP16, the handle's plane kind), self dots and 1/scale.
 tsvm_status launch_dense_tc2_planes(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
                                     long long ld_out, cudaStream_t st) {
-    return launch_pair_any<false>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, km->rows_end_dev}, st);
+    return launch_pair_any<false>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, 0, km->rows_end_dev}, st);
 }
 
 // Prediction form: the m staged rows are test rows, the kernel matrix holds the support vectors; adds
@@ -679,7 +699,7 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
     const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
     const RowPlanes staged{km->Whi, km->Wlo, km->sd_rows, km->w_unscale};
     const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes};
-    return launch_pair_any<true>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, nullptr}, st);
+    return launch_pair_any<true>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, 0, nullptr}, st);
 }
 
 // Requested rows = the m rows staged in the handle's scratch.

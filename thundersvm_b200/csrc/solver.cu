@@ -1183,7 +1183,12 @@ struct tsvm_solver {
             const RowPlanes new_members{reinterpret_cast<const float *>(reinterpret_cast<const char *>(ws_hi) + (size_t) q * rb),
                                         reinterpret_cast<const float *>(reinterpret_cast<const char *>(ws_lo) + (size_t) q * rb),
                                         ws_sd + q, ws_unscale + q};
-            TSVM_TRY(km_rows_planes_on(km, members, new_members, q, kww + (size_t) q * ws, ws, st2));
+            // (spread over all SM pairs it is done sooner, but the big launch waits for them: with more than four rounds of
+            // tiles that one is the longer path, 200,000 x 2,000 457 ms per solve against 460)
+            km->whole_blocks = (long long) ceil_div(n, 256) * ceil_div(q, 256) > 4 * (device_sm_count() / 2);
+            const tsvm_status bs = km_rows_planes_on(km, members, new_members, q, kww + (size_t) q * ws, ws, st2);
+            km->whole_blocks = false;
+            TSVM_TRY(bs);
             TSVM_TRY(launch_local_smo(kind, ws, kww, diag_ws, y_ws, f_ws, a_ws, alpha_diff, Cp, Cn, eps, local_max_iter,
                                       diff, ids, alpha, st2, stop, times));
         }
