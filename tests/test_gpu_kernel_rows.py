@@ -298,3 +298,28 @@ def test_dense_rows_block_widths(capi, n, q, d):
     want = P.kernel_rows_idx(P.Csr(dense=X), ids, kernel="rbf", gamma=0.3 / d)
     assert rel_err(km.get_rows(torch.from_numpy(ids).cuda()).cpu().numpy(), want) < REL_TOL
     km.close()
+
+
+@pytest.mark.parametrize("engine", ["simt", "tensor2", "tensor_f16"])
+@pytest.mark.parametrize("m,dt", [(1, 41), (33, 46), (130, 38), (3600, 41)])
+def test_batches_of_new_rows(capi, engine, m, dt):
+    """Self dots and operand form of a batch in one launch: fewer and more features than the matrix, rows that are not
+    16-byte aligned, empty CSR rows, more rows than warps of the launch, one row."""
+    import torch
+    rng = np.random.default_rng(m + dt)
+    n, d = 150, 41
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    T = (rng.standard_normal((m, dt)) * (rng.random((m, dt)) < 0.6)).astype(np.float32)
+    T[m // 2] = 0
+    km = capi.KernelMatrix(dense=torch.from_numpy(X).cuda(), kernel="rbf", gamma=0.02)
+    km.set_dense_engine(engine)
+    want = P.kernel_rows_ins(P.Csr(dense=X), P.Csr(dense=T), kernel="rbf", gamma=0.02)
+    wide = np.zeros((m, dt + 3), np.float32)
+    wide[:, 1:dt + 1] = T
+    dev = torch.from_numpy(wide).cuda()
+    nz = T != 0
+    rp = np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32)
+    csr = tuple(torch.from_numpy(a).cuda() for a in (T[nz], rp, np.nonzero(nz)[1].astype(np.int32)))
+    for batch in (dict(dense=torch.from_numpy(T).cuda()), dict(dense=dev[:, 1:dt + 1]), dict(csr=csr)):
+        assert rel_err(km.get_rows_instances(**batch).cpu().numpy(), want) < REL_TOL
+    km.close()

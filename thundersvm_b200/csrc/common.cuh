@@ -274,9 +274,16 @@ tsvm_status km_rows_staged_on(tsvm_km *km, const InstancePlanes &X, int q, float
                               cudaStream_t st);
 tsvm_status km_rows_planes_on(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int q, float *out,
                               long long ld_out, cudaStream_t st);
-tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt, int ldt, cudaStream_t st);
+// What the fused prediction's contraction adds its sums to: -rho of the pair, [row][pair] (pair_stride 1) or [pair][row].
+struct SumPreset {
+    double *sums = nullptr;
+    const double *rho = nullptr;
+    long long total = 0, pair_stride = 1;
+    int n_pairs = 1;
+};
+tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt, int ldt, const SumPreset &preset, cudaStream_t st);
 tsvm_status km_stage_instances_csr(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int mm,
-                                   cudaStream_t st);
+                                   const SumPreset &preset, cudaStream_t st);
 tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev, const int *sv_class_dev,
                                      int n_classes, double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st);
 tsvm_status km_stage_rows_features(tsvm_km *km, const float *T_dev, int ldt, const float *sd_T_dev, int m,

@@ -253,10 +253,9 @@ __global__ void self_dot_csr_kernel(const float *__restrict__ val, const int *__
 // made from its own row. VEC: 16-byte copies (aligned rows), else 4-byte ones.
 constexpr int SEQ_COLS = 64, SEQ_STAGES = 4, SEQ_LD = SEQ_COLS + 4;      // row stride: 16-byte reads without bank conflicts
 template <bool VEC>
-__global__ void __launch_bounds__(32) self_dot_seq_dense_kernel(const float *__restrict__ T, int m, int dt, int ldt,
-                                                                float *__restrict__ out) {
-    __shared__ __align__(16) float tile[SEQ_STAGES][32][SEQ_LD];
-    const int lane = threadIdx.x, r0 = blockIdx.x * 32, blocks = (dt + SEQ_COLS - 1) / SEQ_COLS;
+__device__ __forceinline__ void self_dots_of_32_rows(const float *__restrict__ T, int r0, int m, int dt, int ldt,
+                                                     float (*tile)[32][SEQ_LD], float *__restrict__ out) {
+    const int lane = threadIdx.x & 31, blocks = (dt + SEQ_COLS - 1) / SEQ_COLS;
     auto fetch = [&](int kb) {
         if (kb < blocks) {
             constexpr int W = VEC ? 4 : 1, PER_ROW = SEQ_COLS / W;
@@ -291,6 +290,13 @@ __global__ void __launch_bounds__(32) self_dot_seq_dense_kernel(const float *__r
     if (r0 + lane < m) out[r0 + lane] = s;
 }
 
+template <bool VEC>
+__global__ void __launch_bounds__(32) self_dot_seq_dense_kernel(const float *__restrict__ T, int m, int dt, int ldt,
+                                                                float *__restrict__ out) {
+    __shared__ __align__(16) float tile[SEQ_STAGES][32][SEQ_LD];
+    self_dots_of_32_rows<VEC>(T, blockIdx.x * 32, m, dt, ldt, tile, out);
+}
+
 static tsvm_status launch_self_dot_seq_dense(const float *T, int m, int dt, int ldt, float *out, cudaStream_t st) {
     if ((ldt & 3) == 0 && ((uintptr_t) T & 15) == 0)
         TSVM_LAUNCH(self_dot_seq_dense_kernel<true>, ceil_div(m, 32), 32, 0, st, T, m, dt, ldt, out);
@@ -298,13 +304,15 @@ static tsvm_status launch_self_dot_seq_dense(const float *T, int m, int dt, int 
     return TSVM_OK;
 }
 
+__device__ __forceinline__ float self_dot_seq_csr(const float *__restrict__ val, int begin, int end) {
+    float s = 0;
+    for (int p = begin; p < end; ++p) s = fmaf(val[p], val[p], s);
+    return s;
+}
 __global__ void self_dot_seq_csr_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, int m,
                                         float *__restrict__ out) {
     int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= m) return;
-    float s = 0;
-    for (int p = row_ptr[r]; p < row_ptr[r + 1]; ++p) s = fmaf(val[p], val[p], s);
-    out[r] = s;
+    if (r < m) out[r] = self_dot_seq_csr(val, row_ptr[r], row_ptr[r + 1]);
 }
 
 // TF32 split x = hi + lo (+ <= 2^-22 |x|): hi = x rounded to TF32, lo = (x - hi) rounded to
@@ -490,27 +498,116 @@ __global__ void dense_from_csr_kernel(const float *__restrict__ val, const int *
     }
 }
 
-// CSR rows -> zero-initialised dense rows for the dense engines.
-__global__ void scatter_csr_to_w_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr,
-                                        const int *__restrict__ col, const int *__restrict__ idx, int m, int d,
-                                        RowDst dst) {
-    int i = blockIdx.x;
-    if (i >= m) return;
-    int r = idx ? idx[i] : i;
-    float scale = 1.0f, unscale = 1.0f;
-    if (dst.kind == 2) {
-        float amax = 0.0f;
-        for (int p = row_ptr[r] + threadIdx.x; p < row_ptr[r + 1]; p += blockDim.x)
-            if (col[p] < d) amax = fmaxf(amax, fabsf(val[p]));
-        row_scale_from_max(block_max_abs(amax), scale, unscale);
-        if (threadIdx.x == 0) dst.unscale[i] = unscale;
+// A batch of new instances as the requested rows of a dense engine, in one launch whose blocks do different things: the
+// self dots (a chain per row: the longest part, so these blocks come first), the rows in the engine's operand form (a warp
+// per row; features >= d are dropped) and, for the fused prediction, -rho into the sums that the contraction adds to.
+// Separate launches took the sum of their times and a launch each: 8 + 8.5 + 2 us per 4,096 rows of 784 features, most
+// of it latency, against MEASURED.
+constexpr int BATCH_THREADS = 128, BATCH_WARPS = BATCH_THREADS / 32;
+__device__ __forceinline__ void preset_sums(const SumPreset &p, int block) {
+    const long long e = (long long) block * BATCH_THREADS + threadIdx.x;
+    if (e < p.total) p.sums[e] = -p.rho[p.pair_stride == 1 ? e % p.n_pairs : e / p.pair_stride];
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(BATCH_THREADS)
+stage_batch_dense_kernel(const float *__restrict__ T, int ldt, int dt, int d, int m, RowDst dst, float *__restrict__ sd,
+                         int dot_blocks, int row_blocks, const SumPreset preset) {
+    __shared__ __align__(16) float tile[SEQ_STAGES][32][SEQ_LD];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int) blockIdx.x < dot_blocks) {
+        if (warp == 0) self_dots_of_32_rows<VEC>(T, blockIdx.x * 32, m, dt, ldt, tile, sd);
+        return;
     }
-    for (int p = row_ptr[r] + threadIdx.x; p < row_ptr[r + 1]; p += blockDim.x) {
-        int c = col[p];
-        if (c >= d) continue;
-        float v = val[p];
-        if (dst.W) dst.W[(size_t) i * dst.ld + c] = v;
-        else store_planes(dst.kind, dst.hi, dst.lo, (size_t) i * dst.ld + c, v, scale);
+    const int block = blockIdx.x - dot_blocks;
+    if (block >= row_blocks) return preset_sums(preset, block - row_blocks);
+    const int lim = d < dt ? d : dt;
+    for (int i = block * BATCH_WARPS + warp; i < m; i += row_blocks * BATCH_WARPS) {
+        const float *x = T + (size_t) i * ldt;
+        // four features at a time (VEC: one 16-byte load)
+        auto four = [&](int k, float (&v)[4]) {
+            if (VEC && k + 3 < lim) {
+                const float4 t = *reinterpret_cast<const float4 *>(x + k);
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = k + u < lim ? x[k + u] : 0.0f;
+            }
+        };
+        float scale = 1.0f, unscale = 1.0f;
+        if (dst.kind == 2) {
+            float amax = 0.0f;
+#pragma unroll 4
+            for (int k = 4 * lane; k < lim; k += 128) {
+                float v[4];
+                four(k, v);
+                amax = fmaxf(fmaxf(fmaxf(amax, fabsf(v[0])), fmaxf(fabsf(v[1]), fabsf(v[2]))), fabsf(v[3]));
+            }
+            amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+            row_scale_from_max(amax, scale, unscale);
+            if (lane == 0) dst.unscale[i] = unscale;
+        }
+#pragma unroll 4
+        for (int k = 4 * lane; k < dst.ld; k += 128) {          // (a row of the destination is a multiple of four long)
+            float v[4];
+            four(k, v);
+            const size_t at = (size_t) i * dst.ld + k;
+            if (dst.W) *reinterpret_cast<float4 *>(dst.W + at) = make_float4(v[0], v[1], v[2], v[3]);
+            else if (dst.kind == 2) {
+                __half h[4], l[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) split_f16(v[u] * scale, h[u], l[u]);
+                *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(dst.hi) + at) = *reinterpret_cast<const uint2 *>(h);
+                *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(dst.lo) + at) = *reinterpret_cast<const uint2 *>(l);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) store_planes(dst.kind, dst.hi, dst.lo, at + u, v[u], scale);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(BATCH_THREADS)
+stage_batch_csr_kernel(const float *__restrict__ val, const int *__restrict__ row_ptr, const int *__restrict__ col, int m, int d,
+                       RowDst dst, float *__restrict__ sd, int dot_blocks, int row_blocks, const SumPreset preset) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int) blockIdx.x < dot_blocks) {
+        const int r = blockIdx.x * BATCH_THREADS + threadIdx.x;
+        if (r < m) sd[r] = self_dot_seq_csr(val, row_ptr[r], row_ptr[r + 1]);
+        return;
+    }
+    const int block = blockIdx.x - dot_blocks;
+    if (block >= row_blocks) return preset_sums(preset, block - row_blocks);
+    for (int i = block * BATCH_WARPS + warp; i < m; i += row_blocks * BATCH_WARPS) {
+        const int b = row_ptr[i], e = row_ptr[i + 1];
+        float amax = 0.0f, scale = 1.0f, unscale = 1.0f;
+        const size_t at = (size_t) i * dst.ld;
+        if (dst.W) {
+            for (int k = 4 * lane; k < dst.ld; k += 128) *reinterpret_cast<float4 *>(dst.W + at + k) = make_float4(0, 0, 0, 0);
+        } else if (dst.kind == 2) {
+            for (int p = b + lane; p < e; p += 32)
+                if (col[p] < d) amax = fmaxf(amax, fabsf(val[p]));
+            amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+            row_scale_from_max(amax, scale, unscale);
+            if (lane == 0) dst.unscale[i] = unscale;
+            for (int k = 8 * lane; k < dst.ld; k += 256) {      // (a multiple of eight halves)
+                *reinterpret_cast<uint4 *>(reinterpret_cast<__half *>(dst.hi) + at + k) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4 *>(reinterpret_cast<__half *>(dst.lo) + at + k) = make_uint4(0, 0, 0, 0);
+            }
+        } else {
+            for (int k = 4 * lane; k < dst.ld; k += 128) {
+                *reinterpret_cast<float4 *>(dst.hi + at + k) = make_float4(0, 0, 0, 0);
+                *reinterpret_cast<float4 *>(dst.lo + at + k) = make_float4(0, 0, 0, 0);
+            }
+        }
+        __syncwarp();                                           // the zeros are in place before the entries
+        for (int p = b + lane; p < e; p += 32) {
+            const int c = col[p];
+            if (c >= d) continue;
+            if (dst.W) dst.W[at + c] = val[p];
+            else store_planes(dst.kind, dst.hi, dst.lo, at + c, val[p], scale);
+        }
+        __syncwarp();
     }
 }
 
@@ -881,9 +978,6 @@ static inline RowDst row_dst(const tsvm_km *km) {
     if (use_tensor_engine(km)) return RowDst{nullptr, km->Whi, km->Wlo, km->w_unscale, km->plane_kind, km->plane_ld};
     return RowDst{km->W, nullptr, nullptr, nullptr, 0, km->d_pad};
 }
-static inline size_t row_dst_bytes(const RowDst &r, int m) {
-    return (size_t) m * r.ld * (r.kind == 2 ? sizeof(__half) : sizeof(float));
-}
 
 static tsvm_status inspect_entries(tsvm_km *km, const float *val, const int *row_ptr, const int *col, int n, bool batch,
                                    cudaStream_t st, bool *exact) {
@@ -1041,11 +1135,20 @@ tsvm_status km_stage_rows_features(tsvm_km *km, const float *T_dev, int ldt, con
 // Stages mm new instances as the requested rows of a dense kernel matrix (self dots accumulated in storage
 // order as kernelmatrix.cpp:288-296 does, rows in the engine's operand form): the first half of
 // tsvm_km_rows_by_instances_*, shared with the fused prediction.
-tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt, int ldt, cudaStream_t st) {
+static inline int batch_row_blocks(int mm) {
+    const int all = ceil_div(mm, BATCH_WARPS), most = 6 * device_sm_count();
+    return all < most ? all : most;
+}
+tsvm_status km_stage_instances_dense(tsvm_km *km, const float *T, int mm, int dt, int ldt, const SumPreset &preset, cudaStream_t st) {
     TSVM_TRY(ensure_scratch(km, mm, false));
-    TSVM_TRY(launch_self_dot_seq_dense(T, mm, dt, ldt, km->sd_rows, st));
     TSVM_TRY(ensure_planes(km, st));
-    TSVM_LAUNCH(stage_rows_dense_kernel, mm, 256, 0, st, T, ldt, dt, km->d, mm, row_dst(km));
+    const int dots = ceil_div(mm, 32), rows = batch_row_blocks(mm), grid = dots + rows + ceil_div(preset.total, BATCH_THREADS);
+    if ((ldt & 3) == 0 && ((uintptr_t) T & 15) == 0)
+        TSVM_LAUNCH(stage_batch_dense_kernel<true>, grid, BATCH_THREADS, 0, st, T, ldt, dt, km->d, mm, row_dst(km), km->sd_rows,
+                    dots, rows, preset);
+    else
+        TSVM_LAUNCH(stage_batch_dense_kernel<false>, grid, BATCH_THREADS, 0, st, T, ldt, dt, km->d, mm, row_dst(km), km->sd_rows,
+                    dots, rows, preset);
     return TSVM_OK;
 }
 
@@ -1062,17 +1165,12 @@ tsvm_status km_pair_engine_takes(tsvm_km *km, const float *tval, const int *rp, 
 }
 
 tsvm_status km_stage_instances_csr(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int mm,
-                                   cudaStream_t st) {
+                                   const SumPreset &preset, cudaStream_t st) {
     TSVM_TRY(ensure_scratch(km, mm, false));
-    TSVM_LAUNCH(self_dot_seq_csr_kernel, ceil_div(mm, 128), 128, 0, st, tval, rp, mm, km->sd_rows);
     TSVM_TRY(ensure_planes(km, st));
-    const RowDst dst = row_dst(km);
-    if (dst.W) TSVM_CUDA(cudaMemsetAsync(dst.W, 0, row_dst_bytes(dst, mm), st));
-    else {
-        TSVM_CUDA(cudaMemsetAsync(dst.hi, 0, row_dst_bytes(dst, mm), st));
-        TSVM_CUDA(cudaMemsetAsync(dst.lo, 0, row_dst_bytes(dst, mm), st));
-    }
-    TSVM_LAUNCH(scatter_csr_to_w_kernel, mm, 128, 0, st, tval, rp, tcol, (const int *) nullptr, mm, km->d, dst);
+    const int dots = ceil_div(mm, BATCH_THREADS), rows = batch_row_blocks(mm), grid = dots + rows + ceil_div(preset.total, BATCH_THREADS);
+    TSVM_LAUNCH(stage_batch_csr_kernel, grid, BATCH_THREADS, 0, st, tval, rp, tcol, mm, km->d, row_dst(km), km->sd_rows, dots, rows,
+                preset);
     return TSVM_OK;
 }
 
@@ -1239,7 +1337,7 @@ tsvm_status tsvm_km_rows_by_instances_dense(tsvm_km *km, const float *T_dev, int
         const float *T = T_dev + (size_t) r0 * ldt;
         float *o = out_dev + (size_t) r0 * ld_out;
         if (dense) {
-            TSVM_TRY(km_stage_instances_dense(km, T, mm, dt, ldt, st));
+            TSVM_TRY(km_stage_instances_dense(km, T, mm, dt, ldt, SumPreset{}, st));
             TSVM_TRY(rows_common(km, mm, o, ld_out, st));
         } else {
             TSVM_TRY(ensure_scratch(km, mm, true));
@@ -1287,7 +1385,7 @@ tsvm_status tsvm_km_rows_by_instances_csr(tsvm_km *km, const float *tval_dev, co
         const int *rp = trow_ptr_dev + r0;     // row_ptr entries stay absolute offsets into tval/tcol
         float *o = out_dev + (size_t) r0 * ld_out;
         if (dense) {
-            TSVM_TRY(km_stage_instances_csr(km, tval_dev, rp, tcol_dev, mm, st));
+            TSVM_TRY(km_stage_instances_csr(km, tval_dev, rp, tcol_dev, mm, SumPreset{}, st));
             TSVM_TRY(rows_common(km, mm, o, ld_out, st));
         } else {
             TSVM_TRY(ensure_scratch(km, mm, true));

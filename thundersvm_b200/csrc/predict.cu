@@ -48,13 +48,6 @@ sum_kernel_values_kernel(const double *__restrict__ coef, int n_sv, const int *_
         }
 }
 
-// What the fused contraction adds its sums to: -rho of the pair. [row][pair] (pair_stride 1) or [pair][row].
-__global__ void preset_dec_kernel(double *__restrict__ dec, long long total, int nb, long long pair_stride,
-                                  const double *__restrict__ rho) {
-    const long long e = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < total) dec[e] = -rho[pair_stride == 1 ? e % nb : e / pair_stride];
-}
-
 // Three to SLAB_CLASSES classes: the contraction adds to a slab [pair][row], where the rows that a warp adds to at a time lie
 // side by side (to [row][pair] every one is a memory sector of its own: ten classes, 8,003 x 784, 173 -> 157 us per
 // 4,096 rows). This kernel turns the slab into decision values [row][pair] and / or votes (the first maximum wins).
@@ -198,9 +191,10 @@ static tsvm_status fused_slab(tsvm_km *km_sv, const double *coef_dev, const int 
                               long long pair_stride, cudaStream_t st) {
     const int nb = n_classes * (n_classes - 1) / 2;
     const long long total = pair_stride == 1 ? (long long) mm * nb : pair_stride * nb;
-    TSVM_LAUNCH(preset_dec_kernel, ceil_div(total, 256), 256, 0, st, dec, total, nb, pair_stride, rho_dev);
-    if (T_dev) TSVM_TRY(km_stage_instances_dense(km_sv, T_dev + (size_t) r0 * ldt, mm, dt, ldt, st));
-    else TSVM_TRY(km_stage_instances_csr(km_sv, tval_dev, trow_ptr_dev + r0, tcol_dev, mm, st));
+    SumPreset preset;
+    preset.sums = dec; preset.rho = rho_dev; preset.total = total; preset.pair_stride = pair_stride; preset.n_pairs = nb;
+    if (T_dev) TSVM_TRY(km_stage_instances_dense(km_sv, T_dev + (size_t) r0 * ldt, mm, dt, ldt, preset, st));
+    else TSVM_TRY(km_stage_instances_csr(km_sv, tval_dev, trow_ptr_dev + r0, tcol_dev, mm, preset, st));
     return launch_dense_tc2_predict(km_sv, mm, coef_dev, sv_class, n_classes, dec, pair_stride == 1 ? nb : 1, pair_stride, st);
 }
 
