@@ -268,37 +268,37 @@ __global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ di
         ids[threadIdx.x] = staying;
     }
     if (threadIdx.x != 0) return;
-    const double d = diff[0];
-    c->diff0 = d;
-    c->local_iter += (long long) diff[1];
-    // csmosolver.cpp:86-111
-    if (fabs(d - c->prev) < eps * 0.001) c->same_cnt++;
-    else { c->same_cnt = 0; c->prev = d; }
-    if (fabs(d - c->second_last) < eps * 0.001) c->swap_cnt++;
-    else c->swap_cnt = 0;
-    c->second_last = c->last;
-    c->last = d;
-    int stop = 0;
-    if ((c->same_cnt >= 10 && fabs(d - 2.0) > eps) || d < eps || (c->swap_cnt >= 10 && fabs(d - 2.0) > eps)) {
-        c->done = 1;
-        stop = 1;
-    }
-    c->iter++;
-    if (max_iter != -1 && c->iter - 1 == max_iter) stop = 1;      // iteration cap (csmosolver.cpp:110)
-    if (*got < wanted) { c->short_got = *got; c->short_wanted = wanted; stop = 1; }
-    if (engine_status && *engine_status) { c->engine_status = *engine_status; stop = 1; }
+    // everything is read before anything is written, so that the reads are in flight together (5.2 -> 4.4 us against
+    // reads that each waited for the write before them)
+    SolverCtl v = *c;
+    const double d = diff[0], steps = diff[1];
+    const int found = *got, engine = engine_status ? *engine_status : 0;
     if (cache_ctr)
-        for (int k = 0; k < CACHE_CTRS; ++k) c->ctr[k] = cache_ctr[k];
-    c->stop = stop;
+#pragma unroll
+        for (int k = 0; k < CACHE_CTRS; ++k) v.ctr[k] = cache_ctr[k];
+    v.diff0 = d;
+    v.local_iter += (long long) steps;
+    // csmosolver.cpp:86-111
+    if (fabs(d - v.prev) < eps * 0.001) v.same_cnt++;
+    else { v.same_cnt = 0; v.prev = d; }
+    if (fabs(d - v.second_last) < eps * 0.001) v.swap_cnt++;
+    else v.swap_cnt = 0;
+    v.second_last = v.last;
+    v.last = d;
+    if ((v.same_cnt >= 10 && fabs(d - 2.0) > eps) || d < eps || (v.swap_cnt >= 10 && fabs(d - 2.0) > eps)) v.stop = v.done = 1;
+    v.iter++;
+    if (max_iter != -1 && v.iter - 1 == max_iter) v.stop = 1;     // iteration cap (csmosolver.cpp:110)
+    if (found < wanted) { v.short_got = found; v.short_wanted = wanted; v.stop = 1; }
+    if (engine) { v.engine_status = engine; v.stop = 1; }
     if (progress) {
         // how far the solve is, for the host that waits for it: a word of pinned host memory
-        *progress = ((unsigned long long) c->iter << 1) | (unsigned) stop;
-        const PhaseTimes t = c->times;
-        c->ns_select += t.select_end - t.select_begin;
-        c->ns_rows += t.rows_end - t.select_end;
-        c->ns_local += t.local_end - t.local_begin;
-        c->ns_update += now - t.update_begin;
+        *progress = ((unsigned long long) v.iter << 1) | (unsigned) v.stop;
+        v.ns_select += v.times.select_end - v.times.select_begin;
+        v.ns_rows += v.times.rows_end - v.times.select_end;
+        v.ns_local += v.times.local_end - v.times.local_begin;
+        v.ns_update += now - v.times.update_begin;
     }
+    *c = v;
 }
 
 // *any becomes non-zero if one of a[0..n) is
