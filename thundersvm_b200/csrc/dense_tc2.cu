@@ -456,6 +456,82 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                     cls_lo = __reduce_min_sync(0xffffffffu, cls_own);
                     cls_hi = __reduce_max_sync(0xffffffffu, cls_own);
                 }
+                // the own instance's kernel values with test rows cbase .. cbase + 15, whose sums are in `priv`
+                auto values = [&](int cbase, float *kv) {
+                    if constexpr (EPI == EPI_RBF) {
+                        float a_i[EPI_CHUNK], s_i[EPI_CHUNK];
+#pragma unroll
+                        for (int c4 = 0; c4 < EPI_CHUNK; c4 += 4) {
+                            const float4 av = *reinterpret_cast<const float4 *>(rowc + cbase + c4);
+                            const float4 sv = *reinterpret_cast<const float4 *>(rowc + COLS_PER_THREAD + cbase + c4);
+                            a_i[c4] = av.x; a_i[c4 + 1] = av.y; a_i[c4 + 2] = av.z; a_i[c4 + 3] = av.w;
+                            s_i[c4] = sv.x; s_i[c4 + 1] = sv.y; s_i[c4 + 2] = sv.z; s_i[c4 + 3] = sv.w;
+                        }
+#pragma unroll
+                        for (int c = 0; c < EPI_CHUNK; ++c) {
+                            float dot = priv[c * (EPI_WARPS * 32)];
+                            if constexpr (F16) dot *= uxj;
+                            const float arg = fmaf(dot, s_i[c], a_i[c]) + pred_b;
+                            float e;
+                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(arg));
+                            kv[c] = j < n ? e : 0.0f;
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < EPI_CHUNK; ++c) {
+                            float dot = priv[c * (EPI_WARPS * 32)];
+                            if constexpr (F16) dot = dot * uxj * rowc[COLS_PER_THREAD + cbase + c];
+                            kv[c] = j < n ? epilogue_value<EPI>(fn, dot, rowc[cbase + c], sdj) : 0.0f;
+                        }
+                    }
+                };
+                if constexpr (PREDICT) if (nc == 1) {
+                    // One coefficient per instance: 32 columns at a time, every value times the instance's coefficient and
+                    // then added up over the 32 lanes with exchanges that halve the number of live columns per step (16 + 8
+                    // + 4 + 2 + 1 shuffles); lane c ends with column c and adds the warp's sum to the row's place. No
+                    // exchange between warps. What bounds it is the chain of the steps, with two such warps per scheduler,
+                    // so that 32 columns per chain beat 16: 12,001 x 123 per 4,096 rows 87 -> 64 us, 200,000 x 2,000 7.45 -> 7.3 ms.
+                    static_assert(EPI_CHUNK == 16 && COLS_PER_THREAD == 128, "four groups of two chunks");
+#pragma unroll 1
+                    for (int group = 0; group < COLS_PER_THREAD / 32; ++group) {
+                        if (half * COLS_PER_THREAD + group * 32 >= n_cols) break;
+                        float kv[32];
+                        switch (group) {
+                            case 0: stage_chunk<0>(sum, priv); break;
+                            case 1: stage_chunk<2>(sum, priv); break;
+                            case 2: stage_chunk<4>(sum, priv); break;
+                            default: stage_chunk<6>(sum, priv); break;
+                        }
+                        values(group * 32, kv);
+                        switch (group) {
+                            case 0: stage_chunk<1>(sum, priv); break;
+                            case 1: stage_chunk<3>(sum, priv); break;
+                            case 2: stage_chunk<5>(sum, priv); break;
+                            default: stage_chunk<7>(sum, priv); break;
+                        }
+                        values(group * 32 + 16, kv + 16);
+                        // (both classes add to the one pair; a lane beyond the last instance has coefficient 0)
+                        float w[16];
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) {
+                            const bool upper = (lane & 16) != 0;
+                            const float send = coef_one * (upper ? kv[c] : kv[c + 16]);
+                            w[c] = fmaf(coef_one, upper ? kv[c + 16] : kv[c], __shfl_xor_sync(0xffffffffu, send, 16));
+                        }
+#pragma unroll
+                        for (int n_left = 8; n_left >= 1; n_left >>= 1)
+#pragma unroll
+                            for (int c = 0; c < n_left; ++c) {
+                                const bool upper = (lane & n_left) != 0;
+                                const float send = upper ? w[c] : w[c + n_left];
+                                w[c] = (upper ? w[c + n_left] : w[c]) + __shfl_xor_sync(0xffffffffu, send, n_left);
+                            }
+                        const int r = i0 + group * 32 + lane;
+                        if (r < m) atomicAdd(pa.dec + r, (double) w[0]);
+                    }
+                    __syncwarp();          // the next item's copies overwrite rowc
+                    continue;
+                }
 #pragma unroll 1
                 for (int ch = 0; ch < COLS_PER_THREAD / EPI_CHUNK; ++ch) {
                     if (half * COLS_PER_THREAD + ch * EPI_CHUNK >= n_cols) break;
@@ -491,39 +567,10 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                             }
                         }
                     } else {
-                        // Kernel values of the own instance for the chunk's 16 test rows, times the instance's
-                        // coefficient; then the 32 lanes' products are added column by column with a butterfly
-                        // that halves the number of live columns per step (16 -> 8 -> 4 -> 2 -> 1 values per
-                        // lane, 31 shuffles for 16 columns), and one lane of every pair adds the warp's sum of
-                        // its column to the decision value. No exchange between warps: every warp adds the sums
-                        // of its own 32 instances.
+                        // Several coefficients per instance: the sums of the warp's 32 instances for the chunk's 16 test
+                        // rows, as above but once per coefficient where shared memory does not hold them all.
                         float kv[EPI_CHUNK];
-                        if constexpr (EPI == EPI_RBF) {
-                            float a_i[EPI_CHUNK], s_i[EPI_CHUNK];
-#pragma unroll
-                            for (int c4 = 0; c4 < EPI_CHUNK; c4 += 4) {
-                                const float4 av = *reinterpret_cast<const float4 *>(rowc + cbase + c4);
-                                const float4 sv = *reinterpret_cast<const float4 *>(rowc + COLS_PER_THREAD + cbase + c4);
-                                a_i[c4] = av.x; a_i[c4 + 1] = av.y; a_i[c4 + 2] = av.z; a_i[c4 + 3] = av.w;
-                                s_i[c4] = sv.x; s_i[c4 + 1] = sv.y; s_i[c4 + 2] = sv.z; s_i[c4 + 3] = sv.w;
-                            }
-#pragma unroll
-                            for (int c = 0; c < EPI_CHUNK; ++c) {
-                                float dot = priv[c * (EPI_WARPS * 32)];
-                                if constexpr (F16) dot *= uxj;
-                                const float arg = fmaf(dot, s_i[c], a_i[c]) + pred_b;
-                                float e;
-                                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(arg));
-                                kv[c] = j < n ? e : 0.0f;
-                            }
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < EPI_CHUNK; ++c) {
-                                float dot = priv[c * (EPI_WARPS * 32)];
-                                if constexpr (F16) dot = dot * uxj * rowc[COLS_PER_THREAD + cbase + c];
-                                kv[c] = j < n ? epilogue_value<EPI>(fn, dot, rowc[cbase + c], sdj) : 0.0f;
-                            }
-                        }
+                        values(cbase, kv);
                         if (nc > 1 && nc <= PRED_NC_SMEM) {
                             // Several coefficients per instance: the butterfly below would repeat its 31 shuffles for
                             // each of them. Instead the warp's 32 x 16 kernel values go back to shared memory and a lane
@@ -533,8 +580,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                             // 4,096 rows: 290 us with the butterfly, 247 with one column and 16 instances per lane (36
                             // instead of 18 reads of coefficients, each as long as four stores), 189 with two, 177 with a
                             // fixed number of coefficients, 173 without branches around the additions, 157 with the
-                            // additions side by side. (With one coefficient the butterfly is faster, 93 against 109 us at
-                            // 12,001 x 123.)
+                            // additions side by side.
                             float *block = priv - lane;
                             const float *cf_block = coef_priv - lane;
                             __syncwarp();                    // everyone has read its own sums
@@ -557,9 +603,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                         const int r = i0 + cbase + col;
                         for (int cl = cls_lo; cl <= cls_hi; ++cl)
                             for (int cr = 0; cr < nc; ++cr) {
-                                float cf;
-                                if (nc == 1) cf = coef_one;
-                                else cf = j < n ? (float) pa.coef[(size_t) cr * n + j] : 0.0f;
+                                float cf = j < n ? (float) pa.coef[(size_t) cr * n + j] : 0.0f;
                                 if (cls_own != cl) cf = 0.0f;
                                 float w[EPI_CHUNK];
 #pragma unroll
@@ -579,11 +623,8 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
 #pragma unroll
                                 for (int o = REST >> 1; o >= 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
                                 if ((lane & (REST - 1)) == 0 && r < m && total != 0.0f) {
-                                    if (nc == 1) atomicAdd(pa.dec + r, (double) total);          // (one pair: its sums lie side by side)
-                                    else {
-                                        const int k = cr < cl ? pair_index(pa.n_classes, cr, cl) : pair_index(pa.n_classes, cl, cr + 1);
-                                        atomicAdd(pa.dec + r * pa.row_stride + k * pa.pair_stride, (double) total);
-                                    }
+                                    const int k = cr < cl ? pair_index(pa.n_classes, cr, cl) : pair_index(pa.n_classes, cl, cr + 1);
+                                    atomicAdd(pa.dec + r * pa.row_stride + k * pa.pair_stride, (double) total);
                                 }
                             }
                     }
