@@ -97,16 +97,19 @@ void DataSet::load_from_sparse(int row_size, float *val, int *row_ptr, int *col_
     node2d &instances_ = *rows_;
     y_.clear(); total_count_ = 0; n_features_ = 0;
     instances_.resize(row_size);
+    if (label) y_.assign(label, label + row_size);
+    int largest = 0;
+#pragma omp parallel for schedule(static) reduction(max : largest) if (row_size > 1024)
     for (int r = 0; r < row_size; ++r) {
-        if (label) y_.push_back(label[r]);
         auto &row = instances_[r];
         row.reserve(row_ptr[r + 1] - row_ptr[r]);
         for (int p = row_ptr[r]; p < row_ptr[r + 1]; ++p) {
             const int idx = col_ptr[p] + 1;                 // to the one-based convention
             row.emplace_back(idx, val[p]);
-            if ((size_t) idx > n_features_) n_features_ = idx;
+            if (idx > largest) largest = idx;
         }
     }
+    n_features_ = (size_t) largest;
     total_count_ = row_size;
     LOG(INFO) << "#instances = " << n_instances() << ", #features = " << n_features();
 }

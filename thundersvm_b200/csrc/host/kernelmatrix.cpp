@@ -4,6 +4,7 @@
 #include <thundersvm/solver/csmosolver.h>
 #include <thundersvm/solver/nusmosolver.h>
 #include <cuda_runtime.h>
+#include <mutex>
 #include "../common.cuh"
 
 namespace {
@@ -42,8 +43,6 @@ KernelMatrix::KernelMatrix(const DataSet::node2d &instances, SvmParam param) : p
         km_->nnz = (long long) nnz_;
     }
     thundersvm::total_memory_size() += (dense_ ? (size_t) dense_bytes : nnz_ * 8 + n_instances_ * 12);
-    diag_.resize(n_instances_);
-    thundersvm::copy_to_host(diag_.host_data(), km_->diag, sizeof(kernel_type) * n_instances_);
 }
 
 KernelMatrix::KernelMatrix(const float *X_dev, size_t d, size_t ld, size_t r0, size_t n0, size_t r1, size_t n1,
@@ -60,8 +59,6 @@ KernelMatrix::KernelMatrix(const float *X_dev, size_t d, size_t ld, size_t r0, s
                                      param.degree, (float) param.gamma, (float) param.coef0, thundersvm::work_stream(), &km_));
     const double dense_bytes = 3.0 * n_instances_ * ((n_features_ + 3) & ~3ul) * 4.0 + 1024.0 * n_instances_ * 4.0;
     thundersvm::total_memory_size() += (size_t) dense_bytes;
-    diag_.resize(n_instances_);
-    thundersvm::copy_to_host(diag_.host_data(), km_->diag, sizeof(kernel_type) * n_instances_);
 }
 
 KernelMatrix::~KernelMatrix() {
@@ -88,7 +85,16 @@ void KernelMatrix::get_rows(const DataSet::node2d &instances, SyncArray<kernel_t
     cudaStreamSynchronize(thundersvm::work_stream());
 }
 
-const SyncArray<kernel_type> &KernelMatrix::diag() const { return diag_; }
+// (copied when someone asks: a solve does not, and the copy is a wait)
+const SyncArray<kernel_type> &KernelMatrix::diag() const {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    if (diag_.size() != n_instances_) {
+        diag_.resize(n_instances_);
+        thundersvm::copy_to_host(diag_.host_data(), km_->diag, sizeof(kernel_type) * n_instances_);
+    }
+    return diag_;
+}
 
 int CSMOSolver::solver_kind() const { return TSVM_SOLVER_C; }
 int NuSMOSolver::solver_kind() const { return for_svr ? TSVM_SOLVER_NU_SVR : TSVM_SOLVER_NU_SVC; }
