@@ -16,10 +16,13 @@ void set_error(const char *fmt, ...);
 long long launch_count();
 void count_launch(int k = 1);
 
+// A failed call leaves its error behind for the next cudaPeekAtLastError of the thread (TSVM_LAUNCH), which would report
+// it as a failure of its own launch: what has been reported here is cleared. (An error that ends the context comes back.)
 #define TSVM_CUDA(expr)                                                                          \
     do {                                                                                         \
         cudaError_t e__ = (expr);                                                                \
         if (e__ != cudaSuccess) {                                                                \
+            cudaGetLastError();                                                                  \
             tsvm::set_error("%s failed at %s:%d: %s", #expr, __FILE__, __LINE__,                 \
                             cudaGetErrorString(e__));                                            \
             return e__ == cudaErrorMemoryAllocation ? TSVM_ERR_OOM : TSVM_ERR_CUDA;              \

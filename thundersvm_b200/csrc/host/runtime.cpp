@@ -14,6 +14,7 @@ void set_verbose(bool on) { g_verbose = on; }
 
 static void cuda_ok(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return;
+    cudaGetLastError();                                               // reported here, not by the next launch too
     if (e == cudaErrorMemoryAllocation) throw std::bad_alloc();       // reference: util/common.h:33-39
     LOG(FATAL) << what << ": " << cudaGetErrorString(e);
 }
