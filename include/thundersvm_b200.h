@@ -318,7 +318,8 @@ tsvm_status tsvm_update_f(double *f_dev, int n, const double *alpha_diff_dev, in
  * batch is dense (T_dev != NULL) or CSR. Batching over the test rows is internal. With dense support
  * vectors of more than 32 features the coefficient sums are part of the contraction's epilogue (FP32
  * partial sums over 128 support vectors, combined in FP64) and the test x SV kernel block is never stored;
- * otherwise it is computed in slabs of at most max_mem_bytes (0 = a sixteenth of the device's memory). */
+ * otherwise it is computed in slabs of at most max_mem_bytes (0 = a sixteenth of the device's memory).
+ * Where a slab does not fit what the device has left, it is halved until it does. */
 tsvm_status tsvm_predict_dec(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host,
                              const double *rho_dev, int n_classes, int m, const float *T_dev, int dt, int ldt,
                              const float *tval_dev, const int *trow_ptr_dev, const int *tcol_dev, long long tnnz,

@@ -33,3 +33,54 @@ s, S, keep = solver(h, 20000)
 check(s)
 assert F.fake_largest_refused() > 1400 * MB, F.fake_largest_refused()
 """)
+
+
+PREDICT = """
+def predict(h, n_sv, m, classes=2, budget=0, dense=None, csr=None, labels=False):
+    count = np.full(classes, n_sv // classes, np.int32)
+    count[-1] += n_sv - count.sum()
+    coef, rho = np.ones((classes - 1, n_sv)), np.zeros(classes * (classes - 1) // 2)
+    out = np.zeros(m * max(1, len(rho)))
+    batch = (p(dense), dense.shape[1], dense.shape[1], None, None, None) if csr is None else (None, 0, 0) + tuple(map(p, csr))
+    nnz = 0 if csr is None else len(csr[0])
+    f = L.tsvm_predict_labels if labels else L.tsvm_predict_dec
+    return f(h, p(coef), p(count), p(rho), classes, m, *batch, C.c_longlong(nnz), p(out), C.c_size_t(budget), None)
+"""
+
+
+@pytest.mark.parametrize("free_mb", [300, 205, 64])
+def test_prediction_takes_smaller_slabs(runtime, free_mb):
+    """The stored kernel block of 10,000 x 20,000 (800 MB) does not fit; neither does the largest one that would leave no
+    room for the staging panel (20 MB)."""
+    fake_device.run_python(runtime, PREDICT + """
+s, h, keep = csr(20000, 5000, 70)
+check(s)
+s, h2, rows = csr(10000, 5000, 70)
+F.fake_set_free(%d * MB)
+check(predict(h, 20000, 10000, csr=rows))
+assert F.fake_largest_refused() >= 800000000
+F.fake_set_free(0)
+L.tsvm_release_cached_memory()
+""" % free_mb)
+
+
+def test_fused_prediction_takes_smaller_slabs(runtime):
+    """4,096 staged rows of 4,096 features take 200 MB."""
+    fake_device.run_python(runtime, PREDICT + """
+s, h = dense(np.ones((2000, 4096), np.float32))
+check(s)
+F.fake_set_free(100 * MB)
+check(predict(h, 2000, 5000, classes=3, dense=np.ones((5000, 4096), np.float32), labels=True))
+""")
+
+
+def test_prediction_without_room_for_one_row_is_refused(runtime):
+    fake_device.run_python(runtime, PREDICT + """
+s, h, keep = csr(20000, 5000, 70)
+check(s)
+s, h2, rows = csr(300, 5000, 70)
+F.fake_set_free(0)
+check(predict(h, 20000, 300, csr=rows), OOM)
+F.fake_set_free(100 * MB)
+check(predict(h, 20000, 300, csr=rows))
+""")

@@ -264,40 +264,12 @@ static tsvm_status predict_few(tsvm_km *km, const double *coef_dev, const int *s
     return TSVM_OK;
 }
 
-// labels_dev != nullptr: only the vote leaves the slab (sum_kernel_values_instant); dec_dev is then unused.
-static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host, const double *rho_dev,
-                                int n_classes, int m, const float *T_dev, int dt, int ldt, const float *tval_dev,
-                                const int *trow_ptr_dev, const int *tcol_dev, long long tnnz, double *dec_dev,
-                                int *labels_dev, size_t max_mem_bytes, cudaStream_t st) {
-    const int n_sv = km_sv->n;
-    int total = 0;
-    std::vector<int> start(n_classes), count(n_classes);
-    for (int c = 0; c < n_classes; ++c) { start[c] = total; count[c] = sv_count_host[c]; total += count[c]; }
-    TSVM_REQUIRE(total == n_sv, "predict: support-vector counts sum to %d but the matrix holds %d", total, n_sv);
-    km_sv->launched(st);
-    bool taken = false;
-    TSVM_TRY(predict_few(km_sv, coef_dev, sv_count_host, rho_dev, n_classes, m, T_dev, dt, ldt, tval_dev, trow_ptr_dev,
-                         tcol_dev, tnnz, dec_dev, labels_dev, st, &taken));
-    if (taken) { km_sv->waited(st); return TSVM_OK; }
-    const int nb = n_classes * (n_classes - 1) / 2;
-    bool fused = false;
-    TSVM_TRY(km_pair_engine_takes(km_sv, T_dev ? nullptr : tval_dev, T_dev ? nullptr : trow_ptr_dev, tcol_dev, m, st, &fused));
-    const long long ldk = ((long long) n_sv + 3) & ~3ll;
-    long long batch = FUSED_ROWS;
-    if (!fused) {
-        // the kernel block of a slab must fit the budget (svmmodel.cpp:86-89 caps a batch at 10000 rows)
-        size_t budget = max_mem_bytes;
-        if (!budget) {
-            // what all rows need, if that is no more than a sixteenth of the device
-            budget = (size_t) (m < 10000 ? m : 10000) * (size_t) ldk * sizeof(float);
-            const size_t most = device_memory_bytes() / 16;
-            if (budget > most) budget = most;
-        }
-        batch = (long long) (budget / sizeof(float) / (size_t) ldk);
-        if (batch > 10000) batch = 10000;
-    }
-    if (batch > m) batch = m;
-    if (batch < 1) batch = 1;
+// All m rows, `batch` at a time, and a wait for the last of them.
+static tsvm_status predict_slabs(tsvm_km *km_sv, const double *coef_dev, const std::vector<int> &start, const std::vector<int> &count,
+                                 const double *rho_dev, int m, const float *T_dev, int dt, int ldt, const float *tval_dev,
+                                 const int *trow_ptr_dev, const int *tcol_dev, double *dec_dev, int *labels_dev, bool fused,
+                                 long long batch, long long ldk, cudaStream_t st) {
+    const int n_sv = km_sv->n, n_classes = (int) start.size(), nb = n_classes * (n_classes - 1) / 2;
     float *K = nullptr;
     int *meta = nullptr, *sv_class = nullptr;
     double *dec_slab = nullptr;
@@ -353,6 +325,51 @@ static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const in
         }
     } else cudaStreamSynchronize(st);
     pool_free_many({K, meta, sv_class, dec_slab}, s == TSVM_OK);      // (only this stream has used them)
+    return s;
+}
+
+// labels_dev != nullptr: only the vote leaves the slab (sum_kernel_values_instant); dec_dev is then unused.
+static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host, const double *rho_dev,
+                                int n_classes, int m, const float *T_dev, int dt, int ldt, const float *tval_dev,
+                                const int *trow_ptr_dev, const int *tcol_dev, long long tnnz, double *dec_dev,
+                                int *labels_dev, size_t max_mem_bytes, cudaStream_t st) {
+    const int n_sv = km_sv->n;
+    int total = 0;
+    std::vector<int> start(n_classes), count(n_classes);
+    for (int c = 0; c < n_classes; ++c) { start[c] = total; count[c] = sv_count_host[c]; total += count[c]; }
+    TSVM_REQUIRE(total == n_sv, "predict: support-vector counts sum to %d but the matrix holds %d", total, n_sv);
+    km_sv->launched(st);
+    bool taken = false;
+    TSVM_TRY(predict_few(km_sv, coef_dev, sv_count_host, rho_dev, n_classes, m, T_dev, dt, ldt, tval_dev, trow_ptr_dev,
+                         tcol_dev, tnnz, dec_dev, labels_dev, st, &taken));
+    if (taken) { km_sv->waited(st); return TSVM_OK; }
+    bool fused = false;
+    TSVM_TRY(km_pair_engine_takes(km_sv, T_dev ? nullptr : tval_dev, T_dev ? nullptr : trow_ptr_dev, tcol_dev, m, st, &fused));
+    const long long ldk = ((long long) n_sv + 3) & ~3ll;
+    long long batch = FUSED_ROWS;
+    if (!fused) {
+        // the kernel block of a slab must fit the budget (svmmodel.cpp:86-89 caps a batch at 10000 rows)
+        size_t budget = max_mem_bytes;
+        if (!budget) {
+            // what all rows need, if that is no more than a sixteenth of the device
+            budget = (size_t) (m < 10000 ? m : 10000) * (size_t) ldk * sizeof(float);
+            const size_t most = device_memory_bytes() / 16;
+            if (budget > most) budget = most;
+        }
+        batch = (long long) (budget / sizeof(float) / (size_t) ldk);
+        if (batch > 10000) batch = 10000;
+    }
+    if (batch > m) batch = m;
+    if (batch < 1) batch = 1;
+    // The size of the slab is a guess at what is free. Where the device has less (for the slab or for the staging scratch of
+    // its rows), half of it will do: every slab writes all of its rows' results, so starting over is safe.
+    tsvm_status s;
+    for (;;) {
+        s = predict_slabs(km_sv, coef_dev, start, count, rho_dev, m, T_dev, dt, ldt, tval_dev, trow_ptr_dev, tcol_dev, dec_dev,
+                          labels_dev, fused, batch, ldk, st);
+        if (s != TSVM_ERR_OOM || batch == 1) break;
+        batch = (batch + 1) / 2;
+    }
     if (s == TSVM_OK) km_sv->waited(st);
     return s;
 }
