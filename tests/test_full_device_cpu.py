@@ -84,3 +84,58 @@ check(predict(h, 20000, 300, csr=rows), OOM)
 F.fake_set_free(100 * MB)
 check(predict(h, 20000, 300, csr=rows))
 """)
+
+
+@pytest.mark.parametrize("free_mb", [20, 35])
+def test_sparse_data_without_room_for_a_dense_copy(runtime, free_mb):
+    """30,000 x 200 as dense rows: 24 MB and two planes of 12 MB; the entries take 3.4 MB."""
+    fake_device.run_python(runtime, """
+F.fake_set_free(%d * MB)
+s, h, keep = csr(30000, 200, 14)
+check(s)
+idx, out = np.arange(64, dtype=np.int32), np.zeros((64, 30000), np.float32)
+check(L.tsvm_km_rows_by_index(h, p(idx), 64, p(out), C.c_longlong(30000), None))
+""" % free_mb)
+
+
+def test_a_solver_takes_the_room_of_a_dense_copy(runtime):
+    """The smallest row buffer of a solve (184 MB) fits next to the entries, not next to the dense copy (48 MB) too. A
+    solver that holds the handle keeps its storage as it is."""
+    fake_device.run_python(runtime, """
+s, h, keep = csr(30000, 200, 14)
+check(s)
+assert F.fake_used() > 48 * MB
+F.fake_set_free(170 * MB)
+s, S, keep2 = solver(h, 30000, 1024)
+check(s)
+L.tsvm_solver_destroy(S)
+L.tsvm_km_destroy(h)
+L.tsvm_release_cached_memory()
+s, h, keep = csr(30000, 200, 14)
+F.fake_set_free(250 * MB)
+s, S, keep2 = solver(h, 30000, 1024)
+check(s)
+F.fake_set_free(170 * MB)
+s, S2, keep3 = solver(h, 30000, 1024)
+check(s, OOM)
+L.tsvm_solver_destroy(S)
+L.tsvm_km_destroy(h)
+""")
+
+
+def test_dense_data_without_room_for_planes(runtime):
+    """The planes are for the engines that read them: without room the handle is made, and a CUDA-core row can be asked for."""
+    fake_device.run_python(runtime, """
+X = np.ones((30000, 200), np.float32)
+F.fake_set_free(28 * MB)
+s, h = dense(X)
+check(s)
+idx, out = np.arange(64, dtype=np.int32), np.zeros((64, 30000), np.float32)
+rows = lambda: L.tsvm_km_rows_by_index(h, p(idx), 64, p(out), C.c_longlong(30000), None)
+check(rows(), OOM)
+check(L.tsvm_km_set_dense_engine(h, 1))
+check(rows())
+F.fake_set_free(100 * MB)
+check(L.tsvm_km_set_dense_engine(h, 0))
+check(rows())
+""")

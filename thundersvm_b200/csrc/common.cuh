@@ -8,6 +8,7 @@
 #include <math.h>
 #include <atomic>
 #include <initializer_list>
+#include <memory>
 #include "../../include/thundersvm_b200.h"
 
 namespace tsvm {
@@ -205,6 +206,7 @@ struct tsvm_km {
     long long nnz = 0;
     bool dense = true;
     bool from_csr = false;          // X is a copy made of CSR data, which stays next to it
+    std::shared_ptr<char> storage_users = std::make_shared<char>();     // copied by every solver, which relies on the storage
     tsvm::KernelFn fn{};
     // 0 = automatic, 1 = CUDA-core FP32, 2 = tcgen05 TF32 planes single CTA, 3 = tcgen05 TF32 planes CTA pairs,
     // 4 = tcgen05 row-scaled FP16 planes CTA pairs
@@ -263,6 +265,7 @@ namespace tsvm {
 // Pieces of tsvm_km_rows_by_index (km.cu) for callers that overlap them with other work.
 tsvm_status km_create_dense(const float *X, int n, int d, int ld, int loc, bool zero_padded, int kernel_type, int degree,
                             float gamma, float coef0, void *stream, tsvm_km **out);
+void km_drop_dense_copy(tsvm_km *km);          // from_csr: back to the entries, e.g. where a solver needs the room
 bool km_pair_engine(tsvm_km *km, cudaStream_t st);
 tsvm_status km_pair_engine_takes(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int m, cudaStream_t st,
                                  bool *takes);

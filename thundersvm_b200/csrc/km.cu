@@ -990,7 +990,17 @@ static tsvm_status inspect_entries(tsvm_km *km, const float *val, const int *row
     return TSVM_OK;
 }
 
-// Makes the dense copy of CSR data whose kernel rows the tensor-core engine computes faster and as exactly.
+// Back to the CSR form of the data (nothing uses the dense copy any more): pool_free_many waits for the device.
+void km_drop_dense_copy(tsvm_km *km) {
+    pool_free_many({km->X_owned, km->Xhi, km->Xlo, km->x_unscale, km->W, km->Whi, km->Wlo, km->w_unscale});
+    km->X_owned = km->Xhi = km->Xlo = km->x_unscale = km->W = km->Whi = km->Wlo = km->w_unscale = nullptr;
+    km->X = nullptr;
+    km->w_cap = km->plane_kind = km->plane_ld = km->d_pad = km->ldx = 0;
+    km->dense = km->from_csr = false;
+}
+
+// Makes the dense copy of CSR data whose kernel rows the tensor-core engine computes faster and as exactly. Where the
+// device has no room for it and its planes the entries do as well.
 static tsvm_status choose_csr_storage(tsvm_km *km, cudaStream_t st) {
     const int d_pad = (km->d + 3) & ~3;
     const double dense_bytes = (double) km->n * d_pad * 8.0;             // the rows and their two planes
@@ -1002,11 +1012,16 @@ static tsvm_status choose_csr_storage(tsvm_km *km, cudaStream_t st) {
     TSVM_TRY(inspect_entries(km, km->val, km->row_ptr, km->col, km->n, false, st, &exact));
     km->nnz = km->status_host[3];
     if (!exact || (km->d > CSR_DENSE_ANY_D && km->nnz < CSR_DENSE_SHARE * (double) km->n * km->d)) return TSVM_OK;
-    TSVM_TRY(dev_alloc(&km->X_owned, (size_t) km->n * d_pad));
-    TSVM_LAUNCH(dense_from_csr_kernel, prepare_grid(km->n), 256, 0, st, km->val, km->row_ptr, km->col, km->n, d_pad, km->X_owned);
-    km->X = km->X_owned;
     km->ldx = km->d_pad = d_pad;
     km->dense = km->from_csr = true;
+    tsvm_status s = dev_alloc(&km->X_owned, (size_t) km->n * d_pad);
+    if (s == TSVM_OK) s = alloc_planes(km, wanted_plane_kind(km));
+    if (s != TSVM_OK) {
+        km_drop_dense_copy(km);
+        return s == TSVM_ERR_OOM ? TSVM_OK : s;
+    }
+    km->X = km->X_owned;
+    TSVM_LAUNCH(dense_from_csr_kernel, prepare_grid(km->n), 256, 0, st, km->val, km->row_ptr, km->col, km->n, d_pad, km->X_owned);
     return TSVM_OK;
 }
 
@@ -1021,8 +1036,12 @@ static tsvm_status finish_create(tsvm_km *km, cudaStream_t st) {
                     km->fn, km->self_dot, km->diag, km->status_dev);
         return TSVM_OK;
     }
-    const int kind = wanted_plane_kind(km);
-    if (kind) TSVM_TRY(alloc_planes(km, kind));
+    int kind = wanted_plane_kind(km);
+    if (kind && !km->Xhi) {
+        const tsvm_status s = alloc_planes(km, kind);
+        if (s == TSVM_ERR_OOM) kind = 0;         // ensure_planes asks again when an engine that reads them is used
+        else if (s != TSVM_OK) return s;
+    }
     TSVM_LAUNCH(prepare_rows_kernel, prepare_grid(km->n), 256, 0, st, km->X, km->n, km->d, km->ldx, kind, km->plane_ld,
                 km->Xhi, km->Xlo, km->x_unscale, km->fn, km->self_dot, km->diag, km->status_dev);
     km->plane_kind = kind;

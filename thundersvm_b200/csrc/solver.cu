@@ -974,6 +974,7 @@ static inline void cpu_pause() {
 
 struct tsvm_solver {
     tsvm_km *km = nullptr;
+    std::shared_ptr<char> storage_user;
     int kind = 0, ws = 0, q = 0, n = 0;
     const int *y = nullptr;
     double *alpha = nullptr, *f = nullptr;
@@ -1075,7 +1076,7 @@ struct tsvm_solver {
         return TSVM_OK;
     }
 
-    tsvm_status init() {
+    tsvm_status allocate() {
         idle = false;
         TSVM_TRY(dev_alloc(&ids, (size_t) ws));
         TSVM_TRY(dev_alloc(&y_ws, (size_t) ws));
@@ -1102,7 +1103,7 @@ struct tsvm_solver {
         st2 = streams->st2; ev_fork = streams->ev_fork; ev_fork2 = streams->ev_fork2; ev_join = streams->ev_join;
         // local iteration cap: max(100000, 100 * ws) (csmosolver.cpp:49)
         local_max_iter = ws > INT_MAX / 100 ? INT_MAX : (100 * ws > 100000 ? 100 * ws : 100000);
-        return init_f();
+        return TSVM_OK;
     }
 
     // init_f (csmosolver.cpp:189-214): f -= sum over the initially non-zero alphas
@@ -1376,17 +1377,23 @@ tsvm_status tsvm_solver_create(tsvm_km *km, int solver_kind, const int *y_dev, d
     TSVM_REQUIRE(ws_size >= 2 && ws_size <= 1024 && ws_size <= n && (ws_size & (ws_size - 1)) == 0,
                  "solver_create: working-set size %d must be a power of two in [2, min(n, 1024)]", ws_size);
     *out = nullptr;
-    tsvm_solver *S = new tsvm_solver;
-    S->km = km; S->kind = solver_kind; S->y = y_dev; S->alpha = alpha_dev; S->f = f_dev;
-    S->eps = eps; S->Cp = Cp; S->Cn = Cn; S->ws = ws_size; S->q = ws_size / 2; S->n = n;
-    S->ld = ((long long) n + 3) & ~3ll;
-    S->st = (cudaStream_t) stream;
-    S->launches0 = launch_count();
-    S->t_begin = std::chrono::steady_clock::now();
-    tsvm_status s = S->init();
-    if (s != TSVM_OK) { delete S; return s; }
-    *out = S;
-    return TSVM_OK;
+    for (;;) {
+        tsvm_solver *S = new tsvm_solver;
+        S->km = km; S->storage_user = km->storage_users;
+        S->kind = solver_kind; S->y = y_dev; S->alpha = alpha_dev; S->f = f_dev;
+        S->eps = eps; S->Cp = Cp; S->Cn = Cn; S->ws = ws_size; S->q = ws_size / 2; S->n = n;
+        S->ld = ((long long) n + 3) & ~3ll;
+        S->st = (cudaStream_t) stream;
+        S->launches0 = launch_count();
+        S->t_begin = std::chrono::steady_clock::now();
+        const tsvm_status s = S->allocate();
+        const tsvm_status r = s == TSVM_OK ? S->init_f() : s;
+        if (r == TSVM_OK) { *out = S; return TSVM_OK; }
+        delete S;
+        // a dense copy of CSR data makes the solve faster, but a solve without it is better than none
+        if (s != TSVM_ERR_OOM || !km->from_csr || km->storage_users.use_count() > 1) return r;
+        km_drop_dense_copy(km);
+    }
 }
 
 tsvm_status tsvm_solver_iterate(tsvm_solver *S, int n_iters, int *done_host) {
