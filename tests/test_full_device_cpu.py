@@ -139,3 +139,16 @@ F.fake_set_free(100 * MB)
 check(L.tsvm_km_set_dense_engine(h, 0))
 check(rows())
 """)
+
+
+def test_row_cache_leaves_room_for_the_rest(runtime):
+    """A quarter of the rows wanted (384 MB) fits to within 2 MB, and the working set's block alone takes 4 MB."""
+    fake_device.run_python(runtime, """
+s, h = dense(np.ones((20000, 64), np.float32))
+check(s)
+F.fake_set_free(386 * MB)
+s, S, keep = solver(h, 20000)
+check(s)
+idx, out = np.arange(512, dtype=np.int32), np.zeros((512, 20000), np.float32)
+check(L.tsvm_km_rows_by_index(h, p(idx), 512, p(out), C.c_longlong(20000), None))
+""")

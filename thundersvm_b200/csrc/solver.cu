@@ -1047,14 +1047,29 @@ struct tsvm_solver {
     }
 
     // Row buffer = kernel-row cache: as many rows as the budget allows (tsvm_set_row_cache_bytes), at least the
-    // working set plus one batch of new rows, at most one row per instance. A failed allocation halves the request.
+    // working set plus one batch of new rows, at most one row per instance. A failed allocation halves the request, and so
+    // does one that leaves no room for the solve's other buffers (looked at only after a failure: the device is nearly full).
+    bool room_for_the_rest() const {
+        const size_t staged = km->dense ? (size_t) 8 * km->d_pad : (size_t) km->d;        // floats per working-set member
+        void *probe = nullptr;
+        if (pool_alloc(&probe, ((size_t) 16 << 20) + sizeof(float) * ((size_t) (ws > 128 ? ws : 128) * (staged + ws) + (size_t) 8 * n)) != TSVM_OK)
+            return false;
+        pool_free_many({probe}, true);
+        return true;
+    }
     tsvm_status alloc_rows() {
         const long long floor_rows = (long long) ws + q;
         long long want = (long long) (row_cache_budget() / (sizeof(float) * (size_t) ld));
         if (want > n) want = n;
         if (want < floor_rows) want = floor_rows;
-        for (;;) {
-            const tsvm_status s = dev_alloc(&rows, (size_t) want * ld);
+        km_pair_engine(km, st);                  // (operand planes that found no room before are built first)
+        for (const long long first = want;;) {
+            tsvm_status s = dev_alloc(&rows, (size_t) want * ld);
+            if (s == TSVM_OK && want < first && want > floor_rows && !room_for_the_rest()) {
+                pool_free_many({rows}, true);
+                rows = nullptr;
+                s = TSVM_ERR_OOM;
+            }
             if (s == TSVM_OK) break;
             if (s != TSVM_ERR_OOM || want == floor_rows) return s;
             want = want / 2 > floor_rows ? want / 2 : floor_rows;
