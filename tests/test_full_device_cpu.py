@@ -152,3 +152,35 @@ check(s)
 idx, out = np.arange(512, dtype=np.int32), np.zeros((512, 20000), np.float32)
 check(L.tsvm_km_rows_by_index(h, p(idx), 512, p(out), C.c_longlong(20000), None))
 """)
+
+
+HOST_MODEL = """
+import host_api
+H = host_api.load()
+rng = np.random.default_rng(0)
+def model(n_sv, d, per_row):
+    rows = [" ".join("%d:1" % c for c in np.sort(rng.choice(d, per_row, replace=False)) + 1) for _ in range(n_sv)]
+    head = ["svm_type c_svc", "kernel_type rbf", "gamma 0.5", "nr_class 2", "total_sv %d" % n_sv, "rho 0.1", "label 0 1",
+            "nr_sv %d %d" % (n_sv // 2, n_sv - n_sv // 2), "SV"]
+    m = H.model_new(0)
+    H.load_from_string_scikit(m, "\\n".join(head + ["1 " + r for r in rows] + [""]).encode())
+    assert H.n_sv(m) == n_sv
+    return m
+def label(m, n_rows, d, per_row):
+    rp = np.arange(0, n_rows * per_row + 1, per_row, dtype=np.int32)
+    col = np.tile(np.arange(1, per_row + 1, dtype=np.int32), n_rows)
+    val, out = np.ones(len(col), np.float32), np.zeros(n_rows, np.float32)
+    return H.sparse_predict(n_rows, host_api.p(val, host_api.f32p), host_api.p(rp, host_api.i32p),
+                            host_api.p(col, host_api.i32p), m, host_api.p(out, host_api.f32p), 0)
+"""
+
+
+def test_host_prediction_keeps_to_the_entries(runtime):
+    """4,000 support vectors of 2,000 features, 2 % set: 32 MB as dense rows and as much for the planes, 1.3 MB as entries."""
+    fake_device.run_python(runtime, HOST_MODEL + """
+m = model(4000, 2000, 42)
+for free in (20, 45, 200):
+    F.fake_set_free(free * MB)
+    assert label(m, 100, 2000, 42) == 0
+    L.tsvm_release_cached_memory()
+""")

@@ -1,0 +1,102 @@
+"""The same results with most of the device's memory taken by someone else: what the library chose freely before has to
+give way (storage of the instances, row cache, prediction slabs). A child process takes the memory, so that it goes back
+with the process."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import sys
+sys.path[:0] = [%r, %r]
+import numpy as np, torch
+from thundersvm_b200 import capi
+import host_api
+H = host_api.load()
+rng = np.random.default_rng(5)
+def leave(mb):
+    # takes all of the device but mb
+    capi.lib().tsvm_release_cached_memory()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - (mb << 20), dtype=torch.uint8, device="cuda")
+def sparse(n, d=2000, k=42):
+    col = np.sort(rng.permuted(np.tile(np.arange(d, dtype=np.int32), (n, 1)), axis=1)[:, :k], axis=1)
+    col[:, 0] = np.minimum(col[:, 0], d // 2)
+    val = rng.random((n, k)).astype(np.float32) + 0.1
+    return val.ravel(), np.arange(0, n * k + 1, k, dtype=np.int32), col.astype(np.int32).ravel()
+def score(csr, d=2000):
+    w = np.random.default_rng(9).standard_normal(d)
+    return (csr[0] * w[csr[2]]).reshape(len(csr[1]) - 1, -1).sum(1)
+""" % (os.path.dirname(HERE), HERE)
+
+
+def run(body):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + body], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout[-3000:]
+
+
+@pytest.mark.parametrize("svm,classes,n", [(0, 2, 6000), (0, 3, 6000), (3, 1, 4000)])
+def test_fit_and_predict(capi, svm, classes, n):
+    """Instances of 2,000 features, 2.1 % set: 48 MB as dense rows (SVR: twice 32 MB) and as much for the planes, 2 MB as
+    entries, which both sides hold; 100 MB are enough for these and the row buffer. The solver stops at eps, so the two
+    storages' rounding may show in the predictions up to that."""
+    run("""
+svm, classes, n = %d, %d, %d
+csr, new = sparse(n), sparse(500)
+s, s_new = score(csr), score(new)
+y = s if svm == 3 else np.searchsorted(np.quantile(s, np.arange(1, classes) / classes), s)
+kw = dict(csr=csr, y=y, gamma=0.05, C_=10.0)
+m, *_ = host_api.train(H, svm, **kw)
+want = host_api.predict_sparse(H, m, new)
+want_sv = H.n_sv(m)
+H.model_free(m)
+taken = leave(100)
+m, *_ = host_api.train(H, svm, **kw)
+got = host_api.predict_sparse(H, m, new)
+assert abs(H.n_sv(m) - want_sv) <= 0.005 * n, (H.n_sv(m), want_sv)
+if svm == 3: assert np.abs(got - want).max() < 0.01 * np.abs(want).max(), np.abs(got - want).max()
+else: assert (got != want).mean() <= 0.01, (got != want).mean()
+""" % (svm, classes, n))
+
+
+def test_prediction_slabs(capi):
+    """A stored kernel block of 10,000 x 20,000 (800 MB) with 150 MB left: the same sums in the same order."""
+    run("""
+n_sv, m, d = 20000, 10000, 5000
+csr, new = sparse(n_sv, d), sparse(m, d)
+cuda = lambda t: tuple(torch.from_numpy(a).cuda() for a in t)
+km = capi.KernelMatrix(csr=cuda(csr), d=d, gamma=0.05)
+coef, rho = torch.from_numpy(rng.standard_normal((1, n_sv))).cuda(), torch.zeros(1, dtype=torch.float64, device="cuda")
+batch = cuda(new)
+predict = lambda: capi.predict_dec(km, coef, [n_sv // 2, n_sv // 2], rho, 2, csr=batch)
+want = predict().clone()
+taken = leave(150)
+assert torch.equal(predict(), want)
+""")
+
+
+def test_row_cache(capi):
+    """20,000 instances: 1.6 GB of rows wanted, 500 MB left. The cache's size changes no result."""
+    run("""
+n, d = 20000, 64
+X = rng.standard_normal((n, d)).astype(np.float32)
+X /= np.linalg.norm(X, axis=1, keepdims=True)
+y = np.where(X @ rng.standard_normal(d) + 0.3 * rng.standard_normal(n) > 0, 1, -1).astype(np.int32)
+km = capi.KernelMatrix(dense=torch.from_numpy(X).cuda(), gamma=0.5)
+yd = torch.from_numpy(y).cuda()
+def solve():
+    a, f = torch.zeros(n, dtype=torch.float64, device="cuda"), -yd.double()
+    rho, st = capi.smo_solve(km, yd, a, f, 1e-3, 1.0, 1.0, 1024)
+    return a, rho, st
+a0, rho0, st0 = solve()
+taken = leave(500)
+a1, rho1, st1 = solve()
+assert st1["cache_rows"] < st0["cache_rows"], (st0["cache_rows"], st1["cache_rows"])
+assert torch.equal(a0, a1) and rho0 == rho1
+""")

@@ -6,6 +6,7 @@
 #include <thundersvm/dataset.h>
 #include <thundersvm/svmparam.h>
 #include <thundersvm/kernelmatrix.h>
+#include <functional>
 #include <memory>
 
 class SvmModel {
@@ -49,7 +50,9 @@ protected:
     /// Kernel matrix of the support vectors, built on the first prediction and kept until the support vectors
     /// change (the reference rebuilds it on every predict call, svmmodel.cpp:84).
     const KernelMatrix &sv_matrix() const;
-    void invalidate_sv_matrix() { sv_kmat_.reset(); }
+    void invalidate_sv_matrix() const { sv_kmat_.reset(); }
+    /// work(sv_matrix()); where the device runs out of memory, again with the matrix in the storage that fits
+    void with_sv_matrix(const std::function<void(const KernelMatrix &)> &work) const;
 
     SvmParam param;
     SyncArray<float_type> coef;

@@ -14,7 +14,22 @@
 namespace thundersvm {
 void *device_alloc(size_t bytes);                 // throws std::bad_alloc when the device is out of memory
 void device_free(void *p);
-bool device_has_room(double bytes);               // less than 60 % of the free device memory
+// Less than 60 % of the free device memory. The driver is asked from 1 % of the device on, or (RoomAsked) always.
+bool device_has_room(double bytes);
+struct RoomAsked {                                // for this host thread, while it lives
+    RoomAsked();
+    ~RoomAsked();
+};
+// Runs work(); if the device runs out of memory in it, runs it again with every device_has_room answered by the driver, so
+// that what chose the larger storage without asking chooses the smaller one.
+template <typename Work> void with_room(Work work) {
+    try {
+        work();
+        return;
+    } catch (const std::bad_alloc &) {}
+    RoomAsked asked;
+    work();
+}
 void copy_to_device(void *dst, const void *src, size_t bytes);
 void copy_to_host(void *dst, const void *src, size_t bytes);
 void copy_on_device(void *dst, const void *src, size_t bytes);

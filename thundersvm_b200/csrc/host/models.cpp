@@ -67,6 +67,15 @@ const KernelMatrix &SvmModel::sv_matrix() const {
     return *sv_kmat_;
 }
 
+void SvmModel::with_sv_matrix(const std::function<void(const KernelMatrix &)> &work) const {
+    bool again = false;
+    thundersvm::with_room([&] {
+        if (again) invalidate_sv_matrix();       // its storage was chosen without asking
+        again = true;
+        work(sv_matrix());
+    });
+}
+
 int SvmModel::get_working_set_size(int n_instances, int n_features) {
     const int ws = tsvm_working_set_size(n_instances, n_features, param.max_mem_size, thundersvm::total_memory_size());
     if (ws < 0) throw std::bad_alloc();          // the budget is already exceeded (svmmodel.cpp:440-442)
@@ -103,13 +112,14 @@ void SvmModel::predict_dec_values(const DataSet::node2d &instances, SyncArray<fl
             for (size_t k = 0; k < n_binary_models; ++k) d[r * n_binary_models + k] = -rho.host_data()[k];
         return;
     }
-    const KernelMatrix &k_mat = sv_matrix();
-    const thundersvm::DeviceCsr batch(instances);
     size_t budget = 0;                      // 0 = library default; a positive batch size bounds the K buffer
     if (batch_size > 0) budget = (size_t) batch_size * (((size_t) sv.size() + 3) & ~3ul) * sizeof(kernel_type);
-    b200_check(tsvm_predict_dec(k_mat.handle(), coef.device_data(), n_sv.host_data(), rho.device_data(), n_classes,
-                                (int) m, nullptr, 0, 0, batch.val(), batch.row_ptr(), batch.col(), (long long) batch.nnz(),
-                                dec_values.device_data(), budget, nullptr));
+    with_sv_matrix([&](const KernelMatrix &k_mat) {
+        const thundersvm::DeviceCsr batch(instances);
+        b200_check(tsvm_predict_dec(k_mat.handle(), coef.device_data(), n_sv.host_data(), rho.device_data(), n_classes,
+                                    (int) m, nullptr, 0, 0, batch.val(), batch.row_ptr(), batch.col(), (long long) batch.nnz(),
+                                    dec_values.device_data(), budget, nullptr));
+    });
 }
 
 void SvmModel::predict_dec_values_instant(const DataSet::node2d &instances, SyncArray<float_type> &predict_instant,
@@ -129,14 +139,15 @@ void SvmModel::predict_dec_values_instant(const DataSet::node2d &instances, Sync
         }
         return;
     }
-    const KernelMatrix &k_mat = sv_matrix();
-    const thundersvm::DeviceCsr batch(instances);
     size_t budget = 0;
     if (batch_size > 0) budget = (size_t) batch_size * (((size_t) sv.size() + 3) & ~3ul) * sizeof(kernel_type);
     SyncArray<int> winner(m);
-    b200_check(tsvm_predict_labels(k_mat.handle(), coef.device_data(), n_sv.host_data(), rho.device_data(), n_classes,
-                                   (int) m, nullptr, 0, 0, batch.val(), batch.row_ptr(), batch.col(),
-                                   (long long) batch.nnz(), winner.device_data(), budget, nullptr));
+    with_sv_matrix([&](const KernelMatrix &k_mat) {
+        const thundersvm::DeviceCsr batch(instances);
+        b200_check(tsvm_predict_labels(k_mat.handle(), coef.device_data(), n_sv.host_data(), rho.device_data(), n_classes,
+                                       (int) m, nullptr, 0, 0, batch.val(), batch.row_ptr(), batch.col(),
+                                       (long long) batch.nnz(), winner.device_data(), budget, nullptr));
+    });
     const int *w = winner.host_data();
     for (size_t r = 0; r < m; ++r) out[r] = w[r];
 }
@@ -349,7 +360,11 @@ void SVC::build_device_rows(const DataSet &ds) {
     if (!((density >= 0.02 || d <= 256) && thundersvm::device_has_room(bytes))) return;
     const vector<int> perm = ds.original_index();
     const DataSet::node2d &ins = ds.instances();
-    dev_rows_.X = static_cast<float *>(thundersvm::device_alloc(n * ld * sizeof(float)));
+    try {
+        dev_rows_.X = static_cast<float *>(thundersvm::device_alloc(n * ld * sizeof(float)));
+    } catch (const std::bad_alloc &) {
+        return;                              // every sub-problem makes its own from the host instances
+    }
     thundersvm::upload_dense(dev_rows_.X, n, ld, [&](size_t k) -> const vector<DataSet::node> & { return ins[perm[k]]; });
     dev_rows_.n = n; dev_rows_.d = d; dev_rows_.ld = ld;
 }
@@ -382,9 +397,10 @@ void SVC::train(const DataSet &dataset, SvmParam param) {
         if (n_threads < 1) n_threads = 1;
         if (n_threads > (int) pairs.size()) n_threads = (int) pairs.size();
     }
-    if (n_threads <= 1) {
+    const auto solve_in_turn = [&] {
         for (size_t k = 0; k < pairs.size(); ++k) train_binary(ds, pairs[k].first, pairs[k].second, *alpha[k], rho_h[k]);
-    } else {
+    };
+    const auto solve_in_threads = [&] {
         int dev = 0;
         cudaGetDevice(&dev);
         std::atomic<size_t> next{0};
@@ -410,7 +426,15 @@ void SVC::train(const DataSet &dataset, SvmParam param) {
             });
         for (auto &th : pool) th.join();
         if (err) std::rethrow_exception(err);
-    }
+    };
+    // (a device without room for that: one pair at a time, each in the storage that fits)
+    bool again = false;
+    thundersvm::with_room([&] {
+        if (again) free_device_rows();
+        const bool threads = n_threads > 1 && !again;
+        again = true;
+        if (threads) solve_in_threads(); else solve_in_turn();
+    });
     for (size_t k = 0; k < pairs.size(); ++k) {
         const vector<int> ids = ds.original_index(pairs[k].first, pairs[k].second);
         CHECK_EQ(ids.size(), alpha[k]->size());
@@ -748,19 +772,21 @@ void SVR::train(const DataSet &dataset, SvmParam param) {
     const int n = (int) dataset.n_instances();
     DataSet::node2d twice(dataset.instances());                 // the dual runs over 2n duplicated instances
     twice.insert(twice.end(), dataset.instances().begin(), dataset.instances().end());
-    KernelMatrix k_mat(twice, param);
     SyncArray<float_type> f_val(2 * n), alpha_2(2 * n);
     SyncArray<int> y(2 * n);
-    alpha_2.mem_set(0);
-    for (int i = 0; i < n; ++i) {
-        f_val.host_data()[i] = param.p - dataset.y()[i];
-        y.host_data()[i] = +1;
-        f_val.host_data()[i + n] = -param.p - dataset.y()[i];
-        y.host_data()[i + n] = -1;
-    }
-    const int ws_size = get_working_set_size(2 * n, (int) k_mat.n_features());
-    CSMOSolver solver;
-    solver.solve(k_mat, y, alpha_2, rho.host_data()[0], f_val, param.epsilon, param.C, param.C, ws_size, max_iter);
+    thundersvm::with_room([&] {
+        KernelMatrix k_mat(twice, param);
+        alpha_2.mem_set(0);
+        for (int i = 0; i < n; ++i) {
+            f_val.host_data()[i] = param.p - dataset.y()[i];
+            y.host_data()[i] = +1;
+            f_val.host_data()[i + n] = -param.p - dataset.y()[i];
+            y.host_data()[i + n] = -1;
+        }
+        const int ws_size = get_working_set_size(2 * n, (int) k_mat.n_features());
+        CSMOSolver solver;
+        solver.solve(k_mat, y, alpha_2, rho.host_data()[0], f_val, param.epsilon, param.C, param.C, ws_size, max_iter);
+    });
     save_svr_coef(alpha_2, dataset.instances());
     if (param.kernel_type == SvmParam::LINEAR) compute_linear_coef_single_model(dataset.n_features(), dataset.is_zero_based());
 }
@@ -775,21 +801,23 @@ void NuSVR::train(const DataSet &dataset, SvmParam param) {
     const int n = (int) dataset.n_instances();
     DataSet::node2d twice(dataset.instances());
     twice.insert(twice.end(), dataset.instances().begin(), dataset.instances().end());
-    KernelMatrix k_mat(twice, param);
     SyncArray<float_type> f_val(2 * n), alpha_2(2 * n);
     SyncArray<int> y(2 * n);
-    float_type mass = param.C * param.nu * n / 2;               // nusvr.cpp:24-32
-    for (int i = 0; i < n; ++i) {
-        const float_type a = std::min(mass, param.C);
-        alpha_2.host_data()[i] = alpha_2.host_data()[i + n] = a;
-        mass -= a;
-        f_val.host_data()[i] = f_val.host_data()[i + n] = -dataset.y()[i];
-        y.host_data()[i] = +1;
-        y.host_data()[i + n] = -1;
-    }
-    const int ws_size = get_working_set_size(2 * n, (int) k_mat.n_features());
-    NuSMOSolver solver(true);
-    solver.solve(k_mat, y, alpha_2, rho.host_data()[0], f_val, param.epsilon, param.C, param.C, ws_size, max_iter);
+    thundersvm::with_room([&] {
+        KernelMatrix k_mat(twice, param);
+        float_type mass = param.C * param.nu * n / 2;               // nusvr.cpp:24-32
+        for (int i = 0; i < n; ++i) {
+            const float_type a = std::min(mass, param.C);
+            alpha_2.host_data()[i] = alpha_2.host_data()[i + n] = a;
+            mass -= a;
+            f_val.host_data()[i] = f_val.host_data()[i + n] = -dataset.y()[i];
+            y.host_data()[i] = +1;
+            y.host_data()[i + n] = -1;
+        }
+        const int ws_size = get_working_set_size(2 * n, (int) k_mat.n_features());
+        NuSMOSolver solver(true);
+        solver.solve(k_mat, y, alpha_2, rho.host_data()[0], f_val, param.epsilon, param.C, param.C, ws_size, max_iter);
+    });
     save_svr_coef(alpha_2, dataset.instances());
     if (param.kernel_type == SvmParam::LINEAR) compute_linear_coef_single_model(dataset.n_features(), dataset.is_zero_based());
 }
@@ -804,16 +832,18 @@ void OneClassSVC::train(const DataSet &dataset, SvmParam param) {
     const int n = (int) dataset.n_instances();
     SyncArray<float_type> alpha(n), f_val(n);
     SyncArray<int> y(n);
-    KernelMatrix k_mat(dataset.instances(), param);
-    alpha.mem_set(0);
-    f_val.mem_set(0);
-    const int full = static_cast<int>(param.nu * n);            // oneclass_svc.cpp:18-24
-    for (int i = 0; i < full; ++i) alpha.host_data()[i] = 1;
-    if (full < n) alpha.host_data()[full] = param.nu * n - full;
-    for (int i = 0; i < n; ++i) y.host_data()[i] = 1;
-    const int ws_size = get_working_set_size(n, (int) k_mat.n_features());
-    CSMOSolver solver;
-    solver.solve(k_mat, y, alpha, rho.host_data()[0], f_val, param.epsilon, 1, 1, ws_size, max_iter);
+    thundersvm::with_room([&] {
+        KernelMatrix k_mat(dataset.instances(), param);
+        alpha.mem_set(0);
+        f_val.mem_set(0);
+        const int full = static_cast<int>(param.nu * n);            // oneclass_svc.cpp:18-24
+        for (int i = 0; i < full; ++i) alpha.host_data()[i] = 1;
+        if (full < n) alpha.host_data()[full] = param.nu * n - full;
+        for (int i = 0; i < n; ++i) y.host_data()[i] = 1;
+        const int ws_size = get_working_set_size(n, (int) k_mat.n_features());
+        CSMOSolver solver;
+        solver.solve(k_mat, y, alpha, rho.host_data()[0], f_val, param.epsilon, 1, 1, ws_size, max_iter);
+    });
     LOG(INFO) << "rho = " << rho.host_data()[0];
     vector<float_type> cf;
     const float_type *a = alpha.host_data();

@@ -50,9 +50,12 @@ void device_free(void *p) {
     tsvm::pool_free_many({p}, true);
 }
 // The driver is asked for the free memory only where it matters (a driver lock, at times tens of milliseconds): what fits
-// a hundredth of the device is allocated in any case, and a device that full fails the allocation.
+// a hundredth of the device is tried first, and a device that full fails the allocation (with_room tries again).
+static thread_local int tl_room_asked = 0;
+RoomAsked::RoomAsked() { ++tl_room_asked; }
+RoomAsked::~RoomAsked() { --tl_room_asked; }
 bool device_has_room(double bytes) {
-    if (bytes < 0.01 * (double) tsvm::device_memory_bytes()) return true;
+    if (!tl_room_asked && bytes < 0.01 * (double) tsvm::device_memory_bytes()) return true;
     size_t free_b = 0, total_b = 0;
     return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes < 0.6 * (double) free_b;
 }
