@@ -184,3 +184,15 @@ for free in (20, 45, 200):
     assert label(m, 100, 2000, 42) == 0
     L.tsvm_release_cached_memory()
 """)
+
+
+def test_uploads_without_page_locked_memory(runtime):
+    """The host may refuse page-locked memory (a limit, a full machine): the instances go through ordinary memory then."""
+    fake_device.run_python(runtime, HOST_MODEL + """
+m = model(400, 2000, 42)
+assert label(m, 100, 2000, 42) == 0
+L.tsvm_release_cached_memory()
+F.fake_refuse_pinned(1)
+assert label(m, 100, 2000, 42) == 0
+assert label(m, 40000, 2000, 42) == 0           # more than one block
+""")

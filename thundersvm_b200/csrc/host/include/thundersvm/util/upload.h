@@ -16,7 +16,7 @@ template <typename T> DevicePtr<T> device_array(size_t count) {
     return DevicePtr<T>(static_cast<T *>(device_alloc(std::max<size_t>(count, 1) * sizeof(T))));
 }
 
-// Two page-locked blocks of at least `bytes` and what is needed to take turns with them
+// Two blocks of at least `bytes`, page-locked if the host has such memory, and what is needed to take turns with them
 class UploadBlocks {
 public:
     explicit UploadBlocks(size_t bytes, bool two);
@@ -29,7 +29,7 @@ public:
 private:
     char *block_[2] = {nullptr, nullptr};
     cudaEvent_t sent_[2] = {nullptr, nullptr};
-    bool busy_[2] = {false, false};
+    bool busy_[2] = {false, false}, pinned_[2] = {false, false};
     int at_ = 1;
 };
 

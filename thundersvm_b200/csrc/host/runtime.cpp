@@ -63,8 +63,11 @@ void device_zero(void *p, size_t bytes) { cuda_ok(cudaMemsetAsync(p, 0, bytes, t
 
 UploadBlocks::UploadBlocks(size_t bytes, bool two) {
     for (int b = 0; b < (two ? 2 : 1); ++b) {
-        if (tsvm::pinned_alloc(reinterpret_cast<void **>(block_ + b), bytes) != TSVM_OK)
-            LOG(FATAL) << "page-locked memory: " << tsvm_last_error();
+        pinned_[b] = tsvm::pinned_alloc(reinterpret_cast<void **>(block_ + b), bytes) == TSVM_OK;
+        if (!pinned_[b]) {                        // the host has none to give: copies through the driver's own, slower
+            block_[b] = static_cast<char *>(std::malloc(bytes));
+            if (!block_[b]) throw std::bad_alloc();
+        }
         if (two) cuda_ok(cudaEventCreateWithFlags(sent_ + b, cudaEventDisableTiming), "event");
     }
 }
@@ -72,7 +75,7 @@ UploadBlocks::~UploadBlocks() {
     if (busy_[0] || busy_[1]) cudaStreamSynchronize(tl_stream);
     for (int b = 0; b < 2; ++b) {
         if (sent_[b]) cudaEventDestroy(sent_[b]);
-        if (block_[b]) tsvm::pinned_free(block_[b]);
+        if (block_[b]) { if (pinned_[b]) tsvm::pinned_free(block_[b]); else std::free(block_[b]); }
     }
 }
 char *UploadBlocks::next() {
