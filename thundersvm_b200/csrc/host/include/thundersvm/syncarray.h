@@ -13,7 +13,10 @@
 
 namespace thundersvm {
 void *device_alloc(size_t bytes);                 // throws std::bad_alloc when the device is out of memory
-void device_free(void *p);
+// Files the block as free, once nothing can use it any more. used_on: the one stream it has been used on - where that is the
+// calling thread's work stream, this is all there is to wait for; the default stream says nothing about who uses the block
+// (so does nullptr for "several"), and the device is waited for.
+void device_free(void *p, cudaStream_t used_on = nullptr);
 // Less than 60 % of the free device memory. The driver is asked from 1 % of the device on, or (RoomAsked) always.
 bool device_has_room(double bytes);
 struct RoomAsked {                                // for this host thread, while it lives
@@ -64,12 +67,13 @@ public:
     const T *host_data() const { to_host(); return hptr(); }
     T *host_data() { to_host(); head_ = HOST; return hptr(); }
     const T *device_data() const { to_device(); return dev_; }
-    T *device_data() { to_device(); head_ = DEVICE; return dev_; }
+    T *device_data() { to_device(); head_ = DEVICE; return dev_; }      // for work on work_stream() (see device_free)
 
     void to_host() const {
         if (head_ == DEVICE && dev_) { thundersvm::copy_to_host(hptr(), dev_, mem_size()); head_ = BOTH; }
     }
     void to_device() const {
+        used();
         if (!dev_ && size_) {
             dev_ = static_cast<T *>(thundersvm::device_alloc(mem_size()));
             own_dev_ = true;
@@ -84,7 +88,10 @@ public:
     }
     void copy_from(const SyncArray<T> &source) {
         CHECK_EQ(size_, source.size()) << "copy_from: size mismatch";
-        if (source.head_ == DEVICE && source.dev_) thundersvm::copy_on_device(device_data(), source.dev_, mem_size());
+        if (source.head_ == DEVICE && source.dev_) {
+            source.used();
+            thundersvm::copy_on_device(device_data(), source.dev_, mem_size());
+        }
         else std::memcpy(host_data(), source.hptr(), mem_size());
     }
     void mem_set(const T &value) {
@@ -94,15 +101,24 @@ public:
     // alias foreign buffers (no ownership)
     void set_host_data(T *p) { ext_host_ = p; head_ = HOST; }
     void set_device_data(T *p) {
-        if (own_dev_ && dev_) thundersvm::device_free(dev_);
+        free_device();
         dev_ = p; own_dev_ = false; head_ = DEVICE;
     }
 
 private:
     enum Head { HOST, DEVICE, BOTH };
+    // (one array is not used by two threads at a time, but one may fill it and another release it)
+    void used() const {
+        const cudaStream_t s = thundersvm::work_stream();
+        if (!dev_) { stream_ = s; mixed_ = false; }
+        else if (s != stream_) mixed_ = true;
+    }
+    void free_device() {
+        if (own_dev_ && dev_) thundersvm::device_free(dev_, mixed_ ? nullptr : stream_);
+    }
     T *hptr() const { return ext_host_ ? ext_host_ : const_cast<T *>(host_.data()); }
     void release() {
-        if (own_dev_ && dev_) thundersvm::device_free(dev_);
+        free_device();
         dev_ = nullptr; own_dev_ = false; ext_host_ = nullptr;
         if (size_) thundersvm::total_memory_size() -= mem_size();
         size_ = 0;
@@ -111,7 +127,8 @@ private:
     mutable vector<T> host_;
     T *ext_host_ = nullptr;
     mutable T *dev_ = nullptr;
-    mutable bool own_dev_ = false;
+    mutable bool own_dev_ = false, mixed_ = false;
+    mutable cudaStream_t stream_ = nullptr;           // the stream of every use so far, unless mixed_
     mutable Head head_ = HOST;
 };
 #endif

@@ -10,10 +10,14 @@
 #include <memory>
 
 namespace thundersvm {
-struct DeviceFree { void operator()(void *p) const { device_free(p); } };
+struct DeviceFree {
+    cudaStream_t used_on = nullptr;
+    void operator()(void *p) const { device_free(p, used_on); }
+};
 template <typename T> using DevicePtr = std::unique_ptr<T, DeviceFree>;
+// for the work stream of the thread that makes it; what else reads it waits by itself, as the handles do
 template <typename T> DevicePtr<T> device_array(size_t count) {
-    return DevicePtr<T>(static_cast<T *>(device_alloc(std::max<size_t>(count, 1) * sizeof(T))));
+    return DevicePtr<T>(static_cast<T *>(device_alloc(std::max<size_t>(count, 1) * sizeof(T))), DeviceFree{work_stream()});
 }
 
 // Two blocks of at least `bytes`, page-locked if the host has such memory, and what is needed to take turns with them

@@ -43,11 +43,11 @@ void copy_to_host(void *dst, const void *src, size_t bytes) {
 void copy_on_device(void *dst, const void *src, size_t bytes) {
     cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, tl_stream), "D2D copy");
 }
-// The owner of such memory works on its thread's stream only, so that is all there is to wait for.
-void device_free(void *p) {
+void device_free(void *p, cudaStream_t used_on) {
     if (!p) return;
-    cudaStreamSynchronize(tl_stream);
-    tsvm::pool_free_many({p}, true);
+    const bool own = used_on && used_on == tl_stream;
+    if (own) cudaStreamSynchronize(tl_stream);
+    tsvm::pool_free_many({p}, own);
 }
 // The driver is asked for the free memory only where it matters (a driver lock, at times tens of milliseconds): what fits
 // a hundredth of the device is tried first, and a device that full fails the allocation (with_room tries again).
