@@ -160,6 +160,26 @@ def test_local_smo_matches_oracle(capi, solver, ws):
     assert np.allclose(ad_got.cpu().numpy(), ad_exp, rtol=0, atol=1e-9)
 
 
+@pytest.mark.parametrize("ws", [256, 512, 1024])
+def test_local_smo_rows_copied_ahead_hold_the_same_values(capi, ws):
+    """A block whose rows are 16-byte aligned is read through the ring in shared memory, one that is not straight from
+    memory: the same steps, bit for bit, over some thousand of them."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(ws)
+    X = torch.randn(ws, 12, device="cuda", generator=g)
+    K = torch.exp(-0.05 * torch.cdist(X, X).square()).contiguous()
+    y = torch.where(torch.rand(ws, device="cuda", generator=g) < 0.5, 1, -1).int()
+    f = -y.double() + 0.01 * torch.randn(ws, device="cuda", generator=g).double()
+    diag, alpha = torch.ones(ws, device="cuda"), torch.zeros(ws, dtype=torch.float64, device="cuda")
+    shifted = torch.empty(ws * ws + 1, device="cuda")[1:].view(ws, ws).copy_(K)
+    assert K.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 != 0
+    want = capi.local_smo(shifted, diag, y, f, alpha, 100.0, 100.0, 1e-9, max_iter=20000)
+    assert want[2][1].item() > 1000
+    for _ in range(3):
+        got = capi.local_smo(K, diag, y, f, alpha, 100.0, 100.0, 1e-9, max_iter=20000)
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
 @pytest.mark.parametrize("n,ws", [(10007, 1024), (333, 64), (4096, 512), (5, 2)])
 def test_update_f_matches_oracle(capi, n, ws):
     rng = np.random.default_rng(n)
