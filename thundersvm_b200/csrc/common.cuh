@@ -270,6 +270,7 @@ bool km_pair_engine(tsvm_km *km, cudaStream_t st);
 tsvm_status km_pair_engine_takes(tsvm_km *km, const float *tval, const int *rp, const int *tcol, int m, cudaStream_t st,
                                  bool *takes);
 bool km_automatic_engine(const tsvm_km *km);
+tsvm_status km_count_entries(tsvm_km *km, cudaStream_t st);     // km->nnz, read from the device the first time it matters
 size_t km_plane_row_bytes(const tsvm_km *km);
 tsvm_status km_stage_rows_by_index(tsvm_km *km, const int *idx_dev, int q, cudaStream_t st);
 tsvm_status km_rows_staged(tsvm_km *km, int q, float *out, long long ld_out, cudaStream_t st);

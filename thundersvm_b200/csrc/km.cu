@@ -1097,9 +1097,17 @@ static tsvm_status rows_common(tsvm_km *km, int m, float *out, long long ld_out,
 tsvm_status launch_dense_tc2_on(tsvm_km *km, const InstancePlanes &X, int m, float *out, long long ld_out,
                                 cudaStream_t st);   // dense_tc2.cu
 
+tsvm_status km_count_entries(tsvm_km *km, cudaStream_t st) {
+    if (km->nnz >= 0) return TSVM_OK;
+    int last = 0;
+    TSVM_CUDA(cudaMemcpyAsync(&last, km->row_ptr + km->n, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TSVM_CUDA(cudaStreamSynchronize(st));
+    km->nnz = last;
+    return TSVM_OK;
+}
+bool km_automatic_engine(const tsvm_km *km) { return km->engine == 0; }
 // True when kernel rows of this matrix run on the CTA-pair tensor engine, whose requested-row staging and
 // launch can be issued separately and against a caller-chosen subset of instances.
-bool km_automatic_engine(const tsvm_km *km) { return km->engine == 0; }
 bool km_pair_engine(tsvm_km *km, cudaStream_t st) {
     if (!km->dense || !use_tensor_engine(km)) return false;
     return ensure_planes(km, st) == TSVM_OK && km->plane_kind != 0;
@@ -1258,7 +1266,7 @@ tsvm_status tsvm_km_create_csr(const float *val, const int *row_ptr, const int *
     km->fn = KernelFn{kernel_type, degree, gamma, coef0};
     tsvm_status s = TSVM_OK;
     if (loc == TSVM_DEVICE) {
-        km->nnz = -1;                     // read from row_ptr when someone asks (tsvm_km_nnz)
+        km->nnz = -1;                     // read from row_ptr when someone asks (tsvm_km_nnz, km_count_entries)
         km->val = val; km->row_ptr = row_ptr; km->col = col;
     } else {
         const int last = row_ptr[n];

@@ -229,8 +229,10 @@ static tsvm_status predict_few(tsvm_km *km, const double *coef_dev, const int *s
     const bool dense = km->dense && !km->from_csr;      // few rows: the entries are read once, and there are fewer of them
     const int R = m == 1 ? 1 : (m == 2 ? 2 : (m <= 4 ? 4 : 8)), tiles = ceil_div(m, R);
     if (n_classes > FEW_CLASSES || tiles > FEW_TILES || (dense && !km_automatic_engine(km))) return TSVM_OK;
-    const double per_sv = dense ? (double) km->d_pad : (double) km->nnz / km->n;
-    if (tiles > 1 && (double) tiles * km->n * (km->nnz < 0 ? 64.0 : per_sv) > 1.6e7) return TSVM_OK;
+    if (tiles > 1) {
+        if (!dense) TSVM_TRY(km_count_entries(km, st));
+        if ((double) tiles * (dense ? (double) km->n * km->d_pad : (double) km->nnz) > 1.6e7) return TSVM_OK;
+    }
     const int n_pairs = n_classes * (n_classes - 1) / 2;
     if (dense) {
         if (sizeof(float) * (size_t) R * km->d_pad + FewShared<8>::bytes(n_pairs) > 190 * 1024) return TSVM_OK;
