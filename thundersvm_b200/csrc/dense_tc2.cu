@@ -39,22 +39,15 @@ constexpr uint32_t STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;   // 64 KB per CTA
 // flight, and its epilogue is shorter.
 constexpr int MAX_STAGES = 5, MIN_WIDTH = 32;
 // Warpgroup 0 holds the TMA producer (warp 0), the MMA issuer (warp 1) and two idle warps and gives most of its
-// registers back; the other warpgroups are the promotion / epilogue warps and take them. Default: 8 epilogue
-// warps (two per tensor-memory lane quarter, 128 columns = 128 sums per thread; a 384-thread CTA is compiled
-// for 168 registers: 128 * 56 + 256 * 224). TSVM_EPI_WARPS = 16 (four per quarter, 64 sums per thread, 640
-// threads) builds and passes the same tests; measured on the 400,000 x 2,000 launch it changes nothing
-// (1.90 ms against 1.88 ms) - the kernel waits for the tensor pipe, not for its epilogue.
-#ifndef TSVM_EPI_WARPS
-#define TSVM_EPI_WARPS 8
-#endif
-constexpr int EPI_WARPS = TSVM_EPI_WARPS, EPI_WARP0 = 4, THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
+// registers back; the other two warpgroups are the promotion / epilogue warps and take them: two warps per tensor-memory
+// lane quarter, 128 columns = 128 sums per thread. (Four warps per quarter with 64 sums each changed nothing on the
+// 400,000 x 2,000 launch, 1.90 against 1.88 ms: it waits for the tensor pipe, not for its epilogue.)
+constexpr int EPI_WARPS = 8, EPI_WARP0 = 4, THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
 constexpr int COLS_PER_THREAD = BN / (EPI_WARPS / 4);
 // Registers can only move inside the CTA: what the epilogue warps take (setmaxnreg.inc blocks until it is there)
 // must have been given back by the control warps, counted from the per-thread figure the kernel is compiled and
-// launched with (168 for 384 threads, 96 for 640: the largest multiples of 8 that fit 65,536 registers).
-constexpr int REGS_LAUNCH = EPI_WARPS == 8 ? 168 : 96;
-constexpr int REGS_CONTROL = EPI_WARPS == 8 ? 56 : 32, REGS_EPILOGUE = EPI_WARPS == 8 ? 224 : 112;
-static_assert(EPI_WARPS == 8 || EPI_WARPS == 16, "two or four epilogue warps per tensor-memory lane quarter");
+// launched with (168: the largest multiple of 8 with which 384 threads fit 65,536 registers).
+constexpr int REGS_LAUNCH = 168, REGS_CONTROL = 56, REGS_EPILOGUE = 224;
 static_assert(128 * REGS_CONTROL + 32 * EPI_WARPS * REGS_EPILOGUE <= THREADS * REGS_LAUNCH,
               "the epilogue warps would wait for registers that nobody releases");
 static_assert(THREADS * REGS_LAUNCH <= 65536, "register file of an SM");
@@ -64,7 +57,7 @@ constexpr int EPI_CHUNK = COLS_PER_THREAD / 8;
 constexpr uint32_t EPI_STAGE_BYTES = EPI_CHUNK * EPI_WARPS * 32 * 4;
 constexpr uint32_t EPI_CONST_BYTES = EPI_WARPS * 2 * COLS_PER_THREAD * 4;
 // prediction form: up to PRED_NC_SMEM coefficients of every epilogue thread's own instance (thread-private columns)
-constexpr int PRED_NC_SMEM = EPI_WARPS == 8 ? 9 : 4;
+constexpr int PRED_NC_SMEM = 9;
 constexpr uint32_t PRED_BYTES = PRED_NC_SMEM * EPI_WARPS * 32 * 4;
 // kernel-row form: output row (slot of the caller's row buffer) of every requested row, per epilogue warp
 constexpr uint32_t SLOT_BYTES = EPI_WARPS * COLS_PER_THREAD * 4;
