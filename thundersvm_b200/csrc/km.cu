@@ -948,7 +948,8 @@ static inline int wanted_plane_kind(const tsvm_km *km) {
     return (km->engine == 2 || km->engine == 3) ? 1 : 2;
 }
 
-static inline int prepare_grid(int n) { const int b = ceil_div(n, 8); return b < 148 * 8 ? b : 148 * 8; }
+// eight blocks of eight warps (a row each) per SM
+static inline int prepare_grid(int n) { const int b = ceil_div(n, 8), most = 8 * device_sm_count(); return b < most ? b : most; }
 
 // Buffers of the planes the selected engine reads.
 static tsvm_status alloc_planes(tsvm_km *km, int kind) {

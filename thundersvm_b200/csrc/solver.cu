@@ -1083,8 +1083,9 @@ struct tsvm_solver {
         TSVM_TRY(dev_alloc(&miss_slot, (size_t) ws));
         TSVM_TRY(dev_alloc(&victims, (size_t) ws));
         TSVM_TRY(dev_alloc(&cache_ctr, (size_t) CACHE_CTRS));
-        TSVM_LAUNCH(fill_int_kernel, 296, 256, 0, st, slot_of, (long long) n, -1);
-        TSVM_LAUNCH(fill_int_kernel, 296, 256, 0, st, inst_of, cache_cap, -1);
+        const int blocks = 2 * device_sm_count();
+        TSVM_LAUNCH(fill_int_kernel, blocks, 256, 0, st, slot_of, (long long) n, -1);
+        TSVM_LAUNCH(fill_int_kernel, blocks, 256, 0, st, inst_of, cache_cap, -1);
         TSVM_CUDA(cudaMemsetAsync(stamp, 0, sizeof(int) * (size_t) cache_cap, st));
         TSVM_CUDA(cudaMemsetAsync(row_slots, 0, sizeof(int) * (size_t) 2 * ws, st));
         TSVM_CUDA(cudaMemsetAsync(cache_ctr, 0, sizeof(long long) * CACHE_CTRS, st));
@@ -1126,7 +1127,8 @@ struct tsvm_solver {
         // all zero, as C-SVC starts: nothing to add, and no need for the alphas on the host
         int *nonzero = reinterpret_cast<int *>(red);
         TSVM_CUDA(cudaMemsetAsync(nonzero, 0, sizeof(int), st));
-        TSVM_LAUNCH(any_nonzero_kernel, ceil_div(n, 4096) < 296 ? ceil_div(n, 4096) : 296, 256, 0, st, alpha, n, nonzero);
+        const int blocks = 2 * device_sm_count();
+        TSVM_LAUNCH(any_nonzero_kernel, ceil_div(n, 4096) < blocks ? ceil_div(n, 4096) : blocks, 256, 0, st, alpha, n, nonzero);
         TSVM_CUDA(cudaMemcpyAsync(diff_host, nonzero, sizeof(int), cudaMemcpyDeviceToHost, st));
         TSVM_CUDA(cudaStreamSynchronize(st));
         if (*reinterpret_cast<const int *>(diff_host) == 0) { idle = true; return TSVM_OK; }
