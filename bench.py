@@ -14,8 +14,8 @@ f update. The metric is kernel rows per second (rows of length n = 400,000):
 plus the whole training run to eps = 1e-3, the prediction of the 100,000 test rows, the HBM-bound
 kernels one by one (`rooflines`), and the four smaller configurations end to end (`configs`).
 `--impl reference` times the reference's own CPU implementation (oracle/_ref, built from the
-reference sources with the Eigen products restated) or, if that library is absent, the C
-restatement, on a bounded sample. Prints exactly one JSON line on rank 0.
+reference sources with the Eigen products restated) on a bounded sample; where that library has
+not been built it says so instead of a number. Prints exactly one JSON line on rank 0.
 """
 import argparse
 import hashlib
@@ -160,6 +160,11 @@ def cpu_train_config(tag):
 def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    from oracle import ref_binding as R
+    if not R.available():
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libthundersvm_ref.so has not been built: it is compiled "
+                          "from the reference's sources, which are not on this machine"}))
         return
     s = cpu_sample(args.cpu_sample_rows, max(1, args.steps))
     line = {
