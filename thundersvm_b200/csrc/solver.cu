@@ -1268,6 +1268,7 @@ struct tsvm_solver {
         long long queued = iter;
         idle = false;
         uncollected = true;
+        km->launched(st);                // (the overlapped iteration reads the handle's planes by itself); collect() ends it
         while (!stopped && iter < end) {
             const int ahead = iter == 0 ? 1 : queue_depth();      // (many small solves end with their first iteration)
             while (queued < end && queued < iter + ahead) TSVM_TRY(enqueue_iteration(queued++));
