@@ -14,8 +14,9 @@
  *     labels and ids are int.
  *   - Kernel rows are written row-major, out[i * ld + j] = K(x_idx[i], x_j), the layout the
  *     reference's consumers read (src/thundersvm/kernel/smo_kernel.cu:62,298).
- *   - Handles own every device allocation they make; there is no process-global device
- *     state.
+ *   - Handles own every device allocation they make. What a destroyed handle leaves goes to a pool of the
+ *     process (tsvm_release_cached_memory); the only other device state that handles do not own is the
+ *     scratch of tsvm_select_working_set_static.
  */
 #ifndef THUNDERSVM_B200_H
 #define THUNDERSVM_B200_H
@@ -59,14 +60,17 @@ void tsvm_release_cached_memory(void);
 typedef struct tsvm_km tsvm_km;
 
 /* Constructor for dense instances: X is n x d row-major with row stride ld (floats).
- * loc = TSVM_HOST: X is copied to the device. loc = TSVM_DEVICE: if ld is a multiple of 4 and
+ * loc = TSVM_HOST: X is copied to the device. loc = TSVM_DEVICE: if d and ld are multiples of 4 and
  * X is 16-byte aligned the buffer is used in place (the caller keeps it alive), else copied.
  * Computes self dots (double accumulate, float store) and the diagonal as
  * kernelmatrix.cpp:194-247 does. Replaces KernelMatrix::KernelMatrix (kernelmatrix.cpp:183). */
 tsvm_status tsvm_km_create_dense(const float *X, int n, int d, int ld, int loc, int kernel_type, int degree,
                                  float gamma, float coef0, void *stream, tsvm_km **out);
 
-/* Constructor for CSR instances (0-based column ids < d, ascending inside a row).
+/* Constructor for CSR instances (0-based column ids < d, ascending inside a row). Data that one FP16 number per
+ * entry holds exactly (one-hot and binary features, small counts), with 33 to 256 features or up to 4,096 of which
+ * 2 % are set, is also kept as dense rows, from which the tensor-core engine computes its kernel rows (if the device
+ * has room for them, at most an eighth of its memory); the caller's arrays stay in use.
  * Replaces KernelMatrix::KernelMatrix + CSR_DenseCSR (kernelmatrix.cpp:16-249). */
 tsvm_status tsvm_km_create_csr(const float *val, const int *row_ptr, const int *col, int n, int d, int loc,
                                int kernel_type, int degree, float gamma, float coef0, void *stream,
@@ -115,9 +119,9 @@ tsvm_status tsvm_km_rows_for_features_dense(tsvm_km *km, const float *T_dev, int
  * pipeline), 1 = FP32 CUDA-core tiles, 3 = tcgen05 CTA pairs on two TF32 planes (2 is accepted as an
  * alias), 4 = tcgen05 CTA pairs on two row-scaled FP16 planes (every row is multiplied by a power of
  * two that brings its largest magnitude to [2^14, 2^15) before the split; same accuracy class as
- * engine 3 at twice the tensor-core rate and half the operand bytes). The operand planes are built on
- * the first call that needs them; changing the engine rebuilds them. On a CSR matrix the setting is
- * ignored. */
+ * engine 3 at twice the tensor-core rate and half the operand bytes). The operand planes of the automatic
+ * choice are built when the handle is created (where the device has no room for them: on the first call that
+ * needs them); changing the engine rebuilds them. On a CSR matrix the setting is ignored. */
 tsvm_status tsvm_km_set_dense_engine(tsvm_km *km, int engine);
 
 /* ------------------------------------------------------------------------------------------
@@ -316,10 +320,14 @@ tsvm_status tsvm_update_f(double *f_dev, int n, const double *alpha_diff_dev, in
  * (n_classes - 1) x n_sv layout of include/thundersvm/model/svmmodel.h:155-164, sv_count_host
  * the per-class support-vector counts, rho_dev[nb]. km_sv holds the support vectors. The test
  * batch is dense (T_dev != NULL) or CSR. Batching over the test rows is internal. With dense support
- * vectors of more than 32 features the coefficient sums are part of the contraction's epilogue (FP32
- * partial sums over 128 support vectors, combined in FP64) and the test x SV kernel block is never stored;
+ * vectors of more than 32 features - and with CSR support vectors and test rows whose values one FP16 number
+ * each holds exactly, where a dense copy pays - the coefficient sums are part of the contraction's epilogue
+ * (FP32 partial sums over 32 support vectors, combined in FP64) and the test x SV kernel block is never stored;
  * otherwise it is computed in slabs of at most max_mem_bytes (0 = a sixteenth of the device's memory).
- * Where a slab does not fit what the device has left, it is halved until it does. */
+ * Where a slab does not fit what the device has left, it is halved until it does.
+ * Up to 64 test rows may go through one launch of FP32 dot products instead (up to 32 classes; CSR support vectors:
+ * CSR test rows of at most 2,048 entries together): all three forms hold FP32 accuracy, but a row's decision value
+ * may differ in its last digits (3e-6 relative at 3,001 x 100) with the number of rows it is predicted with. */
 tsvm_status tsvm_predict_dec(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host,
                              const double *rho_dev, int n_classes, int m, const float *T_dev, int dt, int ldt,
                              const float *tval_dev, const int *trow_ptr_dev, const int *tcol_dev, long long tnnz,

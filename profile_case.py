@@ -40,8 +40,8 @@ def main():
     ap.add_argument("--no-overlap", action="store_true", help="solver case: run the steps one after the other")
     ap.add_argument("--engine", default="auto", help="dense engine: auto, simt, tensor2 (TF32 planes), tensor (FP16 planes)")
     ap.add_argument("--csr-config", default="c4", choices=["c2", "c4"],
-                    help="csr_rows case: config 4 (47,236 features, L2-panel engine) or config 2 (123 features, "
-                         "shared-memory-panel engine)")
+                    help="csr_rows case: config 4 (47,236 features, CSR engine) or config 2 (123 one-hot features, "
+                         "worked on as dense rows)")
     args = ap.parse_args()
     capi.lib()
     if args.case == "predict":

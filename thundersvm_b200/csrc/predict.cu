@@ -4,11 +4,13 @@
 // SVC::predict_label (src/thundersvm/model/svc.cpp:265-289) and the vote-only form
 // sum_kernel_values_instant (kernelmatrix_kernel.cu:99-138).
 //
-// Dense support vectors on the CTA-pair tensor engine take the fused path: the test x SV contraction
-// multiplies its kernel values by the coefficients in its epilogue and adds them to the decision values
-// (dense_tc2.cu, prediction form), so the kernel block is never written. Other storages (CSR support
-// vectors, at most 32 features) compute the block in slabs of test rows and reduce it with
-// sum_kernel_values_kernel.
+// Three paths:
+//   * a few test rows (predict_few.cuh): one launch, FP32 dot products on CUDA cores;
+//   * dense support vectors of more than 32 features, and CSR ones that the handle also keeps as dense rows
+//     (choose_csr_storage) if the test rows qualify too: the test x SV contraction multiplies its kernel values by
+//     the coefficients in its epilogue and adds them to the decision values (dense_tc2.cu, prediction form), so the
+//     kernel block is never written;
+//   * the rest compute the block in slabs of test rows and reduce it with sum_kernel_values_kernel.
 #include "common.cuh"
 #include "predict_few.cuh"
 #include <vector>
