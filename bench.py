@@ -33,7 +33,7 @@ sys.path.insert(0, ROOT)
 
 N_FULL, D_FULL, WS, Q = 400000, 2000, 1024, 512
 GAMMA, C_SVC, EPS = 0.5, 1.0, 1e-3
-TRAFFIC_37888 = 388.7e6   # dram read + write bytes of one 37,888-instance launch of the kernel (ncu capture summarised in profiles/)
+TRAFFIC_37888 = 387.8e6   # dram read + write bytes of one 37,888-instance launch of the kernel (ncu capture summarised in profiles/)
 WORKLOAD = ("config5: binary C-SVC, RBF gamma=0.5 C=1 eps=1e-3, %dx%d dense fp32, ws=1024, 512 new kernel rows per "
             "outer iteration")
 NO_CPU_CONVERGENCE = ("the CPU build cannot converge this configuration in bounded time (26,042 s published for the "
@@ -338,10 +338,10 @@ def extra_rooflines(torch, capi, synth, hbm_peak, peak_src, n):
     flags = torch.zeros(n, dtype=torch.uint8, device="cuda")
     sel = capi.WorkingSetSelector(n, WS)
     us = time_calls(torch, lambda: sel.select(fv, av, yv, 1.0, 1.0, Q, in_ws=flags), 50)
-    out.append(hbm_roofline("working-set selection (radix top-k + merge, config 5: 512 of %d)" % n, n * 21, us, hbm_peak,
+    out.append(hbm_roofline("working-set selection (top-k + merge, config 5: 512 of %d)" % n, n * 21, us, hbm_peak,
                             peak_src, "bytes = n*(8 f + 8 alpha + 4 y + 1 flag) read once; the selection is one cooperative "
-                                      "launch of two or three sweeps separated by grid barriers plus an exact sort of the "
-                                      "candidates by one block: a latency chain, not bandwidth-bound"))
+                                      "launch of one sweep from sampled pivots, ranks counted by the whole grid and a walk "
+                                      "over the lists by its last block: a latency chain, not bandwidth-bound"))
     sel.close()
     del yv, fv, av, flags, f
     # CSR kernel rows, 512 rows per call
@@ -359,7 +359,8 @@ def extra_rooflines(torch, capi, synth, hbm_peak, peak_src, n):
         nnz, nnz_ws = int(rp[-1]), int(np.diff(rp)[idx_np].sum())
         r = hbm_roofline("CSR kernel rows (%s: 512 rows x %d, nnz %d)" % (tag, nn, nnz),
                          Q * nn * 4 + nnz * 8 + (nn + 1) * 4 + nnz_ws * 8, us, hbm_peak, peak_src,
-                         "bytes = q*n*4 out + nnz*8 + (n+1)*4 CSR read once + nnz(requested rows)*8")
+                         "bytes = q*n*4 out + nnz*8 + (n+1)*4 CSR read once + nnz(requested rows)*8" +
+                         ("; one-hot data: worked on as dense rows" if tag == "c2" else ""))
         r["kernel_rows_per_s"] = Q / (us * 1e-6)
         out.append(r)
         km.close()

@@ -22,8 +22,8 @@
 // written in every iteration, FP64 keys and one exact division per thread in the second-order choice); where most
 // values tie (a kernel close to the identity) 1.39 against 2.07; nu 1.48 against 2.58. Of the 1,900 cycles about 740 are
 // the two L2 round trips (372 cycles each), 440 the first reduction, 250 the second. Inside a solve, where other kernels use
-// the L2, the rows copied ahead (copy_rows_ahead) count more: 10,000 x 20 339 -> 303 us per call, next to the kernel-row
-// launch of 200,000 x 2,000 817 -> 588 us.
+// the L2, the rows copied ahead (copy_rows_ahead) count more: 10,000 x 20 339 -> 307 us per call, next to the kernel-row
+// launch of 200,000 x 2,000 817 -> 597 us.
 #pragma once
 #include "common.cuh"
 
