@@ -100,3 +100,29 @@ a1, rho1, st1 = solve()
 assert st1["cache_rows"] < st0["cache_rows"], (st0["cache_rows"], st1["cache_rows"])
 assert torch.equal(a0, a1) and rho0 == rho1
 """)
+
+
+def test_a_solver_takes_the_room_of_a_dense_copy(capi):
+    """One-hot data, 30,000 x 200: the handle keeps a dense copy and planes (48 MB), the smallest row buffer takes 184 MB.
+    With 160 MB left the solve goes back to the entries; the same handle then predicts and gives rows from them."""
+    run("""
+n, d, k = 30000, 200, 14
+col = np.sort(rng.permuted(np.tile(np.arange(d, dtype=np.int32), (n, 1)), axis=1)[:, :k], axis=1).astype(np.int32)
+csr = (np.ones(n * k, np.float32), np.arange(0, n * k + 1, k, dtype=np.int32), col.ravel())
+s = rng.standard_normal(d)[col].sum(1) + rng.standard_normal(n)
+yd = torch.from_numpy(np.where(s > 0, 1, -1).astype(np.int32)).cuda()
+km = capi.KernelMatrix(csr=tuple(torch.from_numpy(a).cuda() for a in csr), d=d, gamma=0.05)
+idx = torch.arange(0, 64, dtype=torch.int32, device="cuda")
+a0, f0, a1, f1 = (torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(4))
+f0 -= yd; f1 -= yd
+rows = torch.empty((64, n), dtype=torch.float32, device="cuda")
+km.get_rows(idx, rows)
+rows0 = rows.cpu()
+rho0, st0 = capi.smo_solve(km, yd, a0, f0, 1e-3, 1.0, 1.0, 1024)
+taken = leave(160)
+rho1, st1 = capi.smo_solve(km, yd, a1, f1, 1e-3, 1.0, 1.0, 1024)
+assert st1["cache_rows"] == 1536 < st0["cache_rows"], (st0["cache_rows"], st1["cache_rows"])
+assert abs(st1["objective"] / st0["objective"] - 1) < 1e-6 and abs(rho1 - rho0) < 2e-3, (st0, st1, rho0, rho1)
+km.get_rows(idx, rows)
+assert float(((rows.cpu() - rows0).abs() / rows0).max()) < 1e-5
+""")
