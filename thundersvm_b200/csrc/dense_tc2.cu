@@ -21,10 +21,6 @@
 // destination CTA; every load is addressed to one CTA's shared memory only. Every mbarrier wait is bounded.
 #include "tc_common.cuh"
 
-#ifndef TSVM_PROMO
-#define TSVM_PROMO 2
-#endif
-
 namespace tsvm {
 
 namespace tc2 {
@@ -247,7 +243,9 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     // the same value in every thread of the grid: the launch's m, or the smaller count found on the device
     const int m = ex.m_dev ? min(m_launch, max(*ex.m_dev, 0)) : m_launch;
     constexpr int BK = F16 ? 64 : 32;          // elements per k slab
-    constexpr int PROMO = F16 ? TSVM_PROMO : 1;   // k slabs summed in tensor memory before the FP32 promotion
+    // k slabs summed in tensor memory before the FP32 promotion (longer units fail the bound on kernel values of 784
+    // features in [0, 1])
+    constexpr int PROMO = F16 ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
