@@ -160,10 +160,70 @@ def test_local_smo_matches_oracle(capi, solver, ws):
     assert np.allclose(ad_got.cpu().numpy(), ad_exp, rtol=0, atol=1e-9)
 
 
+def _local_smo_both(capi, solver, kww, y, f, alpha, C, eps=1e-3, max_iter=100000):
+    ids = np.arange(len(y), dtype=np.int32)
+    diag = np.ascontiguousarray(np.diagonal(kww))
+    exp = P.local_smo("c" if solver == "c" else "nu", y, f, alpha, ids, C, C, kww, diag, eps, max_iter=max_iter, cuda_semantics=1)
+    got = capi.local_smo(_t(kww), _t(diag), _t(y), _t(f), _t(alpha), C, C, eps, max_iter=max_iter, solver=solver)
+    return [g.cpu().numpy() for g in got], exp
+
+
+@pytest.mark.parametrize("solver", ["c", "nu_svc"])
+@pytest.mark.parametrize("ws", [2, 31, 33, 128, 130, 256, 257, 500, 513, 1000, 1023])
+def test_local_smo_odd_sizes(capi, solver, ws):
+    """Working sets that do not fill the threads' slots, on either side of every change of the number of slots per thread:
+    the oracle's steps, to the rounding of the sums."""
+    rng = np.random.default_rng(ws)
+    X = rng.standard_normal((ws, 6))
+    kww = np.exp(-0.1 * ((X[:, None] - X[None]) ** 2).sum(2)).astype(np.float32)
+    y = np.where(np.arange(ws) % 2 == 0, 1, -1).astype(np.int32)
+    alpha = np.zeros(ws) if solver == "c" else np.where(rng.random(ws) < 0.5, 1.0, 0.0)
+    f = -y + 0.01 * rng.standard_normal(ws) if solver == "c" else 0.3 * rng.standard_normal(ws)
+    (a, ad, diff), (a_exp, ad_exp, diff_exp) = _local_smo_both(capi, solver, kww, y, f, alpha, 1.0)
+    assert diff[1] == diff_exp[1] and diff[0] == pytest.approx(diff_exp[0], rel=1e-12)
+    assert np.allclose(a, a_exp, rtol=0, atol=1e-9) and np.allclose(ad, ad_exp, rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("case", ["duplicates", "large_values", "huge_C", "tiny_values", "negative_curvature", "infinite"])
+@pytest.mark.parametrize("ws", [64, 1024])
+def test_local_smo_values_at_the_ends_of_the_range(capi, ws, case):
+    """What the single-precision choice of j, the scaled f and the division by a reciprocal do not cover takes the general
+    form: curvature of zero or below, kernel values and C beyond single precision's square or the scale, infinite values."""
+    rng = np.random.default_rng(ws)
+    X = rng.standard_normal((ws, 5))
+    if case == "duplicates":
+        X[ws // 2:] = X[:ws // 2]                               # each instance twice, with either label
+    kww = np.exp(-0.1 * ((X[:, None] - X[None]) ** 2).sum(2)).astype(np.float32)
+    y = np.where(np.arange(ws) % 2 == 0, 1, -1).astype(np.int32)
+    f = -y + 0.01 * rng.standard_normal(ws)
+    C, steps = 1.0, 40
+    if case == "duplicates":
+        y[ws // 2:] = -y[:ws // 2]
+        f = -y + 0.01 * rng.standard_normal(ws)
+    elif case == "large_values":
+        kww *= np.float32(1e33)
+    elif case == "huge_C":
+        kww, C = kww * np.float32(1e-36), 1e40
+    elif case == "tiny_values":
+        kww *= np.float32(1e-41)                                # denormals
+    elif case == "negative_curvature":
+        kww[0, 1] = kww[1, 0] = 3.0
+    elif case == "infinite":
+        kww[3, 5] = kww[5, 3] = np.inf
+        steps = 1
+        f[3] = -9.0
+        f[7] = 9.0
+        y[3], y[7] = 1, -1
+    (a, ad, diff), (a_exp, ad_exp, diff_exp) = _local_smo_both(capi, "c", np.ascontiguousarray(kww), y, f, np.zeros(ws), C, max_iter=steps - 1)
+    assert diff[1] == diff_exp[1]
+    # (alphas of the order of C: sums of `steps` steps, each to a few ulp)
+    assert np.allclose(a, a_exp, rtol=1e-9, atol=1e-9 * max(1.0, np.abs(a_exp).max()))
+
+
 @pytest.mark.parametrize("ws", [256, 512, 1024])
 def test_local_smo_rows_copied_ahead_hold_the_same_values(capi, ws):
-    """A block whose rows are 16-byte aligned is read through the ring in shared memory, one that is not straight from
-    memory: the same steps, bit for bit, over some thousand of them."""
+    """A block whose rows are 16-byte aligned and one that is not, while other warps read rows ahead: the same steps, bit
+    for bit, over some thousand of them."""
     import torch
     g = torch.Generator(device="cuda").manual_seed(ws)
     X = torch.randn(ws, 12, device="cuda", generator=g)

@@ -13,17 +13,25 @@
 //     reduction over the doubles' high words finds the winner, and only if two lanes share the high word the low words
 //     are looked at.
 //   * The largest f over I_low is needed for the stopping rule only. Its high word gives a lower bound of it; the
-//     exact value is reduced when the bound cannot show that the gap is still open.
+//     exact value is reduced when the bound cannot show that the gap is still open. The rule is applied after the second
+//     argmin, next to the loads for the step: nothing has been changed by then.
 //   * The second-order values b^2 / a are compared in FP32 (error below 1e-6 relative: b truncated to 24 bits, a rounded
 //     once, an approximate reciprocal). If the best value of the block stands out by more than 8e-6 it is the
 //     winner in FP64 too; otherwise - near-equal instances, mostly - or if an operand leaves the range in which that
 //     error bound holds, the block repeats the comparison in FP64 (a few ulp), ties to the lower slot.
-// Measured (RBF block, 1,024 slots): 1.00 us per iteration, 1.74 before (512 threads with two slots each, every mirror
-// written in every iteration, FP64 keys and one exact division per thread in the second-order choice); where most
-// values tie (a kernel close to the identity) 1.39 against 2.07; nu 1.48 against 2.58. Of the 1,900 cycles about 740 are
-// the two L2 round trips (372 cycles each), 440 the first reduction, 250 the second. Inside a solve, where other kernels use
-// the L2, the rows copied ahead (copy_rows_ahead) count more: 10,000 x 20 339 -> 307 us per call, next to the kernel-row
-// launch of 200,000 x 2,000 817 -> 597 us.
+//   * No conversion instructions on the chain (16 of them took 160 cycles): f is held times 2^-896, which makes a float's
+//     bits a double's and a double's a float's by shifts. A value of f below 2^-126 loses digits that way, sums of kernel
+//     values do not get there.
+//   * The step is divided by a reciprocal corrected once, its result by its remainder: within an ulp of the division.
+//   * Two more warps read the rows that the next iterations will want into the L1 cache (read_rows_ahead). In most calls every
+//     row is wanted about once, so a cache alone finds a tenth of them; the best six of an argmin's list hold the next
+//     iteration's winner nine times in ten.
+// Measured per iteration at 1,024 slots inside a solve, before (conversions, an exact division, 32 rows copied to shared
+// memory by one more warp and looked up there) and now: 10,000 x 20 1.05 -> 0.86 us, 12,003 x 784 1.00 -> 0.85, text
+// 1.00 -> 0.85, one-hot records, where many values tie, 1.10 -> 0.93, 200,000 x 2,000 next to the kernel-row launch
+// 1.44 -> 1.28, nu (without the reading warps) 1.38 -> 1.17. With every row found in L1 an iteration takes 0.67 us: 486
+// instructions per warp (604 before) at 2.7 cycles, dependent ones mostly. Two floats per instruction in the second-order
+// values (16 instructions fewer) changed nothing; masks instead of compares where a slot joins or leaves a list cost 5 %.
 #pragma once
 #include "common.cuh"
 
@@ -57,388 +65,464 @@ __device__ __forceinline__ double reciprocal(double a) {
     return a != 0.0 && fabs(a) < 1e300 ? r : r0;
 }
 
-// Row ring: rows of kww that the next iterations are likely to need, copied to shared memory by a warp of its own.
-constexpr int RING = 32;                // one ring slot per lane of the copying warp
-constexpr int RING_SPARE = 10;          // slots kept free for the next copies
-constexpr int NOT_THERE = -1, ON_THE_WAY = -2;
-
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
-__device__ __forceinline__ int load_acquire(const int *p) {
-    int v;
-    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
-    return v;
-}
-__device__ __forceinline__ void store_release(int *p, int v) {
-    asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
-}
-__device__ __forceinline__ bool copy_done(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
+// Reading ahead: how many slots of an argmin are looked after (the bounds), and for how many iterations a row that was read
+// is taken to be there. The cache does not keep rows for long: KEEP 24 / 8 / 4 / 2 / 1 / 0 make 0.92 / 0.91 / 0.88 / 0.87 / 0.86 /
+// 0.90 us (12,003 x 784); with 3 to 6 or 6 to 12 slots 0.89.
+constexpr int KEEP = 1, LO = 4, HI = 8;
 template <int T>
 __device__ __forceinline__ void solver_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory"); }
 
-struct First { double f; int slot; float low; };        // a warp's smallest f over I_up, its slot; high word of max f over I_low
-struct Second { float best, next; int slot, pad; };     // a warp's largest and second-largest estimate of b^2 / a
+// What a warp leaves for the others
+struct __align__(16) First { double f; int slot, pad; };            // its smallest f over I_up and that slot
+struct __align__(16) Second { float best; int slot; float low[2]; };    // its largest estimate of b^2 / a; max f over I_low (high word, per class)
+constexpr int SLOT_MASK = 0x7ff, TIED = 0x800;                      // TIED: another value of the warp is too close
 
-// The copying warp. Which rows the next iterations need can be guessed: the winner of an argmin is usually among the best
-// few of the argmin before. Every warp of the solver leaves its best two slots of both argmins in `cand` (n_cand ids);
-// whichever of them has no row in the ring is copied there, and a row that has not been wanted for longest makes room.
-//   where[t]: ring slot of row t, NOT_THERE or ON_THE_WAY. It is set only when the copy has arrived, so a solver thread
-//   either finds the row or reads kww; both hold the same values. The copying warp's wait on the mbarrier makes the row
-//   visible to itself; its release of `where` and the solver threads' acquire pass that on.
-//   A row is taken out of `where` first, and the fence before `window` is read has that seen by the whole block; its slot is
-//   overwritten three windows later (a window: from one barrier of the solver to the next). A row that a solver thread finds
-//   in a window is read in that window and the next; the barrier orders those reads before thread 0's release of a later
-//   `window`, which the copying warp acquires before it copies.
-//   Measured: the two acquires and the two releases cost 0.5 - 1 % of a solve (10,000 x 20: 33.9 -> 34.3 ms). Letting thread 0
-//   read a count of removals and hand it back with `window` cost 2 - 3 % more.
-__device__ void copy_rows_ahead(const float *__restrict__ kww, int ws, float *ring, int *where, const int *cand, int n_cand,
-                                const int *window, const int *done, unsigned long long *bars, int *stamp, int *stage) {
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max_abs3(float a, float b, float c) {        // NaN if one of them is
+    float r;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+template <int S>
+__device__ __forceinline__ float max_of(const float (&v)[S]) {
+    if constexpr (S == 8) return max3(max3(v[0], v[1], v[2]), max3(v[3], v[4], v[5]), fmaxf(v[6], v[7]));
+    if constexpr (S == 4) return max3(v[0], v[1], fmaxf(v[2], v[3]));
+    if constexpr (S == 2) return fmaxf(v[0], v[1]);
+    return v[0];
+}
+template <int S>
+__device__ __forceinline__ float min_of(const float (&v)[S]) {
+    if constexpr (S == 8) return min3(min3(v[0], v[1], v[2]), min3(v[3], v[4], v[5]), fminf(v[6], v[7]));
+    if constexpr (S == 4) return min3(v[0], v[1], fminf(v[2], v[3]));
+    if constexpr (S == 2) return fminf(v[0], v[1]);
+    return v[0];
+}
+template <int S>
+__device__ __forceinline__ float max_abs_of(const float (&v)[S]) {
+    if constexpr (S == 8) return max_abs3(max_abs3(v[0], v[1], v[2]), max_abs3(v[3], v[4], v[5]), max_abs3(v[6], v[7], v[7]));
+    if constexpr (S == 4) return max_abs3(v[0], v[1], max_abs3(v[2], v[3], v[3]));
+    return max_abs3(v[0], v[S - 1], v[S - 1]);
+}
+__device__ __forceinline__ float mul_ftz(float a, float b) {
+    float r;
+    asm("mul.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// k * 2^-896, exact for every finite float (denormals and zeros too): the float's bits, moved to where a double has them
+constexpr double DOWN = 0x1p-896, BACK = 0x1p896;
+__device__ __forceinline__ double widened(float k) {
+    const int u = __float_as_int(k);
+    return __hiloint2double((u >> 3) & 0x8fffffff, u << 29);
+}
+
+// The reading warps, one for each argmin. Every thread of the solver leaves the best of its slots (best: value, slot); those
+// that are close to the best of all are read, unless that was just done. What is close is adjusted until LO to HI slots are.
+// A row is read by asynchronous copies of one word of every 32-byte sector to a place nobody looks at (sink): they put the
+// sectors into the L1 cache, and unlike loads nothing waits for them (loads: 10 % slower; prefetch.global.L1: no effect).
+// Nothing but time depends on what these warps see: `best`, `window` and `last` are read while they are written. Words copied
+// are words of kww, x is a slot at any time, and a row past ws is not read.
+template <int T, bool LARGEST>
+__device__ void read_rows_ahead(const float *__restrict__ kww, int ws, const float2 *best, const int *window, const int *done,
+                                int *last, float *sink) {
+    constexpr int E = T / 32;
     const int lane = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu, bar = smem_addr(bars + lane), row_bytes = (unsigned) ws * 4;
-    enum { FREE, COMING, READY };
-    int state = FREE, row = 0, freed = -4, used = 0, seen = -1;
-    unsigned parity = 0;
-    auto arrived = [&](int now) {
-        if (state == COMING && copy_done(bar, parity)) {
-            parity ^= 1;
-            state = READY;
-            used = now;
-            store_release(where + row, lane);
-        }
-    };
-    // (bounded: a solver that runs longer than this goes on without new rows)
+    const unsigned full = 0xffffffffu;
+    int seen = 0;
+    float width = LARGEST ? 0.5f : 1e-3f;
+    // (bounded: a solver that runs longer than this goes on without)
     for (int polls = 0; polls < (1 << 26); ++polls) {
-        const int now = load_acquire(window);
-        if (load_acquire(done)) break;
-        arrived(now);
-        if (__all_sync(full, now == seen)) { __nanosleep(32); continue; }
+        const int now = *(volatile const int *) window;
+        if (__any_sync(full, *(volatile const int *) done)) break;
+        if (__all_sync(full, now == seen)) { continue; }
         seen = now;
-        // candidates without a row, each once
-        const int x = lane < n_cand ? *(volatile const int *) (cand + lane) : -1;
-        const bool valid = (unsigned) x < (unsigned) ws;
-        const int at = valid ? *(volatile int *) (where + x) : (int) ON_THE_WAY;
-        const unsigned same = __match_any_sync(full, valid ? x : -1 - lane);
-        const bool need = valid && at == NOT_THERE && lane == __ffs(same) - 1;
-        if (valid && at >= 0) stamp[at] = now;
-        const unsigned needs = __ballot_sync(full, need);
-        if (need) stage[__popc(needs & ((1u << lane) - 1))] = x;
-        __syncwarp();
-        if (state == READY && stamp[lane] == now) used = now;
-        const bool open = state == FREE && now - freed >= 3;
-        const unsigned opens = __ballot_sync(full, open);
-        const int k = __popc(opens & ((1u << lane) - 1));
-        if (open && k < __popc(needs)) {
-            row = stage[k];
-            *(volatile int *) (where + row) = ON_THE_WAY;
-            state = COMING;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(row_bytes) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(smem_addr(ring + (size_t) lane * ws)), "l"(kww + (size_t) row * ws), "r"(row_bytes), "r"(bar) : "memory");
+        float v[E];
+        int x[E], before[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float2 b = best[e * 32 + lane];
+            // the first argmin's values are the high words of doubles
+            v[e] = LARGEST ? b.x : (float) (__hiloint2double(__float_as_int(b.x), 0) * BACK);
+            x[e] = __float_as_int(b.y);
         }
-        // make room: the row that has not been wanted for longest
-        const int spare = __popc(__ballot_sync(full, state == FREE));
-        const int oldest = __reduce_min_sync(full, state == READY ? used : 0x7fffffff);
-        const unsigned olds = __ballot_sync(full, state == READY && used == oldest);
-        if (spare < RING_SPARE && state == READY && used == oldest && oldest < now &&
-            __popc(olds & ((1u << lane) - 1)) < RING_SPARE - spare) {
-            store_release(where + row, NOT_THERE);
-            __threadfence_block();
-            state = FREE;
-            freed = load_acquire(window);
+#pragma unroll
+        for (int e = 0; e < E; ++e) before[e] = last[x[e]];
+        float m = v[0];
+#pragma unroll
+        for (int e = 1; e < E; ++e) m = LARGEST ? fmaxf(m, v[e]) : fminf(m, v[e]);
+        m = LARGEST ? warp_max_f32(m) : warp_min_f32(m);
+        const float limit = LARGEST ? m * width : m + width;
+        int count = 0;
+        unsigned needs[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const bool near = LARGEST ? v[e] > limit : v[e] < limit;
+            count += __popc(__ballot_sync(full, near));
+            const bool need = near && now - before[e] > KEEP && x[e] < ws;
+            needs[e] = __ballot_sync(full, need);
+            if (need) last[x[e]] = now;
         }
-        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            for (unsigned n = needs[e]; n; n &= n - 1) {
+                const float *row = kww + __shfl_sync(full, x[e], __ffs(n) - 1) * ws;
+                // one word of a sector of 32 bytes; where it is put does not matter
+                for (int t = lane * 8; t < ws; t += 32 * 8)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(sink + lane)), "l"(row + t) : "memory");
+            }
+        if (LARGEST) width = count < LO ? width * 0.8f : count > HI ? 1.0f - (1.0f - width) * 0.8f : width;
+        else width = count < LO ? width * 1.25f : count > HI ? width * 0.8f : width;
     }
-    for (int polls = 0; polls < (1 << 24) && __any_sync(full, state == COMING); ++polls) arrived(0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 }  // namespace smo
 
-// Slot t of the working set belongs to thread t % T. S slots per thread; 32 more threads copy rows ahead.
+// Slot t of the working set belongs to thread t % 32 of warp t / (32 S): a warp holds a run of 32 S slots, so that of equal
+// values the lower slot is in the lower warp. S slots per thread; in the C form two more warps read rows ahead.
+// f is held as f * 2^-896: a float's bits are then a double's without a conversion (widened), and a double's are a float's.
 template <bool NU, int S, int T>
-__global__ void __launch_bounds__(T + 32, 1)
+__global__ void __launch_bounds__(T + (NU ? 0 : 64), 1)
 local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict__ diag_ws,
                  const int *__restrict__ y_ws, const double *__restrict__ f_ws, double *__restrict__ alpha_ws,
                  double *__restrict__ alpha_diff, double Cp_in, double Cn_in, double eps, int max_iter,
                  double *__restrict__ diff, const int *__restrict__ ids, double *__restrict__ alpha_global,
-                 const int *__restrict__ stop, int use_ring, PhaseTimes *times) {
+                 const int *__restrict__ stop, int ahead, PhaseTimes *times) {
     using namespace smo;
     constexpr int W = T / 32, CLS = NU ? 2 : 1;             // nu: the lists of I_up and I_low are split by class
-    constexpr bool AHEAD = !NU;                             // (nu reads two rows i and guesses j badly: 5 % slower with the ring)
+    constexpr int RUN = 32 * S;                             // slots of a warp
     if (stop && *stop) {            // queued past the end of a solve: no step, so the f update that follows adds zero
-        for (int t = threadIdx.x; t < ws; t += T + 32) alpha_diff[t] = 0;
+        for (int t = threadIdx.x; t < ws; t += blockDim.x) alpha_diff[t] = 0;
         return;
     }
     if (times && threadIdx.x == 0) times->local_begin = device_ns();
-    __shared__ double f_sm[S * T], a_sm[S * T];
-    __shared__ float kd_sm[S * T];
-    __shared__ int y_sm[S * T];
+    __shared__ __align__(16) double f_sm[S * T];
+    __shared__ double a_sm[S * T];
+    __shared__ float2 ky_sm[S * T];                         // diagonal, label
     __shared__ First e1[CLS][W];
     __shared__ Second e2[W];
     __shared__ unsigned long long exact_key[CLS][W];
     __shared__ int exact_slot[CLS][W];
     __shared__ double exact_low[CLS][W];
-    // row ring (use_ring): ring [RING][ws] floats in dynamic shared memory
-    extern __shared__ __align__(128) float ring[];
-    constexpr int N_CAND = 2 * (CLS + 1) * W;
-    __shared__ int where[S * T], cand[N_CAND], ring_stamp[RING], ring_stage[32], window, done;
-    __shared__ __align__(8) unsigned long long ring_bar[RING];
-    static_assert(N_CAND <= 32, "one candidate per lane of the copying warp");
+    // what the reading warps look at: every thread's best value of the two argmins with its slot; when it changed
+    constexpr bool AHEAD = !NU;                             // (nu reads two rows i and guesses j badly: 1.216 us without, 1.228 with)
+    __shared__ float2 best[2][T];
+    __shared__ int last[S * T], window[2], done;
+    __shared__ float sink[2][32];
+    static_assert(S * T <= SLOT_MASK, "a slot fits its field");
     const double Cp = NU ? (double) (float) Cp_in : Cp_in;
     const double Cn = NU ? Cp : Cn_in;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid >= T) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(ring_bar + lane)) : "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        ring_stamp[lane] = -1;
-        if (lane < N_CAND) cand[lane] = -1;
-        if (lane == 0) { window = 0; done = 0; }
-        for (int t = lane; t < S * T; t += 32) where[t] = NOT_THERE;
+    if (AHEAD && tid >= T) {
+        for (int t = tid - T; t < S * T; t += 64) last[t] = -KEEP - 1;
+        for (int t = tid - T; t < 2 * T; t += 64) best[0][t] = make_float2(0.0f, 0.0f);
+        if (tid == T) { window[0] = window[1] = 0; done = 0; }
         __syncthreads();
-        if (AHEAD && use_ring) copy_rows_ahead(kww, ws, ring, where, cand, N_CAND, &window, &done, ring_bar, ring_stamp, ring_stage);
+        if (ahead) {
+            if (warp == W) read_rows_ahead<T, false>(kww, ws, best[0], &window[0], &done, last, sink[0]);
+            else read_rows_ahead<T, true>(kww, ws, best[1], &window[1], &done, last, sink[1]);
+        }
         return;
     }
 
+    // the thread's slots: runs of V, 32 V apart
+    constexpr int V = NU && S >= 4 ? 4 : 1;
+    const int t0 = warp * RUN + lane * V;
+    auto nth = [](int s) { return s / V * (32 * V) + s % V; };
     double f[S];
-    float kd[S], pen_up[S], pen_low[S];     // +-FAR_POS: what clamps a non-member's f out of the list
+    float kd[S], pen_up[CLS][S], pen_low[S];    // +-FAR_POS: what clamps a non-member's f out of the list
     bool pos[S];                            // nu: class of the slot
-    int off[S];                             // column of the slot in a row of kww (any valid one where there is no slot)
+    float kd_most = 0;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-        const int t = tid + s * T;
+        const int t = t0 + nth(s);
         double a = 0;
         int y = 0;                          // y = 0: member of no set
         f[s] = 0; kd[s] = 0;
-        if (t < ws) { f[s] = f_ws[t]; a = alpha_ws[t]; y = y_ws[t]; kd[s] = diag_ws[t]; }
-        f_sm[t] = f[s]; a_sm[t] = a; y_sm[t] = y; kd_sm[t] = kd[s];
-        pen_up[s] = in_I_up(a, y, Cp, Cn) ? -FAR_POS : FAR_POS;
+        if (t < ws) { f[s] = f_ws[t] * DOWN; a = alpha_ws[t]; y = y_ws[t]; kd[s] = diag_ws[t]; }
+        f_sm[t] = f[s]; a_sm[t] = a; ky_sm[t] = make_float2(kd[s], __int_as_float(y));
+        const float up_s = in_I_up(a, y, Cp, Cn) ? -FAR_POS : FAR_POS;
+#pragma unroll
+        for (int c = 0; c < CLS; ++c) pen_up[c][s] = !NU || (y > 0) == (c == 0) ? up_s : FAR_POS;
         pen_low[s] = in_I_low(a, y, Cp, Cn) ? FAR_POS : -FAR_POS;
         pos[s] = y > 0;
-        off[s] = t < ws ? t : 0;
+        kd_most = max_abs3(kd_most, kd[s], kd[s]);
     }
     __syncthreads();
-    auto read_row = [&](int r, int at, float (&k)[S]) {
-        if (at >= 0) {
+    const bool whole = ws == S * T && (V == 1 || ((unsigned long long) kww & 15) == 0);
+    auto read_row = [&](int r, float (&k)[S]) {
+        const float *p = kww + r * ws + t0;
+        if (whole) {
+            if constexpr (V == 4) {
 #pragma unroll
-            for (int s = 0; s < S; ++s) k[s] = ring[at * ws + off[s]];
+                for (int s = 0; s < S; s += 4) {
+                    const float4 x = __ldg((const float4 *) (p + nth(s)));
+                    k[s] = x.x; k[s + 1] = x.y; k[s + 2] = x.z; k[s + 3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int s = 0; s < S; ++s) k[s] = __ldg(p + nth(s));
+            }
         } else {
 #pragma unroll
-            for (int s = 0; s < S; ++s) k[s] = __ldg(kww + r * ws + off[s]);
+            for (int s = 0; s < S; ++s) k[s] = t0 + nth(s) < ws ? __ldg(p + nth(s)) : 0.0f;
         }
     };
+    const bool mild = Cp < 0x1p100 && Cn < 0x1p100;         // steps stay in a double's range when scaled
 
-    double local_eps = 0;
+    double local_eps = 0;                   // (scaled like f)
     int it = 0;
     // the last step, written to a_sm once every thread has read what it needs for that step
     int step_i = 0, step_j = 0;
-    double step_ai = a_sm[0], step_aj = step_ai;
+    double step_vi = a_sm[0], step_vj = step_vi;
     for (;;) {
-        float first_h[CLS];                 // the lane's best, without the warp's winner
+        // ---- smallest f over I_up, with its slot -------------------------------------------------------------
+        float first_h[CLS];                 // the thread's best
         int first_slot[CLS];
-        // ---- smallest f over I_up (with its slot), high word of the largest f over I_low ---------------------
-        float low_h[S];                     // high word of f, clamped to -FAR_POS outside I_low
-#pragma unroll
-        for (int s = 0; s < S; ++s) low_h[s] = fminf(high_as_float(f[s]), pen_low[s]);
 #pragma unroll
         for (int c = 0; c < CLS; ++c) {
+            float hs[S];
             double v[S];
             int slot[S];
-            float lo = -FAR_POS;
 #pragma unroll
             for (int s = 0; s < S; ++s) {
-                const float h = fmaxf(high_as_float(f[s]), pen_up[s]);
-                const bool mine = !NU || pos[s] == (c == 0);
-                v[s] = with_high(mine ? h : FAR_POS, f[s]);
-                slot[s] = tid + s * T;
-                lo = fmaxf(lo, mine ? low_h[s] : -FAR_POS);
+                hs[s] = fmaxf(high_as_float(f[s]), pen_up[c][s]);
+                v[s] = with_high(hs[s], f[s]);
+                slot[s] = t0 + nth(s);
             }
             // The warp's reduction runs over the high words and needs only their minimum; the exact minimum and its slot
             // are found next to it. Neighbouring slots first: the left operand always holds the lower slots and wins ties.
-            float h = high_as_float(v[0]);
-#pragma unroll
-            for (int s = 1; s < S; ++s) h = fminf(h, high_as_float(v[s]));
-            const float h_min = warp_min_f32(h), lo_max = warp_max_f32(lo);
+            const float h = min_of(hs), h_min = warp_min_f32(h);
 #pragma unroll
             for (int d = 1; d < S; d <<= 1)
 #pragma unroll
                 for (int s = 0; s + d < S; s += 2 * d)
                     if (v[s + d] < v[s]) { v[s] = v[s + d]; slot[s] = slot[s + d]; }
             bool winner = h == h_min;
-            First e;
-            e.f = v[0]; e.slot = slot[0]; e.low = lo_max;
-            if (winner) { e1[c][warp] = e; if (AHEAD) cand[c * W + warp] = slot[0]; }
             const unsigned at_min = __ballot_sync(0xffffffffu, winner);
-            if (at_min & (at_min - 1)) {            // several lanes share the high word: the lane with the exact minimum writes again
+            if ((at_min ^ (at_min - 1)) <= at_min - 1) {        // not one lane: the exact minimum, ties to the lower slot
                 unsigned long long key = ordered_key(v[0]);
                 int sl = slot[0];
                 warp_argmin_u64(key, sl);
                 winner = slot[0] == sl;
-                __syncwarp();
-                if (winner) { e1[c][warp] = e; if (AHEAD) cand[c * W + warp] = slot[0]; }
             }
-            first_h[c] = winner ? FAR_POS : h;
-            first_slot[c] = slot[0];
+            if (winner) e1[c][warp] = First{v[0], slot[0], 0};
+            first_h[c] = h; first_slot[c] = slot[0];
         }
         solver_barrier<T>();
-        if (AHEAD && tid == 0) store_release(&window, 2 * it + 1);
         double up[CLS];
         int iu[CLS];
-        float lowf[CLS];
 #pragma unroll
         for (int c = 0; c < CLS; ++c) {
             double v[W];
-            int slot[W];
-            float lo[W];
+            int sl[W];
 #pragma unroll
-            for (int w = 0; w < W; ++w) { const First e = e1[c][w]; v[w] = e.f; slot[w] = e.slot; lo[w] = e.low; }
+            for (int w = 0; w < W; ++w) { const First e = e1[c][w]; v[w] = e.f; sl[w] = e.slot; }
 #pragma unroll
             for (int d = 1; d < W; d <<= 1)
 #pragma unroll
-                for (int w = 0; w + d < W; w += 2 * d) {
-                    lo[w] = fmaxf(lo[w], lo[w + d]);
-                    if (v[w + d] < v[w] || (v[w + d] == v[w] && slot[w + d] < slot[w])) { v[w] = v[w + d]; slot[w] = slot[w + d]; }
-                }
-            up[c] = v[0]; iu[c] = (unsigned) slot[0] < (unsigned) ws ? slot[0] : 0; lowf[c] = lo[0];
+                for (int w = 0; w + d < W; w += 2 * d)
+                    if (v[w + d] < v[w]) { v[w] = v[w + d]; sl[w] = sl[w + d]; }
+            up[c] = v[0]; iu[c] = min(sl[0], ws - 1);           // (an empty list)
         }
-        float kI[CLS][S];
-        int at_i[CLS];
+        float kI[CLS][S], kd_i[CLS];
 #pragma unroll
-        for (int c = 0; c < CLS; ++c) { at_i[c] = AHEAD ? load_acquire(where + iu[c]) : (int) NOT_THERE; read_row(iu[c], at_i[c], kI[c]); }
-        // second-best lanes of the first argmin: rows to copy ahead
-#pragma unroll
-        for (int c = 0; c < CLS; ++c)
-            if (AHEAD && first_h[c] == warp_min_f32(first_h[c])) cand[(CLS + 1 + c) * W + warp] = first_slot[c];
-        // mirrors of the state after the last step (its readers have passed the barrier above)
-#pragma unroll
-        for (int s = 0; s < S; ++s) f_sm[tid + s * T] = f[s];
-        if (tid == 0) { a_sm[step_i] = step_ai; a_sm[step_j] = step_aj; }
-
-        // ---- stopping rule ---------------------------------------------------------------------------------
-        bool open = it > 0 && it <= max_iter;
-        {
-            double gap = 0;
-#pragma unroll
-            for (int c = 0; c < CLS; ++c) {
-                // the smallest double with this high word
-                const int h = __float_as_int(lowf[c]);
-                const double g = __hiloint2double(h, h < 0 ? -1 : 0) - up[c];
-                gap = c == 0 ? g : fmax(gap, g);
-            }
-            open = open && gap >= local_eps;
+        for (int c = 0; c < CLS; ++c) {
+            kd_i[c] = ky_sm[iu[c]].x;
+            read_row(iu[c], kI[c]);
         }
-        if (!open) {
-            // the exact gap: at the first iteration, near the end, and at the end
 #pragma unroll
-            for (int c = 0; c < CLS; ++c) {
-                double m = -INFINITY;
+        for (int s = 0; s < S; s += V) {
+            if constexpr (V == 4) {
+                *(double2 *) (f_sm + t0 + nth(s)) = make_double2(f[s], f[s + 1]);
+                *(double2 *) (f_sm + t0 + nth(s + 2)) = make_double2(f[s + 2], f[s + 3]);
+            } else f_sm[t0 + nth(s)] = f[s];
+        }
+        if (tid == 64) { a_sm[step_i] = step_vi; a_sm[step_j] = step_vj; }
+        if (AHEAD) {
+            best[0][tid] = make_float2(first_h[0], __int_as_float(first_slot[0]));
+            if (tid == 96) *(volatile int *) &window[0] = it + 1;
+        }
+        // the largest f over I_low: high words, clamped to -FAR_POS outside
+        float low_h[S], low_most[2] = {-FAR_POS, -FAR_POS};
 #pragma unroll
-                for (int s = 0; s < S; ++s)
-                    if (pen_low[s] > 0 && (!NU || pos[s] == (c == 0))) m = fmax(m, f[s]);
-                const double wm = key_to_double(~warp_min_u64(~ordered_key(m)));
-                if (lane == 0) exact_low[c][warp] = wm;
-            }
-            solver_barrier<T>();
-            double local_diff = 0;
+        for (int s = 0; s < S; ++s) low_h[s] = fminf(high_as_float(f[s]), pen_low[s]);
 #pragma unroll
-            for (int c = 0; c < CLS; ++c) {
-                double m = exact_low[c][0];
-                for (int w = 1; w < W; ++w) m = fmax(m, exact_low[c][w]);
-                const double d = m - (up[c] > NO_MEMBER ? INFINITY : up[c]);
-                local_diff = c == 0 ? d : fmax(local_diff, d);
-            }
-            if (it == 0) {
-                local_eps = NU ? fmax(eps, 0.1 * local_diff) : fmax(eps, (double) 0.1f * local_diff);
-                if (tid == 0) diff[0] = local_diff;
-            }
-            if (it > max_iter || local_diff < local_eps) break;
+        for (int c = 0; c < CLS; ++c) {
+            float m[S];
+#pragma unroll
+            for (int s = 0; s < S; ++s) m[s] = !NU || pos[s] == (c == 0) ? low_h[s] : -FAR_POS;
+            low_most[c] = warp_max_f32(max_of(m));
         }
 
         // ---- second-order choice of j ------------------------------------------------------------------------
-        float q[S], q2[S], q0[S];
-        int qs[S];
-        float kd_i[CLS];
+        // b in FP32, truncated, straight from the double's bits (zero below 2^-126 and outside I_low; the gap bounds it above).
+        // A curvature that is no positive float gives a value beyond what is accepted below.
+        float q[S], k_most;
+        {
+            float m[S];
 #pragma unroll
-        for (int c = 0; c < CLS; ++c) kd_i[c] = kd_sm[iu[c]];
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-            const bool second = NU && !pos[s];
-            const float k = second ? kI[CLS - 1][s] : kI[0][s];
-            const double b = with_high(low_h[s], f[s]) - (second ? up[CLS - 1] : up[0]);    // far below zero outside I_low
-            // b in FP32, truncated, straight from the double's bits; [2^-50, 2^50) keeps its square in range
-            const int bh = __double2hiint(b);
-            const float b32 = __int_as_float(__funnelshift_l((unsigned) __double2loint(b), (unsigned) (bh - 0x38000000), 3));
-            const bool b_ok = (unsigned) (bh - 0x3cd00000) < 0x06400000u;
-            const float a32 = fmaf(-2.0f, k, (second ? kd_i[CLS - 1] : kd_i[0]) + kd[s]);
-            const bool a_ok = a32 > 1e-30f && a32 < 1e30f;
-            float r;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a32));
-            q[s] = b_ok && a_ok ? b32 * b32 * r : (b > 0 ? INFINITY : 0.0f);
-            q0[s] = q[s];
-            q2[s] = 0.0f;
-            qs[s] = tid + s * T;
+            for (int s = 0; s < S; ++s) {
+                const bool second = NU && !pos[s];
+                const float k = second ? kI[CLS - 1][s] : kI[0][s];
+                const double b = with_high(low_h[s], f[s]) - (second ? up[CLS - 1] : up[0]);
+                const float b32 = __int_as_float(__funnelshift_l((unsigned) __double2loint(b), (unsigned) max(__double2hiint(b), 0), 3));
+                const float a32 = fmaf(-2.0f, k, (second ? kd_i[CLS - 1] : kd_i[0]) + kd[s]);
+                float r;
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(a32, 0x1p-126f)));
+                q[s] = mul_ftz(mul_ftz(b32, r), b32);
+                m[s] = k;
+            }
+            k_most = max_abs3(max_abs_of(m), kd_most, kd_most);
+            q[0] = k_most < 1e30f ? q[0] : INFINITY;
         }
+        float q2[S];
+        int qs[S];
+        const float best_w = warp_max_f32(max_of(q));
+#pragma unroll
+        for (int s = 0; s < S; ++s) { q2[s] = 0.0f; qs[s] = t0 + nth(s); }
 #pragma unroll
         for (int d = 1; d < S; d <<= 1)
 #pragma unroll
             for (int s = 0; s + d < S; s += 2 * d) {
-                q2[s] = fmaxf(fminf(q[s], q[s + d]), fmaxf(q2[s], q2[s + d]));
-                if (q[s + d] > q[s]) { q[s] = q[s + d]; qs[s] = qs[s + d]; }
+                q2[s] = d == 1 ? fminf(q[s], q[s + d]) : max3(fminf(q[s], q[s + d]), q2[s], q2[s + d]);
+                qs[s] = q[s + d] > q[s] ? qs[s + d] : qs[s];
+                q[s] = fmaxf(q[s], q[s + d]);
             }
         {
-            const float best = warp_max_f32(q[0]);
-            const unsigned at_best = __ballot_sync(0xffffffffu, q[0] == best);
-            const float mine = q[0] == best ? q2[0] : q[0];
-            const float next = warp_max_f32(mine);
-            if (AHEAD && mine == next && q[0] != best) cand[(2 * CLS + 1) * W + warp] = qs[0];
-            if (lane == (int) __ffs(at_best) - 1) {
-                Second e;
-                e.best = best; e.next = (at_best & (at_best - 1)) ? best : next; e.slot = qs[0]; e.pad = 0;
-                e2[warp] = e;
-                if (AHEAD) cand[CLS * W + warp] = qs[0];
-            }
+            const float thr = best_w * (1.0f - 8e-6f);
+            const unsigned near = __ballot_sync(0xffffffffu, q[0] >= thr), nears = __ballot_sync(0xffffffffu, q2[0] >= thr);
+            if (q[0] == best_w)
+                e2[warp] = Second{best_w, (near & (near - 1)) | nears ? qs[0] | TIED : qs[0], {low_most[0], low_most[1]}};
         }
         solver_barrier<T>();
-        if (AHEAD && tid == 0) store_release(&window, 2 * it + 2);
         int j;
+        float most[W], next[W], low[CLS];
+        double dI[S];
         {
-            float best[W], next[W];
-            int slot[W];
+            int sl[W];
+            float lw[2][W];
 #pragma unroll
-            for (int w = 0; w < W; ++w) { const Second e = e2[w]; best[w] = e.best; next[w] = e.next; slot[w] = e.slot; }
+            for (int w = 0; w < W; ++w) {
+                const Second e = e2[w];
+                most[w] = e.best; sl[w] = e.slot; lw[0][w] = e.low[0]; lw[1][w] = e.low[1];
+                next[w] = 0;
+            }
+#pragma unroll
+            for (int s = 0; s < S; ++s) dI[s] = NU ? 0.0 : widened(kI[0][s]);
 #pragma unroll
             for (int d = 1; d < W; d <<= 1)
 #pragma unroll
                 for (int w = 0; w + d < W; w += 2 * d) {
-                    next[w] = fmaxf(fminf(best[w], best[w + d]), fmaxf(next[w], next[w + d]));
-                    if (best[w + d] > best[w]) { best[w] = best[w + d]; slot[w] = slot[w + d]; }
+                    next[w] = d == 1 ? fminf(most[w], most[w + d]) : max3(fminf(most[w], most[w + d]), next[w], next[w + d]);
+                    sl[w] = most[w + d] > most[w] ? sl[w + d] : sl[w];
+                    most[w] = fmaxf(most[w], most[w + d]);
                 }
-            j = slot[0];
-            if (!(best[0] > 0.0f && best[0] < INFINITY && next[0] < best[0] * (1.0f - 8e-6f))) {
-                // too close to call in FP32, or out of its range: the same values in FP64, ties to the lower slot
-                const float thr = best[0] < INFINITY ? best[0] * (1.0f - 8e-6f) : 0.0f;
-                double most[CLS];
-                int sl[CLS];
+            j = min(sl[0] & SLOT_MASK, ws - 1);
+            if (sl[0] & TIED) next[0] = most[0];
 #pragma unroll
-                for (int c = 0; c < CLS; ++c) { most[c] = -INFINITY; sl[c] = NO_SLOT; }
+            for (int c = 0; c < CLS; ++c) low[c] = max_of(lw[c]);
+        }
+        // what the step needs of i and j; read before j is certain
+        float kJ[S], kij;
+        float2 kyj;
+        double fj, aj, ai;
+        int yi;
+        auto read_step = [&] {
+            kyj = ky_sm[j];
+            fj = f_sm[j];
+            aj = a_sm[j];
+            const int i = NU && __float_as_int(kyj.y) < 0 ? iu[CLS - 1] : iu[0];
+            kij = __ldg(kww + i * ws + j);          // row i has just been read
+            read_row(j, kJ);
+            ai = a_sm[i];
+            yi = __float_as_int(ky_sm[i].y);
+        };
+        read_step();
+        if (AHEAD) {
+            best[1][tid] = make_float2(q[0], __int_as_float(qs[0]));
+            if (tid == 96) *(volatile int *) &window[1] = it + 1;
+        }
+        double gap = 0;
 #pragma unroll
-                for (int s = 0; s < S; ++s) {
-                    const bool second = NU && !pos[s];
-                    const double b = -(second ? up[CLS - 1] : up[0]) + f[s];
-                    const float k = second ? kI[CLS - 1][s] : kI[0][s], kdi = second ? kd_i[CLS - 1] : kd_i[0];
-                    const double a = NU ? (double) (kdi + kd[s] - 2 * k) : (double) (kdi + kd[s]) - 2.0 * (double) k;
-                    const double e = b * b * reciprocal(a);
-                    const bool asked = q0[s] > 0.0f && q0[s] >= thr;
-#pragma unroll
-                    for (int c = 0; c < CLS; ++c)
-                        if (asked && second == (c > 0) && e > most[c]) { most[c] = e; sl[c] = tid + s * T; }
-                }
-                unsigned long long key[CLS];
-#pragma unroll
-                for (int c = 0; c < CLS; ++c) key[c] = ordered_key(-most[c]);
+        for (int c = 0; c < CLS; ++c) {
+            // the smallest double with this high word
+            const int h = __float_as_int(low[c]);
+            const double g = __hiloint2double(h, h < 0 ? -1 : 0) - up[c];
+            gap = c == 0 ? g : fmax(gap, g);
+        }
+        // ---- the unusual: first and last iteration, a gap that may be closed, values too close to call in FP32 or out of its
+        // range (1e-20 .. 3e7, gap below 2^50)
+        const bool ranged = (most[0] > 1e-20f) & (most[0] < 3e7f) & (__double2hiint(gap) < (127 + 50) << 20);
+        const float tied = most[0] * (1.0f - 8e-6f);
+        const bool called = ranged & (next[0] < tied);
+        const bool open = ((unsigned) (it - 1) < (unsigned) max_iter) & (gap >= local_eps);
+        if (!(called & open)) {
+            if (!open) {
+                // the exact gap
 #pragma unroll
                 for (int c = 0; c < CLS; ++c) {
+                    double m = -INFINITY;
+#pragma unroll
+                    for (int s = 0; s < S; ++s)
+                        if (pen_low[s] > 0 && (!NU || pos[s] == (c == 0))) m = fmax(m, f[s]);
+                    const double wm = key_to_double(~warp_min_u64(~ordered_key(m)));
+                    if (lane == 0) exact_low[c][warp] = wm;
+                }
+                solver_barrier<T>();
+                double local_diff = 0;
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) {
+                    double m = exact_low[c][0];
+                    for (int w = 1; w < W; ++w) m = fmax(m, exact_low[c][w]);
+                    const double d = m - (up[c] > NO_MEMBER ? INFINITY : up[c]);
+                    local_diff = c == 0 ? d : fmax(local_diff, d);
+                }
+                if (it == 0) {
+                    const double first = local_diff * BACK;
+                    local_eps = (NU ? fmax(eps, 0.1 * first) : fmax(eps, (double) 0.1f * first)) * DOWN;
+                    if (tid == 0) diff[0] = first;
+                }
+                if (it > max_iter || local_diff < local_eps) break;
+            }
+            if (!called) {
+                // the same values in FP64, ties to the lower slot; of a thread with one value that is close enough, only that
+                double e_most[CLS];
+                int sl[CLS];
+                unsigned long long key[CLS];
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) { e_most[c] = -INFINITY; sl[c] = NO_SLOT; }
+                auto weigh = [&](int slot, double fs, float kds, float k, bool second) {
+                    const double b = (-(second ? up[CLS - 1] : up[0]) + fs) * BACK;
+                    const float kdi = second ? kd_i[CLS - 1] : kd_i[0];
+                    const double a = NU ? (double) (kdi + kds - 2 * k) : (double) (kdi + kds) - 2.0 * (double) k;
+                    const double e = b * b * reciprocal(a);
+#pragma unroll
+                    for (int c = 0; c < CLS; ++c)
+                        if (b > 0 && second == (c > 0) && e > e_most[c]) { e_most[c] = e; sl[c] = slot; }
+                };
+                if (!ranged || q2[0] >= tied) {
+#pragma unroll
+                    for (int s = 0; s < S; ++s) {
+                        const bool second = NU && !pos[s];
+                        if (pen_low[s] > 0) weigh(t0 + nth(s), f[s], kd[s], second ? kI[CLS - 1][s] : kI[0][s], second);
+                    }
+                } else if (q[0] >= tied) {
+                    const float2 ky = ky_sm[qs[0]];
+                    const bool second = NU && __float_as_int(ky.y) < 0;
+                    weigh(qs[0], f_sm[qs[0]], ky.x, __ldg(kww + (second ? iu[CLS - 1] : iu[0]) * ws + qs[0]), second);
+                }
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) {
+                    key[c] = ordered_key(-e_most[c]);
                     warp_argmin_u64(key[c], sl[c]);
                     if (lane == 0) { exact_key[c][warp] = key[c]; exact_slot[c][warp] = sl[c]; }
                 }
@@ -453,51 +537,78 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                 // the positive-class pair wins only if its value is strictly smaller (smo_kernel.cu:220-233)
                 if (NU && !(key_to_double(key[0]) < key_to_double(key[CLS - 1]))) j = sl[CLS - 1];
                 if (j == NO_SLOT) j = 0;
+                read_step();
             }
         }
-        // ---- step, repeated by every thread in the shadow of row j -------------------------------------------
-        float kJ[S];
-        read_row(j, AHEAD ? load_acquire(where + j) : (int) NOT_THERE, kJ);
-        const int yj = y_sm[j];
+        // ---- step, repeated by every thread ------------------------------------------------------------------
+        const int yj = __float_as_int(kyj.y);
         const bool second = NU && yj < 0;
         const int i = second ? iu[CLS - 1] : iu[0];
-        const int yi = y_sm[i];
-        const double u = second ? up[CLS - 1] : up[0];
-        const double ai = a_sm[i], aj = a_sm[j], fj = f_sm[j];
-        const int at = second ? at_i[CLS - 1] : at_i[0];
-        const float kij = at >= 0 ? ring[at * ws + j] : __ldg(kww + i * ws + j);      // row i has just been read: from L1
-        const double room_i = yi > 0 ? Cp - ai : ai;
-        const double curv = NU ? (double) (kd_sm[i] + kd_sm[j] - 2 * kij)
-                               : (double) (kd_sm[i] + kd_sm[j]) - 2.0 * (double) kij;
-        const double room_j = fmin(yj > 0 ? aj : Cn - aj, (-u + fj) / curv);
-        const double l = fmin(room_i, room_j);
-        step_i = i; step_j = j;
-        step_ai = ai + l * yi; step_aj = aj - l * yj;
-        const float up_i = in_I_up(step_ai, yi, Cp, Cn) ? -FAR_POS : FAR_POS, up_j = in_I_up(step_aj, yj, Cp, Cn) ? -FAR_POS : FAR_POS;
-        const float lo_i = in_I_low(step_ai, yi, Cp, Cn) ? FAR_POS : -FAR_POS, lo_j = in_I_low(step_aj, yj, Cp, Cn) ? FAR_POS : -FAR_POS;
+        const double ci = yi > 0 ? Cp : Cn, cj = yj > 0 ? Cp : Cn;
+        const double b = (-(second ? up[CLS - 1] : up[0]) + fj) * BACK;
+        const float kdi = second ? kd_i[CLS - 1] : kd_i[0];
+        const double a = NU ? (double) (kdi + kyj.x - 2 * kij) : (double) (kdi + kyj.x) - 2.0 * (double) kij;
+        // b / a: the quotient by a reciprocal of half the digits, corrected once (within an ulp of the division)
+        double r;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+        r = fma(r, fma(-a, r, 1.0), r);
+        double l = b * r;
+        l = fma(fma(-a, l, b), r, l);
+        const double room_i = yi > 0 ? Cp - ai : ai, room_j = yj > 0 ? aj : Cn - aj;
+        const double room = room_j < room_i ? room_j : room_i;
+        l = room < l ? room : l;
+        double d[S];
+        float m[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-            const int t = tid + s * T;
-            if (t == i) { pen_up[s] = up_i; pen_low[s] = lo_i; }
-            if (t == j) { pen_up[s] = up_j; pen_low[s] = lo_j; }
+            d[s] = NU ? widened(kJ[s] - (second ? kI[CLS - 1][s] : kI[0][s])) : widened(kJ[s]) - dI[s];
+            m[s] = NU ? kJ[s] - (second ? kI[CLS - 1][s] : kI[0][s]) : kJ[s];
+        }
+        const float k_all = NU ? max_abs_of(m) : max_abs3(max_abs_of(m), k_most, k_most);
+        const bool usual = ((unsigned) (__double2hiint(a) - 0x03000000) < 0x79000000u) & mild & (k_all < INFINITY);
+        double g[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) g[s] = fma(-l, d[s], f[s]);
+        if (!usual) {           // curvature not positive or at the ends of the range, infinite kernel values, a huge C
+            l = fmin(room, b / a);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const float k = second ? kI[CLS - 1][s] : kI[0][s];
+                g[s] = fma(-l, NU ? (double) (kJ[s] - k) : (double) kJ[s] - (double) k, f[s] * BACK) * DOWN;
+            }
         }
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            const float k = second ? kI[CLS - 1][s] : kI[0][s];
-            const double d = NU ? (double) (kJ[s] - k) : (double) kJ[s] - (double) k;
-            f[s] = fma(-l, d, f[s]);
+        for (int s = 0; s < S; ++s) f[s] = g[s];
+        const double step_ai = ai + (yi > 0 ? l : -l), step_aj = aj - (yj > 0 ? l : -l);
+        const bool i_up0 = step_ai < ci, i_dn0 = step_ai > 0, j_up0 = step_aj < cj, j_dn0 = step_aj > 0;
+        const bool were_free = (ai > 0) & (ai < ci) & (aj > 0) & (aj < cj);
+        if (!(were_free & i_up0 & i_dn0 & j_up0 & j_dn0)) {
+            const float up_i = in_I_up(step_ai, yi, Cp, Cn) ? -FAR_POS : FAR_POS, up_j = in_I_up(step_aj, yj, Cp, Cn) ? -FAR_POS : FAR_POS;
+            const float lo_i = in_I_low(step_ai, yi, Cp, Cn) ? FAR_POS : -FAR_POS, lo_j = in_I_low(step_aj, yj, Cp, Cn) ? FAR_POS : -FAR_POS;
+            const int mine_i = i - t0, mine_j = j - t0;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+#pragma unroll
+                for (int c = 0; c < CLS; ++c) {
+                    if (mine_i == nth(s) && (!NU || second == (c > 0))) pen_up[c][s] = up_i;
+                    if (mine_j == nth(s) && (!NU || second == (c > 0))) pen_up[c][s] = up_j;
+                }
+                if (mine_i == nth(s)) pen_low[s] = lo_i;
+                if (mine_j == nth(s)) pen_low[s] = lo_j;
+            }
         }
+        step_i = i; step_j = j; step_vi = step_ai; step_vj = step_aj;
         ++it;
     }
-    if (tid == 0) store_release(&done, 1);
+    if (AHEAD && tid == 0) *(volatile int *) &done = 1;
     solver_barrier<T>();            // (the last step's alphas are in a_sm)
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-        const int t = tid + s * T;
+        const int t = t0 + nth(s);
         if (t < ws) {
             const double a = a_sm[t], a_old = alpha_ws[t];
             alpha_ws[t] = a;
-            alpha_diff[t] = -(a - a_old) * y_sm[t];
+            alpha_diff[t] = -(a - a_old) * __float_as_int(ky_sm[t].y);
             if (alpha_global && ids[t] >= 0) alpha_global[ids[t]] = a;
         }
     }

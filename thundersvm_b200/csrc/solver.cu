@@ -586,18 +586,18 @@ static tsvm_status launch_local_smo(int solver_kind, int ws, const float *kww, c
                                     double eps, int max_iter, double *diff, const int *ids, double *alpha_global,
                                     cudaStream_t st, const int *stop = nullptr, PhaseTimes *times = nullptr) {
     const bool nu = solver_kind != TSVM_SOLVER_C;
-    // four warps at every size, one to eight slots per thread: measured at 1,024 / 512 / 256 slots 1.00 / 0.84 / 0.73 us
-    // per iteration against 1.12 / 0.99 / 0.86 with eight warps and 1.73 with sixteen (512 slots)
+    // four warps at every size, one to eight slots per thread: with eight warps every one repeats the reductions and the
+    // step next to another on its scheduler (1,024 slots, rows in L1: 0.74 against 0.93 us per iteration, 1.65 with sixteen).
+    // Blocks below 256 slots are small enough for L1 to hold what is used again.
     constexpr int T = 128;
-    const int use_ring = !nu && ws >= 256 && (ws & 3) == 0 && ((uintptr_t) kww & 15) == 0;
-    const size_t ring_bytes = use_ring ? (size_t) smo::RING * ws * sizeof(float) : 0;
+    const int ahead = ws >= 256;
 #define SMO_LAUNCH(NU, S)                                                                                          \
     do {                                                                                                           \
         TSVM_ONCE_PER_DEVICE(TSVM_CUDA(cudaFuncSetAttribute(local_smo_kernel<NU, S, T>,                            \
-                                                            cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                                                            (int) (smo::RING * S * T * sizeof(float)))));          \
-        TSVM_LAUNCH((local_smo_kernel<NU, S, T>), 1, T + 32, ring_bytes, st, ws, kww, diag_ws, y_ws, f_ws,         \
-                    alpha_ws, alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop, use_ring, times);  \
+                                                            cudaFuncAttributePreferredSharedMemoryCarveout,        \
+                                                            cudaSharedmemCarveoutMaxL1)));                         \
+        TSVM_LAUNCH((local_smo_kernel<NU, S, T>), 1, T + (NU ? 0 : 64), 0, st, ws, kww, diag_ws, y_ws, f_ws,        \
+                    alpha_ws, alpha_diff, Cp, Cn, eps, max_iter, diff, ids, alpha_global, stop, ahead, times);     \
     } while (0)
 #define SMO_CASE(S) do { if (nu) SMO_LAUNCH(true, S); else SMO_LAUNCH(false, S); } while (0)
     if (ws <= T) SMO_CASE(1); else if (ws <= 2 * T) SMO_CASE(2); else if (ws <= 4 * T) SMO_CASE(4); else SMO_CASE(8);
