@@ -27,9 +27,9 @@
 //     row is wanted about once, so a cache alone finds a tenth of them; the best six of an argmin's list hold the next
 //     iteration's winner nine times in ten.
 // Measured per iteration at 1,024 slots inside a solve, before (conversions, an exact division, 32 rows copied to shared
-// memory by one more warp and looked up there) and now: 10,000 x 20 1.05 -> 0.86 us, 12,003 x 784 1.00 -> 0.85, text
-// 1.00 -> 0.85, one-hot records, where many values tie, 1.10 -> 0.93, 200,000 x 2,000 next to the kernel-row launch
-// 1.44 -> 1.28, nu (without the reading warps) 1.38 -> 1.17. With every row found in L1 an iteration takes 0.67 us: 486
+// memory by one more warp and looked up there) and now: 10,000 x 20 1.05 -> 0.82 us, 12,003 x 784 1.00 -> 0.81, text
+// 1.00 -> 0.80, one-hot records, where many values tie, 1.10 -> 0.88, 200,000 x 2,000 next to the kernel-row launch
+// 1.44 -> 1.20, nu (without the reading warps) 1.38 -> 1.15. With every row found in L1 an iteration takes 0.67 us: 486
 // instructions per warp (604 before) at 2.7 cycles, dependent ones mostly. Two floats per instruction in the second-order
 // values (16 instructions fewer) changed nothing; masks instead of compares where a slot joins or leaves a list cost 5 %.
 #pragma once
@@ -66,10 +66,10 @@ __device__ __forceinline__ double reciprocal(double a) {
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
-// Reading ahead: how many slots of an argmin are looked after (the bounds), and for how many iterations a row that was read
-// is taken to be there. The cache does not keep rows for long: KEEP 24 / 8 / 4 / 2 / 1 / 0 make 0.92 / 0.91 / 0.88 / 0.87 / 0.86 /
-// 0.90 us (12,003 x 784); with 3 to 6 or 6 to 12 slots 0.89.
-constexpr int KEEP = 1, LO = 4, HI = 8;
+// Reading ahead: how many slots of an argmin are looked after, how many rows are read at a time at most, and for how many
+// iterations a row that was read is taken to be there (the cache does not keep it for long): KEEP 0 / 1 / 3 make 0.821 / 0.806 /
+// 0.825 us (12,003 x 784), 4 or 8 slots 0.815 or 0.819.
+constexpr int KEEP = 1, WANTED = 6, MOST = 8;
 template <int T>
 __device__ __forceinline__ void solver_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory"); }
 
@@ -125,25 +125,27 @@ __device__ __forceinline__ double widened(float k) {
     return __hiloint2double((u >> 3) & 0x8fffffff, u << 29);
 }
 
-// The reading warps, one for each argmin. Every thread of the solver leaves the best of its slots (best: value, slot); those
-// that are close to the best of all are read, unless that was just done. What is close is adjusted until LO to HI slots are.
-// A row is read by asynchronous copies of one word of every 32-byte sector to a place nobody looks at (sink): they put the
-// sectors into the L1 cache, and unlike loads nothing waits for them (loads: 10 % slower; prefetch.global.L1: no effect).
-// Nothing but time depends on what these warps see: `best`, `window` and `last` are read while they are written. Words copied
-// are words of kww, x is a slot at any time, and a row past ws is not read.
-template <int T, bool LARGEST>
+// The reading warps, one for each argmin. Every thread of the solver leaves the best of its slots (best: value, slot); the rows
+// of those that are closest to the best of all are read, unless that was just done.
+// A row is read by one word of each of its 32-byte sectors, by loads whose results are looked at when the next rows are read.
+// (Asynchronous copies, which need no registers, take 160 cycles a row to issue against 20: a pass over six rows then lasts
+// 1.7 iterations, and 60 - 75 % of the rows are found instead of 83 - 96 %; prefetch.global.L1 has no effect.)
+// Nothing but time depends on what these warps see: `best`, `window` and `last` are read while they are written. A slot in
+// `best` is one at any time, and no row past ws is read.
+template <int S, int T, bool LARGEST>
 __device__ void read_rows_ahead(const float *__restrict__ kww, int ws, const float2 *best, const int *window, const int *done,
-                                int *last, float *sink) {
-    constexpr int E = T / 32;
+                                int *last, int *stage) {
+    constexpr int E = T / 32, G = S * T > 256 ? S * T / 256 : 1;
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
     int seen = 0;
     float width = LARGEST ? 0.5f : 1e-3f;
+    int used = 0, word[MOST][G] = {};
     // (bounded: a solver that runs longer than this goes on without)
     for (int polls = 0; polls < (1 << 26); ++polls) {
         const int now = *(volatile const int *) window;
         if (__any_sync(full, *(volatile const int *) done)) break;
-        if (__all_sync(full, now == seen)) { continue; }
+        if (__all_sync(full, now == seen)) continue;
         seen = now;
         float v[E];
         int x[E], before[E];
@@ -160,29 +162,42 @@ __device__ void read_rows_ahead(const float *__restrict__ kww, int ws, const flo
 #pragma unroll
         for (int e = 1; e < E; ++e) m = LARGEST ? fmaxf(m, v[e]) : fminf(m, v[e]);
         m = LARGEST ? warp_max_f32(m) : warp_min_f32(m);
-        const float limit = LARGEST ? m * width : m + width;
-        int count = 0;
-        unsigned needs[E];
+        // the narrowest of five widths around the last one that has WANTED slots in it
+        const float unit = (LARGEST ? m : 1.0f) * width * 0.25f;
+        int level = 4;
+#pragma unroll
+        for (int k = 3; k >= 0; --k) {
+            int count = 0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) count += fabsf(v[e] - m) <= unit * (float) (1 << k);
+            if (__reduce_add_sync(full, count) >= WANTED) level = k;
+        }
+        const float limit = unit * (float) (1 << level);
+        int n = 0;
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            const bool near = LARGEST ? v[e] > limit : v[e] < limit;
-            count += __popc(__ballot_sync(full, near));
-            const bool need = near && now - before[e] > KEEP && x[e] < ws;
-            needs[e] = __ballot_sync(full, need);
-            if (need) last[x[e]] = now;
+            const bool need = fabsf(v[e] - m) <= limit && now - before[e] > KEEP && x[e] < ws;
+            const unsigned needs = __ballot_sync(full, need);
+            const int k = n + __popc(needs & ((1u << lane) - 1));
+            if (need && k < MOST) { stage[k] = x[e]; last[x[e]] = now; }
+            n += __popc(needs);
         }
+        __syncwarp();
+        // one word of every sector of 32 bytes; the words of the pass before have arrived (they are used for that alone)
 #pragma unroll
-        for (int e = 0; e < E; ++e)
-            for (unsigned n = needs[e]; n; n &= n - 1) {
-                const float *row = kww + __shfl_sync(full, x[e], __ffs(n) - 1) * ws;
-                // one word of a sector of 32 bytes; where it is put does not matter
-                for (int t = lane * 8; t < ws; t += 32 * 8)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(sink + lane)), "l"(row + t) : "memory");
+        for (int k = 0; k < MOST; ++k) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) used |= word[k][g];
+            if (k < n) {
+                const int *row = (const int *) kww + stage[k] * ws + lane * 8;
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    if (g * 256 + lane * 8 < ws) word[k][g] = __ldg(row + g * 256);
             }
-        if (LARGEST) width = count < LO ? width * 0.8f : count > HI ? 1.0f - (1.0f - width) * 0.8f : width;
-        else width = count < LO ? width * 1.25f : count > HI ? width * 0.8f : width;
+        }
+        width = LARGEST ? fminf(limit / m, 1.0f) : limit;
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (used == -1) last[0] = 0;            // (the loads have a use)
 }
 }  // namespace smo
 
@@ -213,10 +228,10 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
     __shared__ int exact_slot[CLS][W];
     __shared__ double exact_low[CLS][W];
     // what the reading warps look at: every thread's best value of the two argmins with its slot; when it changed
-    constexpr bool AHEAD = !NU;                             // (nu reads two rows i and guesses j badly: 1.216 us without, 1.228 with)
+    constexpr bool AHEAD = !NU;                             // (nu: 1.14 us without, 1.24 with three such warps)
     __shared__ float2 best[2][T];
     __shared__ int last[S * T], window[2], done;
-    __shared__ float sink[2][32];
+    __shared__ int stage[2][MOST];
     static_assert(S * T <= SLOT_MASK, "a slot fits its field");
     const double Cp = NU ? (double) (float) Cp_in : Cp_in;
     const double Cn = NU ? Cp : Cn_in;
@@ -227,8 +242,8 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         if (tid == T) { window[0] = window[1] = 0; done = 0; }
         __syncthreads();
         if (ahead) {
-            if (warp == W) read_rows_ahead<T, false>(kww, ws, best[0], &window[0], &done, last, sink[0]);
-            else read_rows_ahead<T, true>(kww, ws, best[1], &window[1], &done, last, sink[1]);
+            if (warp == W) read_rows_ahead<S, T, false>(kww, ws, best[0], &window[0], &done, last, stage[0]);
+            else read_rows_ahead<S, T, true>(kww, ws, best[1], &window[1], &done, last, stage[1]);
         }
         return;
     }
