@@ -123,6 +123,44 @@ def test_fused_prediction_many_classes(capi):
     _fused_case(capi, 20, [17 + 3 * c for c in range(20)], d=64, m=4500)
 
 
+@pytest.mark.parametrize("m", [192, 193, 256, 257, 700])
+@pytest.mark.parametrize("kernel", ["rbf", "linear"])
+@pytest.mark.parametrize("cnt", [[1, 0], [16, 15], [130, 127], [20, 12, 31], [256, 1, 0, 255], [9, 16, 17, 0, 1, 64, 33, 2, 5, 100],
+                                 [40] * 11])
+def test_fused_prediction_rows_on_the_lanes(capi, m, kernel, cnt):
+    """From 193 rows on the test rows lie on the lanes and the support vectors on the columns: row tiles and their remainders,
+    blocks of columns and their remainders, classes that begin and end at a group of 16 columns, inside one, several in one,
+    none in a class; the last number of classes of that form and the first beyond it. Against sums in FP64: kernel values
+    and products are FP32, the error of a sum of n products stays below (n + 20) 2^-24 times the sum of their magnitudes."""
+    rng = np.random.default_rng(m + len(cnt))
+    cnt = np.asarray(cnt, dtype=np.int32)
+    nc, n_sv, d, gamma = len(cnt), int(cnt.sum()), 65, 0.02
+    SV, T = (rng.standard_normal((k, d)).astype(np.float32) for k in (n_sv, m))
+    coef, rho = rng.standard_normal((nc - 1, n_sv)), rng.standard_normal(nc * (nc - 1) // 2)
+    dots = T.astype(np.float64) @ SV.T.astype(np.float64)
+    K = dots
+    if kernel == "rbf":
+        K = np.exp(-gamma * ((T.astype(np.float64) ** 2).sum(1)[:, None] + (SV.astype(np.float64) ** 2).sum(1)[None] - 2 * dots))
+    own = np.repeat(np.arange(nc), cnt)
+    want, size = [], []
+    for i in range(nc):
+        for j in range(i + 1, nc):
+            c = np.where(own == i, coef[j - 1], 0.0) + np.where(own == j, coef[i], 0.0)
+            want.append(K @ c - rho[len(want)])
+            size.append(np.abs(K) @ np.abs(c))
+    want, size = np.stack(want, 1), np.stack(size, 1)
+    # values: up to 2 gamma |x| |y| log2 e 2^-24 relative in the exponent (RBF), the dot's own 2^-24 sum of magnitudes (linear)
+    term = np.abs(T).astype(np.float64) @ np.abs(SV).T.astype(np.float64)
+    loose = (K * gamma * 4 * (term + (T ** 2).sum(1)[:, None] + (SV ** 2).sum(1)[None]) if kernel == "rbf" else 4 * term) * np.abs(coef).sum(0)
+    km = capi.KernelMatrix(dense=_t(SV), kernel=kernel, gamma=gamma)
+    dec = capi.predict_dec(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, dense=_t(T))
+    bound = 2.0 ** -24 * ((n_sv + 20) * size + loose.sum(1)[:, None]) + 1e-12
+    assert np.all(np.abs(dec.cpu().numpy() - want) <= bound), np.max(np.abs(dec.cpu().numpy() - want) / bound)
+    lab = capi.predict_labels(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, dense=_t(T))
+    assert np.array_equal(lab.cpu().numpy(), capi.vote(dec, nc).cpu().numpy())
+    km.close()
+
+
 @pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 64, 65])
 @pytest.mark.parametrize("storage", ["dense", "dense_sv_csr_rows", "csr"])
 @pytest.mark.parametrize("nc,n_sv,d,kernel", [(2, 1, 1, "rbf"), (2, 700, 35, "rbf"), (3, 129, 4, "linear"),

@@ -293,6 +293,8 @@ tsvm_status km_stage_instances_csr(tsvm_km *km, const float *tval, const int *rp
                                    const SumPreset &preset, cudaStream_t st);
 tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev, const int *sv_class_dev,
                                      int n_classes, double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st);
+tsvm_status launch_dense_tc2_predict_lanes(tsvm_km *km, int m, const float *cols, long long cols_ld, int nc_pad, int n_classes,
+                                           double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st);
 tsvm_status km_stage_rows_features(tsvm_km *km, const float *T_dev, int ldt, const float *sd_T_dev, int m,
                                    cudaStream_t st);
 }  // namespace tsvm

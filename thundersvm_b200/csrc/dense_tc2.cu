@@ -47,6 +47,16 @@ constexpr int REGS_LAUNCH = 168, REGS_CONTROL = 56, REGS_EPILOGUE = 224;
 static_assert(128 * REGS_CONTROL + 32 * EPI_WARPS * REGS_EPILOGUE <= THREADS * REGS_LAUNCH,
               "the epilogue warps would wait for registers that nobody releases");
 static_assert(THREADS * REGS_LAUNCH <= 65536, "register file of an SM");
+// Prediction with the test rows on the lanes. Where one promotion unit holds all features (ONE_UNIT) the sums are read from tensor
+// memory as the epilogue needs them, and sixteen warps with 64 columns each fit the registers: four per scheduler, which hide
+// each other's latencies. Otherwise eight warps keep 128 sums as above.
+template <bool ONE_UNIT>
+struct Lanes {
+    static constexpr int WARPS = ONE_UNIT ? 16 : EPI_WARPS, N_THREADS = 32 * (EPI_WARP0 + WARPS), COLS = BN / (WARPS / 4);
+    static constexpr int LAUNCH = ONE_UNIT ? 96 : REGS_LAUNCH, CONTROL = REGS_CONTROL, EPILOGUE = ONE_UNIT ? 104 : REGS_EPILOGUE;
+    static_assert(128 * CONTROL + 32 * WARPS * EPILOGUE <= N_THREADS * LAUNCH, "the epilogue warps would wait for registers that nobody releases");
+    static_assert(N_THREADS * LAUNCH <= 65536, "register file of an SM");
+};
 // epilogue staging (see the epilogue): EPI_CHUNK sums of each epilogue thread (eight chunks per thread), and per
 // warp the self dots and 1/scale of its requested rows
 constexpr int EPI_CHUNK = COLS_PER_THREAD / 8;
@@ -60,6 +70,11 @@ constexpr uint32_t SLOT_BYTES = EPI_WARPS * COLS_PER_THREAD * 4;
 constexpr uint32_t SMEM_BASE = STAGES * STAGE_BYTES + 1024 + 256 + EPI_STAGE_BYTES + EPI_CONST_BYTES;
 constexpr uint32_t SMEM_BYTES = SMEM_BASE + SLOT_BYTES;
 constexpr uint32_t SMEM_BYTES_PREDICT = SMEM_BASE + PRED_BYTES;
+// prediction, rows on the lanes: what the epilogue needs of a block's support vectors, COL_ROWS numbers each, twice
+constexpr int COL_ROWS = 3 + PRED_NC_SMEM;
+constexpr uint32_t COL_BYTES = COL_ROWS * BN * 4;
+constexpr uint32_t SMEM_BYTES_LANES = STAGES * STAGE_BYTES + 1024 + 256 + 2 * COL_BYTES;
+static_assert(SMEM_BYTES_LANES <= 227 * 1024, "prediction form, rows on the lanes, does not fit the shared memory of an SM");
 static_assert(SMEM_BYTES <= 227 * 1024, "kernel-row form does not fit the shared memory of an SM");
 static_assert(SMEM_BYTES_PREDICT <= 227 * 1024, "prediction form does not fit the shared memory of an SM");
 constexpr uint32_t TMEM_COLS = 512;
@@ -135,7 +150,16 @@ struct PredictArgs {
     double *dec;               // the sums are added to dec[r * row_stride + pair * pair_stride]
     long long row_stride, pair_stride;
     int n_classes;
+    // rows on the lanes: the support vectors' numbers (predict_columns_kernel), rows of cols_ld floats; nc_pad rows of coefficients
+    const float *cols;
+    long long cols_ld;
+    int nc_pad;
 };
+// form of the kernel: rows, prediction with the instances on the lanes, prediction with the test rows on the lanes and
+// FORM % 16 coefficients, for any number of features or for those of one promotion unit
+enum { FORM_ROWS = 0, FORM_PREDICT = 1, FORM_LANES = 16, FORM_LANES_ONE_UNIT = 32 };
+template <int FORM>
+using LanesOf = tc2::Lanes<(FORM >= FORM_LANES_ONE_UNIT)>;
 
 // Optional indirections of the kernel-row form, both read on the device so that a caller can decide them
 // without a host round trip: the number of requested rows actually wanted (at most the m the launch was
@@ -164,6 +188,24 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 }
 __device__ __forceinline__ int pair_index(int n_classes, int i, int j) {      // i < j, pairs ordered (0,1),(0,2),...
     return i * (2 * n_classes - i - 1) / 2 + (j - i - 1);
+}
+
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long exp2_2(unsigned long long v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(lo));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(hi));
+    return pack2(lo, hi);
 }
 
 // Columns (requested rows) of row block nb that the MMAs cover: all 256, or the rows left rounded up to 32
@@ -231,8 +273,116 @@ __device__ __forceinline__ void reduce_chunk(const float *block, const float *co
     }
 }
 
-template <int EPI, bool F16, bool PREDICT>
-__global__ void __launch_bounds__(tc2::THREADS, 1)
+// Prediction with the test rows on the lanes (FORM_LANES + NC): a thread holds the products of one test row with up to 128
+// support vectors, so that the sum over them needs no other thread. The support vectors' numbers come from shared memory, the
+// same word for all lanes: `col`, rows of BN floats - factor and summand of the exponent (RBF: 2 gamma log2 e / scale, -gamma
+// log2 e |x|^2; linear: 1 / scale), class, NC coefficients (zero beyond the real ones). 16 columns at a time, two per
+// instruction; sums of 32 products in FP32, of more in FP64. At the end of a class the sums go to its pairs.
+template <int I>
+struct Index {
+    static constexpr int value = I;
+    __device__ constexpr operator int() const { return I; }
+};
+// take(g, x): the products of columns 16 g .. 16 g + 15.
+template <int EPI, int NC, bool ONE_UNIT, class Take>
+__device__ __forceinline__ void sum_columns(Take take, const float *col, int n_cols, float unscale, float row_term, long long r,
+                                            bool wanted, const PredictArgs &pa) {
+    using namespace tc2;
+    const unsigned long long u2 = pack2(unscale, unscale), a2 = pack2(row_term, row_term);
+    double total[NC];
+    float part[NC];
+#pragma unroll
+    for (int t = 0; t < NC; ++t) { total[t] = 0; part[t] = 0; }
+    int cls = -1;
+    const int nc = pa.n_classes - 1;
+    auto add_up = [&] {
+#pragma unroll
+        for (int t = 0; t < NC; ++t) { total[t] += (double) part[t]; part[t] = 0; }
+    };
+    auto hand_over = [&] {
+        if (NC > 1) add_up();
+#pragma unroll
+        for (int t = 0; t < NC; ++t) {
+            const int pair = NC == 1 ? 0 : t < cls ? pair_index(pa.n_classes, t, cls) : pair_index(pa.n_classes, cls, t + 1);
+            red_add_if(wanted && t < nc, pa.dec + r * pa.row_stride + pair * pa.pair_stride, total[t]);
+            total[t] = 0;
+        }
+    };
+    auto group = [&](auto g) {
+        float x[16];
+        take(g, x);
+        const float *at = col + g * 16;
+        unsigned long long k[8];
+#pragma unroll
+        for (int p = 0; p < 8; p += 2) {
+            const ulonglong2 f = *reinterpret_cast<const ulonglong2 *>(at + 2 * p);
+            k[p] = mul2(pack2(x[2 * p], x[2 * p + 1]), u2);
+            k[p + 1] = mul2(pack2(x[2 * p + 2], x[2 * p + 3]), u2);
+            if constexpr (EPI == EPI_RBF) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(at + BN + 2 * p);
+                k[p] = exp2_2(add2(fma2(k[p], f.x, b.x), a2));
+                k[p + 1] = exp2_2(add2(fma2(k[p + 1], f.y, b.y), a2));
+            } else {
+                k[p] = mul2(k[p], f.x);
+                k[p + 1] = mul2(k[p + 1], f.y);
+            }
+        }
+        auto accumulate = [&](const unsigned long long (&v)[8]) {
+#pragma unroll
+            for (int t = 0; t < NC; ++t) {
+                unsigned long long w0 = 0ull, w1 = 0ull;
+#pragma unroll
+                for (int p = 0; p < 8; p += 2) {
+                    const ulonglong2 c = *reinterpret_cast<const ulonglong2 *>(at + (3 + t) * BN + 2 * p);
+                    w0 = fma2(c.x, v[p], w0);
+                    w1 = fma2(c.y, v[p + 1], w1);
+                }
+                part[t] += sum2(add2(w0, w1));
+            }
+        };
+        if constexpr (NC == 1) accumulate(k);            // (both classes add to the one pair)
+        else {
+            const int *own = reinterpret_cast<const int *>(at + 2 * BN);
+            const int first = own[0], last = own[15];
+            if (first == last) {
+                if (cls != first && cls >= 0) hand_over();
+                cls = first;
+                accumulate(k);
+            } else
+#pragma unroll 1
+                for (int c = first; c <= last; ++c) {
+                    if (cls != c && cls >= 0) hand_over();
+                    cls = c;
+                    unsigned long long v[8];
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        float lo, hi;
+                        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(k[p]));
+                        v[p] = pack2(own[2 * p] == c ? lo : 0.0f, own[2 * p + 1] == c ? hi : 0.0f);
+                    }
+                    accumulate(v);
+                }
+        }
+    };
+    // (n_cols is a multiple of 32)
+    if constexpr (ONE_UNIT) {
+#pragma unroll 1
+        for (int g = 0; g * 16 < n_cols; g += 2) { group(g); group(g + 1); add_up(); }
+    } else {                                    // register indices must be constants
+        auto two_groups = [&](auto index) {
+            constexpr int g = 2 * decltype(index)::value;
+            if (g * 16 >= n_cols) return;
+            group(Index<g>());
+            group(Index<g + 1>());
+            add_up();
+        };
+        two_groups(Index<0>()); two_groups(Index<1>()); two_groups(Index<2>()); two_groups(Index<3>());
+    }
+    hand_over();
+}
+
+template <int EPI, bool F16, int FORM>
+__global__ void __launch_bounds__(FORM >= FORM_LANES ? LanesOf<FORM>::N_THREADS : tc2::THREADS, 1)
 dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_constant__ CUtensorMap map_xlo,
                       const __grid_constant__ CUtensorMap map_whi, const __grid_constant__ CUtensorMap map_wlo,
                       int n, int m_launch, int row_len, const float *__restrict__ sd, const float *__restrict__ sd_rows,
@@ -240,6 +390,10 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                       KernelFn fn, float *__restrict__ out, long long ld_out, int *__restrict__ status,
                       const PredictArgs pa, const RowsExtra ex) {
     using namespace tc2;
+    constexpr bool PREDICT = FORM == FORM_PREDICT, LANES = FORM >= FORM_LANES;
+    constexpr bool ONE_UNIT = FORM >= FORM_LANES_ONE_UNIT;
+    constexpr int NC = LANES ? FORM % 16 : 1;
+    constexpr int WARPS = LANES ? LanesOf<FORM>::WARPS : EPI_WARPS, COLS = LANES ? LanesOf<FORM>::COLS : COLS_PER_THREAD;      // of the epilogue
     // the same value in every thread of the grid: the launch's m, or the smaller count found on the device
     const int m = ex.m_dev ? min(m_launch, max(*ex.m_dev, 0)) : m_launch;
     constexpr int BK = F16 ? 64 : 32;          // elements per k slab
@@ -254,6 +408,11 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     const uint32_t tfull_bar = empty_bar + 8 * MAX_STAGES, tempty_bar = tfull_bar + 16;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * MAX_STAGES + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    // rows on the lanes: two buffers of columns' numbers, filled by warp 2 and read by the epilogue warps
+    const uint32_t cfull_bar = smem_u32(bars) + 128, cempty_bar = cfull_bar + 16;
+    static_assert(!ONE_UNIT || F16, "one_unit counts halves");
+    static_assert((2 * MAX_STAGES + 4) * 8 + 8 <= 128 && 128 + 32 <= 256, "barriers and flags lie side by side");
+    const float *colbuf = reinterpret_cast<const float *>(ring_ptr + STAGES * STAGE_BYTES + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
@@ -264,11 +423,17 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     const int pair_tiles = (n + 2 * BM - 1) / (2 * BM), n_blocks = (m + width - 1) / width, k_blocks = (row_len + BK - 1) / BK;
     // Work items are (pair tile, row block) with the row block fastest, so neighbouring clusters stream the
     // same instance slabs at the same time and the second reader finds them in L2.
+    // With the test rows on the lanes the tile is the faster one: the support vectors are the larger matrix, and their slabs are
+    // read once per launch (200,000 x 2,000 against 100,000 rows: 222 ms the other way round).
     const int n_items = pair_tiles * n_blocks;
+    auto tile_of = [&](int item) { return LANES ? item % pair_tiles : item / n_blocks; };
+    auto block_of = [&](int item) { return LANES ? item / pair_tiles : item % n_blocks; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar + 8 * a, 1); mbar_init(tempty_bar + 8 * a, 2 * EPI_WARPS); }
+        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar + 8 * a, 1); mbar_init(tempty_bar + 8 * a, 2 * WARPS); }
+        if (LANES)
+            for (int a = 0; a < 2; ++a) { mbar_init(cfull_bar + 8 * a, 1); mbar_init(cempty_bar + 8 * a, WARPS); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -285,14 +450,14 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp < EPI_WARP0) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_CONTROL));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(LANES ? LanesOf<FORM>::CONTROL : REGS_CONTROL));
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         if (lane == 0) {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (int item = cluster_id; item < n_items && ok; item += n_clusters) {
-                    const int pt = item / n_blocks, nb = item - pt * n_blocks;
+                    const int pt = tile_of(item), nb = block_of(item);
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         if (!mbar_wait(empty_bar + 8 * stage, phase ^ 1, abort_flag, 1)) { ok = false; break; }
                         const uint32_t base = ring + stage * stage_bytes;
@@ -314,7 +479,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             for (int item = cluster_id; item < n_items && ok; item += n_clusters) {
-                    const uint32_t idesc_n = (uint32_t) (block_columns(m, item % n_blocks, width) >> 3) << 17;
+                    const uint32_t idesc_n = (uint32_t) (block_columns(m, block_of(item), width) >> 3) << 17;
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         const bool unit_start = kb % PROMO == 0, unit_end = kb % PROMO == PROMO - 1 || kb == k_blocks - 1;
                         if (unit_start && !mbar_wait(tempty_bar + 8 * acc, acc_phase ^ 1, abort_flag, 2)) { ok = false; break; }
@@ -347,9 +512,25 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                     }
             }
         }
+    } else if (LANES && warp == 2) {
+        // ---------------- the columns' numbers, one block per item (both CTAs, each for itself) ----------------
+        if (lane == 0) {
+            const uint32_t rows = 3 + NC;
+            uint32_t buf = 0, phase = 0;
+            for (int item = cluster_id; item < n_items; item += n_clusters) {
+                if (!mbar_wait(cempty_bar + 8 * buf, phase ^ 1, abort_flag, 6)) break;
+                mbar_expect_tx(cfull_bar + 8 * buf, rows * BN * 4);
+                const float *src = pa.cols + (long long) block_of(item) * width;
+                for (uint32_t k = 0; k < rows; ++k)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(smem_u32(colbuf) + buf * COL_BYTES + k * (BN * 4)), "l"(src + k * pa.cols_ld), "r"((uint32_t) BN * 4),
+                                   "r"(cfull_bar + 8 * buf) : "memory");
+                if (++buf == 2) { buf = 0; phase ^= 1; }
+            }
+        }
     }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_EPILOGUE));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(LANES ? LanesOf<FORM>::EPILOGUE : REGS_EPILOGUE));
         // ---------------- slab promotion + epilogue (both CTAs, own 128 instances) ----------------
         const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2;
         float *priv = reinterpret_cast<float *>(ring_ptr + STAGES * STAGE_BYTES + 256) + (warp - EPI_WARP0) * 32 + lane;
@@ -361,10 +542,10 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
         float *coef_priv = reinterpret_cast<float *>(ring_ptr + STAGES * STAGE_BYTES + 256 + EPI_STAGE_BYTES + EPI_CONST_BYTES) +
                            (warp - EPI_WARP0) * 32 + lane;
         const int nc = PREDICT ? pa.n_classes - 1 : 0;
-        uint32_t acc = 0, acc_phase = 0;
+        uint32_t acc = 0, acc_phase = 0, cbuf = 0, cphase = 0;
         bool ok = true;
         for (int item = cluster_id; item < n_items && ok; item += n_clusters) {
-            const int pt = item / n_blocks, nb = item - pt * n_blocks;
+            const int pt = tile_of(item), nb = block_of(item);
             const int j = pt * 2 * BM + (int) rank * BM + quarter * 32 + lane;
             const float sdj = j < n ? sd[j] : 0.0f;
             const float uxj = (F16 && j < n) ? x_unscale[j] : 1.0f;
@@ -385,32 +566,60 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                 // Self dot and 1/scale of this warp's 128 requested rows go to shared memory by asynchronous
                 // copies while the k loop runs: with nearly all of the SM's memory configured as shared, the
                 // L1 left over does not keep them across the epilogue's stores.
-                const int i0 = nb * width + half * COLS_PER_THREAD;
+                const int i0 = nb * width + half * COLS;
 #pragma unroll
                 for (int c = lane; c < COLS_PER_THREAD; c += 32) {
-                    if (i0 + c < m) {
+                    if (!LANES && i0 + c < m) {
                         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(rowc + c)), "l"(sd_rows + i0 + c) : "memory");
                         if constexpr (F16)
                             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(rowc + COLS_PER_THREAD + c)), "l"(w_unscale + i0 + c) : "memory");
-                        if constexpr (!PREDICT)
+                        if constexpr (FORM == FORM_ROWS)
                             if (ex.row_slot)
                                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(slotc + c)), "l"(ex.row_slot + i0 + c) : "memory");
                     }
                 }
-                float sum[COLS_PER_THREAD];
+                float sum[ONE_UNIT ? 1 : COLS];
+                if constexpr (!LANES) {
 #pragma unroll
-                for (int c = 0; c < COLS_PER_THREAD; ++c) sum[c] = 0.0f;
+                    for (int c = 0; c < COLS; ++c) sum[c] = 0.0f;
+                }
+                const float row_term = EPI == EPI_RBF ? -fn.gamma * 1.4426950408889634f * sdj : 0.0f;       // (rows on the lanes)
                 for (int unit = 0; unit < (k_blocks + PROMO - 1) / PROMO; ++unit) {
                     if (!mbar_wait(tfull_bar + 8 * acc, acc_phase, abort_flag, 4)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t taddr = tmem_base + ((uint32_t) (quarter * 32) << 16) + acc * BN + half * COLS_PER_THREAD;
+                    const uint32_t taddr = tmem_base + ((uint32_t) (quarter * 32) << 16) + acc * BN + half * COLS;
+                    if constexpr (ONE_UNIT) {
+                        if (!mbar_wait(cfull_bar + 8 * cbuf, cphase, abort_flag, 5)) { ok = false; break; }
+                        const float *col = colbuf + cbuf * (COL_BYTES / 4) + half * COLS;
+                        const int cols = min(n_cols - half * COLS, COLS);
+                        if (cols > 0)
+                            sum_columns<EPI, NC, true>([&](int g, float (&x)[16]) {
+                                uint32_t v[16];
+                                tmem_ld16(taddr + 16 * g, v);
 #pragma unroll
-                    for (int c0 = 0; c0 < COLS_PER_THREAD; c0 += 32) {
-                        if (half * COLS_PER_THREAD + c0 >= n_cols) break;      // columns the narrow MMAs did not write
+                                for (int c = 0; c < 16; ++c) x[c] = __uint_as_float(v[c]);
+                            }, col, cols, uxj, row_term, j, j < n, pa);
+                    } else {
+#pragma unroll
+                    for (int c0 = 0; c0 < COLS; c0 += 32) {
+                        if (half * COLS + c0 >= n_cols) break;      // columns the narrow MMAs did not write
                         uint32_t v[32];
                         tmem_ld32(taddr + c0, v);
+                        if (LANES && unit == 0) {
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) sum[c0 + c] += __uint_as_float(v[c]);
+                            for (int c = 0; c < 32; ++c) sum[c0 + c] = __uint_as_float(v[c]);
+                        } else if constexpr (LANES) {
+#pragma unroll
+                            for (int c = 0; c < 32; c += 2) {
+                                const unsigned long long t = add2(pack2(sum[c0 + c], sum[c0 + c + 1]),
+                                                                  pack2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])));
+                                asm("mov.b64 {%0, %1}, %2;" : "=f"(sum[c0 + c]), "=f"(sum[c0 + c + 1]) : "l"(t));
+                            }
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 32; ++c) sum[c0 + c] += __uint_as_float(v[c]);
+                        }
+                    }
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -418,6 +627,22 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                     if (++acc == 2) { acc = 0; acc_phase ^= 1; }
                 }
                 if (!ok) break;
+                if constexpr (LANES) {
+                    if constexpr (!ONE_UNIT) {
+                        if (!mbar_wait(cfull_bar + 8 * cbuf, cphase, abort_flag, 5)) { ok = false; break; }
+                        const float *col = colbuf + cbuf * (COL_BYTES / 4) + half * COLS;
+                        const int cols = min(n_cols - half * COLS, COLS);
+                        if (cols > 0)
+                            sum_columns<EPI, NC, false>([&](auto g, float (&x)[16]) {
+#pragma unroll
+                                for (int c = 0; c < 16; ++c) x[c] = sum[16 * decltype(g)::value + c];
+                            }, col, cols, uxj, row_term, j, j < n, pa);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(cempty_bar + 8 * cbuf);
+                    if (++cbuf == 2) { cbuf = 0; cphase ^= 1; }
+                    continue;
+                } else {
                 // The sums live in registers, so a loop over them has to be fully unrolled; with the kernel
                 // function in its body that is 128 copies of it, and the instruction fetch of such an
                 // epilogue cost several times its arithmetic. Instead the sums pass 32 at a time through a
@@ -621,6 +846,7 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                     }
                 }
                 __syncwarp();          // the next item's copies overwrite rowc
+                }
             }
         }
     }
@@ -652,11 +878,13 @@ static int block_width(int pair_tiles, int m, int avail) {
     return width;
 }
 
-template <int EPI, bool F16, bool PREDICT>
+template <int EPI, bool F16, int FORM>
 static tsvm_status launch_pair_kernel(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
                                       long long ld_out, const PredictArgs &pa, const RowsExtra &ex_in, cudaStream_t st) {
-    auto kernel = dense_rows_tc2_kernel<EPI, F16, PREDICT>;
-    constexpr uint32_t smem_bytes = PREDICT ? tc2::SMEM_BYTES_PREDICT : tc2::SMEM_BYTES;
+    auto kernel = dense_rows_tc2_kernel<EPI, F16, FORM>;
+    constexpr uint32_t smem_bytes = FORM >= FORM_LANES ? tc2::SMEM_BYTES_LANES
+                                  : FORM == FORM_PREDICT ? tc2::SMEM_BYTES_PREDICT : tc2::SMEM_BYTES;
+    constexpr int threads = FORM >= FORM_LANES ? LanesOf<FORM>::N_THREADS : tc2::THREADS;
     static int clusters_of_device[MAX_DEVICES] = {0};      // per instantiation and per device ordinal
     int dev = 0;
     TSVM_CUDA(cudaGetDevice(&dev));
@@ -669,7 +897,7 @@ static tsvm_status launch_pair_kernel(tsvm_km *km, const InstancePlanes &X, cons
         cudaLaunchAttribute pattr[1];
         pattr[0].id = cudaLaunchAttributeClusterDimension;
         pattr[0].val.clusterDim.x = 2; pattr[0].val.clusterDim.y = 1; pattr[0].val.clusterDim.z = 1;
-        probe.gridDim = dim3(sms & ~1); probe.blockDim = dim3(tc2::THREADS); probe.dynamicSmemBytes = smem_bytes;
+        probe.gridDim = dim3(sms & ~1); probe.blockDim = dim3(threads); probe.dynamicSmemBytes = smem_bytes;
         probe.attrs = pattr; probe.numAttrs = 1;
         int nc = 0;
         if (cudaOccupancyMaxActiveClusters(&nc, kernel, &probe) != cudaSuccess || nc < 1) {
@@ -694,34 +922,34 @@ static tsvm_status launch_pair_kernel(tsvm_km *km, const InstancePlanes &X, cons
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2 * clusters); cfg.blockDim = dim3(tc2::THREADS); cfg.dynamicSmemBytes = smem_bytes;
+    cfg.gridDim = dim3(2 * clusters); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
     TSVM_CUDA(cudaLaunchKernelEx(&cfg, kernel, mxh, mxl, mwh, mwl, X.n, m, len, X.sd, W.sd, X.unscale, W.unscale,
-                                 km->fn, out, ld_out, PREDICT ? km->status_host : km->status_dev, pa, ex));
+                                 km->fn, out, ld_out, FORM != FORM_ROWS ? km->status_host : km->status_dev, pa, ex));
     count_launch();
     return TSVM_OK;
 }
 
-template <bool PREDICT>
+template <int FORM>
 static tsvm_status launch_pair_any(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
                                    long long ld_out, const PredictArgs &pa, const RowsExtra &ex, cudaStream_t st) {
     TSVM_REQUIRE(km->plane_kind == 1 || km->plane_kind == 2, "tensor engine: operand planes are not built");
     const int epi = epilogue_kind(km->fn);
     if (km->plane_kind == 2) {
-        if (epi == EPI_RBF) return launch_pair_kernel<EPI_RBF, true, PREDICT>(km, X, W, m, out, ld_out, pa, ex, st);
-        if (epi == EPI_LINEAR) return launch_pair_kernel<EPI_LINEAR, true, PREDICT>(km, X, W, m, out, ld_out, pa, ex, st);
-        return launch_pair_kernel<EPI_GENERIC, true, PREDICT>(km, X, W, m, out, ld_out, pa, ex, st);
+        if (epi == EPI_RBF) return launch_pair_kernel<EPI_RBF, true, FORM>(km, X, W, m, out, ld_out, pa, ex, st);
+        if (epi == EPI_LINEAR) return launch_pair_kernel<EPI_LINEAR, true, FORM>(km, X, W, m, out, ld_out, pa, ex, st);
+        return launch_pair_kernel<EPI_GENERIC, true, FORM>(km, X, W, m, out, ld_out, pa, ex, st);
     }
-    if (epi == EPI_RBF) return launch_pair_kernel<EPI_RBF, false, PREDICT>(km, X, W, m, out, ld_out, pa, ex, st);
-    if (epi == EPI_LINEAR) return launch_pair_kernel<EPI_LINEAR, false, PREDICT>(km, X, W, m, out, ld_out, pa, ex, st);
-    return launch_pair_kernel<EPI_GENERIC, false, PREDICT>(km, X, W, m, out, ld_out, pa, ex, st);
+    if (epi == EPI_RBF) return launch_pair_kernel<EPI_RBF, false, FORM>(km, X, W, m, out, ld_out, pa, ex, st);
+    if (epi == EPI_LINEAR) return launch_pair_kernel<EPI_LINEAR, false, FORM>(km, X, W, m, out, ld_out, pa, ex, st);
+    return launch_pair_kernel<EPI_GENERIC, false, FORM>(km, X, W, m, out, ld_out, pa, ex, st);
 }
 
 // Kernel values of the m staged requested rows against a set of instances given by its operand planes
 // (kind 1 = TF32 words, 2 = row-scaled FP16, the handle's plane kind), self dots and 1/scale.
 tsvm_status launch_dense_tc2_planes(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
                                     long long ld_out, cudaStream_t st) {
-    return launch_pair_any<false>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, 0, km->rows_end_dev}, st);
+    return launch_pair_any<FORM_ROWS>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, 0, km->rows_end_dev}, st);
 }
 
 // Prediction form: the m staged rows are test rows, the kernel matrix holds the support vectors; adds
@@ -730,8 +958,35 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
                                      int n_classes, double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st) {
     const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
     const RowPlanes staged{km->Whi, km->Wlo, km->sd_rows, km->w_unscale};
-    const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes};
-    return launch_pair_any<true>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, 0, nullptr}, st);
+    const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes, nullptr, 0, 0};
+    return launch_pair_any<FORM_PREDICT>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, 0, nullptr}, st);
+}
+
+// The same with the test rows on the tensor memory's lanes and the support vectors on its columns. What bounds FORM_PREDICT is
+// its epilogue: the sum over the support vectors crosses the lanes of a warp (19 instructions per warp and kernel value with
+// two classes, 58 with ten); here it stays in a thread, the support vectors' numbers are the same words for all lanes (5 and
+// 18). Kernel times per launch of 4,096 rows and in one launch of all: 16,281 x 12,001 x 123 63 -> 115 us for all (254 in four
+// launches), ten classes, 10,000 x 8,003 x 784 157 -> 323 us for all (380 in three); whole calls 320 -> 162 and 535 -> 397 us,
+// 100,000 x 200,000 x 2,000 180 -> 178 ms (it waits for the tensor pipe). What bounds it now: the products, 2.4 of 2.8 us per
+// tile with 123 features; with ten classes the epilogue (products alone: 240 of 323 us).
+// Sums are no less exact than before: FP32 over four products at a time, FP64 from 32 on; against sums in FP64 the relative
+// errors of ten data sets are 0.96 - 1.03 times the former, 1.00 on average.
+// The price is a tile of 256 test rows, whole or not. The columns' numbers travel by bulk copies into two buffers (warp 2), so
+// that the epilogue's warps need no barrier among themselves.
+tsvm_status launch_dense_tc2_predict_lanes(tsvm_km *km, int m, const float *cols, long long cols_ld, int nc_pad, int n_classes,
+                                           double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st) {
+    const InstancePlanes rows{km->Whi, km->Wlo, km->sd_rows, km->w_unscale, m};
+    const RowPlanes svs{km->Xhi, km->Xlo, km->self_dot, km->x_unscale};
+    const PredictArgs pa{nullptr, nullptr, dec_dev, row_stride, pair_stride, n_classes, cols, cols_ld, nc_pad};
+    const RowsExtra ex{nullptr, nullptr, 0, nullptr};
+    const bool rbf = epilogue_kind(km->fn) == EPI_RBF;
+    const bool one_unit = km->plane_ld <= 128;              // two k slabs
+#define TSVM_LANES(EPI, NC) \
+    (one_unit ? launch_pair_kernel<EPI, true, FORM_LANES_ONE_UNIT + NC>(km, rows, svs, km->n, nullptr, 0, pa, ex, st) \
+              : launch_pair_kernel<EPI, true, FORM_LANES + NC>(km, rows, svs, km->n, nullptr, 0, pa, ex, st))
+    if (rbf) return nc_pad == 1 ? TSVM_LANES(EPI_RBF, 1) : nc_pad == 3 ? TSVM_LANES(EPI_RBF, 3) : TSVM_LANES(EPI_RBF, 9);
+    return nc_pad == 1 ? TSVM_LANES(EPI_LINEAR, 1) : nc_pad == 3 ? TSVM_LANES(EPI_LINEAR, 3) : TSVM_LANES(EPI_LINEAR, 9);
+#undef TSVM_LANES
 }
 
 // Requested rows = the m rows staged in the handle's scratch.

@@ -8,8 +8,9 @@
 //   * a few test rows (predict_few.cuh): one launch, FP32 dot products on CUDA cores;
 //   * dense support vectors of more than 32 features, and CSR ones that the handle also keeps as dense rows
 //     (choose_csr_storage) if the test rows qualify too: the test x SV contraction multiplies its kernel values by
-//     the coefficients in its epilogue and adds them to the decision values (dense_tc2.cu, prediction form), so the
-//     kernel block is never written;
+//     the coefficients in its epilogue and adds them to the decision values (dense_tc2.cu, prediction forms), so the
+//     kernel block is never written; more than LANES_ROWS rows, RBF and linear kernels and up to ten classes: with the
+//     test rows on the accumulator's lanes, otherwise with the support vectors on them;
 //   * the rest compute the block in slabs of test rows and reduce it with sum_kernel_values_kernel.
 #include "common.cuh"
 #include "predict_few.cuh"
@@ -112,7 +113,27 @@ __global__ void class_tables_kernel(const __grid_constant__ ClassCounts cc, int 
     }
 }
 
-// the same from start offsets in memory (more classes than the argument holds)
+// What the contraction with the test rows on the lanes needs of every support vector, one row of `ld` floats each (zero beyond
+// the last support vector): factor and summand of the kernel function's argument, class, nc_pad coefficients.
+constexpr int LANES_CLASSES = 10;
+static int lanes_coefficients(int n_classes) { return n_classes == 2 ? 1 : n_classes <= 4 ? 3 : LANES_CLASSES - 1; }
+__global__ void predict_columns_kernel(const __grid_constant__ ClassCounts cc, int n_classes, int n_sv, long long ld, int nc_pad,
+                                       const double *__restrict__ coef, const float *__restrict__ sd,
+                                       const float *__restrict__ unscale, int rbf, float gamma, float *__restrict__ out) {
+    const long long s = (long long) blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= ld) return;
+    const bool there = s < n_sv;
+    int cls = 0;
+    for (int c = 0, end = 0; c + 1 < n_classes; ++c) { end += cc.count[c]; cls += s >= end; }
+    constexpr float LOG2E = 1.4426950408889634f;
+    const float u = there ? unscale[s] : 0.0f;
+    out[s] = rbf ? 2.0f * gamma * LOG2E * u : u;
+    out[ld + s] = rbf && there ? -gamma * LOG2E * sd[s] : 0.0f;
+    out[2 * ld + s] = __int_as_float(cls);
+    for (int t = 0; t < nc_pad; ++t) out[(3 + t) * ld + s] = there && t < n_classes - 1 ? (float) coef[(size_t) t * n_sv + s] : 0.0f;
+}
+
+// the classes from start offsets in memory (more classes than the argument holds)
 __global__ void sv_class_kernel(int *__restrict__ cls, int n_sv, const int *__restrict__ sv_start, int n_classes) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_sv) return;
@@ -182,13 +203,21 @@ static tsvm_status launch_vote(const double *dec, int m, int n_classes, int *out
 
 using namespace tsvm;
 
-// Rows of test instances handled per launch of the fused contraction (the handle's staging scratch grows
-// to hold them) and per slab of the unfused path.
-static constexpr int FUSED_ROWS = 4096;
+// Rows of test instances handled per launch of the fused contraction (the handle's staging scratch grows to hold them): as
+// many as leave their operand planes in a quarter of the L2 cache, where every block of support vectors reads them again, and
+// at least 4,096. One launch instead of four for 16,281 rows of 123 features: 201 -> 156 us per call.
+static int fused_rows(const tsvm_km *km) {
+    const size_t fit = ((size_t) 32 << 20) / (2 * km_plane_row_bytes(km));
+    return fit < 4096 ? 4096 : fit > 16384 ? 16384 : (int) (fit & ~(size_t) 255);
+}
+// From this number of test rows on the contraction takes them on the lanes of its accumulators (FORM_LANES in dense_tc2.cu): its
+// epilogue is the shorter one, but it computes whole tiles of 256 rows. 40,000 x 2,000, both forms: 157 against 166 us with
+// 129 rows, 164 / 168 with 192, 176 / 169 with 256, 239 / 230 with 257, 399 / 382 with 800; smaller models differ by less.
+static constexpr int LANES_ROWS = 192;
 
 // Decision values of test rows [r0, r0 + mm) into dec (preset here): [row][pair] with pair_stride 1, else [pair][row].
-static tsvm_status fused_slab(tsvm_km *km_sv, const double *coef_dev, const int *sv_class, const double *rho_dev,
-                              int n_classes, long long r0, int mm, const float *T_dev, int dt, int ldt,
+static tsvm_status fused_slab(tsvm_km *km_sv, const double *coef_dev, const int *sv_class, const float *columns, long long columns_ld,
+                              const double *rho_dev, int n_classes, long long r0, int mm, const float *T_dev, int dt, int ldt,
                               const float *tval_dev, const int *trow_ptr_dev, const int *tcol_dev, double *dec,
                               long long pair_stride, cudaStream_t st) {
     const int nb = n_classes * (n_classes - 1) / 2;
@@ -197,7 +226,11 @@ static tsvm_status fused_slab(tsvm_km *km_sv, const double *coef_dev, const int 
     preset.sums = dec; preset.rho = rho_dev; preset.total = total; preset.pair_stride = pair_stride; preset.n_pairs = nb;
     if (T_dev) TSVM_TRY(km_stage_instances_dense(km_sv, T_dev + (size_t) r0 * ldt, mm, dt, ldt, preset, st));
     else TSVM_TRY(km_stage_instances_csr(km_sv, tval_dev, trow_ptr_dev + r0, tcol_dev, mm, preset, st));
-    return launch_dense_tc2_predict(km_sv, mm, coef_dev, sv_class, n_classes, dec, pair_stride == 1 ? nb : 1, pair_stride, st);
+    const long long row_stride = pair_stride == 1 ? nb : 1;
+    if (columns)
+        return launch_dense_tc2_predict_lanes(km_sv, mm, columns, columns_ld, lanes_coefficients(n_classes), n_classes, dec, row_stride,
+                                              pair_stride, st);
+    return launch_dense_tc2_predict(km_sv, mm, coef_dev, sv_class, n_classes, dec, row_stride, pair_stride, st);
 }
 
 // Few rows: one launch (predict_few.cuh; 62 -> 33 us per call at 8 rows x 3,001 x 100, 104 -> 45 us at 1 x 5,000 x 784 with
@@ -277,9 +310,17 @@ static tsvm_status predict_slabs(tsvm_km *km_sv, const double *coef_dev, const s
     float *K = nullptr;
     int *meta = nullptr, *sv_class = nullptr;
     double *dec_slab = nullptr;
-    tsvm_status s = dev_alloc(&meta, (size_t) 2 * n_classes);
+    // test rows on the lanes: what that form needs of the support vectors, in place of their classes
+    const int type = km_sv->fn.type;
+    const bool rbf = type == TSVM_RBF || type == TSVM_PRECOMPUTED;
+    const bool lanes = fused && m > LANES_ROWS && n_classes <= LANES_CLASSES && km_sv->plane_kind == 2 && (rbf || type == TSVM_LINEAR);
+    float *columns = nullptr;
+    const long long columns_ld = ((long long) n_sv + 255) / 256 * 256 + 256;       // (a block may read 255 past the last one)
+    tsvm_status s = TSVM_OK;
+    if (lanes) s = dev_alloc(&columns, (size_t) columns_ld * (3 + lanes_coefficients(n_classes)));
+    else s = dev_alloc(&meta, (size_t) 2 * n_classes);
     if (s == TSVM_OK && !fused) s = dev_alloc(&K, (size_t) batch * ldk);
-    if (s == TSVM_OK && fused) s = dev_alloc(&sv_class, (size_t) n_sv);
+    if (s == TSVM_OK && fused && !lanes) s = dev_alloc(&sv_class, (size_t) n_sv);
     const bool by_pair = fused && n_classes > 2 && n_classes <= SLAB_CLASSES;
     const long long slab_ld = (batch + 3) & ~3ll;
     if (s == TSVM_OK && (labels_dev || by_pair)) s = dev_alloc(&dec_slab, (size_t) slab_ld * nb);
@@ -293,9 +334,12 @@ static tsvm_status predict_slabs(tsvm_km *km_sv, const double *coef_dev, const s
     }
     km_sv->status_host[0] = 0;
     auto run = [&]() -> tsvm_status {
-        if (by_argument) {
-            ClassCounts cc;
-            for (int c = 0; c < n_classes; ++c) cc.count[c] = count[c];
+        ClassCounts cc;
+        for (int c = 0; c < n_classes && by_argument; ++c) cc.count[c] = count[c];
+        if (lanes) {
+            TSVM_LAUNCH(predict_columns_kernel, ceil_div(columns_ld, 256), 256, 0, st, cc, n_classes, n_sv, columns_ld,
+                        lanes_coefficients(n_classes), coef_dev, km_sv->self_dot, km_sv->x_unscale, rbf, km_sv->fn.gamma, columns);
+        } else if (by_argument) {
             TSVM_LAUNCH(class_tables_kernel, ceil_div(fused && n_sv > n_classes ? n_sv : n_classes, 256), 256, 0, st, cc,
                         n_classes, n_sv, meta, meta + n_classes, sv_class);
         } else if (fused) TSVM_LAUNCH(sv_class_kernel, ceil_div(n_sv, 256), 256, 0, st, sv_class, n_sv, meta, n_classes);
@@ -303,7 +347,7 @@ static tsvm_status predict_slabs(tsvm_km *km_sv, const double *coef_dev, const s
             const int mm = (int) ((m - r0) < batch ? (m - r0) : batch);
             double *dec = labels_dev ? dec_slab : dec_dev + (size_t) r0 * nb;
             if (fused) {
-                TSVM_TRY(fused_slab(km_sv, coef_dev, sv_class, rho_dev, n_classes, r0, mm, T_dev, dt, ldt, tval_dev,
+                TSVM_TRY(fused_slab(km_sv, coef_dev, sv_class, columns, columns_ld, rho_dev, n_classes, r0, mm, T_dev, dt, ldt, tval_dev,
                                     trow_ptr_dev, tcol_dev, by_pair ? dec_slab : dec, by_pair ? slab_ld : 1, st));
                 if (by_pair)
                     TSVM_LAUNCH(finish_slab_kernel, ceil_div(mm, 32), SLAB_THREADS, 0, st, dec_slab, slab_ld, mm, n_classes,
@@ -328,7 +372,7 @@ static tsvm_status predict_slabs(tsvm_km *km_sv, const double *coef_dev, const s
             s = TSVM_ERR_DEVICE;
         }
     } else cudaStreamSynchronize(st);
-    pool_free_many({K, meta, sv_class, dec_slab}, s == TSVM_OK);      // (only this stream has used them)
+    pool_free_many({K, meta, sv_class, dec_slab, columns}, s == TSVM_OK);      // (only this stream has used them)
     return s;
 }
 
@@ -350,7 +394,7 @@ static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const in
     bool fused = false;
     TSVM_TRY(km_pair_engine_takes(km_sv, T_dev ? nullptr : tval_dev, T_dev ? nullptr : trow_ptr_dev, tcol_dev, m, st, &fused));
     const long long ldk = ((long long) n_sv + 3) & ~3ll;
-    long long batch = FUSED_ROWS;
+    long long batch = fused ? fused_rows(km_sv) : 0;
     if (!fused) {
         // the kernel block of a slab must fit the budget (svmmodel.cpp:86-89 caps a batch at 10000 rows)
         size_t budget = max_mem_bytes;
@@ -363,6 +407,8 @@ static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const in
         batch = (long long) (budget / sizeof(float) / (size_t) ldk);
         if (batch > 10000) batch = 10000;
     }
+    // slabs of equal size, in whole tiles
+    if (fused && batch < m) batch = (ceil_div(m, ceil_div(m, batch)) + 255) / 256 * 256;
     if (batch > m) batch = m;
     if (batch < 1) batch = 1;
     // The size of the slab is a guess at what is free. Where the device has less (for the slab or for the staging scratch of
