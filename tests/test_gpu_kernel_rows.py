@@ -323,3 +323,21 @@ def test_batches_of_new_rows(capi, engine, m, dt):
     for batch in (dict(dense=torch.from_numpy(T).cuda()), dict(dense=dev[:, 1:dt + 1]), dict(csr=csr)):
         assert rel_err(km.get_rows_instances(**batch).cpu().numpy(), want) < REL_TOL
     km.close()
+
+
+@pytest.mark.parametrize("n,d,q", [(300, 33, 5), (700, 123, 130), (1500, 256, 300), (400, 200, 256)])
+@pytest.mark.parametrize("values", ["ones", "halves"])
+def test_one_product_per_value_where_the_low_planes_are_zero(capi, n, d, q, values):
+    """Sparse data that one FP16 number per entry holds is multiplied without its low planes: the same bits as the same
+    data given as dense rows, which keep all three products. One and several k slabs and promotion units, narrow blocks."""
+    import torch
+    rng = np.random.default_rng(n + d)
+    X = ((rng.random((n, d)) < 0.15) * (1.0 if values == "ones" else 0.5 * rng.integers(1, 60, (n, d)))).astype(np.float32)
+    X[3] = 0.0
+    nz = X != 0
+    rp = np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32)
+    csr = tuple(torch.from_numpy(a).cuda() for a in (X[nz], rp, np.nonzero(nz)[1].astype(np.int32)))
+    ids = torch.from_numpy(rng.choice(n, q, replace=False).astype(np.int32)).cuda()
+    gamma = 0.05 if values == "ones" else 1e-4
+    rows = [km.get_rows(ids) for km in (capi.KernelMatrix(csr=csr, d=d, gamma=gamma), capi.KernelMatrix(dense=torch.from_numpy(X).cuda(), gamma=gamma))]
+    assert torch.equal(rows[0], rows[1])

@@ -168,6 +168,7 @@ struct RowsExtra {
     const int *m_dev;
     const int *row_slot;
     int width;                      // requested rows per block (set by the launch)
+    int hi_only;                    // the low planes of both operands are zero (set by the launch)
     long long *end;                 // device_ns() when the last block left (never taken back), or nullptr
 };
 
@@ -418,7 +419,12 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
     const uint32_t rank = cluster_ctarank();
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const int width = ex.width;
-    const uint32_t b_bytes = (uint32_t) width * 64, stage_bytes = 2 * A_BYTES + 2 * b_bytes;     // half a block's rows of 128 bytes
+    // One product per value instead of three, and half the bytes, where nothing is left for the low planes: the dense copy of CSR
+    // data is made only of values that one FP16 number holds (choose_csr_storage). The products left out are zeros. 16,281 rows
+    // against 12,001 x 123: 115 -> 91 us.
+    const bool hi_only = F16 && ex.hi_only;
+    const uint32_t planes = hi_only ? 1 : 2;
+    const uint32_t b_bytes = (uint32_t) width * 64, b_at = planes * A_BYTES, stage_bytes = planes * (A_BYTES + b_bytes);     // half a block's rows of 128 bytes
     const uint32_t n_stages = min((uint32_t) MAX_STAGES, STAGES * STAGE_BYTES / stage_bytes);
     const int pair_tiles = (n + 2 * BM - 1) / (2 * BM), n_blocks = (m + width - 1) / width, k_blocks = (row_len + BK - 1) / BK;
     // Work items are (pair tile, row block) with the row block fastest, so neighbouring clusters stream the
@@ -466,9 +472,11 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                         // this CTA's half of the block's requested rows (a narrow last block has narrow halves)
                         const int xrow = pt * 2 * BM + (int) rank * BM, wrow = nb * width + (int) rank * (block_columns(m, nb, width) >> 1);
                         tma_load_2d_pair(base, &map_xhi, leader_full, kb * BK, xrow);
-                        tma_load_2d_pair(base + A_BYTES, &map_xlo, leader_full, kb * BK, xrow);
-                        tma_load_2d_pair(base + 2 * A_BYTES, &map_whi, leader_full, kb * BK, wrow);
-                        tma_load_2d_pair(base + 2 * A_BYTES + b_bytes, &map_wlo, leader_full, kb * BK, wrow);
+                        tma_load_2d_pair(base + b_at, &map_whi, leader_full, kb * BK, wrow);
+                        if (!hi_only) {
+                            tma_load_2d_pair(base + A_BYTES, &map_xlo, leader_full, kb * BK, xrow);
+                            tma_load_2d_pair(base + b_at + b_bytes, &map_wlo, leader_full, kb * BK, wrow);
+                        }
                         if (++stage == n_stages) { stage = 0; phase ^= 1; }
                     }
             }
@@ -487,18 +495,21 @@ dense_rows_tc2_kernel(const __grid_constant__ CUtensorMap map_xhi, const __grid_
                         tc_fence_after();
                         const uint32_t d_tmem = tmem_base + acc * BN;
                         const uint32_t base = ring + stage * stage_bytes;
+                        if (!hi_only) {
 #pragma unroll
-                        for (int k = 0; k < K_STEPS; ++k) {
-                            const uint32_t koff = k * 32;
-                            umma_pair<F16>(d_tmem, smem_desc_sw128(base + A_BYTES + koff),
-                                           smem_desc_sw128(base + 2 * A_BYTES + koff), k != 0 || !unit_start, idesc_n);
-                            umma_pair<F16>(d_tmem, smem_desc_sw128(base + koff),
-                                           smem_desc_sw128(base + 2 * A_BYTES + b_bytes + koff), 1, idesc_n);
+                            for (int k = 0; k < K_STEPS; ++k) {
+                                const uint32_t koff = k * 32;
+                                umma_pair<F16>(d_tmem, smem_desc_sw128(base + A_BYTES + koff),
+                                               smem_desc_sw128(base + b_at + koff), k != 0 || !unit_start, idesc_n);
+                                umma_pair<F16>(d_tmem, smem_desc_sw128(base + koff),
+                                               smem_desc_sw128(base + b_at + b_bytes + koff), 1, idesc_n);
+                            }
                         }
 #pragma unroll
                         for (int k = 0; k < K_STEPS; ++k) {
                             const uint32_t koff = k * 32;
-                            umma_pair<F16>(d_tmem, smem_desc_sw128(base + koff), smem_desc_sw128(base + 2 * A_BYTES + koff), 1, idesc_n);
+                            umma_pair<F16>(d_tmem, smem_desc_sw128(base + koff), smem_desc_sw128(base + b_at + koff),
+                                           !hi_only || k != 0 || !unit_start, idesc_n);
                         }
                         // stage free / slab complete, signalled in both CTAs
                         umma_commit_pair(mapa_u32(empty_bar + 8 * stage, 0));
@@ -913,6 +924,7 @@ static tsvm_status launch_pair_kernel(tsvm_km *km, const InstancePlanes &X, cons
     int avail = max_clusters - km->reserve_clusters;     // SM pairs left free for a concurrent stream
     if (avail < 1) avail = 1;
     RowsExtra ex = ex_in;
+    ex.hi_only = km->from_csr;
     ex.width = km->whole_blocks ? tc2::BN : block_width(ceil_div(X.n, 2 * tc2::BM), m, avail);
     TSVM_TRY(make_map(&mwh, W.hi, m, len, len, ex.width / 2, F16));
     TSVM_TRY(make_map(&mwl, W.lo, m, len, len, ex.width / 2, F16));
@@ -949,7 +961,7 @@ static tsvm_status launch_pair_any(tsvm_km *km, const InstancePlanes &X, const R
 // (kind 1 = TF32 words, 2 = row-scaled FP16, the handle's plane kind), self dots and 1/scale.
 tsvm_status launch_dense_tc2_planes(tsvm_km *km, const InstancePlanes &X, const RowPlanes &W, int m, float *out,
                                     long long ld_out, cudaStream_t st) {
-    return launch_pair_any<FORM_ROWS>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, 0, km->rows_end_dev}, st);
+    return launch_pair_any<FORM_ROWS>(km, X, W, m, out, ld_out, PredictArgs{}, RowsExtra{km->rows_m_dev, km->rows_slot_dev, 0, 0, km->rows_end_dev}, st);
 }
 
 // Prediction form: the m staged rows are test rows, the kernel matrix holds the support vectors; adds
@@ -959,7 +971,7 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
     const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
     const RowPlanes staged{km->Whi, km->Wlo, km->sd_rows, km->w_unscale};
     const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes, nullptr, 0, 0};
-    return launch_pair_any<FORM_PREDICT>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, 0, nullptr}, st);
+    return launch_pair_any<FORM_PREDICT>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, 0, 0, nullptr}, st);
 }
 
 // The same with the test rows on the tensor memory's lanes and the support vectors on its columns. What bounds FORM_PREDICT is
@@ -967,8 +979,8 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
 // two classes, 58 with ten); here it stays in a thread, the support vectors' numbers are the same words for all lanes (5 and
 // 18). Kernel times per launch of 4,096 rows and in one launch of all: 16,281 x 12,001 x 123 63 -> 115 us for all (254 in four
 // launches), ten classes, 10,000 x 8,003 x 784 157 -> 323 us for all (380 in three); whole calls 320 -> 162 and 535 -> 397 us,
-// 100,000 x 200,000 x 2,000 180 -> 178 ms (it waits for the tensor pipe). What bounds it now: the products, 2.4 of 2.8 us per
-// tile with 123 features; with ten classes the epilogue (products alone: 240 of 323 us).
+// 100,000 x 200,000 x 2,000 180 -> 178 ms (it waits for the tensor pipe). What bounds it now: with 123 features and three products those,
+// 2.4 of 2.8 us per tile (with one, see hi_only, the epilogue); with ten classes the epilogue (products alone: 240 of 323 us).
 // Sums are no less exact than before: FP32 over four products at a time, FP64 from 32 on; against sums in FP64 the relative
 // errors of ten data sets are 0.96 - 1.03 times the former, 1.00 on average.
 // The price is a tile of 256 test rows, whole or not. The columns' numbers travel by bulk copies into two buffers (warp 2), so
@@ -978,7 +990,7 @@ tsvm_status launch_dense_tc2_predict_lanes(tsvm_km *km, int m, const float *cols
     const InstancePlanes rows{km->Whi, km->Wlo, km->sd_rows, km->w_unscale, m};
     const RowPlanes svs{km->Xhi, km->Xlo, km->self_dot, km->x_unscale};
     const PredictArgs pa{nullptr, nullptr, dec_dev, row_stride, pair_stride, n_classes, cols, cols_ld, nc_pad};
-    const RowsExtra ex{nullptr, nullptr, 0, nullptr};
+    const RowsExtra ex{nullptr, nullptr, 0, 0, nullptr};
     const bool rbf = epilogue_kind(km->fn) == EPI_RBF;
     const bool one_unit = km->plane_ld <= 128;              // two k slabs
 #define TSVM_LANES(EPI, NC) \
