@@ -103,7 +103,7 @@ __device__ __forceinline__ long long device_ns() {
 // When the phases of an outer iteration began and ended (device_ns), noted by the kernels themselves: timing events between
 // launches delay the next kernel by 3 - 4 us each, seven of them took 25 of the 370 us of an iteration at 10,000 x 20.
 struct PhaseTimes {
-    long long select_begin, select_end, rows_end, local_begin, local_end, update_begin;
+    long long select_begin, select_end, rows_end, local_begin, local_end;
 };
 
 // Monotone map double -> uint64 (ascending); -0.0 is folded onto +0.0 so that equal values

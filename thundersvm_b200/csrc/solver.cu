@@ -245,37 +245,50 @@ struct SolverCtl {
     long long local_iter;
     long long ctr[CACHE_CTRS];      // cache counters as of the last iteration that ran
     PhaseTimes times;               // of the running iteration
+    long long update_begin;                                // of the iteration before
     long long ns_select, ns_rows, ns_local, ns_update;     // sums over the iterations that ran
 };
 static_assert(offsetof(SolverCtl, stop) == 0, "kernels read the stop flag through a pointer to the struct");
 
-constexpr int STATUS_THREADS = 512;                               // at least half the largest working set
+struct StatusArgs {
+    SolverCtl *c = nullptr;         // nullptr: nothing to do
+    const double *diff = nullptr;
+    const int *got = nullptr;
+    int wanted = 0;
+    double eps = 0;
+    int max_iter = -1;
+    const long long *cache_ctr = nullptr;
+    const int *engine_status = nullptr;
+    int *ids = nullptr;
+    int q = 0;
+    unsigned char *in_ws = nullptr;
+    volatile unsigned long long *progress = nullptr;
+};
 
-__global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ diff, const int *__restrict__ got,
-                                     int wanted, double eps, int max_iter, const long long *__restrict__ cache_ctr,
-                                     const int *__restrict__ engine_status, int *__restrict__ ids, int q,
-                                     unsigned char *__restrict__ in_ws, volatile unsigned long long *progress) {
+// One block. It reads nothing that the f update writes, so that it runs as one more block of the iteration's last f update
+// (a launch of its own took 4.1 us and 2.2 between launches).
+__device__ __noinline__ void solver_status(const StatusArgs &s) {
+    SolverCtl *c = s.c;
     const int already = c->stop;
     __syncthreads();
     if (already) return;
-    const long long now = device_ns();
     // The working set rotates for the next selection: the old second half becomes the first half and keeps its flags,
     // the old first half leaves. (After the last iteration nothing looks at it again.)
-    if ((int) threadIdx.x < q) {
-        const int leaving = ids[threadIdx.x], staying = ids[q + threadIdx.x];
-        if (leaving >= 0) in_ws[leaving] = 0;
-        if (staying >= 0) in_ws[staying] = 1;
-        ids[threadIdx.x] = staying;
+    for (int t = threadIdx.x; t < s.q; t += blockDim.x) {
+        const int leaving = s.ids[t], staying = s.ids[s.q + t];
+        if (leaving >= 0) s.in_ws[leaving] = 0;
+        if (staying >= 0) s.in_ws[staying] = 1;
+        s.ids[t] = staying;
     }
     if (threadIdx.x != 0) return;
     // everything is read before anything is written, so that the reads are in flight together (5.2 -> 4.4 us against
     // reads that each waited for the write before them)
     SolverCtl v = *c;
-    const double d = diff[0], steps = diff[1];
-    const int found = *got, engine = engine_status ? *engine_status : 0;
-    if (cache_ctr)
+    const double d = s.diff[0], steps = s.diff[1], eps = s.eps;
+    const int found = *s.got, engine = s.engine_status ? *s.engine_status : 0;
+    if (s.cache_ctr)
 #pragma unroll
-        for (int k = 0; k < CACHE_CTRS; ++k) v.ctr[k] = cache_ctr[k];
+        for (int k = 0; k < CACHE_CTRS; ++k) v.ctr[k] = s.cache_ctr[k];
     v.diff0 = d;
     v.local_iter += (long long) steps;
     // csmosolver.cpp:86-111
@@ -287,19 +300,23 @@ __global__ void solver_status_kernel(SolverCtl *c, const double *__restrict__ di
     v.last = d;
     if ((v.same_cnt >= 10 && fabs(d - 2.0) > eps) || d < eps || (v.swap_cnt >= 10 && fabs(d - 2.0) > eps)) v.stop = v.done = 1;
     v.iter++;
-    if (max_iter != -1 && v.iter - 1 == max_iter) v.stop = 1;     // iteration cap (csmosolver.cpp:110)
-    if (found < wanted) { v.short_got = found; v.short_wanted = wanted; v.stop = 1; }
+    if (s.max_iter != -1 && v.iter - 1 == s.max_iter) v.stop = 1;     // iteration cap (csmosolver.cpp:110)
+    if (found < s.wanted) { v.short_got = found; v.short_wanted = s.wanted; v.stop = 1; }
     if (engine) { v.engine_status = engine; v.stop = 1; }
-    if (progress) {
+    if (s.progress) {
         // how far the solve is, for the host that waits for it: a word of pinned host memory
-        *progress = ((unsigned long long) v.iter << 1) | (unsigned) v.stop;
+        *s.progress = ((unsigned long long) v.iter << 1) | (unsigned) v.stop;
         v.ns_select += v.times.select_end - v.times.select_begin;
         v.ns_rows += v.times.rows_end - v.times.select_end;
         v.ns_local += v.times.local_end - v.times.local_begin;
-        v.ns_update += now - v.times.update_begin;
+        // (the update of an iteration ends when the next selection begins; of the last one it is not known)
+        if (v.update_begin) v.ns_update += v.times.select_begin - v.update_begin;
+        v.update_begin = device_ns();
     }
     *c = v;
 }
+
+__global__ void solver_status_kernel(const StatusArgs s) { solver_status(s); }
 
 // *any becomes non-zero if one of a[0..n) is
 __global__ void any_nonzero_kernel(const double *__restrict__ a, int n, int *__restrict__ any) {
@@ -321,17 +338,20 @@ __global__ void fill_int_kernel(int *p, long long n, int v) {
 // sum has the same bits for any number of columns, V and share of them on this GPU. Measured, 512 rows, against one thread
 // per column (four from 300,000 on): 1,000 columns 41 -> 10 us, 10,000 39 -> 12, 32,768 42 -> 20, 100,000 53 -> 45, 200,000
 // 100 -> 78 (5.3 TB/s), 400,000 140 -> 141.
+// Slots [t_begin, t_mid) and [t_mid, t_end) are two sums, subtracted one after the other as two launches would do (one
+// launch for both halves of a working set: 3.9 us less per iteration).
 constexpr int UPD_WARPS = 8, UPD_SLOTS = 1024;
 constexpr int UPD_WIDE_PER_SM = 2;           // blocks of the V = 4 form that fit an SM (registers)
 template <int V>
 __global__ void __launch_bounds__(UPD_WARPS * 32, V == 4 ? UPD_WIDE_PER_SM : 3)
 update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_diff, int q, int first_half_phys,
-                const float *__restrict__ rows, long long ld, int t_begin, int t_end, const int *__restrict__ row_slot,
-                PhaseTimes *times) {
-    if (times && blockIdx.x == 0 && threadIdx.x == 0) times->update_begin = device_ns();
+                const float *__restrict__ rows, long long ld, int t_begin, int t_mid, int t_end, const int *__restrict__ row_slot,
+                const StatusArgs status) {
+    const int other = status.c != nullptr, blocks = gridDim.x - other, block = blockIdx.x - other;
+    if (block < 0) { solver_status(status); return; }               // the first block ends the iteration instead
     constexpr int U = V == 1 ? 16 : 8;
     __shared__ double ad[UPD_SLOTS], part[2][UPD_WARPS][32 * V];
-    __shared__ int prow[UPD_SLOTS], count[UPD_WARPS];
+    __shared__ int prow[UPD_SLOTS], count[UPD_WARPS], count_first[UPD_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // order-preserving compaction of the non-zero entries of slots [t_begin, t_end): 128 slots per warp
     constexpr int PER = UPD_SLOTS / UPD_WARPS / 32;
@@ -343,20 +363,22 @@ update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_
         dv[k] = t < t_end ? alpha_diff[t] : 0.0;
         pr[k] = t < t_end ? (row_slot ? row_slot[t] : (q > 0 ? phys_row(t, q, first_half_phys) : t)) : 0;
     }
-    int mine = 0;
+    int mine = 0, mine_first = 0;
     unsigned ballot[PER];
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         ballot[k] = __ballot_sync(0xffffffffu, dv[k] != 0.0);
         mine += __popc(ballot[k]);
+        mine_first += __popc(__ballot_sync(0xffffffffu, dv[k] != 0.0 && t_begin + (warp * PER + k) * 32 + lane < t_mid));
     }
-    if (lane == 0) count[warp] = mine;
+    if (lane == 0) { count[warp] = mine; count_first[warp] = mine_first; }
     __syncthreads();
-    int base = 0, m = 0;
+    int base = 0, m = 0, m_first = 0;
 #pragma unroll
     for (int w = 0; w < UPD_WARPS; ++w) {
         if (w < warp) base += count[w];
         m += count[w];
+        m_first += count_first[w];
     }
     if (m == 0) return;
 #pragma unroll
@@ -369,10 +391,9 @@ update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_
         base += __popc(ballot[k]);
     }
     __syncthreads();
-    const int run = (m + UPD_WARPS - 1) / UPD_WARPS, r0 = warp * run, r1 = min(m, r0 + run);
     int buf = 0;
-    for (long long c0 = (long long) blockIdx.x * (32 * V); c0 < n; buf ^= 1) {
-        const double f_old = tid < 32 * V && c0 + tid < n ? f[c0 + tid] : 0.0;
+    for (long long c0 = (long long) block * (32 * V); c0 < n;) {
+        double f_now = tid < 32 * V && c0 + tid < n ? f[c0 + tid] : 0.0;
         const float *col = rows + (c0 + lane * V < n ? c0 + lane * V : 0);
         auto load = [&](int r, float (&x)[V]) {
             const float *at = col + (size_t) prow[r] * ld;
@@ -381,40 +402,47 @@ update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_
                 x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
             } else x[0] = __ldcs(at);
         };
-        double s[V];
+        for (int part_no = 0; part_no < 2; ++part_no) {         // the slots before t_mid, then those from there on
+            const int p0 = part_no ? m_first : 0, p1 = part_no ? m : m_first;
+            if (p0 == p1) continue;
+            const int run = (p1 - p0 + UPD_WARPS - 1) / UPD_WARPS, r0 = p0 + warp * run, r1 = min(p1, r0 + run);
+            double s[V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) s[v] = 0;
-        for (int r = r0; r < r1; r += U) {
-            float x[U][V];
-            if (r + U <= r1) {
+            for (int v = 0; v < V; ++v) s[v] = 0;
+            for (int r = r0; r < r1; r += U) {
+                float x[U][V];
+                if (r + U <= r1) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) load(r + u, x[u]);
+                    for (int u = 0; u < U; ++u) load(r + u, x[u]);
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int v = 0; v < V; ++v) s[v] += ad[r + u] * x[u][v];
-            } else {                            // the rest in one go as well
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (r + u < r1) load(r + u, x[u]);
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (r + u < r1)
+                    for (int u = 0; u < U; ++u)
 #pragma unroll
                         for (int v = 0; v < V; ++v) s[v] += ad[r + u] * x[u][v];
+                } else {                            // the rest in one go as well
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (r + u < r1) load(r + u, x[u]);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (r + u < r1)
+#pragma unroll
+                            for (int v = 0; v < V; ++v) s[v] += ad[r + u] * x[u][v];
+                }
             }
-        }
 #pragma unroll
-        for (int v = 0; v < V; ++v) part[buf][warp][lane * V + v] = s[v];
-        __syncthreads();        // (this buffer is written again only after the next barrier)
-        if (tid < 32 * V && c0 + tid < n) {
-            double t = part[buf][0][tid];
+            for (int v = 0; v < V; ++v) part[buf][warp][lane * V + v] = s[v];
+            __syncthreads();        // (this buffer is written again only after the next barrier)
+            if (tid < 32 * V && c0 + tid < n) {
+                double t = part[buf][0][tid];
 #pragma unroll
-            for (int w = 1; w < UPD_WARPS; ++w) t += part[buf][w][tid];
-            f[c0 + tid] = f_old - t;
+                for (int w = 1; w < UPD_WARPS; ++w) t += part[buf][w][tid];
+                f_now -= t;
+            }
+            buf ^= 1;
         }
+        if (tid < 32 * V && c0 + tid < n) f[c0 + tid] = f_now;
         if (V == 1) return;                     // one tile per block
-        c0 += (long long) gridDim.x * (32 * V);
+        c0 += (long long) blocks * (32 * V);
     }
 }
 
@@ -570,14 +598,15 @@ __global__ void shard_scatter_kernel(const int *__restrict__ ids, int ws, int lo
 // 23 us at 32,768 columns, but 18.5 against 16.4 at 20,000. Below that, and for rows that are not aligned, 32 columns per
 // block.
 static tsvm_status launch_update_f(double *f, int n, const double *alpha_diff, int q, int first_half_phys, const float *rows,
-                                   long long ld, int t0, int t1, const int *row_slot, PhaseTimes *times, cudaStream_t st) {
-    const int wide_tiles = ceil_div(n, 128), sms = device_sm_count();
+                                   long long ld, int t0, int t_mid, int t1, const int *row_slot, cudaStream_t st,
+                                   const StatusArgs &status = StatusArgs()) {
+    const int wide_tiles = ceil_div(n, 128), sms = device_sm_count(), more = status.c != nullptr;
     if (((uintptr_t) rows & 15) == 0 && (ld & 3) == 0 && 2 * wide_tiles >= 3 * sms)
-        TSVM_LAUNCH(update_f_kernel<4>, wide_tiles < UPD_WIDE_PER_SM * sms ? wide_tiles : UPD_WIDE_PER_SM * sms, UPD_WARPS * 32,
-                    0, st, f, n, alpha_diff, q, first_half_phys, rows, ld, t0, t1, row_slot, times);
+        TSVM_LAUNCH(update_f_kernel<4>, wide_tiles + more < UPD_WIDE_PER_SM * sms ? wide_tiles + more : UPD_WIDE_PER_SM * sms,
+                    UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows, ld, t0, t_mid, t1, row_slot, status);
     else
-        TSVM_LAUNCH(update_f_kernel<1>, ceil_div(n, 32), UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows,
-                    ld, t0, t1, row_slot, times);
+        TSVM_LAUNCH(update_f_kernel<1>, ceil_div(n, 32) + more, UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows,
+                    ld, t0, t_mid, t1, row_slot, status);
     return TSVM_OK;
 }
 
@@ -863,7 +892,7 @@ tsvm_status tsvm_update_f(double *f_dev, int n, const double *alpha_diff_dev, in
                           long long ld, void *stream) {
     TSVM_REQUIRE(f_dev && alpha_diff_dev && rows_dev && n > 0 && ws_size > 0 && ws_size <= 1024 && ld >= n,
                  "update_f: bad arguments (at most 1024 rows per call)");
-    TSVM_TRY(launch_update_f(f_dev, n, alpha_diff_dev, 0, 0, rows_dev, ld, 0, ws_size, nullptr, nullptr, (cudaStream_t) stream));
+    TSVM_TRY(launch_update_f(f_dev, n, alpha_diff_dev, 0, 0, rows_dev, ld, 0, 0, ws_size, nullptr, (cudaStream_t) stream));
     return TSVM_OK;
 }
 
@@ -1145,7 +1174,7 @@ struct tsvm_solver {
             TSVM_CUDA(cudaMemcpyAsync(ids, bi.data(), sizeof(int) * m, cudaMemcpyHostToDevice, st));
             TSVM_CUDA(cudaMemcpyAsync(alpha_diff, bd.data(), sizeof(double) * m, cudaMemcpyHostToDevice, st));
             TSVM_TRY(tsvm_km_rows_by_index(km, ids, m, rows, ld, st));
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, 0, 0, rows, ld, 0, m, nullptr, nullptr, st));
+            TSVM_TRY(launch_update_f(f, n, alpha_diff, 0, 0, rows, ld, 0, 0, m, nullptr, st));
             TSVM_CUDA(cudaStreamSynchronize(st));
             rows_made += m;
             bi.clear(); bd.clear();
@@ -1225,7 +1254,7 @@ struct tsvm_solver {
             TSVM_CUDA(cudaStreamWaitEvent(st2, ev_fork2, 0));
             // the rows that were in the buffer already can be applied to f at once (HBM-bound, next to the
             // tensor-bound launch); the new rows follow on the first stream
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, q, row_slot, nullptr, st2));
+            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, 0, q, row_slot, st2));
             TSVM_CUDA(cudaEventRecord(ev_join, st2));
             // first stream: the missing rows against all instances, on all SM pairs but one
             const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
@@ -1245,17 +1274,13 @@ struct tsvm_solver {
         } else {
             TSVM_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
         }
-        // f -= sum over the old half's rows, then f -= sum over the new half's rows: two launches in every
-        // form of the iteration, so that all of them round alike (the first iteration has new rows only)
-        if (it == 0) {
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, ws, row_slot, times, st));
-        } else {
-            if (!overlapped)
-                TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, 0, q, row_slot, nullptr, st));
-            TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, q, ws, row_slot, times, st));
-        }
-        TSVM_LAUNCH(solver_status_kernel, 1, STATUS_THREADS, 0, st, ctl, diff, sel->count, n_new, eps, max_iter, cache_ctr,
-                    km->status_dev, ids, q, in_ws, progress());
+        // f -= sum over the old half's rows, then f -= sum over the new half's rows: two sums in every form of the iteration,
+        // so that all of them round alike (the first iteration has new rows only; overlapped, the old half is done)
+        StatusArgs status;
+        status.c = ctl; status.diff = diff; status.got = sel->count; status.wanted = n_new; status.eps = eps; status.max_iter = max_iter;
+        status.cache_ctr = cache_ctr; status.engine_status = km->status_dev; status.ids = ids; status.q = q; status.in_ws = in_ws;
+        status.progress = progress();
+        TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, overlapped ? q : 0, it == 0 ? 0 : q, ws, row_slot, st, status));
         return TSVM_OK;
     }
 
@@ -1676,7 +1701,7 @@ struct tsvm_shard {
                                   nullptr, nullptr, st2, &ctl->stop));
         TSVM_CUDA(cudaEventRecord(E.b1, st2));
         if (it > 0)        // the old half's rows are in the buffer already
-            TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, 0, q, nullptr, nullptr, st2));
+            TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, 0, 0, q, nullptr, st2));
         TSVM_CUDA(cudaEventRecord(ev_join, st2));
         // first stream: the new rows against this rank's columns
         float *new_rows = rows + (size_t) (it == 0 ? 0 : (1 - first_half_phys) * q) * ld;
@@ -1688,10 +1713,12 @@ struct tsvm_shard {
         TSVM_TRY(rs);
         TSVM_CUDA(cudaEventRecord(E.r1, st));
         TSVM_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
-        TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, it == 0 ? 0 : q, ws, nullptr, nullptr, st));
+        TSVM_TRY(launch_update_f(f, n_local, alpha_diff, q, first_half_phys, rows, ld, it == 0 ? 0 : q, it == 0 ? 0 : q, ws, nullptr, st));
         TSVM_LAUNCH(shard_scatter_kernel, ceil_div(ws, 256), 256, 0, st, ids, ws, lo, hi, a_ws, alpha);
-        TSVM_LAUNCH(solver_status_kernel, 1, 32, 0, st, ctl, diff, sel->count, n_new, eps, -1, (const long long *) nullptr,
-                    km->status_dev, (int *) nullptr, 0, (unsigned char *) nullptr, (volatile unsigned long long *) nullptr);
+        StatusArgs status;
+        status.c = ctl; status.diff = diff; status.got = sel->count; status.wanted = n_new; status.eps = eps;
+        status.engine_status = km->status_dev;
+        TSVM_LAUNCH(solver_status_kernel, 1, 32, 0, st, status);
         ++queued;
         phase = 0;
         return TSVM_OK;
