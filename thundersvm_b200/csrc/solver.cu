@@ -23,6 +23,7 @@ __device__ __forceinline__ int phys_row(int t, int q, int first_half_phys) {
     return t < q ? first_half_phys * q + t : (1 - first_half_phys) * q + (t - q);
 }
 
+constexpr int GATHER_AT_A_TIME = 4;
 __global__ void gather_ws_kernel(int ws, int q, int first_half_phys, const int *__restrict__ ids,
                                  const float *__restrict__ rows, long long ld, const float *__restrict__ diag,
                                  const int *__restrict__ y, const double *__restrict__ f,
@@ -37,9 +38,17 @@ __global__ void gather_ws_kernel(int ws, int q, int first_half_phys, const int *
     // a slot without an instance (id -1: fewer eligible instances than slots) is inert: y = 0 puts it in no set
     if (a < block_rows) {
         const float *row = rows + (size_t) (row_slot ? row_slot[a] : phys_row(a, q, first_half_phys)) * ld;
-        for (int b = threadIdx.x; b < ws; b += blockDim.x) {
-            const int id = ids[b];
-            kww[(size_t) a * ws + b] = id >= 0 ? row[id] : 0.0f;
+        // all of a thread's ids first, then all of its values: two latencies instead of eight
+        for (int b0 = threadIdx.x; b0 < ws; b0 += GATHER_AT_A_TIME * blockDim.x) {
+            int id[GATHER_AT_A_TIME];
+            float k[GATHER_AT_A_TIME];
+#pragma unroll
+            for (int u = 0; u < GATHER_AT_A_TIME; ++u) id[u] = b0 + u * blockDim.x < ws ? ids[b0 + u * blockDim.x] : -1;
+#pragma unroll
+            for (int u = 0; u < GATHER_AT_A_TIME; ++u) k[u] = id[u] >= 0 ? row[id[u]] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < GATHER_AT_A_TIME; ++u)
+                if (b0 + u * blockDim.x < ws) kww[(size_t) a * ws + b0 + u * blockDim.x] = k[u];
         }
     }
     if (threadIdx.x == 0) {
