@@ -270,6 +270,22 @@ def test_update_f_runs_and_tiles(capi, n, ws, nonzero):
     assert np.array_equal(got[0], got[1]) and got[0][0] == got[2][0]
 
 
+@pytest.mark.parametrize("n", [14208, 14209, 14273, 20243, 28287])
+@pytest.mark.parametrize("shift", [0, 2, 1])
+def test_update_f_64_column_tiles(capi, n, shift):
+    """Around the column counts from which a block takes 64 columns (with 148 SMs), a last tile of one column; rows that are
+    16-, 8- and 4-byte aligned, the last of which keep to 32 columns. The same bits whatever the form."""
+    import torch
+    rng = np.random.default_rng(n)
+    ld = (n + 4 + 3) // 4 * 4 if shift != 1 else n + 4 + (n % 2 == 0)
+    block = torch.from_numpy(rng.random((130, ld), dtype=np.float32)).cuda()
+    rows = block.view(-1)[shift:shift + 129 * ld].view(129, ld)[:, :n]
+    ad, f = rng.standard_normal(129), rng.standard_normal(n)
+    got = capi.update_f(_t(f), _t(ad), rows).cpu().numpy()
+    assert np.allclose(got, P.update_f(f, ad, np.ascontiguousarray(rows.cpu().numpy())), rtol=0, atol=1e-11)
+    assert got[0] == capi.update_f(_t(f[:1]), _t(ad), rows[:, :1]).cpu().numpy()[0]
+
+
 CASES = {"c1": (lambda: synth.config1(1500), None, None), "c1_soft": (lambda: dict(synth.config1(1500), gamma=0.025), None, None),
          "c2": (lambda: synth.config2(1200), None, None), "c2_dense": (lambda: synth.config2(1200), None, "dense"),
          "c3": (lambda: synth.config3(900), 5, None), "c4": (lambda: synth.config4(700), None, None),

@@ -350,15 +350,15 @@ __global__ void fill_int_kernel(int *p, long long n, int v) {
 // Slots [t_begin, t_mid) and [t_mid, t_end) are two sums, subtracted one after the other as two launches would do (one
 // launch for both halves of a working set: 3.9 us less per iteration).
 constexpr int UPD_WARPS = 8, UPD_SLOTS = 1024;
-constexpr int UPD_WIDE_PER_SM = 2;           // blocks of the V = 4 form that fit an SM (registers)
+constexpr int UPD_WIDE_PER_SM = 2, UPD_NARROW_PER_SM = 3;        // blocks of the V = 4 form and of the others that fit an SM (registers)
 template <int V>
-__global__ void __launch_bounds__(UPD_WARPS * 32, V == 4 ? UPD_WIDE_PER_SM : 3)
+__global__ void __launch_bounds__(UPD_WARPS * 32, V == 4 ? UPD_WIDE_PER_SM : UPD_NARROW_PER_SM)
 update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_diff, int q, int first_half_phys,
                 const float *__restrict__ rows, long long ld, int t_begin, int t_mid, int t_end, const int *__restrict__ row_slot,
                 const StatusArgs status) {
     const int other = status.c != nullptr, blocks = gridDim.x - other, block = blockIdx.x - other;
     if (block < 0) { solver_status(status); return; }               // the first block ends the iteration instead
-    constexpr int U = V == 1 ? 16 : 8;
+    constexpr int U = V == 4 ? 8 : 16;
     __shared__ double ad[UPD_SLOTS], part[2][UPD_WARPS][32 * V];
     __shared__ int prow[UPD_SLOTS], count[UPD_WARPS], count_first[UPD_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -406,7 +406,10 @@ update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_
         const float *col = rows + (c0 + lane * V < n ? c0 + lane * V : 0);
         auto load = [&](int r, float (&x)[V]) {
             const float *at = col + (size_t) prow[r] * ld;
-            if constexpr (V == 4) {
+            if constexpr (V == 2) {
+                const float2 t = __ldcs(reinterpret_cast<const float2 *>(at));
+                x[0] = t.x; x[1] = t.y;
+            } else if constexpr (V == 4) {
                 const float4 t = __ldcs(reinterpret_cast<const float4 *>(at));       // (the row is padded to a multiple of 4)
                 x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
             } else x[0] = __ldcs(at);
@@ -450,7 +453,7 @@ update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_
             buf ^= 1;
         }
         if (tid < 32 * V && c0 + tid < n) f[c0 + tid] = f_now;
-        if (V == 1) return;                     // one tile per block
+        if (V < 4) return;                      // one tile per block
         c0 += (long long) blocks * (32 * V);
     }
 }
@@ -602,10 +605,11 @@ __global__ void shard_scatter_kernel(const int *__restrict__ ids, int ws, int lo
 // =================================================================================================
 // host side
 // =================================================================================================
-// f -= the rows of slots [t0, t1) times their alpha_diff. 16-byte loads, 128 columns at a time by blocks that stay (a tile's
-// reads start while the last one is being added up), where these tiles keep one and a half blocks per SM busy: 20 against
-// 23 us at 32,768 columns, but 18.5 against 16.4 at 20,000. Below that, and for rows that are not aligned, 32 columns per
-// block.
+// f -= the rows of slots [t0, t1) times their alpha_diff, those before t_mid first. 16-byte loads, 128 columns at a time by blocks
+// that stay (a tile's reads start while the last one is being added up), where these tiles keep one and a half blocks per SM
+// busy: 20 against 23 us at 32,768 columns, but 18.5 against 16.4 at 20,000. Below that, and for rows that are not aligned, one
+// tile per block: 32 columns while all blocks are resident at once, else 64 by 8-byte loads (20,242 columns, both halves of a
+// working set inside a solve: 27 us in one and a half rounds of blocks, 16.6 in one).
 static tsvm_status launch_update_f(double *f, int n, const double *alpha_diff, int q, int first_half_phys, const float *rows,
                                    long long ld, int t0, int t_mid, int t1, const int *row_slot, cudaStream_t st,
                                    const StatusArgs &status = StatusArgs()) {
@@ -613,6 +617,9 @@ static tsvm_status launch_update_f(double *f, int n, const double *alpha_diff, i
     if (((uintptr_t) rows & 15) == 0 && (ld & 3) == 0 && 2 * wide_tiles >= 3 * sms)
         TSVM_LAUNCH(update_f_kernel<4>, wide_tiles + more < UPD_WIDE_PER_SM * sms ? wide_tiles + more : UPD_WIDE_PER_SM * sms,
                     UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows, ld, t0, t_mid, t1, row_slot, status);
+    else if (((uintptr_t) rows & 7) == 0 && (ld & 1) == 0 && ceil_div(n, 32) + more > UPD_NARROW_PER_SM * sms)
+        TSVM_LAUNCH(update_f_kernel<2>, ceil_div(n, 64) + more, UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows,
+                    ld, t0, t_mid, t1, row_slot, status);
     else
         TSVM_LAUNCH(update_f_kernel<1>, ceil_div(n, 32) + more, UPD_WARPS * 32, 0, st, f, n, alpha_diff, q, first_half_phys, rows,
                     ld, t0, t_mid, t1, row_slot, status);
