@@ -976,8 +976,8 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
 
 // The same with the test rows on the tensor memory's lanes and the support vectors on its columns. What bounds FORM_PREDICT is
 // its epilogue: the sum over the support vectors crosses the lanes of a warp (19 instructions per warp and kernel value with
-// two classes, 58 with ten); here it stays in a thread, the support vectors' numbers are the same words for all lanes (5 and
-// 18). Kernel times per launch of 4,096 rows and in one launch of all: 16,281 x 12,001 x 123 63 -> 115 us for all (254 in four
+// two classes, 58 with ten); here it stays in a thread, the support vectors' numbers are the same words for all lanes (8 and
+// 44, waiting included). Kernel times per launch of 4,096 rows and in one launch of all: 16,281 x 12,001 x 123 63 -> 115 us for all (254 in four
 // launches), ten classes, 10,000 x 8,003 x 784 157 -> 323 us for all (380 in three); whole calls 320 -> 162 and 535 -> 397 us,
 // 100,000 x 200,000 x 2,000 180 -> 178 ms (it waits for the tensor pipe). What bounds it now: with 123 features and three products those,
 // 2.4 of 2.8 us per tile (with one, see hi_only, the epilogue); with ten classes the epilogue (products alone: 240 of 323 us).
