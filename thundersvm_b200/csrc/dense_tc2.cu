@@ -10,8 +10,8 @@
 //
 // Roles per CTA (384 threads = 3 warpgroups): warp 0 TMA producer for this CTA's operand halves
 // (transaction bytes are reported to the leader's "full" barrier), warp 1 tensor-memory allocation (both
-// CTAs) and MMA issue (leader only), warps 2..3 idle, warps 4..11 slab promotion + epilogue on this CTA's 128
-// instances. Warpgroup 0 hands registers to the other two (setmaxnreg): the epilogue keeps 128 sums per
+// CTAs) and MMA issue (leader only), warps 2..3 idle (prediction with the test rows on the lanes: warp 2 fetches the columns'
+// numbers), warps 4..11 slab promotion + epilogue on this CTA's 128 instances. Warpgroup 0 hands registers to the other two (setmaxnreg): the epilogue keeps 128 sums per
 // thread live, and with the 168 registers a 384-thread CTA is compiled for it spilled a few loop-invariant
 // values - their reloads from local memory (the L1 is tiny next to 222 KB of shared memory) cost 9 % of
 // the kernel.
@@ -976,10 +976,10 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
 
 // The same with the test rows on the tensor memory's lanes and the support vectors on its columns. What bounds FORM_PREDICT is
 // its epilogue: the sum over the support vectors crosses the lanes of a warp (19 instructions per warp and kernel value with
-// two classes, 58 with ten); here it stays in a thread, the support vectors' numbers are the same words for all lanes (8 and
-// 44, waiting included). Kernel times per launch of 4,096 rows and in one launch of all: 16,281 x 12,001 x 123 63 -> 115 us for all (254 in four
-// launches), ten classes, 10,000 x 8,003 x 784 157 -> 323 us for all (380 in three); whole calls 320 -> 162 and 535 -> 397 us,
-// 100,000 x 200,000 x 2,000 180 -> 178 ms (it waits for the tensor pipe). What bounds it now: with 123 features and three products those,
+// two classes, 58 with ten, waiting included); here it stays in a thread, and the support vectors' numbers are the same words
+// for all lanes (8 and 44). Kernel times: 16,281 x 12,001 x 123 254 us in four launches -> 115 us in one (91 with one product),
+// ten classes, 10,000 x 8,003 x 784 380 us in three -> 323 us in one; whole calls 320 -> 142 and 535 -> 405 us, 100,000 x
+// 200,000 x 2,000 184 -> 181 ms (it waits for the tensor pipe). What bounds it now: with 123 features and three products those,
 // 2.4 of 2.8 us per tile (with one, see hi_only, the epilogue); with ten classes the epilogue (products alone: 240 of 323 us).
 // Sums are no less exact than before: FP32 over four products at a time, FP64 from 32 on; against sums in FP64 the relative
 // errors of ten data sets are 0.96 - 1.03 times the former, 1.00 on average.

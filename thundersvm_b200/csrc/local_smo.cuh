@@ -65,7 +65,6 @@ __device__ __forceinline__ double reciprocal(double a) {
     return a != 0.0 && fabs(a) < 1e300 ? r : r0;
 }
 
-__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
 // Reading ahead: how many slots of an argmin are looked after, how many rows are read at a time at most, and for how many
 // iterations a row that was read is taken to be there (the cache does not keep it for long): KEEP 0 / 1 / 3 make 0.821 / 0.806 /
 // 0.825 us (12,003 x 784), 4 or 8 slots 0.815 or 0.819.

@@ -244,7 +244,7 @@ cache_assign_kernel(const int *__restrict__ ids, int t0, int n_new, int now, int
 // Here one thread applies the same rules to the same doubles on the device, so the host can queue several
 // iterations and read the outcome once: every kernel of a queued iteration looks at `stop` first and does
 // nothing once it is set.
-struct SolverCtl {
+struct SolverState {
     int stop;                       // first member: kernels take a pointer to it
     int done;                       // the reference's own termination rules fired
     int iter, same_cnt, swap_cnt;
@@ -257,7 +257,12 @@ struct SolverCtl {
     long long update_begin;                                // of the iteration before
     long long ns_select, ns_rows, ns_local, ns_update;     // sums over the iterations that ran
 };
-static_assert(offsetof(SolverCtl, stop) == 0, "kernels read the stop flag through a pointer to the struct");
+static_assert(offsetof(SolverState, stop) == 0, "kernels read the stop flag through a pointer to the struct");
+// Next to it when the blocks of an iteration's f update left, by the iteration's parity: written while the block that ends the
+// iteration writes the state back, read by the iteration after.
+struct SolverCtl : SolverState {
+    long long update_end[2];
+};
 
 struct StatusArgs {
     SolverCtl *c = nullptr;         // nullptr: nothing to do
@@ -272,6 +277,7 @@ struct StatusArgs {
     int q = 0;
     unsigned char *in_ws = nullptr;
     volatile unsigned long long *progress = nullptr;
+    int parity = 0;                 // of the iteration
 };
 
 // One block. It reads nothing that the f update writes, so that it runs as one more block of the iteration's last f update
@@ -292,7 +298,8 @@ __device__ __noinline__ void solver_status(const StatusArgs &s) {
     if (threadIdx.x != 0) return;
     // everything is read before anything is written, so that the reads are in flight together (5.2 -> 4.4 us against
     // reads that each waited for the write before them)
-    SolverCtl v = *c;
+    SolverState v = *c;
+    const long long update_end = *(volatile const long long *) &c->update_end[s.parity ^ 1];       // (of the iteration before)
     const double d = s.diff[0], steps = s.diff[1], eps = s.eps;
     const int found = *s.got, engine = s.engine_status ? *s.engine_status : 0;
     if (s.cache_ctr)
@@ -318,11 +325,10 @@ __device__ __noinline__ void solver_status(const StatusArgs &s) {
         v.ns_select += v.times.select_end - v.times.select_begin;
         v.ns_rows += v.times.rows_end - v.times.select_end;
         v.ns_local += v.times.local_end - v.times.local_begin;
-        // (the update of an iteration ends when the next selection begins; of the last one it is not known)
-        if (v.update_begin) v.ns_update += v.times.select_begin - v.update_begin;
+        if (update_end > v.update_begin && v.update_begin) v.ns_update += update_end - v.update_begin;
         v.update_begin = device_ns();
     }
-    *c = v;
+    *static_cast<SolverState *>(c) = v;
 }
 
 __global__ void solver_status_kernel(const StatusArgs s) { solver_status(s); }
@@ -453,9 +459,11 @@ update_f_kernel(double *__restrict__ f, int n, const double *__restrict__ alpha_
             buf ^= 1;
         }
         if (tid < 32 * V && c0 + tid < n) f[c0 + tid] = f_now;
-        if (V < 4) return;                      // one tile per block
+        if (V < 4) break;                       // one tile per block
         c0 += (long long) blocks * (32 * V);
     }
+    if (status.c && tid == 0)
+        atomicMax(reinterpret_cast<unsigned long long *>(&status.c->update_end[status.parity]), (unsigned long long) device_ns());
 }
 
 // =================================================================================================
@@ -1295,7 +1303,7 @@ struct tsvm_solver {
         StatusArgs status;
         status.c = ctl; status.diff = diff; status.got = sel->count; status.wanted = n_new; status.eps = eps; status.max_iter = max_iter;
         status.cache_ctr = cache_ctr; status.engine_status = km->status_dev; status.ids = ids; status.q = q; status.in_ws = in_ws;
-        status.progress = progress();
+        status.progress = progress(); status.parity = (int) (it & 1);
         TSVM_TRY(launch_update_f(f, n, alpha_diff, q, 0, rows, ld, overlapped ? q : 0, it == 0 ? 0 : q, ws, row_slot, st, status));
         return TSVM_OK;
     }
@@ -1353,6 +1361,8 @@ struct tsvm_solver {
             return TSVM_ERR_DEVICE;
         }
         t_sel = c.ns_select * 1e-9; t_rows = c.ns_rows * 1e-9; t_loc = c.ns_local * 1e-9; t_upd = c.ns_update * 1e-9;
+        const long long last_end = c.update_end[0] > c.update_end[1] ? c.update_end[0] : c.update_end[1];
+        if (c.update_begin && last_end > c.update_begin) t_upd += (last_end - c.update_begin) * 1e-9;       // (of the last iteration)
         hits = c.ctr[CACHE_HITS]; misses = c.ctr[CACHE_MISSES];
         row_blocks = c.ctr[CACHE_BLOCKS]; row_blocks_saved = c.ctr[CACHE_BLOCKS_SAVED];
         rows_made += (c.iter - iter_collected) * q + (iter_collected == 0 && c.iter > 0 ? ws - q : 0);
