@@ -220,6 +220,40 @@ def test_local_smo_values_at_the_ends_of_the_range(capi, ws, case):
     assert np.allclose(a, a_exp, rtol=1e-9, atol=1e-9 * max(1.0, np.abs(a_exp).max()))
 
 
+@pytest.mark.parametrize("solver", ["c", "nu_svc"])
+@pytest.mark.parametrize("ws", [64, 300, 1024])
+@pytest.mark.parametrize("curvature,scale", [("negative", 0), ("negative", -20), ("zero", 0), ("zero", -30)])
+def test_local_smo_curvature_of_neighbours_whose_f_nearly_ties(capi, solver, ws, curvature, scale):
+    """Candidates j with f a few ulp above the smallest one and a curvature that is not positive: a negative one is the last
+    choice (and a step of no size for ever if it is taken), zero is the first, however small the difference of f. At the
+    smallest scale the square of that difference is far below what the other candidates have."""
+    rng = np.random.default_rng(ws)
+    X = rng.standard_normal((ws, 5))
+    kww = np.exp(-0.1 * ((X[:, None] - X[None]) ** 2).sum(2)).astype(np.float32)
+    y = np.where(np.arange(ws) % 2 == 0, 1, -1).astype(np.int32)
+    if solver == "c":
+        f, alpha = -y + 0.01 * rng.standard_normal(ws), np.zeros(ws)
+        near = np.array([5, ws // 2 + 1, ws - 1])               # of the class that may go down
+    else:
+        f, alpha = rng.random(ws), np.where(np.arange(ws) % 4 < 2, 1.0, 0.0)
+        near = np.array([4, ws // 2 // 4 * 4, ws - 4])          # y > 0, alpha at its bound
+    i = 2 if solver == "nu_svc" else 6                          # y > 0, alpha = 0
+    f[i] = -2.0
+    f[near] = -2.0 + np.array([1, 2, 4]) * 2.0 ** -52         # (doubles below 2 in magnitude)
+    if scale and curvature == "zero":                           # the others keep their differences
+        f = np.abs(f) + 0.5
+        f[i] = 1.0
+        f[near] = 1.0 + np.array([1, 2, 4]) * 2.0 ** -52
+        f[np.r_[i, near]] *= 2.0 ** scale
+    else:
+        f *= 2.0 ** scale
+    kww[i, near] = kww[near, i] = 1.0 if curvature == "zero" else 1.5
+    (a, ad, diff), (a_exp, ad_exp, diff_exp) = _local_smo_both(capi, solver, np.ascontiguousarray(kww), y, f, alpha, 1.0,
+                                                               eps=1e-12, max_iter=39)
+    assert diff[1] == diff_exp[1]
+    assert np.allclose(a, a_exp, rtol=1e-9, atol=1e-9 * np.abs(a_exp - alpha).max())
+
+
 @pytest.mark.parametrize("ws", [256, 512, 1024])
 def test_local_smo_rows_copied_ahead_hold_the_same_values(capi, ws):
     """A block whose rows are 16-byte aligned and one that is not, while other warps read rows ahead: the same steps, bit

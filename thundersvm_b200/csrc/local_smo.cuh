@@ -379,7 +379,10 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
 
         // ---- second-order choice of j ------------------------------------------------------------------------
         // b in FP32, truncated, straight from the double's bits (zero below 2^-126 and outside I_low; the gap bounds it above).
-        // A curvature that is no positive float gives a value beyond what is accepted below.
+        // A curvature of zero (below 2^-126) has the reciprocal infinity: the value is beyond what is accepted below, whatever b
+        // is. A negative one gives a negative value, which counts as zero like that of no candidate: it is chosen only where all
+        // values are so, and then in FP64. So does 0 times infinity, slot i itself (the maximum drops a NaN; NaN in a kernel value
+        // is found by k_most).
         float q[S], k_most;
         {
             float m[S];
@@ -391,8 +394,8 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
                 const float b32 = __int_as_float(__funnelshift_l((unsigned) __double2loint(b), (unsigned) max(__double2hiint(b), 0), 3));
                 const float a32 = fmaf(-2.0f, k, (second ? kd_i[CLS - 1] : kd_i[0]) + kd[s]);
                 float r;
-                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(a32, 0x1p-126f)));
-                q[s] = mul_ftz(mul_ftz(b32, r), b32);
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a32));
+                q[s] = fmaxf(mul_ftz(mul_ftz(b32, r), b32), 0.0f);
                 m[s] = k;
             }
             k_most = max_abs3(max_abs_of(m), kd_most, kd_most);
