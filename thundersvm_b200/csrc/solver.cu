@@ -254,7 +254,7 @@ struct SolverState {
     long long local_iter;
     long long ctr[CACHE_CTRS];      // cache counters as of the last iteration that ran
     PhaseTimes times;               // of the running iteration
-    long long update_begin;                                // of the iteration before
+    long long update_begin;         // of the iteration before
     long long ns_select, ns_rows, ns_local, ns_update;     // sums over the iterations that ran
 };
 static_assert(offsetof(SolverState, stop) == 0, "kernels read the stop flag through a pointer to the struct");
@@ -284,6 +284,7 @@ struct StatusArgs {
 // (a launch of its own took 4.1 us and 2.2 between launches).
 __device__ __noinline__ void solver_status(const StatusArgs &s) {
     SolverCtl *c = s.c;
+    const long long begin = device_ns();        // of the f update that this block runs in: its other blocks start with it
     const int already = c->stop;
     __syncthreads();
     if (already) return;
@@ -326,7 +327,7 @@ __device__ __noinline__ void solver_status(const StatusArgs &s) {
         v.ns_rows += v.times.rows_end - v.times.select_end;
         v.ns_local += v.times.local_end - v.times.local_begin;
         if (update_end > v.update_begin && v.update_begin) v.ns_update += update_end - v.update_begin;
-        v.update_begin = device_ns();
+        v.update_begin = begin;
     }
     *static_cast<SolverState *>(c) = v;
 }
