@@ -254,6 +254,55 @@ def test_local_smo_curvature_of_neighbours_whose_f_nearly_ties(capi, solver, ws,
     assert np.allclose(a, a_exp, rtol=1e-9, atol=1e-9 * np.abs(a_exp - alpha).max())
 
 
+@pytest.mark.parametrize("solver", ["c", "nu_svc"])
+@pytest.mark.parametrize("law", ["ordinary", "cancelling", "wide"])
+def test_local_smo_step_is_within_an_ulp_of_the_division(capi, solver, law):
+    """One step of two instances with room enough moves alpha from zero by b / a: the kernel's quotient against the true
+    division of the same doubles. Ordinary curvatures, such that are the small difference of large kernel values, and both
+    operands over many powers of two."""
+    rng = np.random.default_rng(len(law))
+    worst = 0.0
+    for _ in range(200):
+        s = 2.0 ** rng.integers(-40, 41) if law == "wide" else 1.0
+        kd = (s * (0.5 + rng.random(2))).astype(np.float32)
+        least = np.float32(kd.sum()) / np.float32(2)
+        kij = np.float32(least * (1 - 2.0 ** -rng.integers(15, 20)) if law == "cancelling" else s * (0.5 * rng.random() - 0.2))
+        a = float(np.float32(kd[0] + kd[1]) - np.float32(2) * kij) if solver == "nu_svc" else float(np.float32(kd[0] + kd[1])) - 2.0 * float(kij)
+        f = rng.standard_normal(2) * (2.0 ** rng.integers(-30, 31) if law == "wide" else 1.0)
+        f.sort()
+        b = -f[0] + f[1]
+        assert a > 0 and b > 0
+        y = np.array([1, -1] if solver == "c" else [1, 1], np.int32)
+        C = 2.0 ** 90
+        alpha, _, diff = capi.local_smo(_t(np.array([[kd[0], kij], [kij, kd[1]]], np.float32)), _t(kd), _t(y), _t(f),
+                                        _t(np.array([0.0, 0.0 if solver == "c" else C])), C, C, 0.0, max_iter=0, solver=solver)
+        assert diff[1].item() == 1
+        worst = max(worst, abs(alpha[0].item() - b / a) / np.spacing(b / a))
+    assert worst <= 1.0, worst
+
+
+@pytest.mark.parametrize("swapped", [False, True])
+def test_local_smo_choice_between_nearly_equal_values(capi, swapped):
+    """Two candidates whose b^2 / a differ by 1e-14 relative: equal to single precision, so the choice falls in FP64, whose
+    values are good to a few ulp (b^2 one rounding, the reciprocal two, their product one: below 5 x 2^-53 = 6e-16 each)."""
+    rng = np.random.default_rng(7)
+    for _ in range(100):
+        kI = (0.8 * rng.random(2)).astype(np.float32)
+        a = 2.0 - 2.0 * kI.astype(np.float64)
+        up, b0 = 0.25 * rng.standard_normal(), 0.5 + rng.random()
+        # equal values first, then the winner's f up by single doubles
+        f = np.array([up, up + b0, up + b0 * np.sqrt(a[1] / a[0])])
+        want = 2 if swapped else 1
+        e = (f[1:] - up) ** 2 / a
+        while e[want - 1] / e[2 - want] - 1 < 1e-14:
+            f[want] = np.nextafter(f[want], np.inf)
+            e = (f[1:] - up) ** 2 / a
+        K = np.array([[1, kI[0], kI[1]], [kI[0], 1, 0.5], [kI[1], 0.5, 1]], np.float32)
+        alpha, _, _ = capi.local_smo(_t(K), _t(np.ones(3, np.float32)), _t(np.array([1, -1, -1], np.int32)), _t(f),
+                                     _t(np.zeros(3)), 1e6, 1e6, 0.0, max_iter=0, solver="c")
+        assert alpha[want].item() > 0 and alpha[3 - want].item() == 0
+
+
 @pytest.mark.parametrize("ws", [256, 512, 1024])
 def test_local_smo_rows_copied_ahead_hold_the_same_values(capi, ws):
     """A block whose rows are 16-byte aligned and one that is not, while other warps read rows ahead: the same steps, bit

@@ -22,7 +22,11 @@
 //   * No conversion instructions on the chain (16 of them took 160 cycles): f is held times 2^-896, which makes a float's
 //     bits a double's and a double's a float's by shifts. A value of f below 2^-126 loses digits that way, sums of kernel
 //     values do not get there.
-//   * The step is divided by a reciprocal corrected once, its result by its remainder: within an ulp of the division.
+//   * The step is divided by a reciprocal after one Newton-Raphson iteration, the quotient corrected by its remainder: the method
+//     of P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor" (IBM Journal of Research and
+//     Development 34, 1990), which rests on the fused multiply-add. Within an ulp of the division: the hardware's approximation of
+//     the reciprocal has some 20 bits, the iteration squares its error, and the correction squares that (below 2^-70, beside the last
+//     rounding).
 //   * Two more warps read the rows that the next iterations will want into the L1 cache (read_rows_ahead). In most calls every
 //     row is wanted about once, so a cache alone finds a tenth of them; the best six of an argmin's list hold the next
 //     iteration's winner nine times in ten.
@@ -56,7 +60,8 @@ __device__ __forceinline__ float warp_max_f32(float v) {
     return r;
 }
 
-// 1 / a to a few ulp: two Newton steps on the hardware's approximation (which is kept for zero and infinity)
+// 1 / a to a few ulp: two Newton-Raphson iterations r (2 - a r) on the hardware's approximation (which is kept for zero and
+// infinity), each with its residual by a fused multiply-add
 __device__ __forceinline__ double reciprocal(double a) {
     double r0;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(a));
@@ -565,7 +570,7 @@ local_smo_kernel(int ws, const float *__restrict__ kww, const float *__restrict_
         const double b = (-(second ? up[CLS - 1] : up[0]) + fj) * BACK;
         const float kdi = second ? kd_i[CLS - 1] : kd_i[0];
         const double a = NU ? (double) (kdi + kyj.x - 2 * kij) : (double) (kdi + kyj.x) - 2.0 * (double) kij;
-        // b / a: the quotient by a reciprocal of half the digits, corrected once (within an ulp of the division)
+        // b / a by Markstein's method: a reciprocal of most of the digits, the quotient corrected by its remainder
         double r;
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
         r = fma(r, fma(-a, r, 1.0), r);
