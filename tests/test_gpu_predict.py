@@ -117,10 +117,11 @@ def test_fused_prediction_numbers_of_classes(capi, nc):
     _fused_case(capi, nc, [1 + 32 * (c % 2) for c in range(nc)], d=40, m=97)
 
 
-def test_fused_prediction_many_classes(capi):
-    """20 classes: 19 coefficient rows per support vector (more than the shared-memory table holds) and 190 pairs;
-    several launches over the test rows."""
-    _fused_case(capi, 20, [17 + 3 * c for c in range(20)], d=64, m=4500)
+@pytest.mark.parametrize("d,gamma", [(64, 0.02), (2050, 5e-4)])
+def test_fused_prediction_many_classes(capi, d, gamma):
+    """20 classes: 19 coefficient rows per support vector (more than the shared-memory table holds) and 190 pairs; with 2,050
+    features in two launches over the test rows."""
+    _fused_case(capi, 20, [17 + 3 * c for c in range(20)], d=d, m=4500, gamma=gamma)
 
 
 @pytest.mark.parametrize("m", [192, 193, 256, 257, 700])
@@ -159,6 +160,59 @@ def test_fused_prediction_rows_on_the_lanes(capi, m, kernel, cnt):
     lab = capi.predict_labels(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, dense=_t(T))
     assert np.array_equal(lab.cpu().numpy(), capi.vote(dec, nc).cpu().numpy())
     km.close()
+
+
+def _sums_in_fp64(SV, T, kernel, gamma, cnt, coef, rho):
+    """Decision values in FP64, and the bound on the error of FP32 kernel values and products: (n + 20) 2^-24 times the sum of
+    the magnitudes of a pair's n products, and the values' own errors - the exponent's 2 gamma |x| |y| 2^-24 and more (RBF), the
+    dot's 2^-24 times its sum of magnitudes (linear)."""
+    A, B = T.astype(np.float64), SV.astype(np.float64)
+    dots, squares = A @ B.T, (A ** 2).sum(1)[:, None] + (B ** 2).sum(1)[None]
+    K = np.exp(-gamma * (squares - 2 * dots)) if kernel == "rbf" else dots
+    term = np.abs(A) @ np.abs(B).T
+    loose = (K * gamma * 4 * (term + squares) if kernel == "rbf" else 4 * term) @ np.abs(coef).sum(0)
+    own, want, size = np.repeat(np.arange(len(cnt)), cnt), [], []
+    for i in range(len(cnt)):
+        for j in range(i + 1, len(cnt)):
+            c = np.where(own == i, coef[j - 1], 0.0) + np.where(own == j, coef[i], 0.0)
+            want.append(K @ c - rho[len(want)])
+            size.append(np.abs(K) @ np.abs(c))
+    return np.stack(want, 1), 2.0 ** -24 * ((len(own) + 20) * np.stack(size, 1) + loose[:, None]) + 1e-12
+
+
+def _sums_case(capi, km, SV, T, kernel, gamma, cnt, seed, batch):
+    rng = np.random.default_rng(seed)
+    nc, n_sv = len(cnt), int(np.sum(cnt))
+    coef, rho = rng.standard_normal((nc - 1, n_sv)), rng.standard_normal(nc * (nc - 1) // 2)
+    want, bound = _sums_in_fp64(SV, T, kernel, gamma, cnt, coef, rho)
+    dec = capi.predict_dec(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, **batch)
+    assert np.all(np.abs(dec.cpu().numpy() - want) <= bound), np.max(np.abs(dec.cpu().numpy() - want) / bound)
+    lab = capi.predict_labels(km, _t(coef.reshape(-1)), cnt, _t(rho), nc, **batch).cpu().numpy()
+    # labels are the vote over a second call's sums, whose order may differ: rows without a value in doubt
+    sure = (np.abs(want) > bound).all(1)
+    assert sure.any() and np.array_equal(lab[sure], capi.vote(dec, nc).cpu().numpy()[sure])
+    km.close()
+
+
+@pytest.mark.parametrize("storage", ["dense", "csr"])
+@pytest.mark.parametrize("d,m", [(2050, 4500), (2050, 8200), (260, 33000)])
+@pytest.mark.parametrize("kernel,cnt", [("rbf", [70, 60]), ("rbf", [20, 31, 12]), ("linear", [9, 16, 17, 0, 1, 64, 33, 2, 5, 40]),
+                                        ("rbf", [11] * 12), ("linear", [4] * 33)])
+def test_fused_prediction_over_several_launches(capi, storage, d, m, kernel, cnt):
+    """More test rows than one launch takes (4,096 of 2,050 features, some 31,000 of 260): presets and results of every slab, the
+    last one shorter; test rows and support vectors on the lanes; sums by pair and by row; dense data, and CSR data that is
+    worked on as dense rows."""
+    rng = np.random.default_rng(m)
+    n_sv = sum(cnt)
+    if storage == "dense":
+        SV, T = (rng.standard_normal((k, d)).astype(np.float32) for k in (n_sv, m))
+        km, batch = capi.KernelMatrix(dense=_t(SV), kernel=kernel, gamma=1.0 / d), dict(dense=_t(T))
+    else:
+        SV, T = ((rng.random((k, d)) < 0.03).astype(np.float32) for k in (n_sv, m))
+        csr = [(_t(np.ones(int(a.sum()), np.float32)), _t(np.concatenate([[0], np.cumsum((a != 0).sum(1))]).astype(np.int32)),
+                _t(np.nonzero(a)[1].astype(np.int32))) for a in (SV, T)]
+        km, batch = capi.KernelMatrix(csr=csr[0], d=d, kernel=kernel, gamma=1.0 / d), dict(csr=csr[1])
+    _sums_case(capi, km, SV, T, kernel, 1.0 / d, cnt, len(cnt), batch)
 
 
 @pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 64, 65])

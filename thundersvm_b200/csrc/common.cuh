@@ -79,6 +79,7 @@ void pool_free(void *p);                      // waits for the block's device, l
 void pool_free_many(std::initializer_list<void *> blocks, bool idle = false);
 int device_sm_count();                        // SMs of the current device (asked once per device)
 size_t device_memory_bytes();                 // total memory of the current device (asked once per device)
+size_t device_l2_bytes();                     // its L2 cache (likewise)
 void pool_release();                          // returns every cached block to the driver
 void release_solver_streams();                // solver.cu: destroys the cached streams and events
 tsvm_status pinned_alloc(void **p, size_t bytes);         // at most 64 MB of freed blocks are kept

@@ -121,6 +121,17 @@ int device_sm_count() {
     return sms;
 }
 
+size_t device_l2_bytes() {
+    static std::atomic<int> bytes[MAX_DEVICES];
+    int dev = 0, size = 126 << 20;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return size; }
+    std::atomic<int> &known = bytes[dev & (MAX_DEVICES - 1)];
+    if (const int k = known.load(std::memory_order_relaxed)) return k;
+    if (cudaDeviceGetAttribute(&size, cudaDevAttrL2CacheSize, dev) != cudaSuccess) cudaGetLastError();
+    known.store(size, std::memory_order_relaxed);
+    return size;
+}
+
 size_t device_memory_bytes() {
     static std::atomic<size_t> bytes[MAX_DEVICES];
     int dev = 0;

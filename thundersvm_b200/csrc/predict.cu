@@ -55,6 +55,7 @@ sum_kernel_values_kernel(const double *__restrict__ coef, int n_sv, const int *_
 // side by side (to [row][pair] every one is a memory sector of its own: ten classes, 8,003 x 784, 173 -> 157 us per
 // 4,096 rows). This kernel turns the slab into decision values [row][pair] and / or votes (the first maximum wins).
 constexpr int SLAB_CLASSES = 32, SLAB_THREADS = 256;
+static bool sums_by_pair(int n_classes) { return n_classes > 2 && n_classes <= SLAB_CLASSES; }
 __global__ void __launch_bounds__(SLAB_THREADS)
 finish_slab_kernel(const double *__restrict__ slab, long long ld, int m, int n_classes, double *__restrict__ dec,
                    int *__restrict__ labels) {
@@ -205,10 +206,18 @@ using namespace tsvm;
 
 // Rows of test instances handled per launch of the fused contraction (the handle's staging scratch grows to hold them): as
 // many as leave their operand planes in a quarter of the L2 cache, where every block of support vectors reads them again, and
-// at least 4,096. One launch instead of four for 16,281 rows of 123 features: 201 -> 156 us per call.
-static int fused_rows(const tsvm_km *km) {
-    const size_t fit = ((size_t) 32 << 20) / (2 * km_plane_row_bytes(km));
-    return fit < 4096 ? 4096 : fit > 16384 ? 16384 : (int) (fit & ~(size_t) 255);
+// at least 4,096; `scratch_pairs` decision values per row that the call keeps for itself may take a sixteenth of the device,
+// like the kernel block of the unfused path. Whole calls with 4,096 / 16,384 / as many rows per launch as the planes allow:
+// 60,000 rows against 12,001 x 123 one-hot CSR 630 / 440 / 392 us, 100,000 against 3,000 x 60 588 / 317 / 215, 300,000 against 1,000 x
+// 64, three classes, 1,400 - 2,000 / 650 - 820 / 370 - 440, 60,000 against 2,000 x 100, 20 classes, 3,490 / 2,400 / 2,210, 60
+// classes 18.6 / 15.4 / 15.2 ms. Half and twice the quarter: 100,000 against 3,000 x 60 226 / 214, 40,000 against 40,000 x 2,000 15.1
+// and 15.6 - 17.1 ms against 14.5 - 15.1.
+static int fused_rows(const tsvm_km *km, size_t scratch_pairs) {
+    size_t fit = device_l2_bytes() / 4 / (2 * km_plane_row_bytes(km));
+    if (fit < 4096) fit = 4096;
+    const size_t most = device_memory_bytes() / 16 / (sizeof(double) * (scratch_pairs ? scratch_pairs : 1));
+    if (fit > most) fit = most;
+    return fit < 256 ? 256 : (int) (fit & ~(size_t) 255);
 }
 // From this number of test rows on the contraction takes them on the lanes of its accumulators (FORM_LANES in dense_tc2.cu): its
 // epilogue is the shorter one, but it computes whole tiles of 256 rows. 40,000 x 2,000, both forms: 157 against 166 us with
@@ -321,7 +330,7 @@ static tsvm_status predict_slabs(tsvm_km *km_sv, const double *coef_dev, const s
     else s = dev_alloc(&meta, (size_t) 2 * n_classes);
     if (s == TSVM_OK && !fused) s = dev_alloc(&K, (size_t) batch * ldk);
     if (s == TSVM_OK && fused && !lanes) s = dev_alloc(&sv_class, (size_t) n_sv);
-    const bool by_pair = fused && n_classes > 2 && n_classes <= SLAB_CLASSES;
+    const bool by_pair = fused && sums_by_pair(n_classes);
     const long long slab_ld = (batch + 3) & ~3ll;
     if (s == TSVM_OK && (labels_dev || by_pair)) s = dev_alloc(&dec_slab, (size_t) slab_ld * nb);
     const bool by_argument = n_classes <= ARG_CLASSES;
@@ -394,7 +403,8 @@ static tsvm_status predict_impl(tsvm_km *km_sv, const double *coef_dev, const in
     bool fused = false;
     TSVM_TRY(km_pair_engine_takes(km_sv, T_dev ? nullptr : tval_dev, T_dev ? nullptr : trow_ptr_dev, tcol_dev, m, st, &fused));
     const long long ldk = ((long long) n_sv + 3) & ~3ll;
-    long long batch = fused ? fused_rows(km_sv) : 0;
+    const bool scratch = labels_dev || sums_by_pair(n_classes);
+    long long batch = fused ? fused_rows(km_sv, scratch ? (size_t) n_classes * (n_classes - 1) / 2 : 0) : 0;
     if (!fused) {
         // the kernel block of a slab must fit the budget (svmmodel.cpp:86-89 caps a batch at 10000 rows)
         size_t budget = max_mem_bytes;
