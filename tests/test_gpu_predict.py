@@ -194,6 +194,19 @@ def _sums_case(capi, km, SV, T, kernel, gamma, cnt, seed, batch):
     km.close()
 
 
+@pytest.mark.parametrize("d", [127, 128, 129, 256, 257, 300, 784])
+@pytest.mark.parametrize("m", [193, 513])
+@pytest.mark.parametrize("kernel", ["rbf", "linear"])
+@pytest.mark.parametrize("cnt", [[130, 127], [20, 12, 31], [300, 1, 0, 255], [57] * 10, [9, 16, 17, 0, 1, 64, 33, 2, 5, 300]])
+def test_fused_prediction_rows_on_the_lanes_numbers_of_features(capi, d, m, kernel, cnt):
+    """Test rows on the lanes with one promotion unit (up to 128 features), where the sums are taken from tensor memory, and with
+    several, where they stay in registers: one, three and nine coefficients, more than one block of support vectors."""
+    rng = np.random.default_rng(d + m)
+    SV, T = (rng.standard_normal((k, d)).astype(np.float32) for k in (sum(cnt), m))
+    km = capi.KernelMatrix(dense=_t(SV), kernel=kernel, gamma=1.0 / d)
+    _sums_case(capi, km, SV, T, kernel, 1.0 / d, cnt, len(cnt), dict(dense=_t(T)))
+
+
 @pytest.mark.parametrize("storage", ["dense", "csr"])
 @pytest.mark.parametrize("d,m", [(2050, 4500), (2050, 8200), (260, 33000)])
 @pytest.mark.parametrize("kernel,cnt", [("rbf", [70, 60]), ("rbf", [20, 31, 12]), ("linear", [9, 16, 17, 0, 1, 64, 33, 2, 5, 40]),
