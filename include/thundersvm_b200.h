@@ -326,8 +326,9 @@ tsvm_status tsvm_update_f(double *f_dev, int n, const double *alpha_diff_dev, in
  * otherwise it is computed in slabs of at most max_mem_bytes (0 = a sixteenth of the device's memory).
  * Where a slab does not fit what the device has left, it is halved until it does.
  * Up to 64 test rows may go through one launch of FP32 dot products instead (up to 32 classes; CSR support vectors:
- * CSR test rows of at most 2,048 entries together): all three forms hold FP32 accuracy, but a row's decision value
- * may differ in its last digits (3e-6 relative at 3,001 x 100) with the number of rows it is predicted with. */
+ * CSR test rows of at most 2,048 entries together), and the contraction sums in another order for more than 192 test
+ * rows (RBF and linear kernels, up to ten classes): all forms hold FP32 accuracy, but a row's decision value may differ in its
+ * last digits (3e-6 relative at 3,001 x 100) with the number of rows it is predicted with. */
 tsvm_status tsvm_predict_dec(tsvm_km *km_sv, const double *coef_dev, const int *sv_count_host,
                              const double *rho_dev, int n_classes, int m, const float *T_dev, int dt, int ldt,
                              const float *tval_dev, const int *trow_ptr_dev, const int *tcol_dev, long long tnnz,

@@ -304,7 +304,7 @@ def test_local_smo_choice_between_nearly_equal_values(capi, swapped):
 
 
 @pytest.mark.parametrize("ws", [256, 512, 1024])
-def test_local_smo_rows_copied_ahead_hold_the_same_values(capi, ws):
+def test_local_smo_takes_the_same_steps_while_rows_are_read_ahead(capi, ws):
     """A block whose rows are 16-byte aligned and one that is not, while other warps read rows ahead: the same steps, bit
     for bit, over some thousand of them."""
     import torch

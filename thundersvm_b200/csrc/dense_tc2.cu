@@ -150,10 +150,9 @@ struct PredictArgs {
     double *dec;               // the sums are added to dec[r * row_stride + pair * pair_stride]
     long long row_stride, pair_stride;
     int n_classes;
-    // rows on the lanes: the support vectors' numbers (predict_columns_kernel), rows of cols_ld floats; nc_pad rows of coefficients
+    // rows on the lanes: the support vectors' numbers (predict_columns_kernel), rows of cols_ld floats; FORM % 16 rows of coefficients
     const float *cols;
     long long cols_ld;
-    int nc_pad;
 };
 // form of the kernel: rows, prediction with the instances on the lanes, prediction with the test rows on the lanes and
 // FORM % 16 coefficients, for any number of features or for those of one promotion unit
@@ -970,7 +969,7 @@ tsvm_status launch_dense_tc2_predict(tsvm_km *km, int m, const double *coef_dev,
                                      int n_classes, double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st) {
     const InstancePlanes all{km->Xhi, km->Xlo, km->self_dot, km->x_unscale, km->n};
     const RowPlanes staged{km->Whi, km->Wlo, km->sd_rows, km->w_unscale};
-    const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes, nullptr, 0, 0};
+    const PredictArgs pa{coef_dev, sv_class_dev, dec_dev, row_stride, pair_stride, n_classes, nullptr, 0};
     return launch_pair_any<FORM_PREDICT>(km, all, staged, m, nullptr, 0, pa, RowsExtra{nullptr, nullptr, 0, 0, nullptr}, st);
 }
 
@@ -989,7 +988,7 @@ tsvm_status launch_dense_tc2_predict_lanes(tsvm_km *km, int m, const float *cols
                                            double *dec_dev, long long row_stride, long long pair_stride, cudaStream_t st) {
     const InstancePlanes rows{km->Whi, km->Wlo, km->sd_rows, km->w_unscale, m};
     const RowPlanes svs{km->Xhi, km->Xlo, km->self_dot, km->x_unscale};
-    const PredictArgs pa{nullptr, nullptr, dec_dev, row_stride, pair_stride, n_classes, cols, cols_ld, nc_pad};
+    const PredictArgs pa{nullptr, nullptr, dec_dev, row_stride, pair_stride, n_classes, cols, cols_ld};
     const RowsExtra ex{nullptr, nullptr, 0, 0, nullptr};
     const bool rbf = epilogue_kind(km->fn) == EPI_RBF;
     const bool one_unit = km->plane_ld <= 128;              // two k slabs
