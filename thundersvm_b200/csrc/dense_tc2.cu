@@ -1,9 +1,8 @@
 // Dense kernel rows on tcgen05 with CTA pairs (cta_group::2).
 //
-// Same contraction, same 3xTF32 scheme and same per-slab FP32 promotion as dense_tc.cu, but two
-// CTAs on neighbouring SMs work as one: the pair owns a 256-instance x 256-requested-row tile, each
-// CTA holds the TF32 planes of ITS 128 instances and of ITS 128 requested rows (half of the B
-// operand), and one thread of the leader CTA issues tcgen05.mma.cta_group::2 (M = 256), which reads
+// Every operand is held as two planes (row-scaled FP16, or TF32), a product takes three MMAs, and sums are promoted to FP32
+// registers every few k slabs. Two CTAs on neighbouring SMs work as one: the pair owns a 256-instance x 256-requested-row tile,
+// each CTA holds the planes of ITS 128 instances and of ITS 128 requested rows (half of the B operand), and one thread of the leader CTA issues tcgen05.mma.cta_group::2 (M = 256), which reads
 // both CTAs' shared memory and writes both CTAs' tensor memory. Per CTA a k slab is then 64 KB
 // instead of 96 KB for the same tensor-core time, and three of them fit the ring instead of two - the
 // single-CTA engine was bound by the latency of its one slab in flight, not by any bandwidth.
@@ -11,12 +10,13 @@
 // Roles per CTA (384 threads = 3 warpgroups): warp 0 TMA producer for this CTA's operand halves
 // (transaction bytes are reported to the leader's "full" barrier), warp 1 tensor-memory allocation (both
 // CTAs) and MMA issue (leader only), warps 2..3 idle (prediction with the test rows on the lanes: warp 2 fetches the columns'
-// numbers), warps 4..11 slab promotion + epilogue on this CTA's 128 instances. Warpgroup 0 hands registers to the other two (setmaxnreg): the epilogue keeps 128 sums per
-// thread live, and with the 168 registers a 384-thread CTA is compiled for it spilled a few loop-invariant
+// numbers), warps 4..11 slab promotion + epilogue on this CTA's 128 instances (prediction with the test rows on the lanes and
+// one promotion unit: 640 threads, warps 4..19). Warpgroup 0 hands registers to the others (setmaxnreg): the epilogue keeps 128
+// sums per thread live, and with the 168 registers a 384-thread CTA is compiled for it spilled a few loop-invariant
 // values - their reloads from local memory (the L1 is tiny next to 222 KB of shared memory) cost 9 % of
 // the kernel.
 // Barriers: full[s] (leader; both CTAs' TMA bytes), empty[s] (per CTA; MMAs that read the stage have
-// retired), tfull[a] (per CTA; slab sum complete), tempty[a] (leader; 16 epilogue warps drained it).
+// retired), tfull[a] (per CTA; slab sum complete), tempty[a] (leader; the epilogue warps of both CTAs drained it).
 // Cross-CTA signalling uses mbarrier arrives on shared::cluster addresses and one tcgen05.commit per
 // destination CTA; every load is addressed to one CTA's shared memory only. Every mbarrier wait is bounded.
 #include "tc_common.cuh"
