@@ -207,17 +207,18 @@ using namespace tsvm;
 // Rows of test instances handled per launch of the fused contraction (the handle's staging scratch grows to hold them): as
 // many as leave their operand planes in a quarter of the L2 cache, where every block of support vectors reads them again, and
 // at least 4,096; `scratch_pairs` decision values per row that the call keeps for itself may take a sixteenth of the device,
-// like the kernel block of the unfused path. Whole calls with 4,096 / 16,384 / as many rows per launch as the planes allow:
-// 60,000 rows against 12,001 x 123 one-hot CSR 630 / 440 / 392 us, 100,000 against 3,000 x 60 588 / 317 / 215, 300,000 against 1,000 x
-// 64, three classes, 1,400 - 2,000 / 650 - 820 / 370 - 440, 60,000 against 2,000 x 100, 20 classes, 3,490 / 2,400 / 2,210, 60
-// classes 18.6 / 15.4 / 15.2 ms. Half and twice the quarter: 100,000 against 3,000 x 60 226 / 214, 40,000 against 40,000 x 2,000 15.1
-// and 15.6 - 17.1 ms against 14.5 - 15.1.
+// like the kernel block of the unfused path, or what 16,384 rows need: with more than 128 classes the vote is a thread per row and
+// takes as long for 4,096 rows as for these (16,384 rows, 150 classes: 670 ms in four launches, 180 in one). Whole calls with
+// 4,096 / 16,384 / as many rows per launch as the planes allow: 60,000 rows against 12,001 x 123 one-hot CSR 630 / 440 / 392 us,
+// 100,000 against 3,000 x 60 588 / 317 / 215, 300,000 against 1,000 x 64, three classes, 1,400 - 2,000 / 650 - 820 / 370 - 440, 60,000
+// against 2,000 x 100, 20 classes, 3,490 / 2,400 / 2,210, 60 classes 18.6 / 15.4 / 15.2 ms. Half and twice the quarter: 100,000 against
+// 3,000 x 60 226 / 214, 40,000 against 40,000 x 2,000 15.1 and 15.6 - 17.1 ms against 14.5 - 15.1.
 static int fused_rows(const tsvm_km *km, size_t scratch_pairs) {
     size_t fit = device_l2_bytes() / 4 / (2 * km_plane_row_bytes(km));
     if (fit < 4096) fit = 4096;
-    const size_t most = device_memory_bytes() / 16 / (sizeof(double) * (scratch_pairs ? scratch_pairs : 1));
-    if (fit > most) fit = most;
-    return fit < 256 ? 256 : (int) (fit & ~(size_t) 255);
+    size_t most = device_memory_bytes() / 16 / (sizeof(double) * (scratch_pairs ? scratch_pairs : 1));
+    if (most < 16384) most = 16384;
+    return (int) ((fit < most ? fit : most) & ~(size_t) 255);
 }
 // From this number of test rows on the contraction takes them on the lanes of its accumulators (FORM_LANES in dense_tc2.cu): its
 // epilogue is the shorter one, but it computes whole tiles of 256 rows. 40,000 x 2,000, both forms: 157 against 166 us with
